@@ -60,7 +60,7 @@ constexpr int REDUCE_THREADS = 256;
 // more are swept in passes of ENERGY_PASS (eight threads of four energies).
 constexpr int SWEEP_MAX_ENERGIES = 64;
 constexpr int ENERGY_PASS = 32;
-constexpr int NQ = 48;  // partial-sum slots of the finalize reduction
+constexpr int NQ = 38;  // partial-sum slots of the finalize reduction (four components)
 
 // ------------------------------------------------------------------ kernels --
 
@@ -1171,97 +1171,132 @@ __device__ __forceinline__ void res_add(double *q, double o, double n) {
   q[5] = max_nan(q[5], fabs(o));
 }
 
-// Block reduction of NQ slots: slots listed in max_mask are max-reduced.
-__device__ void block_reduce(double *q, int nq, unsigned long long max_mask, double *out) {
-  __shared__ double sh[REDUCE_THREADS];
-  for (int k = 0; k < nq; ++k) {
-    sh[threadIdx.x] = q[k];
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-      if ((int)threadIdx.x < s) {
-        const double o = sh[threadIdx.x + s];
-        sh[threadIdx.x] = ((max_mask >> k) & 1ull) ? max_nan(sh[threadIdx.x], o) : sh[threadIdx.x] + o;
-      }
-      __syncthreads();
+// Block reduction of N sums held in registers (slots listed in max_mask are
+// maxima), written to out[0..N): a shuffle tree per warp, then one thread per
+// slot adds the warps' values in order.  One barrier for all slots instead of
+// ten per slot: the 48-slot reduction of k_finalize took 44 of its 44 us on a
+// 86 x 86 lattice through 480 barriers.
+template <int N>
+__device__ __forceinline__ void block_reduce(double (&q)[N], unsigned long long max_mask, double *out) {
+  __shared__ double sh[N][REDUCE_THREADS / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const bool mx = (max_mask >> k) & 1ull;
+    double v = q[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double u = __shfl_xor_sync(0xffffffffu, v, o);
+      v = mx ? max_nan(v, u) : v + u;
     }
-    if (threadIdx.x == 0) out[k] = sh[0];
-    __syncthreads();
+    if (lane == 0) sh[k][w] = v;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < N; k += REDUCE_THREADS) {
+    const bool mx = (max_mask >> k) & 1ull;
+    double v = sh[k][0];
+#pragma unroll
+    for (int i = 1; i < REDUCE_THREADS / 32; ++i) v = mx ? max_nan(v, sh[k][i]) : v + sh[k][i];
+    out[k] = v;
   }
 }
 
-// Slot layout of the finalize reduction.
-//   [6c .. 6c+5]  order-parameter residual of component c (c < 4)
-//   [24 .. 29]    current-density residual
-//   30            sum of the free-energy kernel inside the grain
-//   31 .. 34      sum |Delta_c|^2 inside the grain
-//   35            sum B^2 over the lattice
-//   36, 37        sum of the new current density (x, y)
+// Slot layout of the finalize reduction of nc components.
+//   [0 .. 5]      current-density residual
+//   6             sum of the free-energy kernel inside the grain
+//   7             sum B^2 over the lattice
+//   8, 9          sum of the new current density (x, y)
+//   10 + 7c ..    order-parameter residual of component c (six), then
+//                 sum |Delta_c|^2 inside the grain
+constexpr int FIN_HEAD = 10, FIN_COMP = 7;
 constexpr unsigned long long FIN_MAX_MASK =
-    (0x30ull) | (0x30ull << 6) | (0x30ull << 12) | (0x30ull << 18) | (0x30ull << 24);
+    0x30ull | ((0x30ull | (0x30ull << 7) | (0x30ull << 14) | (0x30ull << 21)) << FIN_HEAD);
 
 // ComputeOrderParameter / ComputeCurrent / ComputeFreeEnergy
-// ::computePropertyFromGreens, element-wise part and partial sums.
+// ::computePropertyFromGreens, element-wise part and partial sums.  The
+// component count is fixed at compile time (NC = 0: up to MAX_COMP at run
+// time), so that the sums stay in registers and only used slots are reduced.
+template <int NC>
 __global__ void __launch_bounds__(REDUCE_THREADS) k_finalize(
-    int n0, int nc, double h, double jfactor, int has_vp, const uint8_t *__restrict__ dom,
+    int n0, int nc_, double h, double jfactor, int has_vp, const uint8_t *__restrict__ dom,
     const double *__restrict__ coupling, const double *__restrict__ acc_d,
     const double *__restrict__ acc_j, const double *__restrict__ acc_fe,
     const double *__restrict__ delta, const double *__restrict__ avec, double *delta_new,
     double *j_real, double *partial) {
-  const size_t nn = (size_t)n0 * n0;
-  double q[NQ];
-  for (int k = 0; k < NQ; ++k) q[k] = 0.0;
+  const unsigned nn = (unsigned)n0 * n0;
+  constexpr int NCM = NC > 0 ? NC : MAX_COMP;
+  const int nc = NC > 0 ? NC : nc_;
+  double q[FIN_HEAD + FIN_COMP * NCM];
+#pragma unroll
+  for (int k = 0; k < FIN_HEAD + FIN_COMP * NCM; ++k) q[k] = 0.0;
   const double inv_h = 1.0 / h;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nn;
-       i += (size_t)gridDim.x * blockDim.x) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
     const bool in = dom[i] != 0;
-    for (int c = 0; c < nc; ++c) {
+#pragma unroll
+    for (int c = 0; c < NCM; ++c) {
+      if (c >= nc) break;
+      double *qc = &q[FIN_HEAD + FIN_COMP * c];
       const double lc = coupling[c];
-      for (int p = 0; p < 2; ++p) {
-        const size_t k = (size_t)(2 * c + p) * nn + i;
-        const double nv = in ? acc_d[k] * lc : 0.0;
-        delta_new[k] = nv;
-        res_add(&q[6 * c], delta[k], nv);
-      }
-      if (in) {
-        const double o_re = delta[(size_t)(2 * c) * nn + i], o_im = delta[(size_t)(2 * c + 1) * nn + i];
-        q[31 + c] += o_re * o_re + o_im * o_im;
-      }
+      const size_t kr = (size_t)(2 * c) * nn + i, ki = kr + nn;
+      const double o_re = delta[kr], o_im = delta[ki];
+      const double n_re = in ? acc_d[kr] * lc : 0.0, n_im = in ? acc_d[ki] * lc : 0.0;
+      delta_new[kr] = n_re;
+      delta_new[ki] = n_im;
+      res_add(qc, o_re, n_re);
+      res_add(qc, o_im, n_im);
+      if (in) qc[6] += o_re * o_re + o_im * o_im;
     }
+#pragma unroll
     for (int d = 0; d < 2; ++d) {
       const size_t k = (size_t)d * nn + i;
       const double nv = in ? acc_j[k] * jfactor : 0.0;
-      res_add(&q[24], j_real[k], nv);
+      res_add(&q[0], j_real[k], nv);
       j_real[k] = nv;
-      q[36 + d] += nv;
+      q[8 + d] += nv;
     }
-    if (in) q[30] += acc_fe[i];
+    if (in) q[6] += acc_fe[i];
     if (has_vp) {
       // curl_kernel, GridFunctions_GPU.h:326-352.
-      const int x = (int)(i % n0), y = (int)(i / n0);
+      const int x = (int)(i % (unsigned)n0), y = (int)(i / (unsigned)n0);
       const int xn = min(x + 1, n0 - 1), xp = max(x - 1, 0);
       const int yn = min(y + 1, n0 - 1), yp = max(y - 1, 0);
       const double *ax = avec, *ay = avec + nn;
       const double dAydx = (ay[(size_t)y * n0 + xn] - ay[(size_t)y * n0 + xp]) / (double)(xn - xp);
       const double dAxdy = (ax[(size_t)yn * n0 + x] - ax[(size_t)yp * n0 + x]) / (double)(yn - yp);
       const double bz = (dAydx - dAxdy) * inv_h;
-      q[35] += bz * bz;
+      q[7] += bz * bz;
     }
   }
-  block_reduce(q, NQ, FIN_MAX_MASK, partial + (size_t)blockIdx.x * NQ);
+  block_reduce(q, FIN_MAX_MASK, partial + (size_t)blockIdx.x * NQ);
 }
 
 __global__ void __launch_bounds__(256) k_ldos_finalize(int n0, int n_fields, const uint8_t *__restrict__ dom,
                                                        const double *__restrict__ acc, double *ldos,
                                                        double *partial) {
   double q[6] = {0, 0, 0, 0, 0, 0};
-  const size_t nn = (size_t)n0 * n0, n = nn * n_fields;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const double nv = dom[i % nn] ? -acc[i] : 0.0;
-    res_add(q, ldos[i], nv);
-    ldos[i] = nv;
+  const unsigned nn = (unsigned)n0 * n0;
+  // A thread keeps its site and walks the energies, four at a time in flight
+  // (no division per element).
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
+    const bool in = dom[i] != 0;
+    for (int f = 0; f < n_fields; f += 4) {
+      double a[4], o[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const size_t k = (size_t)(f + u) * nn + i;
+        a[u] = f + u < n_fields ? acc[k] : 0.0;
+        o[u] = f + u < n_fields ? ldos[k] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (f + u < n_fields) {
+          const double nv = in ? -a[u] : 0.0;
+          res_add(q, o[u], nv);
+          ldos[(size_t)(f + u) * nn + i] = nv;
+        }
+    }
   }
-  block_reduce(q, 6, 0x30ull, partial + (size_t)blockIdx.x * 6);
+  block_reduce(q, 0x30ull, partial + (size_t)blockIdx.x * 6);
 }
 
 // Residual partials of a boundary gather (in-place update) or of any (old, new)
@@ -1273,7 +1308,7 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_residual(size_t n, const dou
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
     res_add(q, o[i], nw[i]);
-  block_reduce(q, 6, 0x30ull, partial + (size_t)blockIdx.x * 6);
+  block_reduce(q, 0x30ull, partial + (size_t)blockIdx.x * 6);
 }
 
 // Specular boundary condition through the precomputed gather table
@@ -1308,7 +1343,7 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_boundary(int n_in, int ne,
     res_add(q, (double)ov.im, (double)nv.im);
     in[t] = nv;
   }
-  block_reduce(q, 6, 0x30ull, partial + (size_t)blockIdx.x * 6);
+  block_reduce(q, 0x30ull, partial + (size_t)blockIdx.x * 6);
 }
 
 // Initial boundary values: homogeneous solutions at every exit node
@@ -1526,18 +1561,22 @@ __device__ double residual_from(const double *t, size_t n_elem, int norm) {
   return numer / fmax(denom, eps);
 }
 
-// Sums (or maxima, for the slots set in max_mask) of nq slots over the
-// nblocks rows of block partials: warp w reduces slots w, w + nwarps, ... in a
-// fixed order (lane-strided, then a shuffle tree); results in t[0..nq).
-__device__ void reduce_slots(const double *partial, int nblocks, int nq, unsigned long long max_mask,
+// Sums (or maxima, for the slots set in max_mask) of the first nq of `stride`
+// slots over the nblocks rows of block partials: warp w reduces slots w,
+// w + nwarps, ... in a fixed order (lane-strided with four loads in flight,
+// then a shuffle tree); results in t[0..nq).
+__device__ void reduce_slots(const double *partial, int nblocks, int stride, int nq, unsigned long long max_mask,
                              double *t) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int k = w; k < nq; k += nw) {
     const bool mx = (max_mask >> k) & 1ull;
     double v = 0.0;
-    for (int b = lane; b < nblocks; b += 32) {
-      const double p = partial[(size_t)b * nq + k];
-      v = mx ? max_nan(v, p) : v + p;
+    for (int b0 = lane; b0 < nblocks; b0 += 128) {
+      double p[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) p[u] = b0 + 32 * u < nblocks ? partial[(size_t)(b0 + 32 * u) * stride + k] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v = mx ? max_nan(v, p[u]) : v + p[u];
     }
     for (int o = 16; o > 0; o >>= 1) {
       const double u = __shfl_xor_sync(0xffffffffu, v, o);
@@ -1560,20 +1599,20 @@ struct FinalizeConsts {
 // ComputeCurrent.h:184-211).
 __global__ void k_scalars_a(FinalizeConsts C, const double *partial, int nblocks, Scalars *S) {
   __shared__ double t[NQ];
-  reduce_slots(partial, nblocks, NQ, FIN_MAX_MASK, t);
+  reduce_slots(partial, nblocks, NQ, FIN_HEAD + FIN_COMP * C.nc, FIN_MAX_MASK, t);
   if (threadIdx.x != 0) return;
   double rop = 0.0;
-  for (int c = 0; c < C.nc; ++c) rop = max_nan(rop, residual_from(&t[6 * c], C.n_elem_field, C.norm));
+  for (int c = 0; c < C.nc; ++c) rop = max_nan(rop, residual_from(&t[FIN_HEAD + FIN_COMP * c], C.n_elem_field, C.norm));
   S->res_op = rop;
   S->conv_op = rop < C.conv;
-  const double rj = residual_from(&t[24], C.n_elem_field, C.norm);
+  const double rj = residual_from(&t[0], C.n_elem_field, C.norm);
   S->res_j = S->first_j ? C.conv * 0.1 : rj;
   S->conv_j = S->res_j < C.conv;
   S->first_j = 0;
-  double nonmag = C.temperature * t[30];
-  for (int c = 0; c < C.nc; ++c) nonmag += t[31 + c] * (C.log_t_tc[c] + C.sum_inv);
+  double nonmag = C.temperature * t[6];
+  for (int c = 0; c < C.nc; ++c) nonmag += t[FIN_HEAD + FIN_COMP * c + 6] * (C.log_t_tc[c] + C.sum_inv);
   double mag = 0.0;
-  if (C.has_vp) mag += (0.5 / (C.lambda * C.lambda)) * t[35];
+  if (C.has_vp) mag += (0.5 / (C.lambda * C.lambda)) * t[7];
   const double la = C.h * C.h;
   const double fe_area = (nonmag + mag) / (double)C.n_grain;
   const double actual = fabs(S->fe_area_prev - fe_area) / fmax(fabs(S->fe_area_prev), 1e-4);
@@ -1586,8 +1625,8 @@ __global__ void k_scalars_a(FinalizeConsts C, const double *partial, int nblocks
   S->fe_mag_area = mag / (double)C.n_grain;
   S->fe_area_prev = fe_area;
   S->n_grain = (double)C.n_grain;
-  S->j_mean[0] = t[36] / (double)C.n_grain;
-  S->j_mean[1] = t[37] / (double)C.n_grain;
+  S->j_mean[0] = t[8] / (double)C.n_grain;
+  S->j_mean[1] = t[9] / (double)C.n_grain;
 }
 
 // Boundary and vector-potential residuals, total residual (Context.h:462-483).
@@ -1596,10 +1635,10 @@ __global__ void k_scalars_b(int norm, size_t n_elem_g, size_t n_elem_gt, size_t 
                             const double *p_bgt, int nb_gt, const double *p_vp, int nb_vp, Scalars *S) {
   __shared__ double t[18];
   if (do_bc) {
-    reduce_slots(p_bg, nb_g, 6, 0x30ull, &t[0]);
-    reduce_slots(p_bgt, nb_gt, 6, 0x30ull, &t[6]);
+    reduce_slots(p_bg, nb_g, 6, 6, 0x30ull, &t[0]);
+    reduce_slots(p_bgt, nb_gt, 6, 6, 0x30ull, &t[6]);
   }
-  if (do_vp) reduce_slots(p_vp, nb_vp, 6, 0x30ull, &t[12]);
+  if (do_vp) reduce_slots(p_vp, nb_vp, 6, 6, 0x30ull, &t[12]);
   if (threadIdx.x != 0) return;
   if (do_bc) S->res_bc = max_nan(residual_from(&t[0], n_elem_g, norm), residual_from(&t[6], n_elem_gt, norm));
   if (do_vp) S->res_vp = residual_from(&t[12], n_elem_vp, norm);
@@ -1631,7 +1670,7 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_acc_sums(int nf, size_t nn, 
     q[1] += mv * mv;
     q[2] += d * mv;
   }
-  block_reduce(q, 3, 0, partial + ((size_t)f * gridDim.x + blockIdx.x) * 3);
+  block_reduce(q, 0, partial + ((size_t)f * gridDim.x + blockIdx.x) * 3);
 }
 
 constexpr int AND_MAX_RANK = 16;
@@ -1658,14 +1697,17 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_and_store(size_t tot, int ra
                                                               double *hd, const AccState *st, double *partial) {
   const int it = st->and_iter, slot = it % rank, m = min(it + 1, rank);
   double q[AND_MAX_RANK];
-  for (int j = 0; j < rank; ++j) q[j] = 0.0;
+#pragma unroll
+  for (int j = 0; j < AND_MAX_RANK; ++j) q[j] = 0.0;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < tot; k += (size_t)gridDim.x * blockDim.x) {
     const double d = gx[k] - x[k];
     hx[(size_t)slot * tot + k] = x[k];
     hd[(size_t)slot * tot + k] = d;
-    for (int j = 0; j < m; ++j) q[j] += d * (j == slot ? d : hd[(size_t)j * tot + k]);
+#pragma unroll
+    for (int j = 0; j < AND_MAX_RANK; ++j)
+      if (j < m) q[j] += d * (j == slot ? d : hd[(size_t)j * tot + k]);
   }
-  block_reduce(q, rank, 0, partial + (size_t)blockIdx.x * rank);
+  block_reduce(q, 0, partial + (size_t)blockIdx.x * AND_MAX_RANK);
 }
 
 // Anderson::solve (Anderson.h:291-333): the bordered least-squares system
@@ -1673,7 +1715,7 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_and_store(size_t tot, int ra
 // Gaussian elimination with partial pivoting; then the iteration count.
 __global__ void k_and_solve(int rank, const double *partial, int nblocks, AccState *st) {
   __shared__ double t[AND_MAX_RANK];
-  reduce_slots(partial, nblocks, rank, 0ull, t);
+  reduce_slots(partial, nblocks, AND_MAX_RANK, rank, 0ull, t);
   if (threadIdx.x != 0) return;
   const int it = st->and_iter, slot = it % rank, m = min(it + 1, rank), mt = m + 1;
   for (int j = 0; j < m; ++j) {
@@ -1777,7 +1819,7 @@ struct AccConsts {
 __global__ void k_acc_scalars(AccConsts C, const double *partial, int nblocks, AccState *st) {
   __shared__ double t[48];
   const int nf = C.nf;
-  for (int f = 0; f < nf; ++f) reduce_slots(partial + (size_t)f * nblocks * 3, nblocks, 3, 0ull, &t[3 * f]);
+  for (int f = 0; f < nf; ++f) reduce_slots(partial + (size_t)f * nblocks * 3, nblocks, 3, 3, 0ull, &t[3 * f]);
   if (threadIdx.x != 0) return;
   if (!st->initialized) {
     for (int f = 0; f < nf; ++f) {
@@ -2305,7 +2347,7 @@ void boundary_initial(sc_ctx *c) {
 void launch_scalars_b(sc_ctx *c, int do_bc, int do_vp, int compute_mode, size_t n_elem_vp = 0) {
   const HostSetup &S = c->S;
   if (!n_elem_vp) n_elem_vp = 2 * c->nn0();
-  k_scalars_b<<<1, 256, 0, c->stream>>>(S.norm, (size_t)2 * S.n_in_g * S.ne,
+  k_scalars_b<<<1, 1024, 0, c->stream>>>(S.norm, (size_t)2 * S.n_in_g * S.ne,
                                          (size_t)2 * S.n_in_gt * S.ne, n_elem_vp, do_bc, do_vp,
                                          compute_mode, c->partial_bg.p, c->nb_bnd, c->partial_bgt.p,
                                          c->nb_bnd, c->partial_vp.p, c->nb_vp, c->scalars.p);
@@ -2637,7 +2679,8 @@ void compute_post(sc_ctx *c) {
     double *delta = c->xstate.p, *avec = c->xstate.p + (size_t)2 * S.nc * nn;
     double *delta_new = c->gstate.p;
     const double jfactor = (double)(2 * S.charge_sign) * S.temperature;
-    k_finalize<<<c->nb_fin, REDUCE_THREADS, 0, c->stream>>>(
+    auto fin = S.nc == 1 ? k_finalize<1> : S.nc == 2 ? k_finalize<2> : k_finalize<0>;
+    fin<<<c->nb_fin, REDUCE_THREADS, 0, c->stream>>>(
         S.n0, S.nc, S.h, jfactor, c->has_vp() ? 1 : 0, c->dom.p, c->coupling.p, c->acc_d.p, c->acc_j.p,
         c->acc_fe.p, delta, avec, delta_new, c->j_real.p, c->partial_fin.p);
     check_launch(c);
@@ -2655,7 +2698,7 @@ void compute_post(sc_ctx *c) {
     for (int e = 0; e < S.ne; ++e) si += S.residues[e] / S.e_im[e];
     F.sum_inv = si * S.temperature;
     for (int k = 0; k < S.nc; ++k) F.log_t_tc[k] = std::log(S.temperature / S.tc[k]);
-    k_scalars_a<<<1, 256, 0, c->stream>>>(F, c->partial_fin.p, c->nb_fin, c->scalars.p);
+    k_scalars_a<<<1, 1024, 0, c->stream>>>(F, c->partial_fin.p, c->nb_fin, c->scalars.p);
     check_launch(c);
   }
   boundary_condition<R>(c);
@@ -3014,7 +3057,7 @@ void upload_static(sc_ctx *c) {
   c->partial_bg.alloc((size_t)c->nb_bnd * 6);
   c->partial_bgt.alloc((size_t)c->nb_bnd * 6);
   c->partial_vp.alloc((size_t)c->nb_vp * 6);
-  c->partial_acc.alloc((size_t)16 * c->nb_acc * 3);
+  c->partial_acc.alloc((size_t)AND_MAX_RANK * c->nb_acc * 3);
   c->partial_vp.zero(s);
   if (S.n_filters && !S.keldysh) {
     c->pois_s.alloc(2 * nn);
