@@ -678,34 +678,10 @@ void evaluate_once(sc_ctx *c) {
   const HostSetup &S = c->S;
   if (!c->boundary_initialized) boundary_initial<double>(c);
   extend_reference(c);
-  c->acc_d.zero(c->stream);
-  c->acc_j.zero(c->stream);
-  c->acc_fe.zero(c->stream);
   run_chunks<double>(c, 0);
   const size_t nn = c->nn0();
   double *delta = c->xstate.p, *avec = c->xstate.p + (size_t)2 * S.nc * nn;
-  const double jfactor = (double)(2 * S.charge_sign) * S.temperature;
-  auto fin = S.nc == 1 ? k_finalize<1> : S.nc == 2 ? k_finalize<2> : k_finalize<0>;
-  fin<<<c->nb_fin, REDUCE_THREADS, 0, c->stream>>>(
-      S.n0, S.nc, S.h, jfactor, c->has_vp() ? 1 : 0, c->dom.p, c->coupling.p, c->acc_d.p, c->acc_j.p, c->acc_fe.p,
-      delta, avec, c->gstate.p, c->j_real.p, c->partial_fin.p);
-  check_launch(c);
-  FinalizeConsts F{};
-  F.nc = S.nc;
-  F.norm = S.norm;
-  F.n_grain = S.n_grain;
-  F.has_vp = c->has_vp() ? 1 : 0;
-  F.n_elem_field = 2 * nn;
-  F.temperature = S.temperature;
-  F.h = S.h;
-  F.lambda = S.lambda;
-  F.conv = S.conv_crit;
-  double si = 0.0;
-  for (int e = 0; e < S.ne; ++e) si += S.residues[e] / S.e_im[e];
-  F.sum_inv = si * S.temperature;
-  for (int k = 0; k < S.nc; ++k) F.log_t_tc[k] = std::log(S.temperature / S.tc[k]);
-  k_scalars_a<<<1, 1024, 0, c->stream>>>(F, c->partial_fin.p, c->nb_fin, c->scalars.p);
-  check_launch(c);
+  launch_finalize(c, delta, avec);
 }
 
 struct AdjBuffers {

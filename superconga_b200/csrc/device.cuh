@@ -115,6 +115,81 @@ __device__ __forceinline__ Cx<R> riccati_step(R dre, R dim, R ere, R eim, Cx<R> 
   return Cx<R>{(c2r * den_re + c2i * den_im) * inv, (c2i * den_re - c2r * den_im) * inv};
 }
 
+// Whether the fields of a site allow step_fast for every energy: with
+// |gamma| <= 1 the discriminant's real part (over 4) is at least
+// 1/4 - (h e_re / 2)^2 - 2 (h/4) |D| (the imaginary energies are positive, so
+// (1 + h e_im) / 2 >= 1/2); the factor 2.5 instead of 2 leaves room for
+// rounding.  False for NaN.  At 20 lattice points per xi0 the left side is
+// 0.25 and the right side 0.01.
+__device__ __forceinline__ bool fields_allow_fast(float dre, float dim, float es, float h, float e_re_max) {
+  const float s = 0.5f * h * (fabsf(es) + e_re_max);
+  return 0.25f - s * s > 0.625f * h * (fabsf(dre) + fabsf(dim));
+}
+
+// The midpoint step in the interior of the grain, where fields_allow_fast
+// holds on both sites, in fewer operations than riccati_step: everything is
+// kept at half scale (b/2, the discriminant/4, its real part/8), so that
+//   g1 = c / (sqrt(w) - b/2),  w = (b^2 - 4 a c) / 4,
+//   xh = Re w / 2 = (bh^2 + s0)/2 - Re(a g0),  u = Im w / 2 = bh sh - Im(a g0),
+//   sqrt(w) = (t, u / t),  t = sqrt(|w|/2 + xh),
+// with bh = -(1 + h e_im)/2 of the energy and sh = h e_re / 2,
+// s0 = (h |D| / 2)^2 - sh^2 of the site.  Re w > 0, so the root has no branch
+// and no sign to choose, and the smallest normal number added to |w|^2 keeps
+// every estimate finite with no guard.  43 FP64 operations instead of 59.
+template <typename R>
+struct SiteConst {
+  R ar, ai, hdr, hdi, s0h, sh;  // a, h D, s0 / 2, h e_re / 2 (without the energy's own real part)
+};
+template <typename R>
+__device__ __forceinline__ SiteConst<R> site_const(R dre, R dim, R es, R h) {
+  SiteConst<R> c;
+  const R q = R(0.25) * h;
+  c.ar = q * dim;
+  c.ai = q * dre;
+  c.hdr = R(4) * c.ai;
+  c.hdi = R(4) * c.ar;
+  c.sh = R(0.5) * h * es;
+  c.s0h = R(2) * (c.ar * c.ar + c.ai * c.ai);  // the -sh^2 / 2 is subtracted where sh is final
+  return c;
+}
+// x / sqrt(x) and 1 / sqrt(x) for the step: the estimate refined as in rsqrt_.
+__device__ __forceinline__ double sqrt_pos(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double p = x * r;
+  const double e = fma(-p, r, 1.0);
+  return fma(p, e * fma(0.375, e, 0.5), p);
+}
+__device__ __forceinline__ float sqrt_pos(float x) { return sqrt_(x); }
+// Reciprocal and reciprocal square root of arguments of order one: in FP32 the
+// hardware estimates without the scaling that subnormal arguments need.
+__device__ __forceinline__ double rsqrt_pos(double x) { return rsqrt_(x); }
+__device__ __forceinline__ float rsqrt_pos(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ double rcp_pos(double x) { return rcp_(x); }
+__device__ __forceinline__ float rcp_pos(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+template <typename R>
+__device__ __forceinline__ Cx<R> step_fast(const SiteConst<R> &S, R s0h, R sh, R bh, Cx<R> g) {
+  const R agre = S.ar * g.re - S.ai * g.im, agim = S.ar * g.im + S.ai * g.re;
+  const R br = agre + bh, bi = agim + sh;  // b / 2
+  const R tr = br + (bh + R(2)), ti = bi + sh;
+  const R cre = tr * g.re - (ti * g.im + S.hdi), cim = tr * g.im + (ti * g.re + S.hdr);
+  const R xh = (R(0.5) * bh * bh + s0h) - agre, u = bh * sh - agim;
+  const R m = sqrt_pos(xh * xh + (u * u + R(sizeof(R) == 8 ? 1e-300 : 1e-37)));
+  const R U = m + xh;
+  const R rho = rsqrt_pos(U);
+  const R dr = U * rho - br, di = u * rho - bi;
+  const R inv = rcp_pos(dr * dr + di * di);
+  return Cx<R>{(cre * dr + cim * di) * inv, (cim * dr - cre * di) * inv};
+}
+
 // Two energies of one thread, lane by lane in FP32 pairs:
 // re = (Re z_j, Re z_j+1), im = (Im z_j, Im z_j+1).  sm_100 executes one
 // FFMA2 / FMUL2 / FADD2 instruction for both lanes, so the FP32 arithmetic of
@@ -175,6 +250,65 @@ __device__ __forceinline__ Cx2 riccati_step2(float dre, float dim, float2 ere, f
   // 2 c / den = 2 c conj(den) / |den|^2 (the factor 2 is exact, so it goes with 1/|den|^2).
   const float2 inv2 = mul2(bc2(2.0f), make_float2(rcp_(s.x), rcp_(s.y)));
   return Cx2{mul2(fma2(cre, dr, mul2(cim, di)), inv2), mul2(fma2(cim, dr, mul2(neg2(cre), di)), inv2)};
+}
+
+// The interior step of the FP32 sweep, two energies at a time.  The step is
+// close to the identity, and its terms of order one (1 + h e, the root near
+// 1/2) round off the small numbers that make up the change: in their place it
+// is written for the change itself,
+//   g1 = g0 + (k g0 + i h D) / den,  k = 2 a g0 - 3 d - sg + 3 i sh,
+//   den = 1 + d + sg - a g0 - i sh,  d = h e_im / 2,  sh = h e_re / 2,
+// with the root sqrt(w) = 1/2 + sg of w = 1/4 + om,
+//   om = d + d^2 + (h |D| / 2)^2 - sh^2 - 2 a g0 - i (1 + 2 d) sh,
+// whose small part sg is taken once through sg = om - sg^2 (from
+// sg (1 + sg) = om), which leaves 2 |sg| of the error that sg has as the
+// root's estimate minus 1/2.  Then k, i h D and the change carry relative FP32
+// errors, and only the last addition rounds at the size of g0.
+// Negated quantities (nx = -x) are carried where that saves a sign change:
+// the packed instructions have no operand negation, and a change of sign costs
+// one more.  39 packed operations (a step on the values themselves: 42).
+struct SiteConst2 {
+  float2 ai, nar, nai, hdi, nhdr;
+};
+struct EnergyConst2 {
+  float2 nbh, c1, d2h, d3;  // 1/2 + d, 1 + d, (d + d^2) / 2, 3 d
+};
+__device__ __forceinline__ Cx2 step_fast2(const SiteConst2 &S, float2 s0h, float2 nsh, float2 n3sh,
+                                          const EnergyConst2 &E, Cx2 g) {
+  const float2 m1 = bc2(-1.0f), two = bc2(2.0f);
+  const float2 nur = fma2(S.ai, g.im, mul2(S.nar, g.re)), nui = fma2(S.nar, g.im, mul2(S.nai, g.re));  // -a g0
+  const float2 omr = add2(add2(E.d2h, s0h), nur), y = fma2(E.nbh, nsh, nui);                           // om / 2
+  const float2 xh = add2(omr, bc2(0.125f));
+  const float2 xx = fma2(xh, xh, fma2(y, y, bc2(1e-37f)));
+  const float2 U = add2(make_float2(sqrt_(xx.x), sqrt_(xx.y)), xh);
+  const float2 rho = make_float2(rsqrt_pos(U.x), rsqrt_pos(U.y));
+  const float2 sgr = fma2(U, rho, bc2(-0.5f)), sgi = mul2(y, rho);
+  const float2 dr = add2(add2(nur, E.c1), sgr), di = add2(add2(nui, nsh), sgi);
+  const float2 nsgr = mul2(sgr, m1);
+  const float2 nkr = fma2(sgi, sgi, fma2(nsgr, sgr, fma2(two, add2(omr, nur), E.d3)));
+  const float2 nki = fma2(two, add2(nui, fma2(nsgr, sgi, y)), n3sh);
+  const float2 ngi = mul2(g.im, m1);
+  const float2 nnr = fma2(nkr, g.re, fma2(nki, ngi, S.hdi)), nni = fma2(nkr, g.im, fma2(nki, g.re, S.nhdr));
+  const float2 s = fma2(dr, dr, mul2(di, di));
+  const float2 ninv = make_float2(-rcp_pos(s.x), -rcp_pos(s.y));
+  const float2 ndi = mul2(di, m1);
+  return Cx2{fma2(fma2(nnr, dr, mul2(nni, di)), ninv, g.re), fma2(fma2(nni, dr, mul2(nnr, ndi)), ninv, g.im)};
+}
+// The same for one energy.
+__device__ __forceinline__ Cx<float> step_fast_f32(const SiteConst<float> &S, float s0h, float sh, float d,
+                                                   Cx<float> g) {
+  const float nur = S.ai * g.im - S.ar * g.re, nui = -(S.ar * g.im + S.ai * g.re);
+  const float omr = ((0.5f * d) * (1.0f + d) + s0h) + nur, y = nui - (0.5f + d) * sh;
+  const float xh = omr + 0.125f;
+  const float U = sqrt_(xh * xh + (y * y + 1e-37f)) + xh;
+  const float rho = rsqrt_pos(U);
+  const float sgr = fmaf(U, rho, -0.5f), sgi = y * rho;
+  const float dr = (nur + (1.0f + d)) + sgr, di = (nui - sh) + sgi;
+  const float nkr = fmaf(sgi, sgi, fmaf(-sgr, sgr, fmaf(2.0f, omr + nur, 3.0f * d)));
+  const float nki = fmaf(2.0f, nui + fmaf(-sgr, sgi, y), -3.0f * sh);
+  const float nnr = fmaf(nkr, g.re, fmaf(-nki, g.im, S.hdi)), nni = fmaf(nkr, g.im, fmaf(nki, g.re, -S.hdr));
+  const float ninv = -rcp_pos(dr * dr + di * di);
+  return Cx<float>{fmaf(nnr * dr + nni * di, ninv, g.re), fmaf(nni * dr - nnr * di, ninv, g.im)};
 }
 
 // local_greens<float> of two energies, before the signs: with p = g gt and
@@ -263,6 +397,21 @@ struct Bilinear {
   int i00;  // index of the lower-left corner in the input grid
   double xf, yf;
 };
+// (int)v and v - (int)v of |v| < 2^31 through the low word of v + 3 * 2^51
+// rounded down: two additions where the conversions to an integer and back are
+// quarter-rate instructions.  Rounding down differs from truncation only for
+// v < 0, of which only -1 < v is ever used.
+__device__ __forceinline__ int split(double v, double &frac) {
+  const double magic = 6755399441055744.0;  // 3 * 2^51
+  const double t = __dadd_rd(v, magic);
+  int i = __double2loint(t);
+  frac = v - (t - magic);
+  if (i == -1 && v > -1.0) {
+    i = 0;
+    frac = v;
+  }
+  return i;
+}
 __device__ __forceinline__ bool rotated_lookup(int x, int y, int n_out, int n_in, double c,
                                                double s, Bilinear &b) {
   const double xt = (double)(n_in - n_out) / 2.0;
@@ -270,20 +419,25 @@ __device__ __forceinline__ bool rotated_lookup(int x, int y, int n_out, int n_in
   const double X = (double)x + xt - sh, Y = (double)y + xt - sh;
   const double xr = X * c - Y * s + sh;
   const double yr = X * s + Y * c + sh;
-  const int xi = (int)xr, yi = (int)yr;
+  const int xi = split(xr, b.xf), yi = split(yr, b.yf);
   if (xi >= 0 && xi + 1 < n_in && yi >= 0 && yi + 1 < n_in) {
     b.i00 = yi * n_in + xi;
-    b.xf = xr - (double)xi;
-    b.yf = yr - (double)yi;
     return true;
   }
   return false;
 }
-__device__ __forceinline__ double bilerp(double v00, double v01, double v10, double v11,
-                                         double xf, double yf) {
-  const double x1 = (1.0 - xf) * v00 + xf * v01;
-  const double x2 = (1.0 - xf) * v10 + xf * v11;
-  return (1.0 - yf) * x1 + yf * x2;
+// The four corner weights of a lookup: a field then costs four fused
+// multiply-adds (against nine operations as three interpolations).
+struct Corners {
+  double w00, w01, w10, w11;
+};
+__device__ __forceinline__ Corners corners(const Bilinear &b, double scale = 1.0) {
+  const double y1 = b.yf * scale, y0 = scale - y1;
+  const double w01 = b.xf * y0, w11 = b.xf * y1;
+  return Corners{y0 - w01, w01, y1 - w11, w11};
+}
+__device__ __forceinline__ double weigh(const Corners &w, double v00, double v01, double v10, double v11) {
+  return fma(w.w11, v11, fma(w.w10, v10, fma(w.w01, v01, w.w00 * v00)));
 }
 
 }  // namespace scb

@@ -64,35 +64,14 @@ constexpr int NQ = 38;  // partial-sum slots of the finalize reduction (four com
 
 // ------------------------------------------------------------------ kernels --
 
-// The reference-grid fields the frame lookups gather, one record per site:
-// rf[site * (nc + 1) + c] = (Re, Im) of order-parameter component c and
-// rf[site * (nc + 1) + nc] = (A_x, A_y) of the induced vector potential, so
-// that a bilinear corner costs one 16-byte load per field pair instead of two
-// 8-byte loads from separate planes.  k_pack_reference copies the state
-// (planar, [2 nc + 2][N0 * N0]) into it.
-__global__ void k_pack_reference(int nc, int nn, const double *__restrict__ x, double2 *__restrict__ rf) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nn) return;
-  double2 *r = rf + (size_t)i * (nc + 1);
-  for (int c = 0; c <= nc; ++c) r[c] = make_double2(x[(size_t)(2 * c) * nn + i], x[(size_t)(2 * c + 1) * nn + i]);
-}
-
-// FP32 copy of the records for the mixed-precision lookups (the FP32 sweep
-// rounds the frame fields to FP32 anyway): half the bytes per gathered corner.
-__global__ void k_round_reference(size_t n, const double2 *__restrict__ rf, float2 *__restrict__ rf32) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double2 v = rf[i];
-  rf32[i] = make_float2((float)v.x, (float)v.y);
-}
-
 // Reference-grid extension of the order parameter (domain_ops.h:11-69):
 // the order parameter everywhere, except label-0 sites next to the grain,
 // which get the mean of their nearest grain sites; written into the records
-// of k_pack_reference (field f = 2c + part of component c).
+// of k_advance_pack (field f = 2c + part of component c).
 __global__ void k_extend_reference(int n_fields, int nn, int n_sites, int stride, const int *__restrict__ site,
                                    const int *__restrict__ off, const int *__restrict__ src,
-                                   const double *__restrict__ in, double *__restrict__ out) {
+                                   const double *__restrict__ in, double *__restrict__ out,
+                                   float *__restrict__ out32) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int f = blockIdx.y;
   if (k >= n_sites || f >= n_fields) return;
@@ -100,7 +79,10 @@ __global__ void k_extend_reference(int n_fields, int nn, int n_sites, int stride
   const int b = off[k], e = off[k + 1];
   double acc = v[src[b]];
   for (int i = b + 1; i < e; ++i) acc = __dadd_rn(acc, v[src[i]]);
-  out[((size_t)site[k] * stride + (f >> 1)) * 2 + (f & 1)] = __ddiv_rn(acc, (double)(e - b));
+  const size_t o = ((size_t)site[k] * stride + (f >> 1)) * 2 + (f & 1);
+  const double v_ext = __ddiv_rn(acc, (double)(e - b));
+  out[o] = v_ext;
+  if (out32) out32[o] = (float)v_ext;
 }
 
 // Element of the frame buffers: the per-angle Matsubara sums are accumulated in
@@ -166,6 +148,7 @@ struct SweepArgs {
   int pair;  // angle offset of the mirrored partner angle (n_angles / 2), 0 = unpaired
   int kmax;  // longest column of the chunk: rows of one scratch tile
   double h, lam_scale, flux_b, q, area;
+  float e_re_max;  // largest |real energy| of the sweep (0 for Ozaki energies)
   const int4 *items;  // (angle, x, first row, last row)
   const AngleParams *ang;
   const uint8_t *labels;
@@ -173,22 +156,24 @@ struct SweepArgs {
   const double *dist_in_g, *dist_out_g, *dist_in_gt, *dist_out_gt;
   const Cx<R> *bin_g, *bin_gt;
   Cx<R> *bout_g, *bout_gt;
-  const double2 *rf;   // [n0*n0][nc + 1]: extended order parameter per component, then A (k_pack_reference)
+  const double2 *rf;   // [n0*n0][nc + 1]: extended order parameter per component, then A (k_advance_pack)
   const float2 *rf32;  // the same records in FP32 (mixed precision: the FP32 sweep's lookups read these)
   const double *e_re, *e_im, *res;
+  const double *res2;  // twice the residues
   Cx<R> *scratch;   // [tile][row][energy][item of tile]
   R *scratch2;      // frame-field records [tile][row][item of tile] of (Re D, Im D, energy shift, label), in R
   typename FrameOf<R>::type *fr;  // frame records [slot][n1*n1][2]: (Re F, Im F), (Re g, Re I)
   typename LdosOf<R>::type *ldf;  // LDOS frame buffer [slot][n1*n1][energy]: Im g per real energy
 };
 
-// Scratch tiles: the items of one warp (32 / G trajectory columns, G = 2^lg
-// threads per column) keep their sweep scratch together, row after row, so the
-// rows a warp steps through are contiguous in memory instead of spread over
-// planes the size of the chunk: gammaTilde [tile][row][energy][column of tile].
+// Scratch tiles: the 16 / G trajectory columns that one warp sweeps (G = 2^lg
+// threads per column and coherence function; half a warp per function) keep
+// their sweep scratch together, row after row, so the rows a warp steps
+// through are contiguous in memory instead of spread over planes the size of
+// the chunk: [tile][row][energy][column of tile].
 template <typename R>
 __device__ __forceinline__ size_t scratch_index(const SweepArgs<R> &A, int lg, int item, int r, int e) {
-  const int sh = 5 - lg;
+  const int sh = 4 - lg;
   const size_t tile = (size_t)(item >> sh), k = (size_t)(item & ((1 << sh) - 1));
   return (((tile * A.kmax + r) * A.ne + e) << sh) + k;
 }
@@ -197,22 +182,29 @@ __device__ __forceinline__ size_t scratch_index(const SweepArgs<R> &A, int lg, i
 // thread stores and loads both of its energies with one vector access.
 template <typename R>
 __device__ __forceinline__ size_t scratch_pair_index(const SweepArgs<R> &A, int lg, int item, int r, int p) {
-  const int sh = 5 - lg;
+  const int sh = 4 - lg;
   const size_t tile = (size_t)(item >> sh), k = (size_t)(item & ((1 << sh) - 1));
   return (((tile * A.kmax + r) * (size_t)((A.ne + 1) >> 1) + p) << sh) + k;
 }
 // Frame-field records, one per column site in the same tiles: (Re D, Im D,
-// energy shift, frame label), [tile][row][column of tile], read by the sweep
-// with one vector load per site.
+// energy shift, site code), [tile][row][column of tile], read by the sweep
+// with one vector load per site.  The site code is kept as integer bits: the
+// frame label, plus SITE_GENERAL where the fields are too large for the
+// shortened interior step (step_fast).
 template <typename R> struct Rec4;
 template <> struct Rec4<double> { using type = double4; };
 template <> struct Rec4<float> { using type = float4; };
 template <typename R>
 __device__ __forceinline__ size_t rec_index(const SweepArgs<R> &A, int lg, int item, int r) {
-  const int sh = 5 - lg;
+  const int sh = 4 - lg;
   const size_t tile = (size_t)(item >> sh), k = (size_t)(item & ((1 << sh) - 1));
   return ((tile * A.kmax + r) << sh) + k;
 }
+constexpr int SITE_LABEL = 7, SITE_GENERAL = 8;
+__device__ __forceinline__ double code_bits(double, int code) { return __hiloint2double(0, code); }
+__device__ __forceinline__ float code_bits(float, int code) { return __int_as_float(code); }
+__device__ __forceinline__ int site_code(double w) { return __double2loint(w); }
+__device__ __forceinline__ int site_code(float w) { return __float_as_int(w); }
 
 // Gauges, include/conga/riccati/energy_shift/Gauges.h:25-62.
 __device__ __forceinline__ void gauge_potential(int gauge, double b, double area, double x,
@@ -268,28 +260,26 @@ __device__ __forceinline__ void frame_fields(const SweepArgs<R> &A, const AngleP
   double2 ca[4];
   const bool inD = rotated_lookup(x, y, A.n1, n0, P.cD, P.sD, b);
   if (inD) {
-    double c_re[4] = {0, 0, 0, 0}, c_im[4] = {0, 0, 0, 0};
-    const int off[4] = {b.i00, b.i00 + 1, b.i00 + n0, b.i00 + n0 + 1};
+    const Corners w = corners(b);
+    const size_t o00 = (size_t)b.i00, o01 = o00 + 1, o10 = o00 + n0, o11 = o10 + 1;
     if (one) {
+      double2 v0, v1, v2, v3;
+      ld_rec01(A, o00, v0, ca[0]);
+      ld_rec01(A, o01, v1, ca[1]);
+      ld_rec01(A, o10, v2, ca[2]);
+      ld_rec01(A, o11, v3, ca[3]);
       const double et = P.eta[0];
-      for (int k = 0; k < 4; ++k) {
-        double2 v;
-        ld_rec01(A, (size_t)off[k], v, ca[k]);
-        c_re[k] += v.x * et;
-        c_im[k] += v.y * et;
-      }
+      dre = weigh(w, v0.x, v1.x, v2.x, v3.x) * et;
+      dim = weigh(w, v0.y, v1.y, v2.y, v3.y) * et;
     } else {
       for (int c = 0; c < A.nc; ++c) {
         const double et = P.eta[c];
-        for (int k = 0; k < 4; ++k) {
-          const double2 v = ld_rec(A, (size_t)off[k] * st + c);
-          c_re[k] += v.x * et;
-          c_im[k] += v.y * et;
-        }
+        const double2 v0 = ld_rec(A, o00 * st + c), v1 = ld_rec(A, o01 * st + c), v2 = ld_rec(A, o10 * st + c),
+                      v3 = ld_rec(A, o11 * st + c);
+        dre = fma(et, weigh(w, v0.x, v1.x, v2.x, v3.x), dre);
+        dim = fma(et, weigh(w, v0.y, v1.y, v2.y, v3.y), dim);
       }
     }
-    dre = bilerp(c_re[0], c_re[1], c_re[2], c_re[3], b.xf, b.yf);
-    dim = bilerp(c_im[0], c_im[1], c_im[2], c_im[3], b.xf, b.yf);
   }
   es = 0.0;
   if (A.has_vp || A.has_ext) {
@@ -315,8 +305,9 @@ __device__ __forceinline__ void frame_fields(const SweepArgs<R> &A, const AngleP
           v10 = ld_rec(A, pa + (size_t)(ba.i00 + n0) * st);
           v11 = ld_rec(A, pa + (size_t)(ba.i00 + n0 + 1) * st);
         }
-        rx = bilerp(v00.x, v01.x, v10.x, v11.x, ba.xf, ba.yf);
-        ry = bilerp(v00.y, v01.y, v10.y, v11.y, ba.xf, ba.yf);
+        const Corners w = corners(ba);
+        rx = weigh(w, v00.x, v01.x, v10.x, v11.x);
+        ry = weigh(w, v00.y, v01.y, v10.y, v11.y);
       }
       rx *= A.lam_scale;
       ry *= A.lam_scale;
@@ -331,32 +322,6 @@ __device__ __forceinline__ void group_sum(double &v, int groups, unsigned mask) 
   for (int o = groups >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
 }
 
-// Sum of four values over the G threads of a group, scattered: afterwards the
-// thread whose group index has bits (b1 b0) in the two highest positions holds
-// the total of value 2 b1 + b0 (G >= 4), or of values {2 b0, 2 b0 + 1} in v[0],
-// v[1] (G = 2).  Halving the exchanged set in each of the first two rounds
-// takes 3 (G = 2: 2, G = 8: 4) shuffles instead of 4 log2(G).
-__device__ __forceinline__ void group_sum4_scatter(double v[4], int g, int log_groups, unsigned mask) {
-  if (log_groups == 0) return;
-  int o = 1 << (log_groups - 1);
-  {  // keep two of four
-    const bool up = (g & o) != 0;
-    const double s0 = up ? v[0] : v[2], s1 = up ? v[1] : v[3];
-    const double r0 = __shfl_xor_sync(mask, s0, o), r1 = __shfl_xor_sync(mask, s1, o);
-    v[0] = (up ? v[2] : v[0]) + r0;
-    v[1] = (up ? v[3] : v[1]) + r1;
-  }
-  o >>= 1;
-  if (!o) return;
-  {  // keep one of two
-    const bool up = (g & o) != 0;
-    const double sv = up ? v[0] : v[1];
-    const double r = __shfl_xor_sync(mask, sv, o);
-    v[0] = (up ? v[1] : v[0]) + r;
-  }
-  for (o >>= 1; o > 0; o >>= 1) v[0] += __shfl_xor_sync(mask, v[0], o);
-}
-
 // Rotated order parameter and Doppler shift of every site of every trajectory
 // column of a chunk, written with the site's frame label as one record per
 // site (rec_index) for the sweep.
@@ -365,7 +330,7 @@ __device__ __forceinline__ void group_sum4_scatter(double v[4], int g, int log_g
 // the reference grid (a warp along one row touched ~20 sectors per gather).
 constexpr int FF_COLS = 8, FF_ROWS = 16;
 template <typename R>
-__global__ void __launch_bounds__(FF_COLS * FF_ROWS) k_frame_fields(const SweepArgs<R> A, int rows_per_block) {
+__global__ void __launch_bounds__(FF_COLS * FF_ROWS, sizeof(R) == 4 ? 6 : 1) k_frame_fields(const SweepArgs<R> A, int rows_per_block) {
   const int item = blockIdx.x * FF_COLS + threadIdx.x;
   if (item >= A.n_items) return;
   const int4 it = A.items[item];
@@ -376,587 +341,14 @@ __global__ void __launch_bounds__(FF_COLS * FF_ROWS) k_frame_fields(const SweepA
   for (int r = r0 + threadIdx.y; r < r1; r += FF_ROWS) {
     double dre, dim, es;
     frame_fields(A, P, x, lo + r, dre, dim, es);
-    const uint8_t lab = A.labels[(size_t)a * A.n1 * A.n1 + (size_t)(lo + r) * A.n1 + x];
+    int code = A.labels[(size_t)a * A.n1 * A.n1 + (size_t)(lo + r) * A.n1 + x];
+    if (!fields_allow_fast((float)dre, (float)dim, (float)es, (float)P.hs, A.e_re_max)) code |= SITE_GENERAL;
     typedef typename Rec4<R>::type V4;
-    ((V4 *)A.scratch2)[rec_index(A, A.log_groups, item, r)] = V4{(R)dre, (R)dim, (R)es, (R)lab};
+    ((V4 *)A.scratch2)[rec_index(A, A.log_groups, item, r)] = V4{(R)dre, (R)dim, (R)es, code_bits(R(0), code)};
   }
 }
 
-// One step of one coherence function at one site for EMAX interleaved
-// energies (internal::computeStep, RiccatiSolverConfined.h:129-225): entry
-// sites start from the stored boundary value with the partial step dist*h, grain
-// sites take the midpoint step, exit sites also step on to the boundary and
-// store the out-going value, sites outside the grain reset to zero.
-template <typename R, int EMAX, bool KEL>
-__device__ __forceinline__ void site_step(uint8_t l, uint8_t l_entry, uint8_t l_exit, R dre,
-                                          R dim, R es, R pdre, R pdim, R pes, const R *ere,
-                                          const R *eim, Cx<R> *coh, int ept, int ecount, R h,
-                                          R dist_in, const Cx<R> *bin, R dist_out, Cx<R> *bout) {
-  const bool entry = l == l_entry;
-  const R sdre = entry ? dre : (dre + pdre) * R(0.5);
-  const R sdim = entry ? dim : (dim + pdim) * R(0.5);
-  const R ses = entry ? es : (es + pes) * R(0.5);
-  const R st = entry ? dist_in * h : h;
-#pragma unroll
-  for (int j = 0; j < EMAX; ++j)
-    if (j < ept) {
-      Cx<R> g0 = coh[j];
-      if (entry) g0 = (j < ecount) ? bin[j] : Cx<R>{R(0), R(0)};
-      coh[j] = riccati_step<R>(sdre, sdim, KEL ? ses + ere[j] : ses, eim[j], g0, st);
-    }
-  if (l == l_exit) {
-    const R sb = dist_out * h;
-#pragma unroll
-    for (int j = 0; j < EMAX; ++j)
-      if (j < ept) {
-        const Cx<R> bv = riccati_step<R>(dre, dim, KEL ? es + ere[j] : es, eim[j], coh[j], sb);
-        if (j < ecount) bout[j] = bv;
-      }
-  }
-  if (l == 0) {
-#pragma unroll
-    for (int j = 0; j < EMAX; ++j) coh[j] = Cx<R>{R(0), R(0)};
-  }
-}
-
-// The step at a grain site (label 1) between two grain sites: midpoint fields,
-// full step, no boundary bookkeeping (site_step handles the other labels).
-template <typename R, int EMAX, bool KEL>
-__device__ __forceinline__ void interior_step(R dre, R dim, R es, R pdre, R pdim, R pes,
-                                              const R *ere, const R *eim, Cx<R> *coh, int ept,
-                                              R h) {
-  const R sdre = (dre + pdre) * R(0.5);
-  const R sdim = (dim + pdim) * R(0.5);
-  const R ses = (es + pes) * R(0.5);
-#pragma unroll
-  for (int j = 0; j < EMAX; ++j)
-    if (j < ept) coh[j] = riccati_step<R>(sdre, sdim, KEL ? ses + ere[j] : ses, eim[j], coh[j], h);
-}
-
-// site_step and interior_step of the packed FP32 sweep: energies in pairs
-// (riccati_step2), every thread with its full EMAX energies (the launch
-// guarantees ept = EMAX).
-// The real parts of energies j, j + 1 with the Doppler shift es added (KEL:
-// real energies; Matsubara energies have none).
-template <bool KEL>
-__device__ __forceinline__ float2 ere_pair(const float *ere, int j, float es) {
-  return KEL ? make_float2(es + ere[j], es + ere[j + 1]) : bc2(es);
-}
-template <int EMAX, bool KEL>
-__device__ __forceinline__ void site_step_x2(uint8_t l, uint8_t l_entry, uint8_t l_exit, float dre, float dim,
-                                             float es, float pdre, float pdim, float pes, const float *ere,
-                                             const float *eim, Cx<float> *coh, int ept, int ecount, float h,
-                                             float dist_in, const Cx<float> *bin, float dist_out,
-                                             Cx<float> *bout) {
-  const bool entry = l == l_entry;
-  const float sdre = entry ? dre : (dre + pdre) * 0.5f;
-  const float sdim = entry ? dim : (dim + pdim) * 0.5f;
-  const float ses = entry ? es : (es + pes) * 0.5f;
-  const float st = entry ? dist_in * h : h;
-  const Cx<float> zero{0.0f, 0.0f};
-#pragma unroll
-  for (int j = 0; j < EMAX; j += 2) {
-    if (j >= ept) break;
-    Cx2 g0 = pack2(coh[j], coh[j + 1]);
-    if (entry) g0 = pack2(j < ecount ? bin[j] : zero, j + 1 < ecount ? bin[j + 1] : zero);
-    unpack2(riccati_step2(sdre, sdim, ere_pair<KEL>(ere, j, ses), make_float2(eim[j], eim[j + 1]), g0, st), coh[j],
-            coh[j + 1]);
-  }
-  if (l == l_exit) {
-    const float sb = dist_out * h;
-#pragma unroll
-    for (int j = 0; j < EMAX; j += 2) {
-      if (j >= ept) break;
-      Cx<float> b0, b1;
-      unpack2(riccati_step2(dre, dim, ere_pair<KEL>(ere, j, es), make_float2(eim[j], eim[j + 1]),
-                            pack2(coh[j], coh[j + 1]), sb),
-              b0, b1);
-      if (j < ecount) bout[j] = b0;
-      if (j + 1 < ecount) bout[j + 1] = b1;
-    }
-  }
-  if (l == 0) {
-#pragma unroll
-    for (int j = 0; j < EMAX; ++j) coh[j] = zero;
-  }
-}
-template <int EMAX, bool KEL>
-__device__ __forceinline__ void interior_step_x2(float dre, float dim, float es, float pdre, float pdim, float pes,
-                                                 const float *ere, const float *eim, Cx<float> *coh, int ept,
-                                                 float h) {
-  const float sdre = (dre + pdre) * 0.5f;
-  const float sdim = (dim + pdim) * 0.5f;
-  const float ses = (es + pes) * 0.5f;
-#pragma unroll
-  for (int j = 0; j < EMAX; j += 2)
-    if (j < ept)
-      unpack2(riccati_step2(sdre, sdim, ere_pair<KEL>(ere, j, ses), make_float2(eim[j], eim[j + 1]),
-                            pack2(coh[j], coh[j + 1]), h),
-              coh[j], coh[j + 1]);
-}
-
-// Dispatch of one site's steps to the packed (PK) or the scalar form.
-template <typename R, int EMAX, bool KEL, bool PK>
-__device__ __forceinline__ void interior_any(R dre, R dim, R es, R pdre, R pdim, R pes, const R *ere,
-                                             const R *eim, Cx<R> *coh, int ept, R h) {
-  if constexpr (PK) interior_step_x2<EMAX, KEL>(dre, dim, es, pdre, pdim, pes, ere, eim, coh, ept, h);
-  else interior_step<R, EMAX, KEL>(dre, dim, es, pdre, pdim, pes, ere, eim, coh, ept, h);
-}
-template <typename R, int EMAX, bool KEL, bool PK>
-__device__ __forceinline__ void site_any(uint8_t l, uint8_t l_entry, uint8_t l_exit, R dre, R dim, R es, R pdre,
-                                         R pdim, R pes, const R *ere, const R *eim, Cx<R> *coh, int ept,
-                                         int ecount, R h, R dist_in, const Cx<R> *bin, R dist_out, Cx<R> *bout) {
-  if constexpr (PK)
-    site_step_x2<EMAX, KEL>(l, l_entry, l_exit, dre, dim, es, pdre, pdim, pes, ere, eim, coh, ept, ecount, h,
-                            dist_in, bin, dist_out, bout);
-  else
-    site_step<R, EMAX, KEL>(l, l_entry, l_exit, dre, dim, es, pdre, pdim, pes, ere, eim, coh, ept, ecount, h,
-                            dist_in, bin, dist_out, bout);
-}
-
-// The fused Riccati sweep of one chunk of angles.  G = 2^log_groups threads
-// share one trajectory column (angle, x); thread g integrates Ozaki energies
-// [g*ept, g*ept + ept).  gammaTilde runs down the column first and is kept in
-// scratch; gamma then runs up and the Green sums over all energies are formed
-// site by site (RiccatiSolverConfined.h:129-312, GreensFunctionStatic.h:92-157,
-// ComputeFreeEnergy.h:106-160).  The frame order parameter and the energies come
-// from scratch2; the coherence functions are integrated in R.
-// KEL: real energies e_re + i e_im (the LDOS path, IntegrationIteratorKeldysh.h
-// :219-389); instead of the energy sums, Im g of every energy is written to the
-// LDOS frame buffer (GreensFunctionStatic.h:66-90, ComputeLDOS.h:123-144).
-// One trajectory column (item) for thread g of its group; s_res holds the
-// residues of the energies.
-// STEP_PER_ANGLE: the Riccati step h/|v_F| is read per angle (a non-circular
-// Fermi surface, and the batch); otherwise it is the uniform lattice spacing h
-// of the circle, which stays a kernel parameter.
-// Asynchronous global-to-shared copies of 16 bytes (cp.async.cg, through L2);
-// with pred false nothing is read (the source must still be a valid address)
-// and the 16 bytes are zero-filled.  Each thread waits only for its own
-// copies (cp.async.wait_group), so no barrier is involved.
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool pred) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(pred ? 16 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-// The sweep's staging ring: every thread keeps the inputs of the next NS - 1
-// sites of its column in flight (the site's frame-field record and, going up,
-// the gammaTilde stored going down), copied asynchronously into shared memory
-// ring[stage][16-byte unit][thread], so that the latency of these loads spans
-// several sites' Riccati steps instead of one.  Used by the packed FP32 sweep
-// with at most four energies per thread (128 threads per block; at most 40 KB
-// of shared memory per block: 36 KB at four energies per thread, six stages).
-// Measured on B200: C2 mixed sweep 5.69 -> 5.30 ms, C5 mixed LDOS sweep
-// 79.5 -> 74.9 ms; the FP64 sweep, whose larger records leave room for three
-// stages only, ran 2% (C2) to 18% (C5 LDOS) slower with it and keeps the
-// one-site-ahead register prefetch.
-template <typename R, int EMAX, bool PK>
-struct SweepRing {
-  static constexpr bool on = PK && EMAX <= 4;
-  static constexpr int NV_REC = sizeof(R) == 8 ? 2 : 1;  // record: 32 or 16 bytes
-  static constexpr int NV_GT = PK ? EMAX / 2 : EMAX;      // gammaTilde: one pair or one FP64 energy per unit
-  static constexpr int NV = NV_REC + NV_GT;
-  static constexpr int NS_FIT = (40 * 1024) / (NV * 128 * 16);
-  static constexpr int NS = on ? (NS_FIT < 2 ? 2 : (NS_FIT > 8 ? 8 : NS_FIT)) : 1;
-  static constexpr int NVD = on ? NV : 1;
-};
-
-// PK: the packed FP32 form (energies in pairs: riccati_step2, local_greens2 or
-// greens_g_im2, the scratch in energy-pair records).  Each thread takes an
-// even number of energies (the mapping's count rounded up, at most EMAX), so
-// that every thread's first energy is even.
-template <typename R, int EMAX, bool KEL, bool STEP_PER_ANGLE, int LG = -1, bool PK = false>
-__device__ __forceinline__ void sweep_column(const SweepArgs<R> &A, const double *s_res, int item,
-                                             int g, unsigned gmask) {
-  static_assert(!PK || (std::is_same<R, float>::value && EMAX % 2 == 0), "packed sweep: FP32 pairs");
-  const int lgc = LG >= 0 ? LG : A.log_groups;  // a compile-time group size when the launch knows it
-  const int4 it = A.items[item];
-  const int a = it.x, x = it.y, lo = it.z, hi = it.w;
-  const int n1 = A.n1, ne = A.ne;
-  const size_t nn1 = (size_t)n1 * n1;
-  const size_t T = (size_t)(32 >> lgc);
-  const R h = STEP_PER_ANGLE ? (R)A.ang[a].hs : (R)A.h;  // h / |v_F| of this angle
-  // A compile-time group size comes with a full load (EMAX energies per
-  // thread), a sweep that stores its frame sums, and no energy passes.
-  const int ept = LG >= 0 ? EMAX : (PK ? ((A.ept + 1) & ~1) : A.ept);
-  const bool burn_in = LG >= 0 ? false : A.burn_in != 0;
-  const bool accumulate = LG >= 0 ? false : A.accumulate != 0;
-  const int e0 = g * ept;
-  int ecount = ne - e0;
-  if (ecount > ept) ecount = ept;
-  if (ecount < 0) ecount = 0;
-
-  R eim[EMAX], ere[EMAX];
-#pragma unroll
-  for (int j = 0; j < EMAX; ++j) {
-    eim[j] = (j < ecount) ? (R)A.e_im[e0 + j] : R(1);
-    ere[j] = (KEL && j < ecount) ? (R)A.e_re[e0 + j] : R(0);
-  }
-
-  Cx<R> coh[EMAX];
-  const size_t sb0 = PK ? scratch_pair_index(A, lgc, item, 0, e0 >> 1) : scratch_index(A, lgc, item, 0, e0);
-  const size_t s_row = PK ? (size_t)((ne + 1) >> 1) * T : (size_t)ne * T;
-  const size_t ax = (size_t)a * n1 + x;
-  // Mirrored partner column (angle + pi, x -> n1 - 1 - x) when paired.
-  const size_t pax = (size_t)(a + A.pair) * n1 + (n1 - 1 - x);
-  // Without the staging ring, the next site's label, fields and stored
-  // gammaTilde are loaded one site ahead so that their latency overlaps the
-  // current site's Riccati steps.
-  typedef typename Rec4<R>::type V4;
-  using RG = SweepRing<R, EMAX, PK>;
-  constexpr bool RING = RG::on;
-  constexpr int NS = RG::NS;
-  __shared__ float4 ring[NS][RG::NVD][128];
-  const int tid = threadIdx.x;
-  const int n_rows = hi - lo + 1;
-  const V4 *fb = (const V4 *)A.scratch2 + rec_index(A, lgc, item, 0);
-  // Copies of row `row` (record, and gammaTilde when with_gt) into the stage
-  // of step `step`; one commit group per step, empty outside the column.
-  auto ring_issue = [&](int step, int row, bool with_gt) {
-    if constexpr (RING) {
-      if (row >= 0 && row < n_rows) {
-        const int sl = step % NS;
-        const char *rp = (const char *)(fb + (size_t)row * T);
-#pragma unroll
-        for (int v = 0; v < RG::NV_REC; ++v) cp_async16(&ring[sl][v][tid], rp + 16 * v, true);
-        if (with_gt) {
-          if constexpr (PK) {
-            const float4 *sc = (const float4 *)A.scratch + sb0 + (size_t)row * s_row;
-#pragma unroll
-            for (int jp = 0; jp < RG::NV_GT; ++jp) {
-              const bool ok = 2 * jp < ecount;
-              cp_async16(&ring[sl][RG::NV_REC + jp][tid], ok ? (const void *)(sc + (size_t)jp * T) : (const void *)rp,
-                         ok);
-            }
-          } else {
-            const Cx<R> *sc = A.scratch + sb0 + (size_t)row * s_row;
-#pragma unroll
-            for (int j = 0; j < RG::NV_GT; ++j) {
-              const bool ok = j < ecount;
-              cp_async16(&ring[sl][RG::NV_REC + j][tid], ok ? (const void *)(sc + (size_t)j * T) : (const void *)rp,
-                         ok);
-            }
-          }
-        }
-      }
-      cp_async_commit();
-    }
-  };
-  auto ring_rec = [&](int step) -> V4 {
-    const int sl = step % NS;
-    if constexpr (sizeof(R) == 4) {
-      const float4 v = ring[sl][0][tid];
-      return V4{(R)v.x, (R)v.y, (R)v.z, (R)v.w};
-    } else {
-      const double2 u = *reinterpret_cast<const double2 *>(&ring[sl][0][tid]);
-      const double2 w = *reinterpret_cast<const double2 *>(&ring[sl][RG::NV_REC - 1][tid]);
-      return V4{(R)u.x, (R)u.y, (R)w.x, (R)w.y};
-    }
-  };
-  auto ring_gt = [&](int step, Cx<R> *gt) {
-    const int sl = step % NS;
-    if constexpr (PK) {
-#pragma unroll
-      for (int jp = 0; jp < RG::NV_GT; ++jp) {
-        const float4 v = ring[sl][RG::NV_REC + jp][tid];
-        gt[2 * jp] = Cx<R>{(R)v.x, (R)v.z};
-        gt[2 * jp + 1] = Cx<R>{(R)v.y, (R)v.w};
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < RG::NV_GT; ++j) {
-        const double2 v = *reinterpret_cast<const double2 *>(&ring[sl][RG::NV_REC + j][tid]);
-        gt[j] = Cx<R>{(R)v.x, (R)v.y};
-      }
-    }
-  };
-  // ------------------------------------------------------ gammaTilde, down --
-  {
-    const int in_base = A.idx_in_gt[ax], out_base = A.idx_out_gt[ax];
-    int nin = 0, nout = 0;
-    R pdre = 0, pdim = 0, pes = 0;
-#pragma unroll
-    for (int j = 0; j < EMAX; ++j) coh[j] = Cx<R>{R(0), R(0)};
-    V4 fr;
-    if constexpr (RING) {
-      for (int st = 0; st < NS - 1; ++st) ring_issue(st, n_rows - 1 - st, false);
-    } else {
-      fr = fb[(size_t)(hi - lo) * T];
-    }
-    for (int y = hi; y >= lo; --y) {
-      const int r = y - lo;
-      if constexpr (RING) {
-        const int st = hi - y;
-        ring_issue(st + NS - 1, r - (NS - 1), false);
-        cp_async_wait<NS - 1>();
-        fr = ring_rec(st);
-      }
-      const uint8_t l = (uint8_t)fr.w;
-      // gammaTilde uses -conj(Delta) (RiccatiSolverConfined.h:74-79).
-      const R dre = (R)(-fr.x), dim = (R)fr.y, es = (R)fr.z;
-      if constexpr (!RING) {
-        if (y > lo) fr = fb[(size_t)(r - 1) * T];
-      }
-      if (l == 1) {
-        interior_any<R, EMAX, KEL, PK>(dre, dim, es, pdre, pdim, pes, ere, eim, coh, ept, h);
-      } else {
-        const bool entry = l == 3, exit = l == 2;
-        const R din = entry ? (R)A.dist_in_gt[in_base + nin] : R(0);
-        const R dout = exit ? (R)A.dist_out_gt[out_base + nout] : R(0);
-        site_any<R, EMAX, KEL, PK>(l, 3, 2, dre, dim, es, pdre, pdim, pes, ere, eim, coh, ept, ecount, h,
-                                   din, A.bin_gt + (size_t)(in_base + nin) * A.ne_stride + e0, dout,
-                                   A.bout_gt + (size_t)(out_base + nout) * A.ne_stride + e0);
-        if (A.pair && exit) {
-          // gamma of the partner angle at its exit is conj(gammaTilde) here.
-          const Cx<R> *src = A.bout_gt + (size_t)(out_base + nout) * A.ne_stride + e0;
-          Cx<R> *dst = A.bout_g + (size_t)(A.idx_out_g[pax] + nout) * A.ne_stride + e0;
-#pragma unroll
-          for (int j = 0; j < EMAX; ++j)
-            if (j < ecount) dst[j] = Cx<R>{src[j].re, -src[j].im};
-        }
-        nin += entry;
-        nout += exit;
-      }
-      if (!burn_in) {
-        if constexpr (PK) {
-          float4 *sc = (float4 *)A.scratch + sb0 + (size_t)r * s_row;
-#pragma unroll
-          for (int j = 0; j < EMAX; j += 2)
-            if (j < ecount) sc[(size_t)(j >> 1) * T] = make_float4(coh[j].re, coh[j + 1].re, coh[j].im, coh[j + 1].im);
-        } else {
-          Cx<R> *sc = A.scratch + sb0 + (size_t)r * s_row;
-#pragma unroll
-          for (int j = 0; j < EMAX; ++j)
-            if (j < ecount) sc[(size_t)j * T] = coh[j];
-        }
-      }
-      pdre = dre;
-      pdim = dim;
-      pes = es;
-    }
-    if constexpr (RING) cp_async_wait<0>();
-  }
-  // ----------------------------------------------------------- gamma, up --
-  {
-    const int in_base = A.idx_in_g[ax], out_base = A.idx_out_g[ax];
-    int nin = 0, nout = 0;
-    R pdre = 0, pdim = 0, pes = 0;
-#pragma unroll
-    for (int j = 0; j < EMAX; ++j) coh[j] = Cx<R>{R(0), R(0)};
-    using Fr = typename FrameOf<R>::type;
-    Fr *frs = A.fr + (size_t)(a - A.slot_base) * nn1 * 2;  // this angle's records
-    // The value this thread stores when four or more threads share a column.
-    auto *vdst = &frs->x + (lgc >= 2 ? (g >> (lgc - 2)) : 0);
-    V4 fr;
-    Cx<R> gt_nx[EMAX];
-    // The stored gammaTilde of row r into gt_nx.
-    auto load_gt = [&](int r) {
-      if constexpr (PK) {
-        const float4 *sc = (const float4 *)A.scratch + sb0 + (size_t)r * s_row;
-#pragma unroll
-        for (int j = 0; j < EMAX; j += 2)
-          if (j < ecount) {
-            const float4 v = sc[(size_t)(j >> 1) * T];
-            gt_nx[j] = Cx<R>{v.x, v.z};
-            gt_nx[j + 1] = Cx<R>{v.y, v.w};
-          }
-      } else {
-        const Cx<R> *sc = A.scratch + sb0 + (size_t)r * s_row;
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j)
-          if (j < ecount) gt_nx[j] = sc[(size_t)j * T];
-      }
-    };
-    if constexpr (RING) {
-      for (int st = 0; st < NS - 1; ++st) ring_issue(st, st, !burn_in);
-    } else {
-      fr = fb[0];
-      if (!burn_in) load_gt(0);
-    }
-    for (int y = lo; y <= hi; ++y) {
-      const int r = y - lo;
-      Cx<R> gt[EMAX];
-      if constexpr (RING) {
-        ring_issue(r + NS - 1, r + NS - 1, !burn_in);
-        cp_async_wait<NS - 1>();
-        fr = ring_rec(r);
-        if (!burn_in) ring_gt(r, gt);
-      }
-      const uint8_t l = (uint8_t)fr.w;
-      const R dre = (R)fr.x, dim = (R)fr.y, es = (R)fr.z;
-      if constexpr (!RING) {
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j) gt[j] = gt_nx[j];
-        if (y < hi) {
-          fr = fb[(size_t)(r + 1) * T];
-          if (!burn_in) load_gt(r + 1);
-        }
-      }
-      if (l == 1) {
-        interior_any<R, EMAX, KEL, PK>(dre, dim, es, pdre, pdim, pes, ere, eim, coh, ept, h);
-      } else {
-        const bool entry = l == 2, exit = l == 3;
-        const R din = entry ? (R)A.dist_in_g[in_base + nin] : R(0);
-        const R dout = exit ? (R)A.dist_out_g[out_base + nout] : R(0);
-        site_any<R, EMAX, KEL, PK>(l, 2, 3, dre, dim, es, pdre, pdim, pes, ere, eim, coh, ept, ecount, h,
-                                   din, A.bin_g + (size_t)(in_base + nin) * A.ne_stride + e0, dout,
-                                   A.bout_g + (size_t)(out_base + nout) * A.ne_stride + e0);
-        if (A.pair && exit) {
-          // gammaTilde of the partner angle at its exit is conj(gamma) here.
-          const Cx<R> *src = A.bout_g + (size_t)(out_base + nout) * A.ne_stride + e0;
-          Cx<R> *dst = A.bout_gt + (size_t)(A.idx_out_gt[pax] + nout) * A.ne_stride + e0;
-#pragma unroll
-          for (int j = 0; j < EMAX; ++j)
-            if (j < ecount) dst[j] = Cx<R>{src[j].re, -src[j].im};
-        }
-        nin += entry;
-        nout += exit;
-      }
-      pdre = dre;
-      pdim = dim;
-      pes = es;
-      if (burn_in) continue;
-      if constexpr (KEL) {
-        if (l != 0) {
-          typename LdosOf<R>::type *o = A.ldf + ((size_t)(a - A.slot_base) * nn1 + (size_t)y * n1 + x) * A.ne_stride + e0;
-          if constexpr (PK) {
-#pragma unroll
-            for (int j = 0; j < EMAX; j += 2)
-              if (j < ecount) {
-                const float2 v = greens_g_im2(pack2(coh[j], coh[j + 1]), pack2(gt[j], gt[j + 1]));
-                o[j] = v.x;
-                if (j + 1 < ecount) o[j + 1] = v.y;
-              }
-          } else {
-#pragma unroll
-            for (int j = 0; j < EMAX; ++j)
-              if (j < ecount) o[j] = greens_g_im<R>(coh[j], gt[j]);
-          }
-        }
-        continue;
-      }
-      double sfr = 0.0, sfi = 0.0, sg = 0.0, si = 0.0;
-      if constexpr (PK) {
-        if (l != 0) {
-          // Signs folded into the FP64 accumulation: sg = -sum r fre,
-          // sfi = -sum r nfim, si = -sum r ni.
-#pragma unroll
-          for (int j = 0; j < EMAX; j += 2)
-            if (j < ecount) {
-              float2 fre, Fre, nfim, ni;
-              local_greens2(pack2(coh[j], coh[j + 1]), pack2(gt[j], gt[j + 1]), dre, dim, fre, Fre, nfim, ni);
-              const double r0 = s_res[e0 + j];
-              sfr += r0 * (double)Fre.x;
-              sfi -= r0 * (double)nfim.x;
-              sg -= r0 * (double)fre.x;
-              si -= r0 * (double)ni.x;
-              if (j + 1 < ecount) {
-                const double r1 = s_res[e0 + j + 1];
-                sfr += r1 * (double)Fre.y;
-                sfi -= r1 * (double)nfim.y;
-                sg -= r1 * (double)fre.y;
-                si -= r1 * (double)ni.y;
-              }
-            }
-        }
-      } else if (l != 0) {
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j)
-          if (j < ecount) {
-            Cx<R> F;
-            R gre, iim;
-            local_greens<R>(coh[j], gt[j], dre, dim, F, gre, iim);
-            const double rr = s_res[e0 + j];
-            sfr += rr * (double)F.re;
-            sfi += rr * (double)F.im;
-            sg += rr * (double)gre;
-            si += rr * (double)iim;
-          }
-      }
-      // The mirrored partner angle is not stored: k_rotate_back reads it
-      // from this frame at the mirrored site.
-      const size_t fi = (size_t)y * n1 + x;
-      double v[4] = {sfr, sfi, sg, -si};
-      const int lg = lgc;
-      group_sum4_scatter(v, g, lg, gmask);
-      Fr *rec = frs + 2 * fi;
-      if (lg == 0) {
-        if (accumulate) {
-          const double2 of = as_d2(rec[0]), og = as_d2(rec[1]);
-          v[0] += of.x;
-          v[1] += of.y;
-          v[2] += og.x;
-          v[3] += og.y;
-        }
-        rec[0] = frame_pair<Fr>(v[0], v[1]);
-        rec[1] = frame_pair<Fr>(v[2], v[3]);
-      } else if (lg == 1) {
-        Fr *dst = rec + g;
-        if (accumulate) {
-          const double2 o = as_d2(*dst);
-          v[0] += o.x;
-          v[1] += o.y;
-        }
-        *dst = frame_pair<Fr>(v[0], v[1]);
-      } else {
-        const int sh = lg - 2;  // low bits below the two value bits
-        if ((g & ((1 << sh) - 1)) == 0) {
-          auto *dst = vdst + 4 * fi;
-          if (accumulate) v[0] += (double)*dst;
-          *dst = (decltype(Fr::x))v[0];
-        }
-      }
-    }
-    if constexpr (RING) cp_async_wait<0>();
-  }
-}
-
-template <typename R, int EMAX, int MINB, bool KEL, bool STEP_PER_ANGLE = false, int LG = -1, bool PK = false>
-__global__ void __launch_bounds__(128, MINB) k_sweep(const SweepArgs<R> A) {
-  __shared__ double s_res[SWEEP_MAX_ENERGIES];  // residues of this pass's energies
-  for (int e = threadIdx.x; e < A.ne && e < SWEEP_MAX_ENERGIES; e += blockDim.x) s_res[e] = A.res[e];
-  __syncthreads();
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lgk = LG >= 0 ? LG : A.log_groups, groups = 1 << lgk;
-  const int item = tid >> lgk;
-  const int g = tid & (groups - 1);
-  const int lane = threadIdx.x & 31;
-  const unsigned gmask = ((groups == 32) ? 0xffffffffu : ((1u << groups) - 1u)) << (lane & ~(groups - 1));
-  if (item >= A.n_items) return;  // whole groups leave together (groups divide the warp)
-  sweep_column<R, EMAX, KEL, STEP_PER_ANGLE, LG, PK>(A, s_res, item, g, gmask);
-}
-
-// The sweep of many grains in one persistent launch.  A work unit is one
-// warp's worth of trajectory columns (32 / G of them) of one grain; warps take
-// units from a global counter, longest columns first (the unit list is sorted
-// by the host), so ragged grains share the GPU without a tail per grain.  All
-// grain has its own G = 2^log_groups threads per column (the warp's unit
-// belongs to one grain, so the mapping is uniform within a warp).
-template <typename R, int EMAX, int MINB, bool PK = false>
-__global__ void __launch_bounds__(128, MINB) k_sweep_batch(const SweepArgs<R> *__restrict__ args,
-                                                           const int2 *__restrict__ units, int n_units,
-                                                           int *counter) {
-  const int lane = threadIdx.x & 31;
-  for (;;) {
-    int u = 0;
-    if (lane == 0) u = atomicAdd(counter, 1);
-    u = __shfl_sync(0xffffffffu, u, 0);
-    if (u >= n_units) break;
-    const int2 wu = units[u];
-    const SweepArgs<R> &A = args[wu.x];
-    const int lg = A.log_groups, groups = 1 << lg;
-    const int g = lane & (groups - 1);
-    const int sub = lane >> lg;
-    const unsigned gmask = ((groups == 32) ? 0xffffffffu : ((1u << groups) - 1u)) << (lane & ~(groups - 1));
-    const int item = wu.y + sub;
-    if (item < A.n_items) sweep_column<R, EMAX, false, true, -1, PK>(A, A.res, item, g, gmask);
-  }
-}
+#include "sweep.cuh"
 
 // Frame extension next to the boundary for the angles of one chunk
 // (ComputeOrderParameter.h:180-181, ComputeCurrent.h:149-150,
@@ -991,11 +383,16 @@ __global__ void k_halo(int n_entries, int entry0, int n1, const int *__restrict_
 // frame of a at the mirrored site (n1-1-x, n1-1-y) with gamma' = conj(gammaTilde),
 // gammaTilde' = conj(gamma): F' = F, Re g' = -Re g, Re I' = Re I.  The angles
 // are then accumulated in the order a, a + pair, a + 1, ...
+// first: the chunk is the iteration's first, the sums start from zero.
+// blockIdx.z takes one of gridDim.z equal parts of the chunk's angles into its
+// own copy of the sums (k_finalize adds them in order), so that lattices of
+// few sites fill the GPU: the kernel waits for its gathers (24 of 29 cycles
+// per issue on a 307 x 307 lattice), and only more threads hide that.
 // NC > 0 fixes the component count at compile time (the sums stay in
 // registers); NC = 0 takes it from nc.  One component: four resident blocks
 // per SM (64 registers) measured fastest on B200; more: three.
 template <typename F2, int NC>
-__global__ void __launch_bounds__(256, NC == 1 ? 4 : 3) k_rotate_back(int n0, int n1, int nc_, int a_begin,
+__global__ void __launch_bounds__(256, NC == 1 ? 4 : 3) k_rotate_back(int n0, int n1, int nc_, int first, int a_begin,
                                                      int a_end, int pair, const AngleParams *__restrict__ ang,
                                                      const F2 *__restrict__ fr,
                                                      double *acc_d, double *acc_j, double *acc_fe) {
@@ -1005,15 +402,20 @@ __global__ void __launch_bounds__(256, NC == 1 ? 4 : 3) k_rotate_back(int n0, in
   const size_t nn0 = (size_t)n0 * n0, nn1 = (size_t)n1 * n1;
   const size_t i = (size_t)y * n0 + x;
   const int nc = NC > 0 ? NC : nc_;
+  acc_d += blockIdx.z * (size_t)(2 * nc) * nn0;
+  acc_j += blockIdx.z * 2 * nn0;
+  acc_fe += blockIdx.z * nn0;
+  const int n_ang = a_end - a_begin;
+  const int k0 = (int)((long long)n_ang * blockIdx.z / gridDim.z), k1 = (int)((long long)n_ang * (blockIdx.z + 1) / gridDim.z);
   double dr[NC > 0 ? NC : MAX_COMP], di[NC > 0 ? NC : MAX_COMP];
 #pragma unroll
   for (int c = 0; c < nc; ++c) {
-    dr[c] = acc_d[(size_t)(2 * c) * nn0 + i];
-    di[c] = acc_d[(size_t)(2 * c + 1) * nn0 + i];
+    dr[c] = first ? 0.0 : acc_d[(size_t)(2 * c) * nn0 + i];
+    di[c] = first ? 0.0 : acc_d[(size_t)(2 * c + 1) * nn0 + i];
   }
-  double jx = acc_j[i], jy = acc_j[nn0 + i], fe = acc_fe[i];
-  const int last = (pair ? 2 : 1) * (a_end - a_begin);
-  for (int k = 0; k < last; ++k) {
+  double jx = first ? 0.0 : acc_j[i], jy = first ? 0.0 : acc_j[nn0 + i], fe = first ? 0.0 : acc_fe[i];
+  const int last = (pair ? 2 : 1) * k1;
+  for (int k = (pair ? 2 : 1) * k0; k < last; ++k) {
     const int a0 = a_begin + (pair ? k >> 1 : k);
     const bool mirrored = pair && (k & 1);
     const int a = mirrored ? a0 + pair : a0;
@@ -1036,22 +438,23 @@ __global__ void __launch_bounds__(256, NC == 1 ? 4 : 3) k_rotate_back(int n0, in
       const size_t m = slot + (nn1 - 1 - (size_t)b.i00);
       r00 = load_rec(fr, m); r01 = load_rec(fr, m - 1); r10 = load_rec(fr, m - n1); r11 = load_rec(fr, m - n1 - 1);
     }
-    const double fre = bilerp(r00.f.x, r01.f.x, r10.f.x, r11.f.x, b.xf, b.yf);
-    const double fim = bilerp(r00.f.y, r01.f.y, r10.f.y, r11.f.y, b.xf, b.yf);
+    const Corners w = corners(b);
+    const double fre = weigh(w, r00.f.x, r01.f.x, r10.f.x, r11.f.x) * pw;
+    const double fim = weigh(w, r00.f.y, r01.f.y, r10.f.y, r11.f.y) * pw;
 #pragma unroll
     for (int c = 0; c < nc; ++c) {
       const double et = P.eta[c];
-      dr[c] += (fre * et) * pw;
-      di[c] += (fim * et) * pw;
+      dr[c] = fma(fre, et, dr[c]);
+      di[c] = fma(fim, et, di[c]);
     }
     // Re g and Re I are interpolated once and weighted afterwards (the same
     // linear map as weighting the corners; the mirrored angle's Re g is minus
     // the stored one).
-    const double gq = bilerp(r00.q.x, r01.q.x, r10.q.x, r11.q.x, b.xf, b.yf);
+    const double gq = weigh(w, r00.q.x, r01.q.x, r10.q.x, r11.q.x);
     const double g = mirrored ? -gq : gq;
-    jx += g * psx;
-    jy += g * psy;
-    fe += bilerp(r00.q.y, r01.q.y, r10.q.y, r11.q.y, b.xf, b.yf) * pw;
+    jx = fma(g, psx, jx);
+    jy = fma(g, psy, jy);
+    fe = fma(weigh(w, r00.q.y, r01.q.y, r10.q.y, r11.q.y), pw, fe);
   }
 #pragma unroll
   for (int c = 0; c < nc; ++c) {
@@ -1098,14 +501,13 @@ __global__ void k_halo_ldos(int n_entries, int entry0, int n1, int ne,
 // consecutive angles overlap.
 constexpr int RB_ANGLES = 32;
 template <int EL, int TX, typename LF>
-__global__ void __launch_bounds__(256) k_rotate_back_ldos(int n0, int n1, int ne, int a_begin, int a_end,
+__global__ void __launch_bounds__(256) k_rotate_back_ldos(int n0, int n1, int ne, int first, int a_begin, int a_end,
                                                           const AngleParams *__restrict__ ang,
                                                           const LF *__restrict__ ldf, double *acc) {
   constexpr int SPB = 256 / EL, TY = SPB / TX;
   static_assert(SPB % TX == 0, "the site tile must fill the block");
   __shared__ int s_i00[RB_ANGLES][SPB];
-  __shared__ double2 s_fxy[RB_ANGLES][SPB];
-  __shared__ double s_w[RB_ANGLES][SPB];
+  __shared__ double2 s_w0[RB_ANGLES][SPB], s_w1[RB_ANGLES][SPB];  // corner weights times the angle's weight
   const int t = threadIdx.x;
   const int s = t / EL;
   const int x = blockIdx.x * TX + s % TX, y = blockIdx.y * TY + s / TX;
@@ -1114,7 +516,7 @@ __global__ void __launch_bounds__(256) k_rotate_back_ldos(int n0, int n1, int ne
   const size_t nn0 = (size_t)n0 * n0, nn1 = (size_t)n1 * n1;
   const size_t i = (size_t)y * n0 + x;
   const size_t dx = (size_t)ne, dy = (size_t)n1 * ne;
-  double v = valid ? acc[(size_t)e * nn0 + i] : 0.0;
+  double v = valid && !first ? acc[(size_t)e * nn0 + i] : 0.0;
   for (int ab = a_begin; ab < a_end; ab += RB_ANGLES) {
     const int na = min(RB_ANGLES, a_end - ab);
     __syncthreads();  // every thread has read the previous angles' lookups
@@ -1125,18 +527,21 @@ __global__ void __launch_bounds__(256) k_rotate_back_ldos(int n0, int n1, int ne
       Bilinear b;
       const bool in = kx < n0 && ky < n0 && rotated_lookup(kx, ky, n0, n1, P.cB, P.sB, b);
       s_i00[ka][ks] = in ? b.i00 : 0;
-      s_fxy[ka][ks] = in ? make_double2(b.xf, b.yf) : make_double2(0.0, 0.0);
-      s_w[ka][ks] = in ? P.w : 0.0;
+      const Corners w = corners(b, P.w);
+      s_w0[ka][ks] = in ? make_double2(w.w00, w.w01) : make_double2(0.0, 0.0);
+      s_w1[ka][ks] = in ? make_double2(w.w10, w.w11) : make_double2(0.0, 0.0);
     }
     __syncthreads();
     if (!valid) continue;
     const LF *f = ldf + (size_t)(ab - a_begin) * nn1 * ne + e;
 #pragma unroll 4
     for (int ka = 0; ka < na; ++ka) {
-      const double2 fxy = s_fxy[ka][s];
-      const double w = s_w[ka][s];
+      const double2 w0 = s_w0[ka][s], w1 = s_w1[ka][s];
       const LF *c = f + (size_t)ka * nn1 * ne + (size_t)s_i00[ka][s] * ne;
-      v += bilerp((double)c[0] * w, (double)c[dx] * w, (double)c[dy] * w, (double)c[dy + dx] * w, fxy.x, fxy.y);
+      v = fma(w0.x, (double)c[0], v);
+      v = fma(w0.y, (double)c[dx], v);
+      v = fma(w1.x, (double)c[dy], v);
+      v = fma(w1.y, (double)c[dy + dx], v);
     }
   }
   if (valid) acc[(size_t)e * nn0 + i] = v;
@@ -1201,6 +606,19 @@ __device__ __forceinline__ void block_reduce(double (&q)[N], unsigned long long 
   }
 }
 
+// Whether this block is the last of `blocks` of its launch to get here; what
+// the others wrote before is then visible to it.  The counter wraps to zero, so
+// the next launch finds it cleared.
+__device__ __forceinline__ bool last_block(unsigned *counter, unsigned blocks) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(counter, blocks - 1) == blocks - 1;
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
 // Slot layout of the finalize reduction of nc components.
 //   [0 .. 5]      current-density residual
 //   6             sum of the free-energy kernel inside the grain
@@ -1212,6 +630,103 @@ constexpr int FIN_HEAD = 10, FIN_COMP = 7;
 constexpr unsigned long long FIN_MAX_MASK =
     0x30ull | ((0x30ull | (0x30ull << 7) | (0x30ull << 14) | (0x30ull << 21)) << FIN_HEAD);
 
+// Scalars of one iteration, reduced from the block partials in a fixed order.
+struct Scalars {
+  double fe, fe_area, fe_mag, fe_mag_area;
+  double res_op, res_j, res_fe, res_vp, res_bc, residual;
+  double n_grain;
+  double j_mean[2];
+  double fe_area_prev;
+  int first_j, first_fe;
+  int conv_op, conv_j, conv_fe;
+};
+
+__device__ double residual_from(const double *t, size_t n_elem, int norm) {
+  double numer, denom, eps = 1e-4;
+  if (norm == NORM_L1) {
+    numer = t[2];
+    denom = t[3];
+    eps *= (double)n_elem;
+  } else if (norm == NORM_L2) {
+    numer = sqrt(t[0]);
+    denom = sqrt(t[1]);
+    eps *= (double)n_elem;
+  } else {
+    numer = max_nan(t[4], 2.2250738585072014e-308);
+    denom = max_nan(t[5], 2.2250738585072014e-308);
+  }
+  return numer / fmax(denom, eps);
+}
+
+// Sums (or maxima, for the slots set in max_mask) of the first nq of `stride`
+// slots over the nblocks rows of block partials: warp w reduces slots w,
+// w + nwarps, ... in a fixed order (lane-strided with four loads in flight,
+// then a shuffle tree); results in t[0..nq).
+__device__ void reduce_slots(const double *partial, int nblocks, int stride, int nq, unsigned long long max_mask,
+                             double *t) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int k = w; k < nq; k += nw) {
+    const bool mx = (max_mask >> k) & 1ull;
+    double v = 0.0;
+    for (int b0 = lane; b0 < nblocks; b0 += 128) {
+      double p[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) p[u] = b0 + 32 * u < nblocks ? partial[(size_t)(b0 + 32 * u) * stride + k] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v = mx ? max_nan(v, p[u]) : v + p[u];
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double u = __shfl_xor_sync(0xffffffffu, v, o);
+      v = mx ? max_nan(v, u) : v + u;
+    }
+    if (lane == 0) t[k] = v;
+  }
+  __syncthreads();
+}
+
+struct FinalizeConsts {
+  int nc, norm, n_grain, has_vp;
+  size_t n_elem_field;  // 2 * n0 * n0
+  double temperature, h, lambda, conv, sum_inv;
+  double log_t_tc[MAX_COMP];
+};
+
+// Free energy and the order-parameter / current residuals
+// (ComputeFreeEnergy.h:281-414, ComputeOrderParameter.h:234-254,
+// ComputeCurrent.h:184-211).
+// By the last block of k_finalize.
+__device__ __forceinline__ void finalize_scalars(const FinalizeConsts &C, const double *partial, int nblocks, Scalars *S) {
+  __shared__ double t[NQ];
+  reduce_slots(partial, nblocks, NQ, FIN_HEAD + FIN_COMP * C.nc, FIN_MAX_MASK, t);
+  if (threadIdx.x != 0) return;
+  double rop = 0.0;
+  for (int c = 0; c < C.nc; ++c) rop = max_nan(rop, residual_from(&t[FIN_HEAD + FIN_COMP * c], C.n_elem_field, C.norm));
+  S->res_op = rop;
+  S->conv_op = rop < C.conv;
+  const double rj = residual_from(&t[0], C.n_elem_field, C.norm);
+  S->res_j = S->first_j ? C.conv * 0.1 : rj;
+  S->conv_j = S->res_j < C.conv;
+  S->first_j = 0;
+  double nonmag = C.temperature * t[6];
+  for (int c = 0; c < C.nc; ++c) nonmag += t[FIN_HEAD + FIN_COMP * c + 6] * (C.log_t_tc[c] + C.sum_inv);
+  double mag = 0.0;
+  if (C.has_vp) mag += (0.5 / (C.lambda * C.lambda)) * t[7];
+  const double la = C.h * C.h;
+  const double fe_area = (nonmag + mag) / (double)C.n_grain;
+  const double actual = fabs(S->fe_area_prev - fe_area) / fmax(fabs(S->fe_area_prev), 1e-4);
+  S->res_fe = S->first_fe ? C.conv * 0.1 : actual;
+  S->conv_fe = S->res_fe < C.conv;
+  S->first_fe = 0;
+  S->fe = (nonmag + mag) * la;
+  S->fe_mag = mag * la;
+  S->fe_area = fe_area;
+  S->fe_mag_area = mag / (double)C.n_grain;
+  S->fe_area_prev = fe_area;
+  S->n_grain = (double)C.n_grain;
+  S->j_mean[0] = t[8] / (double)C.n_grain;
+  S->j_mean[1] = t[9] / (double)C.n_grain;
+}
+
 // ComputeOrderParameter / ComputeCurrent / ComputeFreeEnergy
 // ::computePropertyFromGreens, element-wise part and partial sums.  The
 // component count is fixed at compile time (NC = 0: up to MAX_COMP at run
@@ -1222,7 +737,7 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_finalize(
     const double *__restrict__ coupling, const double *__restrict__ acc_d,
     const double *__restrict__ acc_j, const double *__restrict__ acc_fe,
     const double *__restrict__ delta, const double *__restrict__ avec, double *delta_new,
-    double *j_real, double *partial) {
+    double *j_real, double *partial, FinalizeConsts C, Scalars *S, unsigned *counter, int parts) {
   const unsigned nn = (unsigned)n0 * n0;
   constexpr int NCM = NC > 0 ? NC : MAX_COMP;
   const int nc = NC > 0 ? NC : nc_;
@@ -1239,7 +754,12 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_finalize(
       const double lc = coupling[c];
       const size_t kr = (size_t)(2 * c) * nn + i, ki = kr + nn;
       const double o_re = delta[kr], o_im = delta[ki];
-      const double n_re = in ? acc_d[kr] * lc : 0.0, n_im = in ? acc_d[ki] * lc : 0.0;
+      double s_re = acc_d[kr], s_im = acc_d[ki];  // the parts of k_rotate_back in order
+      for (int p = 1; p < parts; ++p) {
+        s_re += acc_d[p * (size_t)(2 * nc) * nn + kr];
+        s_im += acc_d[p * (size_t)(2 * nc) * nn + ki];
+      }
+      const double n_re = in ? s_re * lc : 0.0, n_im = in ? s_im * lc : 0.0;
       delta_new[kr] = n_re;
       delta_new[ki] = n_im;
       res_add(qc, o_re, n_re);
@@ -1249,12 +769,16 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_finalize(
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
       const size_t k = (size_t)d * nn + i;
-      const double nv = in ? acc_j[k] * jfactor : 0.0;
+      double sj = acc_j[k];
+      for (int p = 1; p < parts; ++p) sj += acc_j[p * 2 * (size_t)nn + k];
+      const double nv = in ? sj * jfactor : 0.0;
       res_add(&q[0], j_real[k], nv);
       j_real[k] = nv;
       q[8 + d] += nv;
     }
-    if (in) q[6] += acc_fe[i];
+    double sf = acc_fe[i];
+    for (int p = 1; p < parts; ++p) sf += acc_fe[p * (size_t)nn + i];
+    if (in) q[6] += sf;
     if (has_vp) {
       // curl_kernel, GridFunctions_GPU.h:326-352.
       const int x = (int)(i % (unsigned)n0), y = (int)(i / (unsigned)n0);
@@ -1268,6 +792,7 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_finalize(
     }
   }
   block_reduce(q, FIN_MAX_MASK, partial + (size_t)blockIdx.x * NQ);
+  if (last_block(counter, gridDim.x)) finalize_scalars(C, partial, gridDim.x, S);
 }
 
 __global__ void __launch_bounds__(256) k_ldos_finalize(int n0, int n_fields, const uint8_t *__restrict__ dom,
@@ -1299,51 +824,47 @@ __global__ void __launch_bounds__(256) k_ldos_finalize(int n0, int n_fields, con
   block_reduce(q, 0x30ull, partial + (size_t)blockIdx.x * 6);
 }
 
-// Residual partials of a boundary gather (in-place update) or of any (old, new)
-// pair of arrays.
-__global__ void __launch_bounds__(REDUCE_THREADS) k_residual(size_t n, const double *__restrict__ o,
-                                                             const double *__restrict__ nw,
-                                                             double *partial) {
-  double q[6] = {0, 0, 0, 0, 0, 0};
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    res_add(q, o[i], nw[i]);
-  block_reduce(q, 0x30ull, partial + (size_t)blockIdx.x * 6);
-}
-
 // Specular boundary condition through the precomputed gather table
 // (BoundaryConditionSpecular.h:245-358): in[k] = sum_s w_s out[src_s] / wsum.
 // The old value is read before it is replaced so the residual comes for free.
+// Both coherence functions in one launch (blockIdx.y).
 template <typename R>
-__global__ void __launch_bounds__(REDUCE_THREADS) k_boundary(int n_in, int ne,
-                                                             const int *__restrict__ src,
-                                                             const double *__restrict__ w,
-                                                             const double *__restrict__ wsum,
-                                                             const Cx<R> *__restrict__ out,
-                                                             Cx<R> *in, double *partial) {
+struct BoundarySide {
+  int n_in;
+  const int *src;
+  const double *w, *wsum;
+  const Cx<R> *out;
+  Cx<R> *in;
+  double *partial;
+};
+template <typename R>
+__global__ void __launch_bounds__(REDUCE_THREADS) k_boundary(int ne, BoundarySide<R> g, BoundarySide<R> gt) {
+  const BoundarySide<R> &B = blockIdx.y ? gt : g;
   double q[6] = {0, 0, 0, 0, 0, 0};
-  const size_t total = (size_t)n_in * ne;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(t / ne), e = (int)(t % ne);
+  const unsigned total = (unsigned)B.n_in * ne;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const unsigned k = t / (unsigned)ne, e = t - k * ne;
+    const int4 src = ((const int4 *)B.src)[k];
+    const double2 w01 = ((const double2 *)B.w)[2 * (size_t)k], w23 = ((const double2 *)B.w)[2 * (size_t)k + 1];
+    const int si[4] = {src.x, src.y, src.z, src.w};
+    const double ws[4] = {w01.x, w01.y, w23.x, w23.y};
     double re = 0.0, im = 0.0;
+#pragma unroll
     for (int s = 0; s < 4; ++s) {
-      const int sidx = src[4 * k + s];
-      if (sidx < 0) continue;
-      const Cx<R> v = out[(size_t)sidx * ne + e];
-      const double ws = w[4 * k + s];
-      re = __dadd_rn(re, __dmul_rn((double)v.re, ws));
-      im = __dadd_rn(im, __dmul_rn((double)v.im, ws));
+      if (si[s] < 0) continue;
+      const Cx<R> v = B.out[(size_t)si[s] * ne + e];
+      re = __dadd_rn(re, __dmul_rn((double)v.re, ws[s]));
+      im = __dadd_rn(im, __dmul_rn((double)v.im, ws[s]));
     }
-    const double W = wsum[k];
+    const double W = B.wsum[k];
     Cx<R> nv{R(0), R(0)};
     if (W > 0.0) nv = Cx<R>{(R)__ddiv_rn(re, W), (R)__ddiv_rn(im, W)};
-    const Cx<R> ov = in[t];
+    const Cx<R> ov = B.in[t];
     res_add(q, (double)ov.re, (double)nv.re);
     res_add(q, (double)ov.im, (double)nv.im);
-    in[t] = nv;
+    B.in[t] = nv;
   }
-  block_reduce(q, 0x30ull, partial + (size_t)blockIdx.x * 6);
+  block_reduce(q, 0x30ull, B.partial + (size_t)blockIdx.x * 6);
 }
 
 // Initial boundary values: homogeneous solutions at every exit node
@@ -1364,16 +885,6 @@ __global__ void k_boundary_initial(int n_out, int ne, int is_g, const int *__res
   bout[t] = is_g ? g : gt;
 }
 
-// Subtracts the mean of each current component (ComputeVectorPotential.h:575-591).
-__global__ void k_subtract_mean(int n0, const double *__restrict__ j, const double *__restrict__ scal,
-                                int mean_slot, double *s) {
-  const size_t nn = (size_t)n0 * n0;
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= 2 * nn) return;
-  const int d = (int)(i / nn);
-  s[i] = j[i] - scal[mean_slot + d];
-}
-
 // ------------------------------------------------------- Poisson by FFT --
 // The separable solve of ComputeVectorPotential::solve
 // (ComputeVectorPotential.h:594-745) is A[r][c] = sum_{u,v} K(u, v) s[r+u][c+v]
@@ -1384,6 +895,12 @@ __global__ void k_subtract_mean(int n0, const double *__restrict__ j, const doub
 // both current components travel in one complex array, s_x + i s_y, the
 // kernel's spectrum is computed once at set-up.  O(P^2 log P) instead of
 // O(K N0^3); the results agree with the direct filter sums to rounding.
+// Three launches per solve: the rows of the current that are not zero
+// (k_pois_rows), every column forward, times the spectrum and back without
+// leaving shared memory (k_pois_cols), and the rows that are read
+// (k_pois_back, with the residual of the vector potential).  The work arrays
+// stay in L2; what bounds a solve is the latency of the launches and of the
+// transforms' stages, so there are as few of both as the transform allows.
 
 // P-point FFT of every row in shared memory, P = 2^a 3^b 5^c <= 4096: the
 // Stockham autosort formulation (Govindaraju et al., "High performance
@@ -1451,182 +968,131 @@ __device__ __forceinline__ void dft_small(double2 *v, double s) {
   }
 }
 
-// One Stockham stage of radix R (registers only: R is a template constant).
+// One Stockham stage of radix R (registers only: R is a template constant) of
+// `cols` transforms of P points each, one after the other in a and b.
 template <int R>
-__device__ __forceinline__ void fft_stage(const double2 *a, double2 *b, int P, int ns,
+__device__ __forceinline__ void fft_stage(const double2 *a, double2 *b, int P, int cols, int ns,
                                           const double2 *__restrict__ tw, int inverse) {
   const int m = P / R, step = P / (ns * R);
   const double s = inverse ? 1.0 : -1.0;
-  for (int j = threadIdx.x; j < m; j += blockDim.x) {
-    const int k = j % ns;
+  const bool pow2 = (ns & (ns - 1)) == 0;  // all but the stages after a radix 3 or 5
+  const int sh = 31 - __clz(ns);
+  for (int t = threadIdx.x; t < cols * m; t += blockDim.x) {
+    const int col = cols == 1 ? 0 : t / m, j = t - col * m;
+    const int jd = pow2 ? j >> sh : j / ns, k = j - jd * ns;
+    const double2 *x = a + col * P;
     double2 v[R];
-    v[0] = a[j];
+    v[0] = x[j];
 #pragma unroll
     for (int r = 1; r < R; ++r) {
       double2 w = tw[r * k * step];
       if (inverse) w.y = -w.y;
-      v[r] = cmul_d2(a[j + r * m], w);
+      v[r] = cmul_d2(x[j + r * m], w);
     }
     dft_small<R>(v, s);
-    const int d = (j / ns) * ns * R + k;
+    double2 *y = b + col * P + jd * ns * R + k;
 #pragma unroll
-    for (int r = 0; r < R; ++r) b[d + r * ns] = v[r];
+    for (int r = 0; r < R; ++r) y[r * ns] = v[r];
   }
 }
 
-__global__ void __launch_bounds__(512) k_fft_rows(FftPlan plan, int P, const double2 *__restrict__ tw,
-                                                  double2 *data, int inverse) {
-  extern __shared__ double2 sm[];
-  double2 *a = sm, *b = sm + P;
-  double2 *row = data + (size_t)blockIdx.x * P;
-  for (int i = threadIdx.x; i < P; i += blockDim.x) a[i] = row[i];
-  __syncthreads();
+// The P-point transforms of `cols` arrays in shared memory, ping-ponging
+// between a and b (the data is in a on return).  The caller has filled a and
+// synchronised.
+__device__ __forceinline__ void fft_shared(const FftPlan &plan, int P, int cols, const double2 *__restrict__ tw,
+                                           double2 *&a, double2 *&b, int inverse) {
   int ns = 1;
   for (int st = 0; st < plan.n_stages; ++st) {
     const int R = plan.radix[st];
-    if (R == 4) fft_stage<4>(a, b, P, ns, tw, inverse);
-    else if (R == 2) fft_stage<2>(a, b, P, ns, tw, inverse);
-    else if (R == 3) fft_stage<3>(a, b, P, ns, tw, inverse);
-    else fft_stage<5>(a, b, P, ns, tw, inverse);
+    if (R == 4) fft_stage<4>(a, b, P, cols, ns, tw, inverse);
+    else if (R == 2) fft_stage<2>(a, b, P, cols, ns, tw, inverse);
+    else if (R == 3) fft_stage<3>(a, b, P, cols, ns, tw, inverse);
+    else fft_stage<5>(a, b, P, cols, ns, tw, inverse);
     __syncthreads();
     double2 *t = a;
     a = b;
     b = t;
     ns *= R;
   }
+}
+
+// Row r of the padded current s_x + i s_y, s = j - mean inside the n x n
+// lattice (ComputeVectorPotential.h:575-591; mean null: j is mean-free),
+// transformed into z[r].  j null: the row of z itself, in place.
+__global__ void __launch_bounds__(512) k_pois_rows(FftPlan plan, int n, int P, const double2 *__restrict__ tw,
+                                                   const double *__restrict__ j, const double *__restrict__ mean,
+                                                   double2 *z) {
+  extern __shared__ double2 fft_sm[];
+  double2 *a = fft_sm, *b = fft_sm + P;
+  double2 *row = z + (size_t)blockIdx.x * P;
+  if (j) {
+    const size_t nn = (size_t)n * n, r = (size_t)blockIdx.x * n;
+    const double mx = mean ? mean[0] : 0.0, my = mean ? mean[1] : 0.0;
+    for (int i = threadIdx.x; i < P; i += blockDim.x)
+      a[i] = i < n ? make_double2(j[r + i] - mx, j[nn + r + i] - my) : make_double2(0.0, 0.0);
+  } else {
+    for (int i = threadIdx.x; i < P; i += blockDim.x) a[i] = row[i];
+  }
+  __syncthreads();
+  fft_shared(plan, P, 1, tw, a, b, 0);
   for (int i = threadIdx.x; i < P; i += blockDim.x) row[i] = a[i];
 }
 
-// out = transpose(in), P x P complex, 32 x 32 tiles.
-__global__ void __launch_bounds__(256) k_fft_transpose(int P, const double2 *__restrict__ in, double2 *out) {
-  __shared__ double2 tile[32][33];
-  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
-  for (int r = threadIdx.y; r < 32; r += 8) tile[r][threadIdx.x] = in[(size_t)(y0 + r) * P + x0 + threadIdx.x];
-  __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += 8) out[(size_t)(x0 + r) * P + y0 + threadIdx.x] = tile[threadIdx.x][r];
-}
-
-// z[r][c] = s_x[r][c] + i s_y[r][c] inside the n x n lattice, 0 in the padding.
-__global__ void k_fft_pack(int n, int P, const double *__restrict__ s, double2 *z) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= (size_t)P * P) return;
-  const int r = (int)(i / P), c = (int)(i % P);
-  const size_t nn = (size_t)n * n;
-  z[i] = (r < n && c < n) ? make_double2(s[(size_t)r * n + c], s[nn + (size_t)r * n + c]) : make_double2(0.0, 0.0);
-}
-
-__global__ void k_fft_mul(size_t count, const double2 *__restrict__ k, double2 *z) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const double2 a = z[i], b = k[i];
-  z[i] = make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
-// a_x = Re z / P^2, a_y = Im z / P^2 on the n x n lattice.
-__global__ void k_fft_unpack(int n, int P, double inv, const double2 *__restrict__ z, double *a) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  const size_t nn = (size_t)n * n;
-  if (i >= nn) return;
-  const int r = (int)(i / n), c = (int)(i % n);
-  const double2 v = z[(size_t)r * P + c];
-  a[i] = v.x * inv;
-  a[nn + i] = v.y * inv;
-}
-
-// Scalars of one iteration, reduced from the block partials in a fixed order.
-struct Scalars {
-  double fe, fe_area, fe_mag, fe_mag_area;
-  double res_op, res_j, res_fe, res_vp, res_bc, residual;
-  double n_grain;
-  double j_mean[2];
-  double fe_area_prev;
-  int first_j, first_fe;
-  int conv_op, conv_j, conv_fe;
-};
-
-__device__ double residual_from(const double *t, size_t n_elem, int norm) {
-  double numer, denom, eps = 1e-4;
-  if (norm == NORM_L1) {
-    numer = t[2];
-    denom = t[3];
-    eps *= (double)n_elem;
-  } else if (norm == NORM_L2) {
-    numer = sqrt(t[0]);
-    denom = sqrt(t[1]);
-    eps *= (double)n_elem;
-  } else {
-    numer = max_nan(t[4], 2.2250738585072014e-308);
-    denom = max_nan(t[5], 2.2250738585072014e-308);
-  }
-  return numer / fmax(denom, eps);
-}
-
-// Sums (or maxima, for the slots set in max_mask) of the first nq of `stride`
-// slots over the nblocks rows of block partials: warp w reduces slots w,
-// w + nwarps, ... in a fixed order (lane-strided with four loads in flight,
-// then a shuffle tree); results in t[0..nq).
-__device__ void reduce_slots(const double *partial, int nblocks, int stride, int nq, unsigned long long max_mask,
-                             double *t) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int k = w; k < nq; k += nw) {
-    const bool mx = (max_mask >> k) & 1ull;
-    double v = 0.0;
-    for (int b0 = lane; b0 < nblocks; b0 += 128) {
-      double p[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) p[u] = b0 + 32 * u < nblocks ? partial[(size_t)(b0 + 32 * u) * stride + k] : 0.0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) v = mx ? max_nan(v, p[u]) : v + p[u];
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double u = __shfl_xor_sync(0xffffffffu, v, o);
-      v = mx ? max_nan(v, u) : v + u;
-    }
-    if (lane == 0) t[k] = v;
+// `cols` neighbouring columns of z, of which the first rows_in rows are not
+// zero: transformed, times their spectrum kf[column][row], transformed back,
+// and the first rows_in rows written in place.  out not null (set-up):
+// transformed only, written to out[column][row].
+__global__ void __launch_bounds__(512) k_pois_cols(FftPlan plan, int P, int rows_in, int cols,
+                                                   const double2 *__restrict__ tw, const double2 *__restrict__ kf,
+                                                   double2 *z, double2 *out) {
+  extern __shared__ double2 fft_sm[];
+  double2 *a = fft_sm, *b = fft_sm + cols * P;
+  const int c0 = blockIdx.x * cols;
+  for (int t = threadIdx.x; t < cols * P; t += blockDim.x) {
+    const int r = t / cols, c = t - r * cols;
+    a[c * P + r] = r < rows_in ? z[(size_t)r * P + c0 + c] : make_double2(0.0, 0.0);
   }
   __syncthreads();
+  fft_shared(plan, P, cols, tw, a, b, 0);
+  if (out) {
+    for (int t = threadIdx.x; t < cols * P; t += blockDim.x) out[(size_t)c0 * P + t] = a[t];
+    return;
+  }
+  for (int t = threadIdx.x; t < cols * P; t += blockDim.x) a[t] = cmul_d2(a[t], kf[(size_t)c0 * P + t]);
+  __syncthreads();
+  fft_shared(plan, P, cols, tw, a, b, 1);
+  for (int t = threadIdx.x; t < cols * rows_in; t += blockDim.x) {
+    const int r = t / cols, c = t - r * cols;
+    z[(size_t)r * P + c0 + c] = a[c * P + r];
+  }
 }
 
-struct FinalizeConsts {
-  int nc, norm, n_grain, has_vp;
-  size_t n_elem_field;  // 2 * n0 * n0
-  double temperature, h, lambda, conv, sum_inv;
-  double log_t_tc[MAX_COMP];
-};
-
-// Free energy and the order-parameter / current residuals
-// (ComputeFreeEnergy.h:281-414, ComputeOrderParameter.h:234-254,
-// ComputeCurrent.h:184-211).
-__global__ void k_scalars_a(FinalizeConsts C, const double *partial, int nblocks, Scalars *S) {
-  __shared__ double t[NQ];
-  reduce_slots(partial, nblocks, NQ, FIN_HEAD + FIN_COMP * C.nc, FIN_MAX_MASK, t);
-  if (threadIdx.x != 0) return;
-  double rop = 0.0;
-  for (int c = 0; c < C.nc; ++c) rop = max_nan(rop, residual_from(&t[FIN_HEAD + FIN_COMP * c], C.n_elem_field, C.norm));
-  S->res_op = rop;
-  S->conv_op = rop < C.conv;
-  const double rj = residual_from(&t[0], C.n_elem_field, C.norm);
-  S->res_j = S->first_j ? C.conv * 0.1 : rj;
-  S->conv_j = S->res_j < C.conv;
-  S->first_j = 0;
-  double nonmag = C.temperature * t[6];
-  for (int c = 0; c < C.nc; ++c) nonmag += t[FIN_HEAD + FIN_COMP * c + 6] * (C.log_t_tc[c] + C.sum_inv);
-  double mag = 0.0;
-  if (C.has_vp) mag += (0.5 / (C.lambda * C.lambda)) * t[7];
-  const double la = C.h * C.h;
-  const double fe_area = (nonmag + mag) / (double)C.n_grain;
-  const double actual = fabs(S->fe_area_prev - fe_area) / fmax(fabs(S->fe_area_prev), 1e-4);
-  S->res_fe = S->first_fe ? C.conv * 0.1 : actual;
-  S->conv_fe = S->res_fe < C.conv;
-  S->first_fe = 0;
-  S->fe = (nonmag + mag) * la;
-  S->fe_mag = mag * la;
-  S->fe_area = fe_area;
-  S->fe_mag_area = mag / (double)C.n_grain;
-  S->fe_area_prev = fe_area;
-  S->n_grain = (double)C.n_grain;
-  S->j_mean[0] = t[8] / (double)C.n_grain;
-  S->j_mean[1] = t[9] / (double)C.n_grain;
+// Row r of the result: a_x = Re z / P^2, a_y = Im z / P^2 on the n x n
+// lattice, and (old not null) the row's residual sums against the old vector
+// potential.
+__global__ void __launch_bounds__(REDUCE_THREADS) k_pois_back(FftPlan plan, int n, int P, double inv,
+                                                              const double2 *__restrict__ tw,
+                                                              const double2 *__restrict__ z,
+                                                              const double *__restrict__ old, double *av,
+                                                              double *partial) {
+  extern __shared__ double2 fft_sm[];
+  double2 *a = fft_sm, *b = fft_sm + P;
+  const double2 *row = z + (size_t)blockIdx.x * P;
+  for (int i = threadIdx.x; i < P; i += blockDim.x) a[i] = row[i];
+  __syncthreads();
+  fft_shared(plan, P, 1, tw, a, b, 1);
+  const size_t nn = (size_t)n * n, r = (size_t)blockIdx.x * n;
+  double q[6] = {0, 0, 0, 0, 0, 0};
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double x = a[i].x * inv, y = a[i].y * inv;
+    av[r + i] = x;
+    av[nn + r + i] = y;
+    if (old) {
+      res_add(q, old[r + i], x);
+      res_add(q, old[nn + r + i], y);
+    }
+  }
+  if (old) block_reduce(q, 0x30ull, partial + (size_t)blockIdx.x * 6);
 }
 
 // Boundary and vector-potential residuals, total residual (Context.h:462-483).
@@ -1653,26 +1119,6 @@ __global__ void k_scalars_b(int norm, size_t n_elem_g, size_t n_elem_gt, size_t 
 }
 
 // ---------------------------------------------------------- accelerators --
-// Per-field sums for CongAcc (CongAcc.h:371-385) and Barzilai-Borwein
-// (BarzilaiBorwein.h:214-229): slots [3f] sum d^2, [3f+1] sum m^2, [3f+2] sum d m,
-// where d = g - x and m is the running mean (CongAcc) or the previous d (BB).
-__global__ void __launch_bounds__(REDUCE_THREADS) k_acc_sums(int nf, size_t nn, const double *__restrict__ x,
-                                                             const double *__restrict__ gx,
-                                                             const double *__restrict__ m,
-                                                             double *partial) {
-  const int f = blockIdx.y;
-  double q[3] = {0, 0, 0};
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nn;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const size_t k = (size_t)f * nn + i;
-    const double d = gx[k] - x[k], mv = m[k];
-    q[0] += d * d;
-    q[1] += mv * mv;
-    q[2] += d * mv;
-  }
-  block_reduce(q, 0, partial + ((size_t)f * gridDim.x + blockIdx.x) * 3);
-}
-
 constexpr int AND_MAX_RANK = 16;
 struct AccState {
   double step[16];
@@ -1688,6 +1134,104 @@ struct AccState {
   double and_dot[AND_MAX_RANK][AND_MAX_RANK];
   double and_w[AND_MAX_RANK];
 };
+
+// CongAcc::computeInertia (CongAcc.h:300-356).
+__device__ double congacc_inertia(double dn, double mn, double dot, double mincos) {
+  double ea = dot / (dn * mn) - mincos, xa = 1.0;
+  double eb = 1.0 - mincos, xb = 0.0;
+  double x = 0.5 * (xa + xb);
+  auto sgn = [](double v) { return (0.0 < v) - (v < 0.0); };
+  for (int it = 0; it < 200; ++it) {
+    const double y = 1.0 - x;
+    const double numer = x * dot + y * dn * dn;
+    const double denom = dn * sqrt(x * x * mn * mn + 2.0 * x * y * dot + y * y * dn * dn);
+    const double err = numer / denom - mincos;
+    const bool conv = fabs(err) < 0.01;
+    if (sgn(err) == sgn(ea)) {
+      ea = err;
+      xa = x;
+    } else {
+      eb = err;
+      xb = x;
+    }
+    if (sgn(ea) == sgn(eb)) break;
+    x = 0.5 * (xa + xb);
+    if (conv) break;
+  }
+  return x;
+}
+
+struct AccConsts {
+  int kind, nf;
+  double step_size, factor, mincos, smax, smin, drag;
+};
+
+// Scalar part of CongAcc::computeInternal (CongAcc.h:371-408) and
+// BarzilaiBorwein::computeInternal (BarzilaiBorwein.h:211-232), by the last
+// block of k_acc_sums: one thread per field.
+__device__ __forceinline__ void acc_scalars(const AccConsts &C, const double *partial, int nblocks, AccState *st) {
+  __shared__ double t[48];
+  const int nf = C.nf;
+  const bool init = !st->initialized;  // read before the barrier in reduce_slots
+  reduce_slots(partial, nblocks, 3 * nf, 3 * nf, 0ull, t);
+  const int f = threadIdx.x;
+  if (f >= nf) return;
+  if (C.kind == ACC_CONGACC) {
+    double step = init ? C.step_size : st->step[f];
+    if (init) st->inertia[f] = 0.0;
+    const double d = sqrt(t[3 * f]), m = sqrt(t[3 * f + 1]);
+    const double den = d * m;
+    if (den > 0.0) {
+      const double dot = t[3 * f + 2];
+      const double cs = dot / den;
+      step *= pow(C.factor, cs);
+      if (cs < C.mincos) st->inertia[f] = congacc_inertia(d, m, dot, C.mincos);
+    }
+    st->step[f] = fmin(fmax(step, C.smin), C.smax);
+  } else if (C.kind == ACC_BB && f == 0) {
+    if (init) {
+      st->bb_step = C.step_size;
+      st->bb_iter = 0;
+    }
+    if (st->bb_iter > 0) {
+      // t: d^2 (= |d|^2), m^2 (= |dprev|^2), d.m (= d . dprev)
+      double dd = 0.0, pp = 0.0, dp = 0.0;
+      for (int k = 0; k < nf; ++k) {
+        dd += t[3 * k];
+        pp += t[3 * k + 1];
+        dp += t[3 * k + 2];
+      }
+      const double dot = fabs(dp - pp);             // |dprev . (d - dprev)|
+      const double ss = dd - 2.0 * dp + pp;         // |d - dprev|^2
+      const double scale = (st->bb_iter % 2 == 0) ? dot / ss : pp / dot;
+      st->bb_step *= scale;
+    }
+    st->bb_step = fmin(fmax(st->bb_step, C.smin), C.smax);
+    st->bb_iter++;
+  }
+  if (f == 0) st->initialized = 1;
+}
+
+// Per-field sums for CongAcc (CongAcc.h:371-385) and Barzilai-Borwein
+// (BarzilaiBorwein.h:214-229): slots [3f] sum d^2, [3f+1] sum m^2, [3f+2] sum d m,
+// where d = g - x and m is the running mean (CongAcc) or the previous d (BB).
+__global__ void __launch_bounds__(REDUCE_THREADS) k_acc_sums(AccConsts C, size_t nn, const double *__restrict__ x,
+                                                             const double *__restrict__ gx,
+                                                             const double *__restrict__ m, double *partial,
+                                                             AccState *st, unsigned *counter) {
+  const int f = blockIdx.y;
+  double q[3] = {0, 0, 0};
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nn;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const size_t k = (size_t)f * nn + i;
+    const double d = gx[k] - x[k], mv = m[k];
+    q[0] += d * d;
+    q[1] += mv * mv;
+    q[2] += d * mv;
+  }
+  block_reduce(q, 0, partial + ((size_t)blockIdx.x * C.nf + f) * 3);
+  if (last_block(counter, gridDim.x * gridDim.y)) acc_scalars(C, partial, gridDim.x, st);
+}
 
 // Anderson::set (Anderson.h:267-289): the iterate and its residual
 // d = g(x) - x go to slot iter mod rank (the oldest once all are used), and
@@ -1783,107 +1327,54 @@ __global__ void k_and_update(size_t tot, int rank, double step, const double *__
   x[k] = v;
 }
 
-// CongAcc::computeInertia (CongAcc.h:300-356).
-__device__ double congacc_inertia(double dn, double mn, double dot, double mincos) {
-  double ea = dot / (dn * mn) - mincos, xa = 1.0;
-  double eb = 1.0 - mincos, xb = 0.0;
-  double x = 0.5 * (xa + xb);
-  auto sgn = [](double v) { return (0.0 < v) - (v < 0.0); };
-  for (int it = 0; it < 200; ++it) {
-    const double y = 1.0 - x;
-    const double numer = x * dot + y * dn * dn;
-    const double denom = dn * sqrt(x * x * mn * mn + 2.0 * x * y * dot + y * y * dn * dn);
-    const double err = numer / denom - mincos;
-    const bool conv = fabs(err) < 0.01;
-    if (sgn(err) == sgn(ea)) {
-      ea = err;
-      xa = x;
-    } else {
-      eb = err;
-      xb = x;
-    }
-    if (sgn(ea) == sgn(eb)) break;
-    x = 0.5 * (xa + xb);
-    if (conv) break;
-  }
-  return x;
-}
-
-struct AccConsts {
-  int kind, nf;
-  double step_size, factor, mincos, smax, smin, drag;
-};
-
-// Scalar part of CongAcc::computeInternal (CongAcc.h:371-408) and
-// BarzilaiBorwein::computeInternal (BarzilaiBorwein.h:211-232).
-__global__ void k_acc_scalars(AccConsts C, const double *partial, int nblocks, AccState *st) {
-  __shared__ double t[48];
-  const int nf = C.nf;
-  for (int f = 0; f < nf; ++f) reduce_slots(partial + (size_t)f * nblocks * 3, nblocks, 3, 3, 0ull, &t[3 * f]);
-  if (threadIdx.x != 0) return;
-  if (!st->initialized) {
-    for (int f = 0; f < nf; ++f) {
-      st->step[f] = C.step_size;
-      st->inertia[f] = 0.0;
-    }
-    st->bb_step = C.step_size;
-    st->bb_iter = 0;
-    st->initialized = 1;
-  }
-  if (C.kind == ACC_CONGACC) {
-    for (int f = 0; f < nf; ++f) {
-      const double d = sqrt(t[3 * f]), m = sqrt(t[3 * f + 1]);
-      const double den = d * m;
-      if (den > 0.0) {
-        const double dot = t[3 * f + 2];
-        const double cs = dot / den;
-        st->step[f] *= pow(C.factor, cs);
-        if (cs < C.mincos) st->inertia[f] = congacc_inertia(d, m, dot, C.mincos);
-      }
-      st->step[f] = fmin(fmax(st->step[f], C.smin), C.smax);
-    }
-  } else if (C.kind == ACC_BB) {
-    if (st->bb_iter > 0) {
-      // t: d^2 (= |d|^2), m^2 (= |dprev|^2), d.m (= d . dprev)
-      double dd = 0.0, pp = 0.0, dp = 0.0;
-      for (int f = 0; f < nf; ++f) {
-        dd += t[3 * f];
-        pp += t[3 * f + 1];
-        dp += t[3 * f + 2];
-      }
-      const double dot = fabs(dp - pp);             // |dprev . (d - dprev)|
-      const double ss = dd - 2.0 * dp + pp;         // |d - dprev|^2
-      const double scale = (st->bb_iter % 2 == 0) ? dot / ss : pp / dot;
-      st->bb_step *= scale;
-    }
-    st->bb_step = fmin(fmax(st->bb_step, C.smin), C.smax);
-    st->bb_iter++;
-  }
-}
-
-// Element-wise accelerator update: CongAcc (CongAcc.h:271-297), Picard
+// One site's new value of field f: CongAcc (CongAcc.h:271-297), Picard
 // (Picard.h:133-138), Polyak (Polyak.h:214-239), Barzilai-Borwein
 // (BarzilaiBorwein.h:234-237).
-__global__ void k_acc_update(AccConsts C, size_t nn, const double *__restrict__ gx, double *x,
-                             double *m, const AccState *st) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= (size_t)C.nf * nn) return;
-  const int f = (int)(i / nn);
-  const double d = gx[i] - x[i];
+__device__ __forceinline__ double acc_advance(const AccConsts &C, const AccState *st, int f, double x, double gx,
+                                              double *m) {
+  const double d = gx - x;
   if (C.kind == ACC_CONGACC) {
     const double in = st->inertia[f];
-    const double mean = m[i] * in + d * (1.0 - in);
-    m[i] = mean;
-    x[i] += st->step[f] * mean;
-  } else if (C.kind == ACC_PICARD) {
-    x[i] += d * C.step_size;
-  } else if (C.kind == ACC_POLYAK) {
-    const double v = m[i] * (1.0 - C.drag) + d * C.step_size;
-    m[i] = v;
-    x[i] += v;
-  } else {  // Barzilai-Borwein: m holds the previous difference
-    m[i] = d;
-    x[i] += d * st->bb_step;
+    const double mean = *m * in + d * (1.0 - in);
+    *m = mean;
+    return x + st->step[f] * mean;
+  }
+  if (C.kind == ACC_PICARD) return x + d * C.step_size;
+  if (C.kind == ACC_POLYAK) {
+    const double v = *m * (1.0 - C.drag) + d * C.step_size;
+    *m = v;
+    return x + v;
+  }
+  *m = d;  // Barzilai-Borwein: m holds the previous difference
+  return x + d * st->bb_step;
+}
+
+// The reference-grid fields the frame lookups gather, one record per site:
+// rf[site * (nc + 1) + c] = (Re, Im) of order-parameter component c and
+// rf[site * (nc + 1) + nc] = (A_x, A_y) of the induced vector potential, so
+// that a bilinear corner costs one 16-byte load per field pair instead of two
+// 8-byte loads from separate planes; rf32 the same records in FP32 for the
+// mixed-precision lookups (the FP32 sweep rounds the frame fields to FP32
+// anyway).  With nf > 0 the first nf of the 2 nc + 2 fields of the state first
+// take the accelerator's step.
+__global__ void __launch_bounds__(256) k_advance_pack(AccConsts C, int nf, int nc, int nn,
+                                                      const double *__restrict__ gx, double *x, double *m,
+                                                      const AccState *st, double2 *__restrict__ rf,
+                                                      float2 *__restrict__ rf32) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nn) return;
+  const size_t r = (size_t)i * (nc + 1);
+  for (int c = 0; c <= nc; ++c) {
+    const size_t k = (size_t)(2 * c) * nn + i, k2 = k + nn;
+    double v0 = x[k], v1 = x[k2];
+    if (2 * c < nf) {
+      v0 = acc_advance(C, st, 2 * c, v0, gx[k], m + k);
+      v1 = acc_advance(C, st, 2 * c + 1, v1, gx[k2], m + k2);
+      x[k] = v0;
+      x[k2] = v1;
+    }
+    rf[r + c] = make_double2(v0, v1);
+    if (rf32) rf32[r + c] = make_float2((float)v0, (float)v1);
   }
 }
 
@@ -1985,7 +1476,8 @@ struct sc_ctx {
   DevArray<int> halo_site, halo_off, halo_src, halo_angle;
   DevArray<int> rext_site, rext_off, rext_src;
   DevArray<int4> items;
-  DevArray<double> e_re, e_im, res, coupling;
+  DevArray<double> e_re, e_im, res, res2, coupling;
+  float e_re_max = 0.0f;  // over all LDOS energies
   DevArray<double> filters;
   DevArray<int> filter_pos;
   DevArray<int> onode_a_g, onode_x_g, onode_y_g, onode_a_gt, onode_x_gt, onode_y_gt;
@@ -1995,28 +1487,28 @@ struct sc_ctx {
   // that the sweep runs in passes of ENERGY_PASS energies that add into the
   // frame sums (low temperatures: T = 0.001 at cutoff 32 takes 281 energies).
   int e_pass = 1;
-  bool emax2 = false;  // two-energies-per-thread sweep variant (tuning)
   int pair = 0;  // > 0: mixed mode sweeps angles [0, n/2) and mirrors them onto [n/2, n)
 
   // state: x = [delta | avec], g = [delta_new | a_new]
   DevArray<double> xstate, gstate, rfields, j_real;
   DevArray<double> rfields32;  // FP32 records (mixed precision), allocated as doubles
   std::vector<int4> h_items;  // trajectory columns (angle, x, first row, last row), host copy
-  DevArray<double> acc_d, acc_j, acc_fe;
+  DevArray<double> acc_d, acc_j, acc_fe;  // [rb_parts] copies
+  int rb_parts = 1;
   DevArray<double> bnd;      // boundary storage (4 arrays), R-typed, viewed through pointers
   size_t bnd_off[4] = {0, 0, 0, 0};
   DevArray<double> scratch, scratch2, frames;
   DevArray<double> partial_fin, partial_bg, partial_bgt, partial_vp, partial_acc;
-  DevArray<double> pois_s;
   // Poisson transform: side P = 32 * 2^a 3^b 5^c (radix plan), twiddles,
   // kernel spectrum, work arrays (complex).
   int fft_p = 0;
   FftPlan fft_plan{};
-  DevArray<double> fft_tw, fft_kf, fft_z, fft_t;
+  DevArray<double> fft_tw, fft_kf, fft_z;
   DevArray<double> acc_m;
   DevArray<double> and_x, and_d;  // Anderson history [rank][fields][N0*N0] (iterates, residuals)
   DevArray<AccState> acc_state;
   DevArray<Scalars> scalars;
+  DevArray<unsigned> counters;  // of finished blocks: k_finalize, k_acc_sums
   DevArray<double> tmp_io;
   int nb_fin = 0, nb_bnd = 0, nb_vp = 0, nb_acc = 0;
 
@@ -2142,6 +1634,8 @@ SweepArgs<R> sweep_args(sc_ctx *c, const Chunk *ch, int burn_in) {
   A.e_re = c->e_re.p;
   A.e_im = c->e_im.p;
   A.res = c->res.p;
+  A.res2 = c->res2.p;
+  A.e_re_max = c->e_re_max;
   A.ldf = (typename LdosOf<R>::type *)c->ldf.p;
   A.scratch = (Cx<R> *)c->w_scratch;
   A.scratch2 = (R *)c->w_scratch2;
@@ -2164,106 +1658,49 @@ void launch_frame_fields(sc_ctx *c, const Chunk &ch, const SweepArgs<R> &A) {
   check_launch(c);
 }
 
+// One launch of the sweep, with the kernel of the context's mapping: EMAX
+// energies per thread on G = 2^lg threads per column and function (plan_mapping).
+template <typename R, int EMAX, int MINB, bool KEL, bool PK>
+void launch_sweep_lg(sc_ctx *c, const SweepArgs<R> &A, unsigned blocks) {
+  constexpr int smem = SweepRing<R, EMAX, MINB, PK>::BYTES;
+  auto go = [&](auto kern) {
+    if (smem > 32 * 1024) CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kern<<<blocks, 128, smem, c->stream>>>(A);
+  };
+  switch (c->log_groups) {
+    case 0: go(k_sweep<R, EMAX, MINB, KEL, 0, PK>); break;
+    case 1: go(k_sweep<R, EMAX, MINB, KEL, 1, PK>); break;
+    case 2: go(k_sweep<R, EMAX, MINB, KEL, 2, PK>); break;
+    case 3: go(k_sweep<R, EMAX, MINB, KEL, 3, PK>); break;
+    default: go(k_sweep<R, EMAX, MINB, KEL, 4, PK>); break;
+  }
+}
+template <typename R, bool KEL>
+void launch_sweep_kel(sc_ctx *c, const SweepArgs<R> &A, unsigned blocks) {
+  if constexpr (sizeof(R) == 8) {
+    if (c->ept == 1) launch_sweep_lg<R, 1, 5, KEL, false>(c, A, blocks);
+    else if (c->ept == 2) launch_sweep_lg<R, 2, 3, KEL, false>(c, A, blocks);
+    else if (c->ept == 4) launch_sweep_lg<R, 4, 3, KEL, false>(c, A, blocks);
+    else launch_sweep_lg<R, 7, 2, KEL, false>(c, A, blocks);
+  } else {
+    if (c->ept == 1) launch_sweep_lg<R, 1, 4, KEL, false>(c, A, blocks);
+    else if (c->ept == 2) launch_sweep_lg<R, 2, 4, KEL, true>(c, A, blocks);
+    else if (c->ept == 4) launch_sweep_lg<R, 4, 3, KEL, true>(c, A, blocks);
+    else launch_sweep_lg<R, 8, 3, KEL, true>(c, A, blocks);
+  }
+}
 template <typename R>
 void launch_sweep_pass(sc_ctx *c, const SweepArgs<R> &A, unsigned blocks) {
-  // Resident blocks per SM, fastest measured on B200 (606 x 606 d-wave square,
-  // 256 angles, 14 energies, fixed-group kernels): FP64 three (four energies
-  // per thread, 168 registers: 21.8 ms against 22.1 with four blocks and 24.4
-  // with two); mixed in the packed FP32 form four (four energies per thread
-  // in two pairs, four threads per column: 5.70 ms, 5.68 with three), or six
-  // with two energies per thread.
-  // The common mappings (four energies per thread and four threads per
-  // column; mixed and LDOS: eight threads per column) are compiled with the
-  // group size fixed, which turns the per-site group reduction, frame store
-  // and tile addressing into straight-line code (C2: FP64 sweep -5%, mixed
-  // -12%); other mappings take it at run time.
-  static const char *minb_env = std::getenv("SCB_SWEEP_MINB");
-  const int variant = minb_env ? std::atoi(minb_env) : (sizeof(R) == 8 ? 3 : (c->emax2 ? 6 : 1));
-  const bool plain = !A.burn_in && !A.accumulate;  // what the fixed-group kernels assume
-  if (c->S.fs_tight_binding) {
-    // Non-circular Fermi surface: per-angle step, generic mappings.
-    if (c->S.keldysh) {
-      if (c->ept <= 4) k_sweep<R, 4, 1, true, true><<<blocks, 128, 0, c->stream>>>(A);
-      else if (c->ept <= 8) k_sweep<R, 8, 1, true, true><<<blocks, 128, 0, c->stream>>>(A);
-      else k_sweep<R, 16, 1, true, true><<<blocks, 128, 0, c->stream>>>(A);
-    } else {
-      if (c->ept <= 4) k_sweep<R, 4, 1, false, true><<<blocks, 128, 0, c->stream>>>(A);
-      else if (c->ept <= 8) k_sweep<R, 8, 1, false, true><<<blocks, 128, 0, c->stream>>>(A);
-      else k_sweep<R, 16, 1, false, true><<<blocks, 128, 0, c->stream>>>(A);
-    }
-  } else if (c->S.keldysh) {
-    static const bool no_packed_kel = std::getenv("SCB_NO_PACKED") != nullptr;
-    if constexpr (std::is_same<R, float>::value) {
-      // Mixed-precision LDOS: four real energies per thread in two FP32 pairs.
-      if (!no_packed_kel && c->ept == 4) {
-        if (plain && c->log_groups == 3) k_sweep<R, 4, 1, true, false, 3, true><<<blocks, 128, 0, c->stream>>>(A);
-        else k_sweep<R, 4, 1, true, false, -1, true><<<blocks, 128, 0, c->stream>>>(A);
-        check_launch(c);
-        return;
-      }
-    }
-    if (plain && c->ept == 4 && c->log_groups == 3) k_sweep<R, 4, 1, true, false, 3><<<blocks, 128, 0, c->stream>>>(A);
-    else if (c->ept <= 4) k_sweep<R, 4, 1, true><<<blocks, 128, 0, c->stream>>>(A);
-    else if (c->ept <= 8) k_sweep<R, 8, 1, true><<<blocks, 128, 0, c->stream>>>(A);
-    else k_sweep<R, 16, 1, true><<<blocks, 128, 0, c->stream>>>(A);
-  } else if (c->ept <= 2 && c->emax2) {
-    const bool g8 = plain && c->log_groups == 3 && c->ept == 2;
-    if constexpr (std::is_same<R, float>::value) {
-      // Two energies per thread: the packed FP32 form (both energies in one
-      // FFMA2 / FMUL2 / FADD2 per operation).
-      static const bool no_packed = std::getenv("SCB_NO_PACKED") != nullptr;
-      if (!no_packed && c->ept == 2 && (variant >= 6 || variant == 4)) {
-        if (variant >= 6 && g8) k_sweep<R, 2, 6, false, false, 3, true><<<blocks, 128, 0, c->stream>>>(A);
-        else if (variant >= 6) k_sweep<R, 2, 6, false, false, -1, true><<<blocks, 128, 0, c->stream>>>(A);
-        else if (g8) k_sweep<R, 2, 4, false, false, 3, true><<<blocks, 128, 0, c->stream>>>(A);
-        else k_sweep<R, 2, 4, false, false, -1, true><<<blocks, 128, 0, c->stream>>>(A);
-        check_launch(c);
-        return;
-      }
-    }
-    if (variant >= 6 && g8) k_sweep<R, 2, 6, false, false, 3><<<blocks, 128, 0, c->stream>>>(A);
-    else if (variant >= 6) k_sweep<R, 2, 6, false><<<blocks, 128, 0, c->stream>>>(A);
-    else if (variant == 4 && g8) k_sweep<R, 2, 4, false, false, 3><<<blocks, 128, 0, c->stream>>>(A);
-    else if (variant == 5 && g8) k_sweep<R, 2, 5, false, false, 3><<<blocks, 128, 0, c->stream>>>(A);
-    else if (variant == 5) k_sweep<R, 2, 5, false><<<blocks, 128, 0, c->stream>>>(A);
-    else if (variant == 3) k_sweep<R, 2, 3, false><<<blocks, 128, 0, c->stream>>>(A);
-    else k_sweep<R, 2, 4, false><<<blocks, 128, 0, c->stream>>>(A);
-  } else if (c->ept <= 4) {
-    if constexpr (std::is_same<R, float>::value) {
-      // Four energies per thread in mixed precision (energy passes of low
-      // temperatures, or a mapping chosen by SCB_ENERGY_GROUPS): two FP32 pairs.
-      static const bool no_packed4 = std::getenv("SCB_NO_PACKED") != nullptr;
-      if (!no_packed4 && c->ept == 4) {
-        const bool g4 = plain && c->log_groups == 2;
-        if (variant == 3 && g4) k_sweep<R, 4, 3, false, false, 2, true><<<blocks, 128, 0, c->stream>>>(A);
-        else if (variant == 3) k_sweep<R, 4, 3, false, false, -1, true><<<blocks, 128, 0, c->stream>>>(A);
-        else if (g4) k_sweep<R, 4, 4, false, false, 2, true><<<blocks, 128, 0, c->stream>>>(A);
-        else k_sweep<R, 4, 4, false, false, -1, true><<<blocks, 128, 0, c->stream>>>(A);
-        check_launch(c);
-        return;
-      }
-    }
-    if (variant == 4 && plain && c->log_groups == 2 && c->ept == 4) k_sweep<R, 4, 4, false, false, 2><<<blocks, 128, 0, c->stream>>>(A);
-    else if (variant == 4) k_sweep<R, 4, 4, false><<<blocks, 128, 0, c->stream>>>(A);
-    else if (variant == 5) k_sweep<R, 4, 5, false><<<blocks, 128, 0, c->stream>>>(A);
-    else if (variant == 3 && plain && c->log_groups == 2 && c->ept == 4) k_sweep<R, 4, 3, false, false, 2><<<blocks, 128, 0, c->stream>>>(A);
-    else if (variant == 2 && plain && c->log_groups == 2 && c->ept == 4) k_sweep<R, 4, 2, false, false, 2><<<blocks, 128, 0, c->stream>>>(A);
-    else if (variant == 3) k_sweep<R, 4, 3, false><<<blocks, 128, 0, c->stream>>>(A);
-    else k_sweep<R, 4, 1, false><<<blocks, 128, 0, c->stream>>>(A);
-  } else if (c->ept <= 8) {
-    k_sweep<R, 8, 1, false><<<blocks, 128, 0, c->stream>>>(A);
-  } else {
-    k_sweep<R, 16, 1, false><<<blocks, 128, 0, c->stream>>>(A);
-  }
+  if (c->S.keldysh) launch_sweep_kel<R, true>(c, A, blocks);
+  else launch_sweep_kel<R, false>(c, A, blocks);
   check_launch(c);
 }
 
 template <typename R>
 void launch_sweep(sc_ctx *c, const Chunk &ch, int burn_in) {
   SweepArgs<R> A = sweep_args<R>(c, &ch, burn_in);
-  const size_t threads = (size_t)A.n_items * c->groups;
-  if (!threads) return;
-  const unsigned blocks = grid1(threads, 128);
+  if (!A.n_items) return;
+  const unsigned blocks = grid1((size_t)A.n_items * 2 * c->groups, 128);  // both functions
   launch_frame_fields<R>(c, ch, A);
   ProfScope prof(c, 0);
   const int ne = c->S.ne, pass = c->e_pass;
@@ -2280,6 +1717,7 @@ void launch_sweep(sc_ctx *c, const Chunk &ch, int burn_in) {
     P.e_re += e;
     P.e_im += e;
     P.res += e;
+    P.res2 += e;
     P.bin_g += e;
     P.bout_g += e;
     P.bin_gt += e;
@@ -2289,22 +1727,36 @@ void launch_sweep(sc_ctx *c, const Chunk &ch, int burn_in) {
   }
 }
 
-void extend_reference(sc_ctx *c) {
+AccConsts acc_consts(const sc_ctx *c) {
+  const HostSetup &S = c->S;
+  AccConsts C{};
+  C.kind = S.acc.kind;
+  C.nf = c->n_fields();
+  C.step_size = S.acc.step_size;
+  C.factor = S.acc.step_size_factor;
+  C.mincos = S.acc.cos_similarity_min;
+  C.smax = S.acc.step_size_max;
+  C.smin = S.acc.step_size_min;
+  C.drag = S.acc.drag;
+  return C;
+}
+
+// The reference records of the state (after the accelerator's element-wise
+// step when advance is set) and their extension past the grain.
+void extend_reference(sc_ctx *c, bool advance = false) {
   const HostSetup &S = c->S;
   const int nn = (int)c->nn0();
-  k_pack_reference<<<grid1(nn, 256), 256, 0, c->stream>>>(S.nc, nn, c->xstate.p, (double2 *)c->rfields.p);
+  const AccConsts C = acc_consts(c);
+  k_advance_pack<<<grid1(nn, 256), 256, 0, c->stream>>>(C, advance ? C.nf : 0, S.nc, nn, c->gstate.p, c->xstate.p,
+                                                       c->acc_m.p, c->acc_state.p, (double2 *)c->rfields.p,
+                                                       (float2 *)c->rfields32.p);
   check_launch(c);
   const int ns = (int)S.rext_site.size();
   if (ns) {
     dim3 grid(grid1(ns, 128), 2 * S.nc);
     k_extend_reference<<<grid, 128, 0, c->stream>>>(2 * S.nc, nn, ns, S.nc + 1, c->rext_site.p, c->rext_off.p,
-                                                    c->rext_src.p, c->xstate.p, c->rfields.p);
-    check_launch(c);
-  }
-  if (c->rfields32.p) {
-    const size_t n = (size_t)(S.nc + 1) * nn;
-    k_round_reference<<<grid1(n, 256), 256, 0, c->stream>>>(n, (const double2 *)c->rfields.p,
-                                                           (float2 *)c->rfields32.p);
+                                                    c->rext_src.p, c->xstate.p, c->rfields.p,
+                                                    (float *)c->rfields32.p);
     check_launch(c);
   }
 }
@@ -2313,13 +1765,11 @@ template <typename R>
 void boundary_condition(sc_ctx *c) {
   const HostSetup &S = c->S;
   ProfScope prof(c, 3);
-  k_boundary<R><<<c->nb_bnd, REDUCE_THREADS, 0, c->stream>>>(
-      S.n_in_g, S.ne, c->bc_src_g.p, c->bc_w_g.p, c->bc_ws_g.p, (const Cx<R> *)c->bnd_ptr(1),
-      (Cx<R> *)c->bnd_ptr(0), c->partial_bg.p);
-  check_launch(c);
-  k_boundary<R><<<c->nb_bnd, REDUCE_THREADS, 0, c->stream>>>(
-      S.n_in_gt, S.ne, c->bc_src_gt.p, c->bc_w_gt.p, c->bc_ws_gt.p, (const Cx<R> *)c->bnd_ptr(3),
-      (Cx<R> *)c->bnd_ptr(2), c->partial_bgt.p);
+  const BoundarySide<R> g{S.n_in_g, c->bc_src_g.p, c->bc_w_g.p, c->bc_ws_g.p, (const Cx<R> *)c->bnd_ptr(1),
+                          (Cx<R> *)c->bnd_ptr(0), c->partial_bg.p};
+  const BoundarySide<R> gt{S.n_in_gt, c->bc_src_gt.p, c->bc_w_gt.p, c->bc_ws_gt.p, (const Cx<R> *)c->bnd_ptr(3),
+                           (Cx<R> *)c->bnd_ptr(2), c->partial_bgt.p};
+  k_boundary<R><<<dim3(c->nb_bnd, 2), REDUCE_THREADS, 0, c->stream>>>(S.ne, g, gt);
   check_launch(c);
 }
 
@@ -2354,57 +1804,39 @@ void launch_scalars_b(sc_ctx *c, int do_bc, int do_vp, int compute_mode, size_t 
   check_launch(c);
 }
 
-// 2D FFT of the P x P array z (rows, transpose into t, rows): the spectrum
-// ends in t in transposed layout [k_col][k_row].  The inverse takes t in that
-// layout and leaves the result in z in the original layout.
-// 2D FFT of a P x P array: rows of `first`, transpose into `second`, rows of
-// `second` (so the spectrum is transposed; the inverse undoes it).  Only the
-// first rows_in rows of `first` can be non-zero (the transform of a zero row is
-// zero, so the others are left as they are), and only the first rows_out rows
-// of the result are needed (the transpose and the last pass stop there).
-void fft2(sc_ctx *c, double2 *z, double2 *t, int inverse, int rows_in, int rows_out) {
-  const int P = c->fft_p;
-  const int thr = std::min(P / 2, 512);
-  const size_t smem = 2 * (size_t)P * sizeof(double2);
-  const dim3 tb(32, 8), tg((rows_out + 31) / 32, P / 32);
-  double2 *first = inverse ? t : z, *second = inverse ? z : t;
-  k_fft_rows<<<rows_in, thr, smem, c->stream>>>(c->fft_plan, P, (const double2 *)c->fft_tw.p, first, inverse);
-  check_launch(c);
-  k_fft_transpose<<<tg, tb, 0, c->stream>>>(P, first, second);
-  check_launch(c);
-  k_fft_rows<<<rows_out, thr, smem, c->stream>>>(c->fft_plan, P, (const double2 *)c->fft_tw.p, second, inverse);
-  check_launch(c);
+// Columns of one block of k_pois_cols: as many as leave a block per SM (four
+// neighbouring columns are a 64-byte run of every row) and about 100 KB of
+// shared memory a block.
+int pois_cols(int P) {
+  int cols = P >= 4 * 148 ? 4 : P >= 2 * 148 ? 2 : 1;
+  while (cols > 1 && (size_t)2 * cols * P * sizeof(double2) > 104 * 1024) cols /= 2;
+  return cols;
 }
 
-void poisson(sc_ctx *c, const double *j, double *a_out, int mean_from_scalars) {
-  const HostSetup &S = c->S;
-  const int n = S.n0;
-  const size_t nn2 = 2 * c->nn0();
-  if (mean_from_scalars) {
-    k_subtract_mean<<<grid1(nn2, 256), 256, 0, c->stream>>>(
-        n, j, (const double *)c->scalars.p, (int)(offsetof(Scalars, j_mean) / sizeof(double)),
-        c->pois_s.p);
-    check_launch(c);
-  } else {
-    CUDA_TRY(cudaMemcpyAsync(c->pois_s.p, j, nn2 * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-  }
+// A of the current j: old not null: its residual against old goes to
+// partial_vp (one row of sums per lattice row), and the mean of j is taken
+// from the scalars; null: j is mean-free.
+void poisson(sc_ctx *c, const double *j, double *a_out, const double *old) {
+  const int n = c->S.n0, P = c->fft_p;
   ProfScope prof(c, 2);
-  const int P = c->fft_p;
-  const size_t pp = (size_t)P * P;
-  double2 *z = (double2 *)c->fft_z.p, *t = (double2 *)c->fft_t.p;
-  k_fft_pack<<<grid1(pp, 256), 256, 0, c->stream>>>(n, P, c->pois_s.p, z);
+  double2 *z = (double2 *)c->fft_z.p;
+  const double2 *tw = (const double2 *)c->fft_tw.p;
+  const int cols = pois_cols(P);
+  const size_t row = 2 * (size_t)P * sizeof(double2);
+  k_pois_rows<<<n, P > 1024 ? 512 : 256, row, c->stream>>>(c->fft_plan, n, P, tw, j,
+                                                           old ? c->scalars.p->j_mean : nullptr, z);
   check_launch(c);
-  fft2(c, z, t, 0, n, P);  // the current fills rows < N0 of z
-  k_fft_mul<<<grid1(pp, 256), 256, 0, c->stream>>>(pp, (const double2 *)c->fft_kf.p, t);
+  k_pois_cols<<<P / cols, 512, cols * row, c->stream>>>(c->fft_plan, P, n, cols, tw, (const double2 *)c->fft_kf.p, z,
+                                                         nullptr);
   check_launch(c);
-  fft2(c, z, t, 1, P, n);  // A is read from rows < N0 of z
-  k_fft_unpack<<<grid1(c->nn0(), 256), 256, 0, c->stream>>>(n, P, 1.0 / ((double)P * (double)P), z, a_out);
+  k_pois_back<<<n, REDUCE_THREADS, row, c->stream>>>(c->fft_plan, n, P, 1.0 / ((double)P * (double)P), tw, z, old,
+                                                    a_out, c->partial_vp.p);
   check_launch(c);
 }
 
 // The kernel K(u, v) = -h^2 scale sum_k (+/-) f_k(u) f_k(v), reflected
 // (A is a correlation, the FFT product a convolution) and wrapped into the
-// P x P array, and its spectrum in the transposed layout of fft2.
+// P x P array, and its spectrum as [column][row].
 void poisson_setup(sc_ctx *c) {
   const HostSetup &S = c->S;
   const int n = S.n0;
@@ -2451,27 +1883,27 @@ void poisson_setup(sc_ctx *c) {
     }
   }
   c->fft_z.alloc(2 * pp);
-  c->fft_t.alloc(2 * pp);
   c->fft_kf.alloc(2 * pp);
   CUDA_TRY(cudaMemcpyAsync(c->fft_z.p, kr.data(), 2 * pp * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  if (2 * P * sizeof(double2) > 48 * 1024)
-    CUDA_TRY(cudaFuncSetAttribute(k_fft_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(2 * P * sizeof(double2))));
-  fft2(c, (double2 *)c->fft_z.p, (double2 *)c->fft_kf.p, 0, P, P);
+  const int cols = pois_cols(P);
+  const size_t row = 2 * (size_t)P * sizeof(double2);
+  for (const void *k : {(const void *)k_pois_rows, (const void *)k_pois_back, (const void *)k_pois_cols})
+    CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+  double2 *z = (double2 *)c->fft_z.p;
+  k_pois_rows<<<P, P > 1024 ? 512 : 256, row, c->stream>>>(c->fft_plan, n, P, (const double2 *)c->fft_tw.p, nullptr,
+                                                           nullptr, z);
+  check_launch(c);
+  k_pois_cols<<<P / cols, 512, cols * row, c->stream>>>(c->fft_plan, P, P, cols, (const double2 *)c->fft_tw.p,
+                                                         nullptr, z, (double2 *)c->fft_kf.p);
+  check_launch(c);
   CUDA_TRY(cudaStreamSynchronize(c->stream));
 }
 
-void accelerate(sc_ctx *c) {
+// The accelerator's step on x, but for the element-wise part of all but
+// Anderson, which extend_reference(c, true) takes: returns whether it is due.
+bool accelerate(sc_ctx *c) {
   const HostSetup &S = c->S;
-  AccConsts C{};
-  C.kind = S.acc.kind;
-  C.nf = c->n_fields();
-  C.step_size = S.acc.step_size;
-  C.factor = S.acc.step_size_factor;
-  C.mincos = S.acc.cos_similarity_min;
-  C.smax = S.acc.step_size_max;
-  C.smin = S.acc.step_size_min;
-  C.drag = S.acc.drag;
+  const AccConsts C = acc_consts(c);
   const size_t nn = c->nn0();
   if (C.kind == ACC_ANDERSON) {
     const size_t tot = (size_t)C.nf * nn;
@@ -2484,19 +1916,15 @@ void accelerate(sc_ctx *c) {
     k_and_update<<<grid1(tot, 256), 256, 0, c->stream>>>(tot, rank, C.step_size, c->and_x.p, c->and_d.p,
                                                          c->acc_state.p, c->xstate.p);
     check_launch(c);
-    return;
+    return false;
   }
   if (C.kind == ACC_CONGACC || C.kind == ACC_BB) {
     dim3 grid(c->nb_acc, C.nf);
-    k_acc_sums<<<grid, REDUCE_THREADS, 0, c->stream>>>(C.nf, nn, c->xstate.p, c->gstate.p, c->acc_m.p,
-                                                        c->partial_acc.p);
-    check_launch(c);
-    k_acc_scalars<<<1, 256, 0, c->stream>>>(C, c->partial_acc.p, c->nb_acc, c->acc_state.p);
+    k_acc_sums<<<grid, REDUCE_THREADS, 0, c->stream>>>(C, nn, c->xstate.p, c->gstate.p, c->acc_m.p,
+                                                        c->partial_acc.p, c->acc_state.p, c->counters.p + 1);
     check_launch(c);
   }
-  k_acc_update<<<grid1((size_t)C.nf * nn, 256), 256, 0, c->stream>>>(C, nn, c->gstate.p, c->xstate.p,
-                                                                       c->acc_m.p, c->acc_state.p);
-  check_launch(c);
+  return true;
 }
 
 // Frame extension and rotation back of one swept chunk.
@@ -2523,10 +1951,10 @@ void frame_to_reference(sc_ctx *c, const Chunk &ch) {
   }
   // A warp covers an 8 x 4 patch of the reference grid (its rotated corners
   // share cache lines of the frame).
-  dim3 blk(8, 32), grid((S.n0 + 7) / 8, (S.n0 + 31) / 32);
+  dim3 blk(8, 32), grid((S.n0 + 7) / 8, (S.n0 + 31) / 32, c->rb_parts);
   ProfScope prof(c, 1);
   auto kern = S.nc == 1 ? k_rotate_back<Fr, 1> : S.nc == 2 ? k_rotate_back<Fr, 2> : k_rotate_back<Fr, 0>;
-  kern<<<grid, blk, 0, c->stream>>>(S.n0, S.n1, S.nc, ch.a_begin, a_stored, pair, c->ang.p, (const Fr *)c->w_fr,
+  kern<<<grid, blk, 0, c->stream>>>(S.n0, S.n1, S.nc, ch.a_begin == 0, ch.a_begin, a_stored, pair, c->ang.p, (const Fr *)c->w_fr,
                                     c->acc_d.p, c->acc_j.p, c->acc_fe.p);
   check_launch(c);
 }
@@ -2539,7 +1967,7 @@ static void launch_rotate_back_ldos(sc_ctx *c, const Chunk &ch) {
   auto go = [&](auto kern, int el, int tx) {
     const int ty = 256 / el / tx;
     dim3 grid((S.n0 + tx - 1) / tx, (S.n0 + ty - 1) / ty, (S.ne + el - 1) / el);
-    kern<<<grid, 256, 0, c->stream>>>(S.n0, S.n1, S.ne, ch.a_begin, ch.a_end, c->ang.p, (const LF *)c->ldf.p,
+    kern<<<grid, 256, 0, c->stream>>>(S.n0, S.n1, S.ne, ch.a_begin == 0, ch.a_begin, ch.a_end, c->ang.p, (const LF *)c->ldf.p,
                                       c->ldos_acc.p);
   };
   if (S.ne <= 8)
@@ -2600,16 +2028,13 @@ void run_chunks(sc_ctx *c, int burn_in) {
 }
 
 // Context::compute in three parts: before the sweep (accelerator step,
-// extended order parameter, cleared accumulators), the sweep with the frame
+// extended order parameter), the sweep with the frame
 // rotation, and after it (finalize, boundary condition, vector potential).
 template <typename R>
 void compute_pre(sc_ctx *c) {
-  if (!c->first_compute) accelerate(c);
-  if (!c->boundary_initialized) boundary_initial<R>(c);
-  extend_reference(c);
-  c->acc_d.zero(c->stream);
-  c->acc_j.zero(c->stream);
-  c->acc_fe.zero(c->stream);
+  const bool advance = !c->first_compute && accelerate(c);
+  extend_reference(c, advance);
+  if (!c->boundary_initialized) boundary_initial<R>(c);  // on the same state
 }
 
 template <typename R>
@@ -2670,6 +2095,30 @@ void compute_iteration(sc_ctx *c) {
   c->launches += c->iter_graph_launches;
 }
 
+void launch_finalize(sc_ctx *c, const double *delta, const double *avec) {
+  const HostSetup &S = c->S;
+  FinalizeConsts F{};
+  F.nc = S.nc;
+  F.norm = S.norm;
+  F.n_grain = S.n_grain;
+  F.has_vp = c->has_vp() ? 1 : 0;
+  F.n_elem_field = 2 * c->nn0();
+  F.temperature = S.temperature;
+  F.h = S.h;
+  F.lambda = S.lambda;
+  F.conv = S.conv_crit;
+  double si = 0.0;
+  for (int e = 0; e < S.ne; ++e) si += S.residues[e] / S.e_im[e];
+  F.sum_inv = si * S.temperature;
+  for (int k = 0; k < S.nc; ++k) F.log_t_tc[k] = std::log(S.temperature / S.tc[k]);
+  const double jfactor = (double)(2 * S.charge_sign) * S.temperature;
+  auto fin = S.nc == 1 ? k_finalize<1> : S.nc == 2 ? k_finalize<2> : k_finalize<0>;
+  fin<<<c->nb_fin, REDUCE_THREADS, 0, c->stream>>>(
+      S.n0, S.nc, S.h, jfactor, c->has_vp() ? 1 : 0, c->dom.p, c->coupling.p, c->acc_d.p, c->acc_j.p, c->acc_fe.p,
+      delta, avec, c->gstate.p, c->j_real.p, c->partial_fin.p, F, c->scalars.p, c->counters.p, c->rb_parts);
+  check_launch(c);
+}
+
 template <typename R>
 void compute_post(sc_ctx *c) {
   const HostSetup &S = c->S;
@@ -2677,37 +2126,13 @@ void compute_post(sc_ctx *c) {
   // Finalize.
   {
     double *delta = c->xstate.p, *avec = c->xstate.p + (size_t)2 * S.nc * nn;
-    double *delta_new = c->gstate.p;
-    const double jfactor = (double)(2 * S.charge_sign) * S.temperature;
-    auto fin = S.nc == 1 ? k_finalize<1> : S.nc == 2 ? k_finalize<2> : k_finalize<0>;
-    fin<<<c->nb_fin, REDUCE_THREADS, 0, c->stream>>>(
-        S.n0, S.nc, S.h, jfactor, c->has_vp() ? 1 : 0, c->dom.p, c->coupling.p, c->acc_d.p, c->acc_j.p,
-        c->acc_fe.p, delta, avec, delta_new, c->j_real.p, c->partial_fin.p);
-    check_launch(c);
-    FinalizeConsts F{};
-    F.nc = S.nc;
-    F.norm = S.norm;
-    F.n_grain = S.n_grain;
-    F.has_vp = c->has_vp() ? 1 : 0;
-    F.n_elem_field = 2 * nn;
-    F.temperature = S.temperature;
-    F.h = S.h;
-    F.lambda = S.lambda;
-    F.conv = S.conv_crit;
-    double si = 0.0;
-    for (int e = 0; e < S.ne; ++e) si += S.residues[e] / S.e_im[e];
-    F.sum_inv = si * S.temperature;
-    for (int k = 0; k < S.nc; ++k) F.log_t_tc[k] = std::log(S.temperature / S.tc[k]);
-    k_scalars_a<<<1, 1024, 0, c->stream>>>(F, c->partial_fin.p, c->nb_fin, c->scalars.p);
-    check_launch(c);
+    launch_finalize(c, delta, avec);
   }
   boundary_condition<R>(c);
   if (c->has_vp()) {
     double *a_new = c->gstate.p + (size_t)2 * S.nc * nn;
     const double *avec = c->xstate.p + (size_t)2 * S.nc * nn;
-    poisson(c, c->j_real.p, a_new, 1);
-    k_residual<<<c->nb_vp, REDUCE_THREADS, 0, c->stream>>>(2 * nn, avec, a_new, c->partial_vp.p);
-    check_launch(c);
+    poisson(c, c->j_real.p, a_new, avec);
   }
   launch_scalars_b(c, 1, c->has_vp() ? 1 : 0, 1);
   c->first_compute = false;
@@ -2753,7 +2178,6 @@ void ldos_once(sc_ctx *c) {
   if (c->ldos_block < 0) ldos_begin_block(c, 0);
   if (!c->boundary_initialized) boundary_initial<R>(c);
   extend_reference(c);
-  c->ldos_acc.zero(c->stream);
   run_chunks<R>(c, 0);
   boundary_condition<R>(c);
   const int nf = ldos_block_count(c, c->ldos_block);
@@ -2835,6 +2259,70 @@ void plan_chunks(sc_ctx *c, std::vector<int4> &items) {
   }
 }
 
+// Threads per column and function (groups = 2^log_groups) and energies per
+// thread (ept) of the context's sweeps.
+void set_mapping(sc_ctx *c, int ept) {
+  while (16 * ept < c->e_pass) ept *= 2;  // at most 16 threads per column and function
+  c->ept = ept;
+  c->log_groups = 0;
+  while ((ept << c->log_groups) < c->e_pass && c->log_groups < 4) c->log_groups++;
+  c->groups = 1 << c->log_groups;
+}
+// The mapping of a single context.  A thread with more energies interleaves
+// more independent recursions and shares the site's loads, reductions and
+// bookkeeping among them; a thread with fewer leaves more warps for a grain of
+// few columns.  Measured on B200 (sweep of the 606 x 606 d-wave square, 14
+// energies, per energy slot, relative): FP64 one energy 1.64, two 1.23, four
+// 1.00, seven 1.06; FP32 two 1.32, four 1.00, eight 0.95 (real energies, whose
+// constants are per energy: eight 1.15).  Slots round the energies up to
+// EMAX * 2^lg, so 14 energies on seven a thread beat 16 slots on four, 20 real
+// energies 21 slots on seven (5.3 ms) 32 slots on four (6.4 ms).  The cheapest
+// product is taken among the mappings that give every scheduler enough warps
+// (1.5 to 5, by the mapping's own parallelism), else the one with the most
+// warps: a 4 xi0 disc in FP32, 0.5 warps per scheduler at two energies, takes
+// 37 us per sweep with one, 46 with two and 55 with four.
+void plan_mapping(sc_ctx *c) {
+  const bool fp32 = c->mode == SC_MODE_MIXED, kel = c->S.keldysh;
+  struct Option {
+    int ept;
+    double cost, warps;  // per energy slot; wanted per scheduler
+  };
+  const Option fp64_opt[] = {{1, 1.64, 0.0}, {2, 1.23, 1.5}, {4, 1.0, 1.5}, {7, 1.06, 3.0}};
+  const Option fp32_opt[] = {{1, 1.6, 0.0}, {2, 1.32, 1.5}, {4, 1.0, 1.5}, {8, kel ? 1.15 : 0.95, 5.0}};
+  const Option *opt = fp32 ? fp32_opt : fp64_opt;
+  const char *eg = std::getenv("SCB_ENERGY_GROUPS");
+  const int cap = fp32 ? 8 : 7;
+  if (eg) {  // tests: at least this many threads per column (as the kernels' energies per thread allow)
+    const int want = std::max(1, std::atoi(eg));
+    const int need = (c->e_pass + want - 1) / want;
+    set_mapping(c, need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : cap);
+    return;
+  }
+  int dev = 0, n_sm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  size_t items = 0;
+  for (const Chunk &ch : c->chunks) items = std::max(items, (size_t)(ch.item_end - ch.item_begin));
+  double best = 1e300;
+  int ept = 1;
+  for (int k = 0; k < 4; ++k) {
+    set_mapping(c, opt[k].ept);
+    if (c->ept != opt[k].ept) continue;  // more than 16 threads per column
+    const double warps = (double)items * 2 * c->groups / 32 / (4.0 * n_sm);
+    if (warps < opt[k].warps) continue;
+    const double cost = opt[k].cost * (opt[k].ept << c->log_groups);
+    if (cost < best) {
+      best = cost;
+      ept = opt[k].ept;
+    }
+  }
+  if (best == 1e300) {  // one energy per thread does not fit 16 threads: the fewest that do
+    ept = 2;
+    while (16 * ept < c->e_pass) ept *= 2;
+  }
+  set_mapping(c, ept);
+}
+
 void upload_static(sc_ctx *c) {
   HostSetup &S = c->S;
   cudaStream_t s = c->stream;
@@ -2888,6 +2376,10 @@ void upload_static(sc_ctx *c) {
   c->e_re.upload(S.e_re, s);
   c->e_im.upload(S.e_im, s);
   c->res.upload(S.residues, s);
+  std::vector<double> res2(S.residues);
+  for (double &v : res2) v *= 2.0;
+  c->res2.upload(res2, s);
+  for (double v : S.ldos_energies) c->e_re_max = std::max(c->e_re_max, (float)std::fabs(v) * 1.001f);
   c->coupling.upload(S.coupling, s);
   if (S.n_filters) {
     c->filters.upload(S.filters, s);
@@ -2958,41 +2450,7 @@ void upload_static(sc_ctx *c) {
   plan_chunks(c, items);
   c->items.upload(items, s);
   c->h_items = items;  // host copy: the batch plans its work units from it
-  // Energy groups per column.
-  c->groups = 1;
-  c->log_groups = 0;
-  const char *eg = std::getenv("SCB_ENERGY_GROUPS");
-  // Default (fastest measured on B200 for 7-14 Ozaki energies): the fewest
-  // threads per column that keep at most four energies per thread; three
-  // (FP64) or four (mixed) resident blocks per SM.  Mixed precision prefers an
-  // even count, which the packed FP32 sweep takes in pairs (C2, 14 energies:
-  // four threads of four energies, sweep 5.70 ms, against eight threads of two
-  // 6.07 ms).
-  const bool fp32_sweep = c->mode == SC_MODE_MIXED && !S.keldysh;
-  const int per_thread = 4;
-  int want = 1;
-  if (eg) want = std::atoi(eg);
-  else {
-    while ((c->e_pass + want - 1) / want > per_thread && want < 8) want *= 2;
-    // Small grains: too few trajectory columns to fill the GPU twice over,
-    // so spread the energies over more threads per column.
-    int dev = 0, n_sm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-    const double resident = (double)n_sm * (fp32_sweep ? 4 : 3) * 128;
-    size_t max_items = 0;
-    for (const Chunk &ch : c->chunks) max_items = std::max(max_items, (size_t)(ch.item_end - ch.item_begin));
-    while ((double)max_items * want < 2.0 * resident && want < 8 && (c->e_pass + want - 1) / want > 1) want *= 2;
-    const int ept_w = (c->e_pass + want - 1) / want;
-    if (fp32_sweep && ept_w > 1 && ept_w % 2 == 1 && want < 8) want *= 2;
-  }
-  while (c->groups < want && c->groups < 8) {
-    c->groups *= 2;
-    c->log_groups++;
-  }
-  c->ept = (c->e_pass + c->groups - 1) / c->groups;
-  if (c->ept > 16) throw EngineError(SC_ERR_ARG, "too many Ozaki energies per thread");
-  c->emax2 = fp32_sweep ? !std::getenv("SCB_SWEEP_EMAX4") : std::getenv("SCB_SWEEP_EMAX2") != nullptr;
+  plan_mapping(c);
 
   // State and work buffers.
   const size_t nn = c->nn0();
@@ -3005,9 +2463,6 @@ void upload_static(sc_ctx *c) {
   if (c->mode == SC_MODE_MIXED) c->rfields32.alloc((size_t)(S.nc + 1) * nn + 1);
   c->j_real.alloc(2 * nn);
   c->j_real.zero(s);
-  c->acc_d.alloc((size_t)2 * S.nc * nn);
-  c->acc_j.alloc(2 * nn);
-  c->acc_fe.alloc(nn);
   size_t off = 0;
   for (int w = 0; w < 4; ++w) {
     c->bnd_off[w] = off;
@@ -3025,6 +2480,18 @@ void upload_static(sc_ctx *c) {
     scr = std::max(scr, ni32 * ch.kmax * (size_t)((c->e_pass + 1) & ~1) * c->esize());
     scr2 = std::max(scr2, ni32 * ch.kmax * 4);
     max_slots = std::max(max_slots, chunk_slots(c, ch));
+  }
+  // Parts of the angles that k_rotate_back sums apart: enough for about 32
+  // blocks per SM, at most eight, at least four stored angles each (606 x 606:
+  // four parts 0.69 ms, one 0.77; 206 x 206: eight 48 us, one 79; 86 x 86: four
+  // 12 us, one 31).
+  if (!S.keldysh) {
+    const size_t tiles = (size_t)((S.n0 + 7) / 8) * ((S.n0 + 31) / 32);
+    const int want = (int)std::min<size_t>(8, (32 * 148 + tiles - 1) / tiles);
+    c->rb_parts = std::max(1, std::min(want, max_slots / 4));
+    c->acc_d.alloc((size_t)2 * S.nc * nn * c->rb_parts);
+    c->acc_j.alloc(2 * nn * c->rb_parts);
+    c->acc_fe.alloc(nn * c->rb_parts);
   }
   c->need_scratch = scr + 8;
   c->need_scratch2 = (scr2 + 1) * sizeof(double);
@@ -3051,7 +2518,7 @@ void upload_static(sc_ctx *c) {
   }
   c->nb_fin = std::min<int>(592, (int)grid1(nn, REDUCE_THREADS));
   c->nb_bnd = std::min<int>(592, (int)grid1((size_t)std::max(S.n_in_g, S.n_in_gt) * S.ne, REDUCE_THREADS));
-  c->nb_vp = std::min<int>(296, (int)grid1(2 * nn, REDUCE_THREADS));
+  c->nb_vp = S.keldysh ? std::min<int>(592, (int)grid1(nn, REDUCE_THREADS)) : S.n0;  // LDOS finalize blocks; Poisson rows
   c->nb_acc = std::min<int>(148, (int)grid1(nn, REDUCE_THREADS));
   c->partial_fin.alloc((size_t)c->nb_fin * NQ);
   c->partial_bg.alloc((size_t)c->nb_bnd * 6);
@@ -3060,7 +2527,6 @@ void upload_static(sc_ctx *c) {
   c->partial_acc.alloc((size_t)AND_MAX_RANK * c->nb_acc * 3);
   c->partial_vp.zero(s);
   if (S.n_filters && !S.keldysh) {
-    c->pois_s.alloc(2 * nn);
     poisson_setup(c);
   }
   c->acc_m.alloc((size_t)std::max(nf, 1) * nn);
@@ -3073,6 +2539,8 @@ void upload_static(sc_ctx *c) {
   c->acc_state.alloc(1);
   c->acc_state.zero(s);
   c->scalars.alloc(1);
+  c->counters.alloc(2);
+  c->counters.zero(s);
   Scalars init{};
   init.first_j = 1;
   init.first_fe = 1;
@@ -3592,7 +3060,7 @@ int sc_poisson(sc_ctx *ctx, const double *j, double *a_out) {
   }
   CUDA_TRY(cudaMemcpyAsync(ctx->tmp_io.p, s.data(), nn2 * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   double *out = ctx->tmp_io.p + nn2;
-  poisson(ctx, ctx->tmp_io.p, out, 0);
+  poisson(ctx, ctx->tmp_io.p, out, nullptr);
   CUDA_TRY(cudaMemcpyAsync(a_out, out, nn2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   API_END
@@ -3678,7 +3146,8 @@ struct sc_batch {
   cudaStream_t stream = nullptr;
   std::string err;
   int ept_max = 4;     // at most this many energies per thread; each grain the fewest threads per column that allow it
-  int minb = 1;        // resident-block variant of the persistent sweep
+  int minb = 1;        // accepted and reported; every mapping has one register variant
+  int ept() const { return ept_max <= 1 ? 1 : ept_max <= 2 ? 2 : ept_max <= 4 ? 4 : mode == SC_MODE_FP64 ? 7 : 8; }
   int n_sm = 148;
   std::vector<char> active;
   std::vector<int> iterations;
@@ -3690,7 +3159,6 @@ struct sc_batch {
   struct Pass {
     DevArray<int2> units;
     int n_units = 0;
-    int ept = 0;  // largest energies per thread among the pass's grains
     DevArray<unsigned char> args;
   };
   struct Wave {
@@ -3778,11 +3246,7 @@ void batch_plan(sc_batch *b) {
     for (int k = 0; k < (int)m.size(); ++k) {
       sc_ctx *c = b->grains[m[k]];
       const int ne = c->e_pass;  // energies per pass: all of them up to 64, else 32
-      c->log_groups = 0;
-      while (((ne + (1 << c->log_groups) - 1) >> c->log_groups) > b->ept_max && c->log_groups < 3)
-        c->log_groups++;
-      c->groups = 1 << c->log_groups;
-      c->ept = (ne + c->groups - 1) / c->groups;
+      set_mapping(c, b->ept());
       n_passes = std::max(n_passes, (c->S.ne + ne - 1) / ne);
     }
     for (int p = 0; p < n_passes; ++p) {
@@ -3794,7 +3258,7 @@ void batch_plan(sc_batch *b) {
         sc_ctx *c = b->grains[m[k]];
         const int e = p * c->e_pass;
         if (e >= c->S.ne) continue;
-        const int per_warp = 32 >> c->log_groups;
+        const int per_warp = 16 >> c->log_groups;
         const Chunk &ch = c->chunks[0];
         SweepArgs<R> A = sweep_args<R>(c, &ch, 0);
         if (c->e_pass < c->S.ne) {
@@ -3803,6 +3267,7 @@ void batch_plan(sc_batch *b) {
           A.e_re += e;
           A.e_im += e;
           A.res += e;
+          A.res2 += e;
           A.bin_g += e;
           A.bout_g += e;
           A.bin_gt += e;
@@ -3810,13 +3275,12 @@ void batch_plan(sc_batch *b) {
         }
         const int slot = (int)args.size();
         args.push_back(A);
-        ps.ept = std::max(ps.ept, c->ept);
         const int n = ch.item_end - ch.item_begin;
         const int4 *items = c->h_items.data() + ch.item_begin;
         for (int i = 0; i < n; i += per_warp) {
           int len = 0;
           for (int j = i; j < std::min(n, i + per_warp); ++j) len = std::max(len, items[j].w - items[j].z + 1);
-          keyed.push_back({len, make_int2(slot, i)});
+          keyed.push_back({len, make_int2(slot, i / per_warp)});
         }
       }
       std::stable_sort(keyed.begin(), keyed.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
@@ -3842,41 +3306,24 @@ void launch_batch_sweep(sc_batch *b, sc_batch::Wave &w, int wi) {
     sc_batch::Pass &ps = *pp;
     const SweepArgs<R> *args = (const SweepArgs<R> *)ps.args.p;
     CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(int), b->stream));
-    const int ept = ps.ept;
-    auto run = [&](auto kernel) {
+    auto run = [&](auto kernel, int smem) {
+      if (smem > 32 * 1024) CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       int per_sm = 1;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, smem);
       const int blocks = std::max(1, per_sm) * b->n_sm;
-      kernel<<<blocks, 128, 0, b->stream>>>(args, ps.units.p, ps.n_units, counter);
+      kernel<<<blocks, 128, smem, b->stream>>>(args, ps.units.p, ps.n_units, counter);
     };
-    // Mixed precision with at most four energies per thread in the pass: the
-    // packed FP32 sweep (each grain's count rounded up to even; a cap of one
-    // energy per thread keeps the scalar form, which that mapping is for).
-    static const bool no_packed = std::getenv("SCB_NO_PACKED") != nullptr;
-    bool packed = false;
-    if constexpr (std::is_same<R, float>::value) packed = !no_packed && b->ept_max >= 2 && ept <= 4;
-    if constexpr (std::is_same<R, float>::value) {
-      if (packed) {
-        if (ept <= 2 && b->minb == 6) run(k_sweep_batch<R, 2, 6, true>);
-        else if (ept <= 2) run(k_sweep_batch<R, 2, 4, true>);
-        else if (b->minb == 4) run(k_sweep_batch<R, 4, 4, true>);
-        else if (b->minb == 3) run(k_sweep_batch<R, 4, 3, true>);
-        else run(k_sweep_batch<R, 4, 1, true>);
-      }
-    }
-    if (packed) {
-    } else if (ept <= 2 && b->minb == 6) {
-      run(k_sweep_batch<R, 2, 6>);
-    } else if (ept <= 2 && b->minb == 4) {
-      run(k_sweep_batch<R, 2, 4>);
-    } else if (ept <= 4) {
-      if (b->minb == 4) run(k_sweep_batch<R, 4, 4>);
-      else if (b->minb == 3) run(k_sweep_batch<R, 4, 3>);
-      else run(k_sweep_batch<R, 4, 1>);
-    } else if (ept <= 8) {
-      run(k_sweep_batch<R, 8, 1>);
+    const int ept = b->ept();
+    if constexpr (sizeof(R) == 8) {
+      if (ept == 1) run(k_sweep_batch<R, 1, 5, false>, SweepRing<R, 1, 5, false>::BYTES);
+      else if (ept == 2) run(k_sweep_batch<R, 2, 3, false>, SweepRing<R, 2, 3, false>::BYTES);
+      else if (ept == 4) run(k_sweep_batch<R, 4, 3, false>, SweepRing<R, 4, 3, false>::BYTES);
+      else run(k_sweep_batch<R, 7, 2, false>, SweepRing<R, 7, 2, false>::BYTES);
     } else {
-      run(k_sweep_batch<R, 16, 1>);
+      if (ept == 1) run(k_sweep_batch<R, 1, 4, false>, SweepRing<R, 1, 4, false>::BYTES);
+      else if (ept == 2) run(k_sweep_batch<R, 2, 4, true>, SweepRing<R, 2, 4, true>::BYTES);
+      else if (ept == 4) run(k_sweep_batch<R, 4, 3, true>, SweepRing<R, 4, 3, true>::BYTES);
+      else run(k_sweep_batch<R, 8, 3, true>, SweepRing<R, 8, 3, true>::BYTES);
     }
     b->launches++;
     cudaError_t e = cudaGetLastError();
