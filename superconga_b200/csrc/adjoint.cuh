@@ -14,23 +14,20 @@
 // derivative starts from seeds on the frame lattice: the transposes of the
 // rotation back (insertRotatedGridAdditive) and of the frame extension
 // (extendValuesAtBoundary) applied to the reference-grid weights.  The adjoint
-// sweep then runs, per trajectory column, the two Riccati recursions forward
-// with gamma and gammaTilde checkpointed every ADJ_K sites, and integrates the
-// adjoint recursions in reverse, recomputing each ADJ_K-site segment from its
-// checkpoint.  Complex sensitivities are carried as G = dL/dRe z + i dL/dIm z:
-// G_z = conj(f'(z)) G_w for holomorphic w = f(z), G_z = k conj(G_w) for
-// w = k conj(z).  The frame-lattice sensitivities of the rotated order
-// parameter and of the Doppler shift are finally scattered back through the
-// transposed bilinear lookups onto the reference grid.
+// sweep then runs, per trajectory column, the two Riccati recursions forward,
+// storing both coherence functions at every site, and integrates the two
+// adjoint recursions in reverse.  Complex sensitivities are carried as
+// G = dL/dRe z + i dL/dIm z: G_z = conj(f'(z)) G_w for holomorphic w = f(z),
+// G_z = k conj(G_w) for w = k conj(z).  The frame-lattice sensitivities of the
+// rotated order parameter and of the Doppler shift are finally scattered back
+// through the transposed bilinear lookups onto the reference grid.
 
 namespace {
 
-constexpr int ADJ_K = 16;  // checkpoint interval in trajectory sites
-
 struct AdjArgs {
   SweepArgs<double> S;
-  Cx<double> *ck_gt, *ck_g;  // [segment][energy][item] state entering each segment
-  int *ck_nin_gt, *ck_nin_g; // [segment][item] entry counters entering each segment
+  int tile0, n_tiles;        // tiles of this launch
+  Cx<double> *g_all;         // gamma of every site, [tile - tile0][row][energy][column of tile]
   const double2 *seed;       // [slot][n1*n1] (seed of Re I, seed of Re g)
   double2 *grad_d;           // [slot][n1*n1] dL/dDelta_frame
   double *grad_e;            // [slot][n1*n1] dL/d(Doppler shift)
@@ -91,427 +88,317 @@ __device__ __forceinline__ void riccati_step_adj(double dre, double dim, double 
   gD = cadd(gD, C{q * Ga.im, q * Ga.re});
 }
 
-__device__ __forceinline__ void fields_at(const SweepArgs<double> &A, size_t ni, int item, int r,
-                                          double &f0, double &f1, double &f2) {
-  (void)ni;
-  const double4 v = ((const double4 *)A.scratch2)[rec_index(A, A.log_groups, item, r)];
-  f0 = v.x;
-  f1 = v.y;
-  f2 = v.z;
+// Reverse mode of step_fast at the same site constants: given gw for g1,
+// returns the sensitivity of g0 and adds those of the step's order parameter
+// and of the real part of its energy to gD and ge.  With the step written as
+//   u = a g0, beta = u + B1, t = beta + B1 + 2, c = t g0 + P, w = B1^2 - a P - 2 u,
+//   s = sqrt(w), g1 = c / (s - beta)      (a = (i h / 4) conj(D), P = i h D,
+//                                          B1 = (i h e - 1) / 2)
+// the reverse is a dozen complex products on values the forward step has too;
+// |w| and 1 / |w| come from one estimate.
+__device__ __forceinline__ Cx<double> step_fast_adj(const SiteConst<double> &S, double s0h, double sh, double bh,
+                                                    double h, Cx<double> g0, Cx<double> gw, Cx<double> &gD,
+                                                    double &ge) {
+  typedef Cx<double> C;
+  const double ure = S.ar * g0.re - S.ai * g0.im, uim = S.ar * g0.im + S.ai * g0.re;
+  const double br = ure + bh, bi = uim + sh;
+  const double tr = br + (bh + 2.0), ti = bi + sh;
+  const double cre = tr * g0.re - (ti * g0.im + S.hdi), cim = tr * g0.im + (ti * g0.re + S.hdr);
+  const double xh = (0.5 * bh * bh + s0h) - ure, y = bh * sh - uim;
+  const double xx = xh * xh + (y * y + 1e-300);  // |w|^2 / 4
+  const double rm = rsqrt_(xx), m = xx * rm;     // 2 / |w|, |w| / 2
+  const double U = m + xh, rho = rsqrt_pos(U);
+  const double sr = U * rho, si = y * rho;
+  const double dr = sr - br, di = si - bi;
+  const double inv = rcp_pos(dr * dr + di * di);
+  // conj(1 / den) = den / |den|^2
+  const C Gc = cmul(C{dr * inv, di * inv}, gw);
+  const C g1{(cre * dr + cim * di) * inv, (cim * dr - cre * di) * inv};
+  const C Gb = cmul(C{g1.re, -g1.im}, Gc);  // of beta: minus the sensitivity of den
+  // s: -Gb; w = s^2: conj(1 / (2 s)) = s / (2 |w|), 1 / (2 |w|) = rm / 4
+  const double q4 = -0.25 * rm;
+  const C Gw = cmul(C{sr * q4, si * q4}, Gb);
+  const C Gt{g0.re * Gc.re + g0.im * Gc.im, g0.re * Gc.im - g0.im * Gc.re};  // conj(g0) Gc
+  C G0{tr * Gc.re + ti * Gc.im, tr * Gc.im - ti * Gc.re};                    // conj(t) Gc
+  const C Gu{Gt.re + Gb.re - 2.0 * Gw.re, Gt.im + Gb.im - 2.0 * Gw.im};
+  G0.re += S.ar * Gu.re + S.ai * Gu.im;  // conj(a) Gu
+  G0.im += S.ar * Gu.im - S.ai * Gu.re;
+  // Re e through i h e: B1 carries half of it, t a further half.
+  //   G of i h e = Gt + Gb / 2 + conj(B1) Gw, B1 = (bh, sh); its imaginary part
+  ge += h * (Gt.im + 0.5 * Gb.im + (bh * Gw.im - sh * Gw.re));
+  // P = (-hdi, hdr): G_P = Gc - conj(a) Gw;  a: G_a = conj(g0) Gu - conj(P) Gw
+  const C GP{Gc.re - (S.ar * Gw.re + S.ai * Gw.im), Gc.im - (S.ar * Gw.im - S.ai * Gw.re)};
+  const C Ga{g0.re * Gu.re + g0.im * Gu.im + (S.hdi * Gw.re - S.hdr * Gw.im),
+             g0.re * Gu.im - g0.im * Gu.re + (S.hdi * Gw.im + S.hdr * Gw.re)};
+  // i h D: G_D = -i h G_P;  (i h / 4) conj(D): G_D += (i h / 4) conj(G_a)
+  gD.re += h * GP.im + 0.25 * h * Ga.im;
+  gD.im += -h * GP.re + 0.25 * h * Ga.re;
+  return G0;
 }
 
-// The adjoint of one trajectory column for the EMAX energies of thread g.
-template <int EMAX>
-__device__ void adjoint_column(const AdjArgs &J, const double *s_res, int item, int g, unsigned gmask) {
+// The adjoint of one tile of trajectory columns, the half-warps as in
+// sweep_tile: gammaTilde down and gamma up first, each storing every site (the
+// sweep's scratch and g_all), then the adjoint of each recursion back along
+// its column, both reading both functions.  A site's sensitivities are written
+// by the half-warp that reaches it first and completed by the other after the
+// middle.  EMAX energies per thread; LG threads per column and function.
+//
+// What bounds it: FP64 issue and the latency of its loads (about 90 bytes per
+// site and energy stored and read).  Storing both functions instead of
+// replaying 16-site segments from checkpoints (twice, in local arrays of 4 KB
+// a thread) halves the Riccati steps.
+template <int EMAX, int LG>
+__global__ void __launch_bounds__(128, 3) k_adjoint(const AdjArgs J) {
   typedef Cx<double> C;
   const SweepArgs<double> &A = J.S;
-  const int4 it = A.items[item];
-  const int a = it.x, x = it.y, lo = it.z, hi = it.w;
-  const int n1 = A.n1, ne = A.ne, len = hi - lo + 1;
-  const size_t nn1 = (size_t)n1 * n1, ni = (size_t)A.n_items;
-  const uint8_t *lab = A.labels + (size_t)a * nn1;
+  const int local = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (local >= J.n_tiles) return;  // whole warps
+  const int tile = J.tile0 + local;
+  const int lane = threadIdx.x & 31, sub = lane & 15;
+  const bool down = lane >= 16;
+  constexpr int G = 1 << LG, T = 16 >> LG;
+  const int g = sub & (G - 1);
+  const int item = tile * T + (sub >> LG);
+  const unsigned gmask = ((1u << G) - 1u) << (lane & ~(G - 1));
+  const int4 it = item < A.n_items ? A.items[item] : make_int4(0, 0, 0, -1);
+  const int a = it.x, x = it.y, lo = it.z, n_rows = it.w - it.z + 1;
+  const int n1 = A.n1, ne = A.ne;
+  const size_t nn1 = (size_t)n1 * n1;
   const double h = A.ang[a].hs;
-  const int e0 = g * A.ept;
-  int ecount = ne - e0;
-  if (ecount > A.ept) ecount = A.ept;
-  if (ecount < 0) ecount = 0;
-  double eim[EMAX], rr[EMAX];
+  const int e0 = g * EMAX, ecount = min(max(ne - e0, 0), EMAX);
+  double bh[EMAX], rr[EMAX];
 #pragma unroll
   for (int j = 0; j < EMAX; ++j) {
-    eim[j] = (j < ecount) ? A.e_im[e0 + j] : 1.0;
-    rr[j] = (j < ecount) ? s_res[e0 + j] : 0.0;
+    bh[j] = -0.5 - 0.5 * h * ((j < ecount) ? A.e_im[e0 + j] : 1.0);
+    rr[j] = (j < ecount) ? A.res[e0 + j] : 0.0;
   }
   const size_t ax = (size_t)a * n1 + x;
-  const int in_g = A.idx_in_g[ax], in_gt = A.idx_in_gt[ax];
-  const size_t slot = (size_t)(a - A.slot_base) * nn1;
-  const int nseg = (len + ADJ_K - 1) / ADJ_K;
-  auto ck = [&](Cx<double> *base, int seg, int j) -> Cx<double> & {
-    return base[((size_t)seg * ne + e0 + j) * ni + item];
-  };
+  const int in_base = (down ? A.idx_in_gt : A.idx_in_g)[ax];
+  const double *dist_in = down ? A.dist_in_gt : A.dist_in_g;
+  const C *bin = down ? A.bin_gt : A.bin_g;
+  const int l_entry = down ? 3 : 2;
 
-  // -------------------------------------------- primal passes, checkpoints --
+  // Records and both functions of row 0 of the column; rows are s_row apart.
+  const double4 *rec = (const double4 *)A.scratch2 + rec_index(A, LG, item, 0);
+  const ptrdiff_t s_row = (ptrdiff_t)ne * T;
+  C *gt_all = A.scratch + scratch_index(A, LG, item, 0, e0);
+  C *g_all = J.g_all + scratch_index(A, LG, item - J.tile0 * T, 0, e0);
+  C *own = down ? gt_all : g_all;
+  const C *other = down ? g_all : gt_all;
+  const int turns = __reduce_max_sync(0xffffffffu, n_rows);
+
   C coh[EMAX];
-  {  // gammaTilde down
-    int nin = 0;
-    double p0 = 0, p1 = 0, p2 = 0;
 #pragma unroll
-    for (int j = 0; j < EMAX; ++j) coh[j] = C{0, 0};
-    for (int r = len - 1; r >= 0; --r) {
-      const int seg = r / ADJ_K;
-      if (r == len - 1 || r % ADJ_K == ADJ_K - 1) {
+  for (int j = 0; j < EMAX; ++j) coh[j] = C{0, 0};
+  bool bounded = true;
+  int n_in = 0, pcode = SITE_GENERAL;
+  double p0 = 0, p1 = 0, p2 = 0;
+  // ------------------------------------------------------------- forward --
+  double4 nx{};
+  if (n_rows > 0) nx = rec[(ptrdiff_t)(down ? n_rows - 1 : 0) * T];
+  for (int k = 0; k < turns; ++k) {
+    __syncwarp();
+    if (k >= n_rows) continue;
+    const int r = down ? n_rows - 1 - k : k;
+    const double4 fr = nx;
+    if (k + 1 < n_rows) nx = rec[(ptrdiff_t)(down ? r - 1 : r + 1) * T];
+    const int code = site_code(fr.w), l = code & SITE_LABEL;
+    const double dre = down ? -fr.x : fr.x, dim = fr.y, es = fr.z;
+    if (code == 1 && pcode < SITE_GENERAL && bounded) {
+      const SiteConst<double> S = site_const<double>((dre + p0) * 0.5, (dim + p1) * 0.5, (es + p2) * 0.5, h);
+      const double s0h = S.s0h - 0.5 * S.sh * S.sh;
 #pragma unroll
-        for (int j = 0; j < EMAX; ++j)
-          if (j < ecount) ck(J.ck_gt, seg, j) = coh[j];
-        if (g == 0) J.ck_nin_gt[(size_t)seg * ni + item] = nin;
-      }
-      double f0, f1, f2;
-      fields_at(A, ni, item, r, f0, f1, f2);
-      const double dre = -f0, dim = f1, es = f2;
-      const uint8_t l = lab[(size_t)(lo + r) * n1 + x];
-      if (l == 0) {
+      for (int j = 0; j < EMAX; ++j) coh[j] = step_fast<double>(S, s0h, S.sh, bh[j], coh[j]);
+    } else {
+      const bool entry = l == l_entry;
+      const double st = entry ? dist_in[in_base + n_in] * h : h;
+      const double mre = entry ? dre : (dre + p0) * 0.5, mim = entry ? dim : (dim + p1) * 0.5,
+                   mes = entry ? es : (es + p2) * 0.5;
 #pragma unroll
-        for (int j = 0; j < EMAX; ++j) coh[j] = C{0, 0};
-      } else if (l == 3) {
-        const double st = A.dist_in_gt[in_gt + nin] * h;
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j)
-          if (j < ecount)
-            coh[j] = riccati_step<double>(dre, dim, es, eim[j], ((const C *)A.bin_gt)[(size_t)(in_gt + nin) * A.ne_stride + e0 + j], st);
-        ++nin;
-      } else {
-        const double mre = (dre + p0) * 0.5, mim = (dim + p1) * 0.5, mes = (es + p2) * 0.5;
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j)
-          if (j < ecount) coh[j] = riccati_step<double>(mre, mim, mes, eim[j], coh[j], h);
-      }
-      p0 = dre;
-      p1 = dim;
-      p2 = es;
-    }
-  }
-  {  // gamma up
-    int nin = 0;
-    double p0 = 0, p1 = 0, p2 = 0;
-#pragma unroll
-    for (int j = 0; j < EMAX; ++j) coh[j] = C{0, 0};
-    for (int r = 0; r < len; ++r) {
-      if (r % ADJ_K == 0) {
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j)
-          if (j < ecount) ck(J.ck_g, r / ADJ_K, j) = coh[j];
-        if (g == 0) J.ck_nin_g[(size_t)(r / ADJ_K) * ni + item] = nin;
-      }
-      double dre, dim, es;
-      fields_at(A, ni, item, r, dre, dim, es);
-      const uint8_t l = lab[(size_t)(lo + r) * n1 + x];
-      if (l == 0) {
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j) coh[j] = C{0, 0};
-      } else if (l == 2) {
-        const double st = A.dist_in_g[in_g + nin] * h;
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j)
-          if (j < ecount)
-            coh[j] = riccati_step<double>(dre, dim, es, eim[j], ((const C *)A.bin_g)[(size_t)(in_g + nin) * A.ne_stride + e0 + j], st);
-        ++nin;
-      } else {
-        const double mre = (dre + p0) * 0.5, mim = (dim + p1) * 0.5, mes = (es + p2) * 0.5;
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j)
-          if (j < ecount) coh[j] = riccati_step<double>(mre, mim, mes, eim[j], coh[j], h);
-      }
-      p0 = dre;
-      p1 = dim;
-      p2 = es;
-    }
-  }
-  __syncwarp(gmask);
-
-  // Segment replays: gamma (up) and gammaTilde (down) of rows [rb, rt].
-  C Lg[ADJ_K][EMAX], Lgt[ADJ_K][EMAX];
-  auto replay = [&](int seg, int rb, int rt) {
-    {  // gamma up from the segment's checkpoint
-      int nin = J.ck_nin_g[(size_t)seg * ni + item];
-      double p0 = 0, p1 = 0, p2 = 0;
-      if (rb > 0) fields_at(A, ni, item, rb - 1, p0, p1, p2);
-      C cc[EMAX];
-#pragma unroll
-      for (int j = 0; j < EMAX; ++j) cc[j] = (j < ecount) ? ck(J.ck_g, seg, j) : C{0, 0};
-      for (int r = rb; r <= rt; ++r) {
-        double dre, dim, es;
-        fields_at(A, ni, item, r, dre, dim, es);
-        const uint8_t l = lab[(size_t)(lo + r) * n1 + x];
-        if (l == 0) {
-#pragma unroll
-          for (int j = 0; j < EMAX; ++j) cc[j] = C{0, 0};
-        } else if (l == 2) {
-          const double st = A.dist_in_g[in_g + nin] * h;
-#pragma unroll
-          for (int j = 0; j < EMAX; ++j)
-            if (j < ecount)
-              cc[j] = riccati_step<double>(dre, dim, es, eim[j], ((const C *)A.bin_g)[(size_t)(in_g + nin) * A.ne_stride + e0 + j], st);
-          ++nin;
-        } else {
-          const double mre = (dre + p0) * 0.5, mim = (dim + p1) * 0.5, mes = (es + p2) * 0.5;
-#pragma unroll
-          for (int j = 0; j < EMAX; ++j)
-            if (j < ecount) cc[j] = riccati_step<double>(mre, mim, mes, eim[j], cc[j], h);
+      for (int j = 0; j < EMAX; ++j) {
+        C g0 = coh[j];
+        if (entry) {
+          g0 = j < ecount ? bin[(size_t)(in_base + n_in) * A.ne_stride + e0 + j] : C{0, 0};
+          if (!(g0.re * g0.re + g0.im * g0.im < 1.002)) bounded = false;
         }
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j) Lg[r - rb][j] = cc[j];
-        p0 = dre;
-        p1 = dim;
-        p2 = es;
+        coh[j] = l == 0 ? C{0, 0} : riccati_step<double>(mre, mim, mes, j < ecount ? A.e_im[e0 + j] : 1.0, g0, st);
       }
+      n_in += entry;
     }
-    {  // gammaTilde down from the segment's checkpoint
-      int nin = J.ck_nin_gt[(size_t)seg * ni + item];
-      double p0 = 0, p1 = 0, p2 = 0;
-      if (rt < len - 1) {
-        fields_at(A, ni, item, rt + 1, p0, p1, p2);
-        p0 = -p0;
+#pragma unroll
+    for (int j = 0; j < EMAX; ++j)
+      if (j < ecount) own[(ptrdiff_t)r * s_row + j * T] = coh[j];
+    pcode = code;
+    p0 = dre;
+    p1 = dim;
+    p2 = es;
+  }
+  __syncwarp();
+
+  // ------------------------------------------------------------- reverse --
+  // The row visited by step k, from the column's end of this function back:
+  // its order-parameter and shift sensitivities collect the step at the row
+  // (half, midpoint) and the step visited before (the other half, in pend).
+  const size_t site0 = (size_t)(a - A.slot_base) * nn1 + (size_t)lo * n1 + x;
+  const int below = n_rows >> 1, odd = n_rows & 1;
+  const int first = down ? below : n_rows - below;  // rows this half-warp reaches before the other one
+  const int delay = down ? odd : 0;
+  const int turns2 = __reduce_max_sync(0xffffffffu, n_rows + odd);
+  C lam[EMAX];
+#pragma unroll
+  for (int j = 0; j < EMAX; ++j) lam[j] = C{0, 0};
+  C pend{0, 0};
+  double pend_e = 0.0;
+  // Inputs one row ahead: the record and seed, the other function, and this
+  // function's value before the row's step (the next row visited).
+  C o_nx[EMAX], in_nx[EMAX], me[EMAX];
+  double4 r_nx{};
+  double2 sd_nx{};
+  auto fetch = [&](int k) {  // inputs of step k (coh of the same row is me)
+    const int r = down ? k : n_rows - 1 - k;
+    const ptrdiff_t before = (ptrdiff_t)(down ? r + 1 : r - 1);  // the row stepped from
+    const bool has = k + 1 < n_rows;
+    sd_nx = J.seed[site0 + (size_t)r * n1];
+    if (has) r_nx = rec[before * T];
+#pragma unroll
+    for (int j = 0; j < EMAX; ++j)
+      if (j < ecount) {
+        o_nx[j] = other[(ptrdiff_t)r * s_row + j * T];
+        in_nx[j] = has ? own[before * s_row + j * T] : C{0, 0};
       }
-      C cc[EMAX];
+  };
 #pragma unroll
-      for (int j = 0; j < EMAX; ++j) cc[j] = (j < ecount) ? ck(J.ck_gt, seg, j) : C{0, 0};
-      for (int r = rt; r >= rb; --r) {
-        double f0, f1, f2;
-        fields_at(A, ni, item, r, f0, f1, f2);
-        const double dre = -f0, dim = f1, es = f2;
-        const uint8_t l = lab[(size_t)(lo + r) * n1 + x];
-        if (l == 0) {
+  for (int j = 0; j < EMAX; ++j) o_nx[j] = in_nx[j] = me[j] = C{0, 0};
+  double4 fr{};
+  if (n_rows > 0) {
+    const int r = down ? 0 : n_rows - 1;
+    fr = rec[(ptrdiff_t)r * T];
 #pragma unroll
-          for (int j = 0; j < EMAX; ++j) cc[j] = C{0, 0};
-        } else if (l == 3) {
-          const double st = A.dist_in_gt[in_gt + nin] * h;
+    for (int j = 0; j < EMAX; ++j)
+      if (j < ecount) me[j] = own[(ptrdiff_t)r * s_row + j * T];
+    fetch(0);
+  }
+  for (int turn = 0; turn < turns2; ++turn) {
+    __syncwarp();
+    const int k = turn - delay;
+    if (k < 0 || k >= n_rows) continue;
+    const int r = down ? k : n_rows - 1 - k;
+    C ot[EMAX], gin[EMAX];
 #pragma unroll
-          for (int j = 0; j < EMAX; ++j)
-            if (j < ecount)
-              cc[j] = riccati_step<double>(dre, dim, es, eim[j], ((const C *)A.bin_gt)[(size_t)(in_gt + nin) * A.ne_stride + e0 + j], st);
-          ++nin;
-        } else {
-          const double mre = (dre + p0) * 0.5, mim = (dim + p1) * 0.5, mes = (es + p2) * 0.5;
+    for (int j = 0; j < EMAX; ++j) {
+      ot[j] = o_nx[j];
+      gin[j] = in_nx[j];
+    }
+    const double4 frp = r_nx;  // the record the step comes from
+    const double2 sd = sd_nx;
+    if (k + 1 < n_rows) fetch(k + 1);
+    const int code = site_code(fr.w), l = code & SITE_LABEL, bcode = site_code(frp.w);
+    const double dre = down ? -fr.x : fr.x, dim = fr.y, es = fr.z;
+    C ownD{0, 0}, nextD{0, 0};
+    double own_e = 0.0, next_e = 0.0;
+    if (l != 0) {
 #pragma unroll
-          for (int j = 0; j < EMAX; ++j)
-            if (j < ecount) cc[j] = riccati_step<double>(mre, mim, mes, eim[j], cc[j], h);
+      for (int j = 0; j < EMAX; ++j) {
+        // Re I = -sum r [Im(conj(D) g - D gt)]: with the sign of this
+        // function's order parameter, G += s r (Im D, -Re D); the direct
+        // dependence on D once, by gamma: s r i (g + conj(gt)).
+        const double sr = sd.x * rr[j];
+        lam[j].re += sr * dim;
+        lam[j].im -= sr * dre;
+        if (!down) {
+          ownD.re -= sr * (me[j].im - ot[j].im);
+          ownD.im += sr * (me[j].re + ot[j].re);
         }
-#pragma unroll
-        for (int j = 0; j < EMAX; ++j) Lgt[r - rb][j] = cc[j];
-        p0 = dre;
-        p1 = dim;
-        p2 = es;
+        // Re g = Im q, q = (1 - p) / (1 + p), p = g gt: G_p = conj(dq/dp) (0, s r).
+        const C p = cmul(me[j], ot[j]);
+        const double nr = 1.0 + p.re, inv = rcp_pos(nr * nr + p.im * p.im);
+        const C ip{nr * inv, -p.im * inv}, i2 = cmul(ip, ip);
+        const double s2 = -2.0 * sd.y * rr[j];
+        const C Gp{s2 * i2.im, s2 * i2.re};
+        lam[j].re += ot[j].re * Gp.re + ot[j].im * Gp.im;
+        lam[j].im += ot[j].re * Gp.im - ot[j].im * Gp.re;
       }
-    }
-  };
-
-  // Local seeds of one site: the sensitivity of the loss to gamma (or
-  // gammaTilde) through Re I and Re g at that site.
-  //   Re I = -sum r [Im(conj(D) g) - Im(D gt)],  Re g = Im((1 - g gt)/(1 + g gt)).
-  auto gp_of = [&](C gm, C gtl, double sg, double r) -> C {
-    const C p = cmul(gm, gtl);
-    const C onep{1.0 + p.re, p.im};
-    const C inv = cinv(onep);
-    const C dq = cscale(cmul(inv, inv), -2.0);          // dQ/dp
-    const C GQ{0.0, sg * r};                             // Re g = Im Q
-    return cmul(cconj(dq), GQ);                          // G_p
-  };
-
-  // ------------------------------------------ adjoint of gamma, top-down --
-  // Row r's order-parameter and shift sensitivities collect the step at r
-  // (half, midpoint) and the step at r + 1 (the other half, carried in pend).
-  {
-    C lam[EMAX];
+      if (l == l_entry) {
+        --n_in;
+        const double st = dist_in[in_base + n_in] * h;
 #pragma unroll
-    for (int j = 0; j < EMAX; ++j) lam[j] = C{0, 0};
-    C pendD{0, 0};
-    double pendE = 0.0;
-    for (int seg = nseg - 1; seg >= 0; --seg) {
-      const int rb = seg * ADJ_K, rt = min(rb + ADJ_K, len) - 1;
-      replay(seg, rb, rt);
-      for (int r = rt; r >= rb; --r) {
-        double dre, dim, es;
-        fields_at(A, ni, item, r, dre, dim, es);
-        const uint8_t l = lab[(size_t)(lo + r) * n1 + x];
-        const size_t site = (size_t)(lo + r) * n1 + x;
-        C ownD{0, 0};
-        double ownE = 0.0;
-        C pendNext{0, 0};
-        double pendNextE = 0.0;
-        if (l != 0) {
-          const double2 sd = J.seed[slot + site];
-          const C D{dre, dim};
+        for (int j = 0; j < EMAX; ++j)
+          if (j < ecount) {
+            C gg0, gD;
+            double ge;
+            riccati_step_adj(dre, dim, es, A.e_im[e0 + j], bin[(size_t)(in_base + n_in) * A.ne_stride + e0 + j], st,
+                             lam[j], gg0, gD, ge);
+            ownD = cadd(ownD, gD);
+            own_e += ge;
+          }
+#pragma unroll
+        for (int j = 0; j < EMAX; ++j) lam[j] = C{0, 0};
+      } else {
+        const bool has = k + 1 < n_rows;
+        const double q0 = has ? (down ? -frp.x : frp.x) : 0.0, q1 = has ? frp.y : 0.0, q2 = has ? frp.z : 0.0;
+        const double mre = (dre + q0) * 0.5, mim = (dim + q1) * 0.5, mes = (es + q2) * 0.5;
+        C nD{0, 0};
+        double nE = 0.0;
+        if (code == 1 && has && bcode < SITE_GENERAL && bounded) {
+          const SiteConst<double> S = site_const<double>(mre, mim, mes, h);
+          const double s0h = S.s0h - 0.5 * S.sh * S.sh;
+#pragma unroll
+          for (int j = 0; j < EMAX; ++j) lam[j] = step_fast_adj(S, s0h, S.sh, bh[j], h, gin[j], lam[j], nD, nE);
+        } else {
 #pragma unroll
           for (int j = 0; j < EMAX; ++j)
             if (j < ecount) {
-              const C gm = Lg[r - rb][j], gtl = Lgt[r - rb][j];
-              // Re I: G_g = -sI r i D ; direct G_D = sI r i (g + conj(gt))
-              const C iD{-D.im, D.re};
-              lam[j] = cadd(lam[j], cscale(iD, -sd.x * rr[j]));
-              const C s1 = cadd(gm, cconj(gtl));
-              ownD = cadd(ownD, cscale(C{-s1.im, s1.re}, sd.x * rr[j]));
-              // Re g: G_g = conj(gt) G_p
-              lam[j] = cadd(lam[j], cmul(cconj(gtl), gp_of(gm, gtl, sd.y, rr[j])));
+              C gg0, gD;
+              double ge;
+              riccati_step_adj(mre, mim, mes, A.e_im[e0 + j], gin[j], h, lam[j], gg0, gD, ge);
+              nD = cadd(nD, gD);
+              nE += ge;
+              lam[j] = gg0;
             }
-          if (l == 2) {
-            int nin = J.ck_nin_g[(size_t)seg * ni + item];
-            for (int r2 = rb; r2 < r; ++r2) nin += lab[(size_t)(lo + r2) * n1 + x] == 2;
-            const double st = A.dist_in_g[in_g + nin] * h;
-#pragma unroll
-            for (int j = 0; j < EMAX; ++j)
-              if (j < ecount) {
-                C gg0, gD;
-                double ge;
-                riccati_step_adj(dre, dim, es, eim[j], ((const C *)A.bin_g)[(size_t)(in_g + nin) * A.ne_stride + e0 + j], st,
-                                 lam[j], gg0, gD, ge);
-                ownD = cadd(ownD, gD);
-                ownE += ge;
-                lam[j] = C{0, 0};
-              }
-          } else {
-            double p0 = 0, p1 = 0, p2 = 0;
-            if (r > 0) fields_at(A, ni, item, r - 1, p0, p1, p2);
-            const double mre = (dre + p0) * 0.5, mim = (dim + p1) * 0.5, mes = (es + p2) * 0.5;
-            C nD{0, 0};
-            double nE = 0.0;
-#pragma unroll
-            for (int j = 0; j < EMAX; ++j)
-              if (j < ecount) {
-                const C gin = (r - 1 >= rb) ? Lg[r - 1 - rb][j] : ck(J.ck_g, seg, j);
-                C gg0, gD;
-                double ge;
-                riccati_step_adj(mre, mim, mes, eim[j], gin, h, lam[j], gg0, gD, ge);
-                nD = cadd(nD, gD);
-                nE += ge;
-                lam[j] = gg0;
-              }
-            ownD = cadd(ownD, cscale(nD, 0.5));
-            ownE += 0.5 * nE;
-            if (r > 0) {
-              pendNext = cscale(nD, 0.5);
-              pendNextE = 0.5 * nE;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < EMAX; ++j) lam[j] = C{0, 0};
         }
-        ownD = cadd(ownD, pendD);
-        ownE += pendE;
-        pendD = pendNext;
-        pendE = pendNextE;
-        if (A.groups > 1) {
-          group_sum(ownD.re, A.groups, gmask);
-          group_sum(ownD.im, A.groups, gmask);
-          group_sum(ownE, A.groups, gmask);
-        }
-        if (g == 0) {
-          if (A.accumulate) {  // a later energy pass adds to the earlier ones
-            const double2 o = J.grad_d[slot + site];
-            J.grad_d[slot + site] = make_double2(o.x + ownD.re, o.y + ownD.im);
-            J.grad_e[slot + site] += ownE;
-          } else {
-            J.grad_d[slot + site] = make_double2(ownD.re, ownD.im);
-            J.grad_e[slot + site] = ownE;
-          }
+        ownD = cadd(ownD, cscale(nD, 0.5));
+        own_e += 0.5 * nE;
+        if (has) {
+          nextD = cscale(nD, 0.5);
+          next_e = 0.5 * nE;
         }
       }
+    } else {
+#pragma unroll
+      for (int j = 0; j < EMAX; ++j) lam[j] = C{0, 0};
     }
-  }
-  __syncwarp(gmask);
-
-  // ---------------------------------------- adjoint of gammaTilde, bottom-up --
-  {
-    C lam[EMAX];
-#pragma unroll
-    for (int j = 0; j < EMAX; ++j) lam[j] = C{0, 0};
-    C pendD{0, 0};
-    double pendE = 0.0;
-    for (int seg = 0; seg < nseg; ++seg) {
-      const int rb = seg * ADJ_K, rt = min(rb + ADJ_K, len) - 1;
-      replay(seg, rb, rt);
-      for (int r = rb; r <= rt; ++r) {
-        double f0, f1, f2;
-        fields_at(A, ni, item, r, f0, f1, f2);
-        const double dre = -f0, dim = f1, es = f2;  // gammaTilde's order parameter -conj(Delta)
-        const uint8_t l = lab[(size_t)(lo + r) * n1 + x];
-        const size_t site = (size_t)(lo + r) * n1 + x;
-        C ownT{0, 0};  // sensitivity to -conj(Delta) at this row
-        double ownE = 0.0;
-        C pendNext{0, 0};
-        double pendNextE = 0.0;
-        if (l != 0) {
-          const double2 sd = J.seed[slot + site];
-          const C D{f0, f1};
-#pragma unroll
-          for (int j = 0; j < EMAX; ++j)
-            if (j < ecount) {
-              const C gm = Lg[r - rb][j], gtl = Lgt[r - rb][j];
-              // Re I: G_gt = sI r i conj(D)
-              const C icD{D.im, D.re};
-              lam[j] = cadd(lam[j], cscale(icD, sd.x * rr[j]));
-              // Re g: G_gt = conj(g) G_p
-              lam[j] = cadd(lam[j], cmul(cconj(gm), gp_of(gm, gtl, sd.y, rr[j])));
-            }
-          if (l == 3) {
-            int nin = J.ck_nin_gt[(size_t)seg * ni + item];
-            for (int rr2 = rt; rr2 > r; --rr2) nin += lab[(size_t)(lo + rr2) * n1 + x] == 3;
-            const double st = A.dist_in_gt[in_gt + nin] * h;
-#pragma unroll
-            for (int j = 0; j < EMAX; ++j)
-              if (j < ecount) {
-                C gg0, gD;
-                double ge;
-                riccati_step_adj(dre, dim, es, eim[j], ((const C *)A.bin_gt)[(size_t)(in_gt + nin) * A.ne_stride + e0 + j], st,
-                                 lam[j], gg0, gD, ge);
-                ownT = cadd(ownT, gD);
-                ownE += ge;
-                lam[j] = C{0, 0};
-              }
-          } else {
-            double p0 = 0, p1 = 0, p2 = 0;
-            if (r < len - 1) {
-              fields_at(A, ni, item, r + 1, p0, p1, p2);
-              p0 = -p0;
-            }
-            const double mre = (dre + p0) * 0.5, mim = (dim + p1) * 0.5, mes = (es + p2) * 0.5;
-            C nD{0, 0};
-            double nE = 0.0;
-#pragma unroll
-            for (int j = 0; j < EMAX; ++j)
-              if (j < ecount) {
-                const C gin = (r + 1 <= rt) ? Lgt[r + 1 - rb][j] : ck(J.ck_gt, seg, j);
-                C gg0, gD;
-                double ge;
-                riccati_step_adj(mre, mim, mes, eim[j], gin, h, lam[j], gg0, gD, ge);
-                nD = cadd(nD, gD);
-                nE += ge;
-                lam[j] = gg0;
-              }
-            ownT = cadd(ownT, cscale(nD, 0.5));
-            ownE += 0.5 * nE;
-            if (r < len - 1) {
-              pendNext = cscale(nD, 0.5);
-              pendNextE = 0.5 * nE;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < EMAX; ++j) lam[j] = C{0, 0};
-        }
-        // -conj(Delta) -> Delta: G_Delta = -conj(G)
-        C ownD{-ownT.re, ownT.im};
-        ownD = cadd(ownD, pendD);
-        ownE += pendE;
-        pendD = C{-pendNext.re, pendNext.im};
-        pendE = pendNextE;
-        if (A.groups > 1) {
-          group_sum(ownD.re, A.groups, gmask);
-          group_sum(ownD.im, A.groups, gmask);
-          group_sum(ownE, A.groups, gmask);
-        }
-        if (g == 0) {
-          const double2 o = J.grad_d[slot + site];
-          J.grad_d[slot + site] = make_double2(o.x + ownD.re, o.y + ownD.im);
-          J.grad_e[slot + site] += ownE;
-        }
+    ownD = cadd(ownD, pend);
+    own_e += pend_e;
+    pend = nextD;
+    pend_e = next_e;
+    // gammaTilde's order parameter is -conj(Delta): G_Delta = -conj(G).
+    double v[4] = {down ? -ownD.re : ownD.re, ownD.im, own_e, 0.0};
+    group_sum4_scatter(v, g, LG, gmask);
+    const size_t site = site0 + (size_t)r * n1;
+    const bool add = A.accumulate || k >= first;  // earlier energy passes, the other half-warp
+    double *gd = (double *)(J.grad_d + site), *gv = J.grad_e + site;
+    if constexpr (LG == 0) {
+      gd[0] = v[0] + (add ? gd[0] : 0.0);
+      gd[1] = v[1] + (add ? gd[1] : 0.0);
+      *gv = v[2] + (add ? *gv : 0.0);
+    } else if constexpr (LG == 1) {
+      if (g == 0) {
+        gd[0] = v[0] + (add ? gd[0] : 0.0);
+        gd[1] = v[1] + (add ? gd[1] : 0.0);
+      } else {
+        *gv = v[0] + (add ? *gv : 0.0);
+      }
+    } else {
+      const int which = g >> (LG - 2);
+      if ((g & ((1 << (LG - 2)) - 1)) == 0 && which < 3) {
+        double *d = which == 2 ? gv : gd + which;
+        *d = v[0] + (add ? *d : 0.0);
       }
     }
+    fr = frp;
+#pragma unroll
+    for (int j = 0; j < EMAX; ++j) me[j] = gin[j];
   }
-}
-
-template <int EMAX>
-__global__ void __launch_bounds__(128) k_adjoint(const AdjArgs J) {
-  __shared__ double s_res[64];
-  for (int e = threadIdx.x; e < J.S.ne && e < 64; e += blockDim.x) s_res[e] = J.S.res[e];
-  __syncthreads();
-  const SweepArgs<double> &A = J.S;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int item = tid >> A.log_groups;
-  const int g = tid & (A.groups - 1);
-  const int lane = threadIdx.x & 31;
-  const unsigned gmask = ((A.groups == 32) ? 0xffffffffu : ((1u << A.groups) - 1u)) << (lane & ~(A.groups - 1));
-  if (item >= A.n_items) return;
-  adjoint_column<EMAX>(J, s_res, item, g, gmask);
 }
 
 // Seeds on the frame lattice of the angles [a_begin, a_end): the transpose of
@@ -685,27 +572,55 @@ void evaluate_once(sc_ctx *c) {
 }
 
 struct AdjBuffers {
-  DevArray<double> ck, grad_e, g_dext, g_avec, g_b, alpha, beta, coef;
-  DevArray<int> ck_nin;
+  DevArray<double> g_all, grad_e, g_dext, g_avec, g_b, alpha, beta, coef;
 };
 void AdjDeleter::operator()(AdjBuffers *p) const { delete p; }
+
+// One launch over the tiles [t0, t0 + n) with four energies in flight per
+// thread pair: EMAX energies per thread, LG threads per column and function.
+template <int EMAX>
+void launch_adjoint(sc_ctx *c, const AdjArgs &J) {
+  const unsigned blocks = grid1((size_t)J.n_tiles * 32, 128);
+  switch (J.S.log_groups) {
+    case 0: k_adjoint<EMAX, 0><<<blocks, 128, 0, c->stream>>>(J); break;
+    case 1: k_adjoint<EMAX, 1><<<blocks, 128, 0, c->stream>>>(J); break;
+    case 2: k_adjoint<EMAX, 2><<<blocks, 128, 0, c->stream>>>(J); break;
+    case 3: k_adjoint<EMAX, 3><<<blocks, 128, 0, c->stream>>>(J); break;
+    default: k_adjoint<EMAX, 4><<<blocks, 128, 0, c->stream>>>(J); break;
+  }
+  check_launch(c);
+}
 
 void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_host, double *g_delta,
                  double *g_a, double *g_b) {
   const HostSetup &S = c->S;
   const size_t nn = c->nn0();
   const size_t nn1 = (size_t)S.n1 * S.n1;
-  // Per-chunk buffers.
-  size_t ck_n = 0, nin_n = 0, slots = 0;
+  // The adjoint's own mapping: two energies per thread, at most 16 threads per
+  // column and function (energy passes above 32); a tile is its own 16 / G
+  // columns.
+  constexpr int ADJ_EMAX = 2;
+  const int pass = std::min(c->e_pass, ADJ_EMAX * 16);
+  int lg = 0;
+  while ((ADJ_EMAX << lg) < pass) ++lg;
+  const int T = 16 >> lg;
+  size_t slots = 0, tile_bytes = 0, tiles = 0;
   for (const Chunk &ch : c->chunks) {
     const size_t ni = (size_t)(ch.item_end - ch.item_begin);
-    const size_t nseg = (size_t)(ch.kmax + ADJ_K - 1) / ADJ_K;
-    ck_n = std::max(ck_n, 2 * nseg * S.ne * ni);
-    nin_n = std::max(nin_n, 2 * nseg * ni);
     slots = std::max(slots, (size_t)(ch.a_end - ch.a_begin));
+    tile_bytes = std::max(tile_bytes, (size_t)ch.kmax * pass * T * sizeof(Cx<double>));
+    tiles = std::max(tiles, (ni + T - 1) / T);
   }
-  if (B.ck.n < 2 * ck_n) B.ck.alloc(2 * ck_n);  // complex: 2 doubles each
-  if (B.ck_nin.n < nin_n) B.ck_nin.alloc(nin_n);
+  // gamma of as many tiles as fit 40% of the free memory (all of them unless
+  // the sweep's own scratch already takes most of the device), at least one.
+  if (!B.g_all.n && tiles) {
+    size_t free_b = 0, total_b = 0;
+    CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+    double budget = 0.4 * (double)free_b;
+    if (const char *env = std::getenv("SCB_SCRATCH_MB")) budget = std::min(budget, std::atof(env) * 1048576.0);
+    const size_t fit = std::max<size_t>(1, (size_t)budget / tile_bytes);
+    B.g_all.alloc(std::min(tiles, fit) * tile_bytes / sizeof(double));
+  }
   if (B.grad_e.n < slots * nn1) B.grad_e.alloc(slots * nn1);
   B.g_dext.alloc((size_t)2 * S.nc * nn);
   B.g_avec.alloc(2 * nn);
@@ -727,6 +642,8 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_ho
     const int nslots = ch.a_end - ch.a_begin;
     SweepArgs<double> A = sweep_args<double>(c, &ch, 0);
     if (!A.n_items) continue;
+    A.log_groups = lg;  // the records in the adjoint's tiles
+    A.groups = 1 << lg;
     launch_frame_fields<double>(c, ch, A);
     // The frame-record buffer (two double2 per site and slot) holds both.
     double2 *seed = (double2 *)c->w_fr, *grad_d = seed + (size_t)nslots * nn1;
@@ -747,37 +664,27 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_ho
     }
     AdjArgs J{};
     J.S = A;
-    const size_t ni = (size_t)A.n_items;
-    const size_t nseg = (size_t)(ch.kmax + ADJ_K - 1) / ADJ_K;
-    J.ck_gt = (Cx<double> *)B.ck.p;
-    J.ck_g = J.ck_gt + nseg * S.ne * ni;
-    J.ck_nin_gt = B.ck_nin.p;
-    J.ck_nin_g = B.ck_nin.p + nseg * ni;
+    J.g_all = (Cx<double> *)B.g_all.p;
     J.seed = seed;
     J.grad_d = grad_d;
     J.grad_e = B.grad_e.p;
-    const size_t threads = ni * c->groups;
-    if (c->ept <= 4 && c->e_pass >= S.ne) {
-      k_adjoint<4><<<grid1(threads, 128), 128, 0, c->stream>>>(J);
-      check_launch(c);
-    } else {
-      // Energy passes of four energies per thread, each from its own slice
-      // of the boundary values, adding into the gradients of the earlier ones.
-      const int pass = 4 * c->groups;
-      for (int e = 0; e < S.ne; e += pass) {
-        AdjArgs P = J;
-        P.S.ne = std::min(pass, S.ne - e);
-        P.S.ept = 4;
-        P.S.accumulate = e > 0;
-        P.S.e_re += e;
-        P.S.e_im += e;
-        P.S.res += e;
-        P.S.bin_g += e;
-        P.S.bin_gt += e;
-        P.S.bout_g += e;
-        P.S.bout_gt += e;
-        k_adjoint<4><<<grid1(threads, 128), 128, 0, c->stream>>>(P);
-        check_launch(c);
+    const size_t ch_tiles = ((size_t)A.n_items + T - 1) / T;
+    for (int e = 0; e < S.ne; e += pass) {
+      // Energies [e, e + pass) of every column from their own boundary
+      // values, adding into the gradients of the earlier passes.
+      AdjArgs P = J;
+      P.S.ne = std::min(pass, S.ne - e);
+      P.S.accumulate = e > 0;
+      P.S.e_im += e;
+      P.S.res += e;
+      P.S.bin_g += e;
+      P.S.bin_gt += e;
+      const size_t per = (size_t)ch.kmax * P.S.ne * T * sizeof(Cx<double>);
+      const size_t most = std::max<size_t>(1, B.g_all.n * sizeof(double) / per);
+      for (size_t t0 = 0; t0 < ch_tiles; t0 += most) {
+        P.tile0 = (int)t0;
+        P.n_tiles = (int)std::min(most, ch_tiles - t0);
+        launch_adjoint<ADJ_EMAX>(c, P);
       }
     }
     dim3 gridf(grid1(nn1, 256), nslots);
