@@ -90,6 +90,9 @@ int sc_burn_in(sc_ctx *ctx, int n, double *residual, int *converged);
  * [2][N0][N0] (internal units).  Any pointer may be NULL. */
 int sc_get_results(sc_ctx *ctx, double *delta_new, double *j, double *a_new);
 
+/* The same into device buffers of the context's GPU. */
+int sc_get_results_device(sc_ctx *ctx, double *d_delta_new, double *d_j, double *d_a_new);
+
 /* out[0..10]: free energy, free energy per area, magnetic free energy,
  * magnetic free energy per area, residuals of order parameter, current, free
  * energy, vector potential and boundary, total residual, grain lattice sites
@@ -133,6 +136,12 @@ int sc_evaluate(sc_ctx *ctx, double *free_energy);
  * *g_b = dL/dB_ext. */
 int sc_adjoint(sc_ctx *ctx, double w_omega, const double *beta_j, double *g_delta, double *g_a,
                double *g_b);
+
+/* The same with beta_j and the gradients in device buffers of the context's
+ * GPU (any of them may be NULL).  The inputs are read on the context's stream;
+ * the gradients are complete on return. */
+int sc_adjoint_device(sc_ctx *ctx, double w_omega, const double *d_beta_j, double *d_g_delta, double *d_g_a,
+                      double *d_g_b);
 
 /* ---- probes used by the parity tests ------------------------------------ */
 

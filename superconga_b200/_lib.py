@@ -37,6 +37,8 @@ SIGNATURES = {
     "sc_get_boundary": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, _c_double_p]),
     "sc_set_boundary": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, _c_double_p]),
     "sc_boundary_initial": (ctypes.c_int, [ctypes.c_void_p]),
+    "sc_get_results_device": (ctypes.c_int, [ctypes.c_void_p] + [ctypes.c_void_p] * 3),
+    "sc_adjoint_device": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_double] + [ctypes.c_void_p] * 4),
     "sc_angle_greens": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, _c_double_p, _c_double_p, _c_double_p]),
     "sc_poisson": (ctypes.c_int, [ctypes.c_void_p, _c_double_p, _c_double_p]),
     "sc_launch_count": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_longlong)]),

@@ -20,41 +20,68 @@ import numpy as np
 import torch
 
 
-def _planar(delta: torch.Tensor) -> np.ndarray:
-    d = delta.detach().to("cpu", torch.complex128).numpy()
-    return np.ascontiguousarray(np.stack([d.real, d.imag], axis=1))
+def _on_gpu(t: torch.Tensor, dtype, size: int, what: str) -> torch.Tensor:
+    """``t`` on the engine's GPU (the current device, where its kernels run)."""
+    if t.numel() != size:
+        raise ValueError(f"FreeEnergy: {what} has {t.numel()} values, the context takes {size}")
+    return t.detach().to(torch.device("cuda", torch.cuda.current_device()), dtype)
+
+
+def _planar(delta: torch.Tensor, ctx) -> torch.Tensor:
+    """[Nc][N0][N0] complex as the engine's [Nc][2][N0][N0], a tensor of its own."""
+    d = ctx.dims
+    z = _on_gpu(delta, torch.complex128, d.n_comp * d.n0 * d.n0, "delta").resolve_conj()
+    z = z.reshape(d.n_comp, d.n0, d.n0)
+    return torch.stack([z.real, z.imag], dim=1).contiguous()
 
 
 class FreeEnergy(torch.autograd.Function):
+    """State and gradients stay on the GPU.  The engine works on a stream of
+    its own: this stream is waited for before the engine reads a tensor, and
+    every engine call here that hands values back is complete when it returns."""
+
     @staticmethod
     def forward(fctx, delta, a, b_ext, ctx, w_omega=1.0, beta_j=None):
-        d = _planar(delta)
-        av = np.ascontiguousarray(a.detach().to("cpu", torch.float64).numpy())
+        d = _planar(delta, ctx)
+        n0 = ctx.dims.n0
+        av = _on_gpu(a, torch.float64, 2 * n0 * n0, "a").resolve_neg().reshape(2, n0, n0).clone(
+            memory_format=torch.contiguous_format)
         b = float(b_ext.detach().cpu())
-        ctx.set_state(d, av)
+        beta = None if beta_j is None else torch.from_numpy(
+            np.array(beta_j, np.float64)).to(d.device)
+        torch.cuda.current_stream().synchronize()
+        ctx.set_state_device(d.data_ptr(), av.data_ptr())
         ctx.set_external_field(b)
         fe = ctx.evaluate()
-        loss = w_omega * fe
-        if beta_j is not None:
-            _, j, _ = ctx.results()
-            loss += float(np.sum(np.asarray(beta_j) * j))
+        if beta is None:
+            loss = torch.tensor(w_omega * fe, dtype=torch.float64, device=delta.device)
+        else:
+            j = torch.empty(2, n0, n0, dtype=torch.float64, device=d.device)
+            ctx.results_device(j_ptr=j.data_ptr())
+            loss = (torch.sum(beta * j) + w_omega * fe).to(delta.device)
         fctx.engine = ctx
-        fctx.args = (d, av, b, w_omega, beta_j)
+        fctx.args = (d, av, b, w_omega, beta)
         fctx.devices = (delta.device, a.device, b_ext.device)
-        return torch.tensor(loss, dtype=torch.float64, device=delta.device)
+        return loss
 
     @staticmethod
     def backward(fctx, grad_out):
         ctx = fctx.engine
-        d, av, b, w_omega, beta_j = fctx.args
-        ctx.set_state(d, av)
+        d, av, b, w_omega, beta = fctx.args
+        n0 = ctx.dims.n0
+        if beta is not None:
+            beta = beta.reshape(2, n0, n0)
+        gd, ga = torch.empty_like(d), torch.empty_like(av)
+        gb = torch.empty((), dtype=torch.float64, device=d.device)
+        torch.cuda.current_stream().synchronize()
+        ctx.set_state_device(d.data_ptr(), av.data_ptr())
         ctx.set_external_field(b)
-        gd, ga, gb = ctx.adjoint(w_omega, beta_j)
-        g = float(grad_out.detach().cpu())
-        gdel = torch.from_numpy(gd[:, 0] + 1j * gd[:, 1]).to(fctx.devices[0]) * g
-        ga_t = torch.from_numpy(ga).to(fctx.devices[1]) * g
-        gb_t = torch.tensor(gb * g, dtype=torch.float64, device=fctx.devices[2])
-        return gdel, ga_t, gb_t, None, None, None
+        ctx.adjoint_device(w_omega, None if beta is None else beta.data_ptr(), gd.data_ptr(), ga.data_ptr(),
+                           gb.data_ptr())
+        g = grad_out.detach().to(d.device, torch.float64)
+        gdel = torch.complex(gd[:, 0], gd[:, 1]) * g
+        return (gdel.to(fctx.devices[0]), (ga * g).to(fctx.devices[1]), (gb * g).to(fctx.devices[2]), None, None,
+                None)
 
 
 def edge_current_weights(domain: np.ndarray, h: float, width: float) -> np.ndarray:

@@ -524,18 +524,22 @@ __global__ void k_adj_rext_t(int n_fields, int nn, int n_sites, const int *__res
   for (int i = b; i < e; ++i) atomicAdd(gf + src[i], v * inv);
 }
 
+struct AdjCoef {
+  double v[MAX_COMP];
+};
+
 // Explicit terms of the free energy: sum_c |Delta_c|^2 (ln(T/Tc_c) + T sum r/e)
 // inside the grain (times h^2 w_omega), and the mask of the order parameter
 // (zero outside the grain, OrderParameter.h:180-199).
 __global__ void k_adj_explicit(int n0, int nc, const uint8_t *__restrict__ dom, const double *__restrict__ x,
-                               const double *__restrict__ coef, double *g) {
+                               AdjCoef coef, double *g) {
   const size_t nn = (size_t)n0 * n0;
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= nn) return;
   for (int c = 0; c < nc; ++c)
     for (int p = 0; p < 2; ++p) {
       const size_t k = (size_t)(2 * c + p) * nn + i;
-      g[k] = dom[i] ? g[k] + 2.0 * coef[c] * x[k] : 0.0;
+      g[k] = dom[i] ? g[k] + 2.0 * coef.v[c] * x[k] : 0.0;
     }
 }
 
@@ -571,8 +575,20 @@ void evaluate_once(sc_ctx *c) {
   launch_finalize(c, delta, avec);
 }
 
+// Reference-grid weights of Re I (free energy) and of the current, zero
+// outside the grain; beta_j null: no current term.
+__global__ void k_adj_weights(size_t nn, const uint8_t *__restrict__ dom, double w_fe, double w_j,
+                              const double *__restrict__ beta_j, double *alpha, double *beta) {
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (i >= nn) return;
+  const bool in = dom[i] != 0;
+  alpha[i] = in ? w_fe : 0.0;
+  beta[i] = in && beta_j ? beta_j[i] * w_j : 0.0;
+  beta[nn + i] = in && beta_j ? beta_j[nn + i] * w_j : 0.0;
+}
+
 struct AdjBuffers {
-  DevArray<double> g_all, grad_e, g_dext, g_avec, g_b, alpha, beta, coef;
+  DevArray<double> g_all, grad_e, g_dext, g_avec, g_b, alpha, beta, beta_in;
 };
 void AdjDeleter::operator()(AdjBuffers *p) const { delete p; }
 
@@ -591,11 +607,15 @@ void launch_adjoint(sc_ctx *c, const AdjArgs &J) {
   check_launch(c);
 }
 
-void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_host, double *g_delta,
-                 double *g_a, double *g_b) {
+// The gradients into the buffers g_dext, g_avec and g_b; beta_j on the device
+// or null.  The buffers are the context's and stay allocated.
+void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_j) {
   const HostSetup &S = c->S;
   const size_t nn = c->nn0();
   const size_t nn1 = (size_t)S.n1 * S.n1;
+  auto ensure = [](DevArray<double> &a, size_t n) {
+    if (a.n < n) a.alloc(n);
+  };
   // The adjoint's own mapping: two energies per thread, at most 16 threads per
   // column and function (energy passes above 32); a tile is its own 16 / G
   // columns.
@@ -622,21 +642,19 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_ho
     B.g_all.alloc(std::min(tiles, fit) * tile_bytes / sizeof(double));
   }
   if (B.grad_e.n < slots * nn1) B.grad_e.alloc(slots * nn1);
-  B.g_dext.alloc((size_t)2 * S.nc * nn);
-  B.g_avec.alloc(2 * nn);
-  B.g_b.alloc(1);
+  ensure(B.g_dext, (size_t)2 * S.nc * nn);
+  ensure(B.g_avec, 2 * nn);
+  ensure(B.g_b, 1);
+  ensure(B.alpha, nn);
+  ensure(B.beta, 2 * nn);
   B.g_dext.zero(c->stream);
   B.g_avec.zero(c->stream);
   B.g_b.zero(c->stream);
-  // Reference-grid weights of Re I (free energy) and of the current.
-  std::vector<double> alpha(nn), beta(2 * nn, 0.0);
   const double la = S.h * S.h;
   const double jfactor = (double)(2 * S.charge_sign) * S.temperature;
-  for (size_t i = 0; i < nn; ++i) alpha[i] = S.domain_ref[i] ? w_omega * la * S.temperature : 0.0;
-  if (beta_host)
-    for (size_t i = 0; i < 2 * nn; ++i) beta[i] = S.domain_ref[i % nn] ? beta_host[i] * jfactor : 0.0;
-  B.alpha.upload(alpha, c->stream);
-  B.beta.upload(beta, c->stream);
+  k_adj_weights<<<grid1(nn, 256), 256, 0, c->stream>>>(nn, c->dom.p, w_omega * la * S.temperature, jfactor, beta_j,
+                                                      B.alpha.p, B.beta.p);
+  check_launch(c);
   extend_reference(c);
   for (const Chunk &ch : c->chunks) {
     const int nslots = ch.a_end - ch.a_begin;
@@ -702,10 +720,9 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_ho
   }
   double si = 0.0;
   for (int e = 0; e < S.ne; ++e) si += S.residues[e] / S.e_im[e];
-  std::vector<double> coef(S.nc);
-  for (int k = 0; k < S.nc; ++k) coef[k] = w_omega * la * (std::log(S.temperature / S.tc[k]) + si * S.temperature);
-  B.coef.upload(coef, c->stream);
-  k_adj_explicit<<<grid1(nn, 256), 256, 0, c->stream>>>(S.n0, S.nc, c->dom.p, c->xstate.p, B.coef.p, B.g_dext.p);
+  AdjCoef coef{};
+  for (int k = 0; k < S.nc; ++k) coef.v[k] = w_omega * la * (std::log(S.temperature / S.tc[k]) + si * S.temperature);
+  k_adj_explicit<<<grid1(nn, 256), 256, 0, c->stream>>>(S.n0, S.nc, c->dom.p, c->xstate.p, coef, B.g_dext.p);
   check_launch(c);
   if (c->has_vp() && w_omega != 0.0) {
     const double scale = w_omega * la * 0.5 / (S.lambda * S.lambda);
@@ -713,12 +730,38 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_ho
                                                           B.g_avec.p);
     check_launch(c);
   }
+}
+
+// sc_adjoint and sc_adjoint_device: beta_j and the results where `from` and
+// `to` say.
+int adjoint_call(sc_ctx *ctx, const char *name, double w_omega, const double *beta_j, cudaMemcpyKind from,
+                 double *g_delta, double *g_a, double *g_b, cudaMemcpyKind to) {
+  if (!ctx) return SC_ERR_ARG;
+  ctx->drop_graph();
+  if (ctx->mode != SC_MODE_FP64 || ctx->S.keldysh || ctx->batch_member) {
+    ctx->err = std::string(name) + ": FP64 self-consistency contexts only";
+    return SC_ERR_STATE;
+  }
+  if (!ctx->boundary_initialized) {
+    ctx->err = std::string(name) + ": the boundary values are not set (run an iteration or sc_boundary_initial first)";
+    return SC_ERR_STATE;
+  }
+  API_BEGIN
+  if (!ctx->adj) ctx->adj.reset(new AdjBuffers());
+  AdjBuffers &B = *ctx->adj;
+  const size_t nn = ctx->nn0();
+  if (beta_j && from == cudaMemcpyHostToDevice) {
+    if (B.beta_in.n < 2 * nn) B.beta_in.alloc(2 * nn);
+    CUDA_TRY(cudaMemcpyAsync(B.beta_in.p, beta_j, 2 * nn * sizeof(double), from, ctx->stream));
+    beta_j = B.beta_in.p;
+  }
+  adjoint_run(ctx, B, w_omega, beta_j);
   if (g_delta)
-    CUDA_TRY(cudaMemcpyAsync(g_delta, B.g_dext.p, (size_t)2 * S.nc * nn * sizeof(double), cudaMemcpyDeviceToHost,
-                             c->stream));
-  if (g_a) CUDA_TRY(cudaMemcpyAsync(g_a, B.g_avec.p, 2 * nn * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  if (g_b) CUDA_TRY(cudaMemcpyAsync(g_b, B.g_b.p, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  CUDA_TRY(cudaStreamSynchronize(c->stream));
+    CUDA_TRY(cudaMemcpyAsync(g_delta, B.g_dext.p, (size_t)2 * ctx->S.nc * nn * sizeof(double), to, ctx->stream));
+  if (g_a) CUDA_TRY(cudaMemcpyAsync(g_a, B.g_avec.p, 2 * nn * sizeof(double), to, ctx->stream));
+  if (g_b) CUDA_TRY(cudaMemcpyAsync(g_b, B.g_b.p, sizeof(double), to, ctx->stream));
+  CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  API_END
 }
 
 }  // namespace
@@ -754,20 +797,14 @@ int sc_evaluate(sc_ctx *ctx, double *free_energy) {
 
 int sc_adjoint(sc_ctx *ctx, double w_omega, const double *beta_j, double *g_delta, double *g_a,
                double *g_b) {
-  if (!ctx) return SC_ERR_ARG;
-  ctx->drop_graph();
-  if (ctx->mode != SC_MODE_FP64 || ctx->S.keldysh || ctx->batch_member) {
-    ctx->err = "sc_adjoint: FP64 self-consistency contexts only";
-    return SC_ERR_STATE;
-  }
-  if (!ctx->boundary_initialized) {
-    ctx->err = "sc_adjoint: the boundary values are not set (run an iteration or sc_boundary_initial first)";
-    return SC_ERR_STATE;
-  }
-  API_BEGIN
-  if (!ctx->adj) ctx->adj.reset(new AdjBuffers());
-  adjoint_run(ctx, *ctx->adj, w_omega, beta_j, g_delta, g_a, g_b);
-  API_END
+  return adjoint_call(ctx, "sc_adjoint", w_omega, beta_j, cudaMemcpyHostToDevice, g_delta, g_a, g_b,
+                      cudaMemcpyDeviceToHost);
+}
+
+int sc_adjoint_device(sc_ctx *ctx, double w_omega, const double *d_beta_j, double *d_g_delta, double *d_g_a,
+                      double *d_g_b) {
+  return adjoint_call(ctx, "sc_adjoint_device", w_omega, d_beta_j, cudaMemcpyDeviceToDevice, d_g_delta, d_g_a, d_g_b,
+                      cudaMemcpyDeviceToDevice);
 }
 
 }  // extern "C"

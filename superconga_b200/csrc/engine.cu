@@ -2298,6 +2298,7 @@ void plan_mapping(sc_ctx *c) {
     set_mapping(c, need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : cap);
     return;
   }
+  if (const char *ee = std::getenv("SCB_EPT")) return set_mapping(c, std::atoi(ee));
   int dev = 0, n_sm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
@@ -2778,6 +2779,17 @@ int sc_get_results(sc_ctx *ctx, double *delta_new, double *j, double *a_new) {
   if (delta_new) CUDA_TRY(cudaMemcpyAsync(delta_new, ctx->gstate.p, nd * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   if (j) CUDA_TRY(cudaMemcpyAsync(j, ctx->j_real.p, 2 * nn * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   if (a_new) CUDA_TRY(cudaMemcpyAsync(a_new, ctx->gstate.p + nd, 2 * nn * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  API_END
+}
+
+int sc_get_results_device(sc_ctx *ctx, double *d_delta_new, double *d_j, double *d_a_new) {
+  if (!ctx) return SC_ERR_ARG;
+  API_BEGIN
+  const size_t nn = ctx->nn0(), nd = (size_t)2 * ctx->S.nc * nn;
+  if (d_delta_new) CUDA_TRY(cudaMemcpyAsync(d_delta_new, ctx->gstate.p, nd * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+  if (d_j) CUDA_TRY(cudaMemcpyAsync(d_j, ctx->j_real.p, 2 * nn * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+  if (d_a_new) CUDA_TRY(cudaMemcpyAsync(d_a_new, ctx->gstate.p + nd, 2 * nn * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   API_END
 }

@@ -516,8 +516,11 @@ __device__ __forceinline__ void sweep_tile(const SweepArgs<R> &A, const double *
       if constexpr (LATE)
         if (green) greens(pdre, pdim, (pcode & SITE_LABEL) != 0);
       if (step) {
+#ifndef NOFASTGEN
         if (fast) fast_steps(dre, dim, es);
-        else general_steps(code & SITE_LABEL, dre, dim, es);
+        else
+#endif
+          general_steps(code & SITE_LABEL, dre, dim, es);
         if (!want_gt && !burn_in) store();
       }
       if constexpr (!LATE)

@@ -160,6 +160,17 @@ class Context:
                                            _p(gd), _p(ga), ctypes.byref(gb)))
         return gd, ga, gb.value
 
+    def adjoint_device(self, w_omega: float, beta_ptr: int | None, delta_ptr: int, a_ptr: int, b_ptr: int):
+        """``adjoint`` on device buffers (float64, the same layouts); complete on return."""
+        self._check(_lib.load().sc_adjoint_device(self._h, float(w_omega), ctypes.c_void_p(beta_ptr),
+                                                  ctypes.c_void_p(delta_ptr), ctypes.c_void_p(a_ptr),
+                                                  ctypes.c_void_p(b_ptr)))
+
+    def results_device(self, delta_ptr: int | None = None, j_ptr: int | None = None, a_ptr: int | None = None):
+        """``results`` into device buffers (None: left out); complete on return."""
+        self._check(_lib.load().sc_get_results_device(self._h, ctypes.c_void_p(delta_ptr), ctypes.c_void_p(j_ptr),
+                                                      ctypes.c_void_p(a_ptr)))
+
     def results(self):
         """g(x): new order parameter, current density, new vector potential."""
         d = np.zeros(self._shape_delta())
