@@ -57,7 +57,9 @@ struct EngineError {
 
 constexpr int REDUCE_THREADS = 256;
 // Ozaki energies one sweep pass takes (the residues sit in shared memory);
-// more are swept in passes of ENERGY_PASS (eight threads of four energies).
+// more are swept in passes of ENERGY_PASS (eight threads of four energies), or
+// on grains of few columns in as few passes as 16 threads per column allow
+// (sweep_pass).
 constexpr int SWEEP_MAX_ENERGIES = 64;
 constexpr int ENERGY_PASS = 32;
 constexpr int NQ = 38;  // partial-sum slots of the finalize reduction (four components)
@@ -242,12 +244,44 @@ __device__ __forceinline__ double2 ld_rec(const SweepArgs<float> &A, size_t idx)
   return make_double2(v.x, v.y);
 }
 
-// Order parameter (OrderParameter::getRotatedGrid) and Doppler shift
-// (computeEnergyShift, RiccatiSolver.h:127-176) at frame site (x, y).
+// The lookups of one frame column (angle P, column x) that do not depend on
+// the row: rotated coordinates (rotated_lookup) of row 0 and their change per
+// row, for the order parameter, the induced vector potential and the position
+// in the external field.
+struct FrameColumn {
+  double y0;                 // row coordinate of row 0, from the rotation centre
+  double xd, yd, xa, ya;     // coordinates at y = 0
+  double xe, ye, sh;
+};
 template <typename R>
-__device__ __forceinline__ void frame_fields(const SweepArgs<R> &A, const AngleParams &P, int x,
+__device__ __forceinline__ FrameColumn frame_column(const SweepArgs<R> &A, const AngleParams &P, int x) {
+  FrameColumn c;
+  c.sh = (double)(A.n0 - 1) / 2.0;
+  const double off = (double)(A.n0 - A.n1) / 2.0 - c.sh;  // = -(n1 - 1) / 2
+  const double X = (double)x + off;
+  c.y0 = off;
+  c.xd = fma(X, P.cD, c.sh);
+  c.yd = fma(X, P.sD, c.sh);
+  c.xa = fma(X, P.cA, c.sh);
+  c.ya = fma(X, P.sA, c.sh);
+  c.xe = X * A.h * P.cE;
+  c.ye = X * A.h * P.sE;
+  return c;
+}
+// rotated_lookup at row offset Y from the column's coordinates (X c, X s).
+__device__ __forceinline__ bool column_lookup(double xc, double xs, double Y, double c, double s, int n, Bilinear &b) {
+  const int xi = split(fma(-Y, s, xc), b.xf), yi = split(fma(Y, c, xs), b.yf);
+  b.i00 = yi * n + xi;
+  return xi >= 0 && xi + 1 < n && yi >= 0 && yi + 1 < n;
+}
+
+// Order parameter (OrderParameter::getRotatedGrid) and Doppler shift
+// (computeEnergyShift, RiccatiSolver.h:127-176) at row y of a frame column.
+template <typename R>
+__device__ __forceinline__ void frame_fields(const SweepArgs<R> &A, const AngleParams &P, const FrameColumn &F,
                                              int y, double &dre, double &dim, double &es) {
   const int n0 = A.n0;
+  const double Y = (double)y + F.y0;
   Bilinear b;
   dre = 0.0;
   dim = 0.0;
@@ -258,7 +292,7 @@ __device__ __forceinline__ void frame_fields(const SweepArgs<R> &A, const AngleP
   // rounding of its own rotation coefficients).
   const bool one = A.nc == 1;
   double2 ca[4];
-  const bool inD = rotated_lookup(x, y, A.n1, n0, P.cD, P.sD, b);
+  const bool inD = column_lookup(F.xd, F.yd, Y, P.cD, P.sD, n0, b);
   if (inD) {
     const Corners w = corners(b);
     const size_t o00 = (size_t)b.i00, o01 = o00 + 1, o10 = o00 + n0, o11 = o10 + 1;
@@ -281,41 +315,30 @@ __device__ __forceinline__ void frame_fields(const SweepArgs<R> &A, const AngleP
       }
     }
   }
-  es = 0.0;
-  if (A.has_vp || A.has_ext) {
-    double ax = 0.0, ay = 0.0;
-    const double off = -0.5 * (double)(A.n1 - 1);
-    const double xp = ((double)x + off) * A.h, yp = ((double)y + off) * A.h;
-    const double xr = xp * P.cE - yp * P.sE, yr = xp * P.sE + yp * P.cE;
-    gauge_potential(A.gauge, A.flux_b, A.area, xr, yr, ax, ay);
-    if (A.has_vp) {
-      double rx = 0.0, ry = 0.0;
-      Bilinear ba;
-      if (rotated_lookup(x, y, A.n1, n0, P.cA, P.sA, ba)) {
-        double2 v00, v01, v10, v11;
-        if (one && inD && ba.i00 == b.i00) {
-          v00 = ca[0];
-          v01 = ca[1];
-          v10 = ca[2];
-          v11 = ca[3];
-        } else {
-          const size_t pa = (size_t)A.nc;
-          v00 = ld_rec(A, pa + (size_t)ba.i00 * st);
-          v01 = ld_rec(A, pa + (size_t)(ba.i00 + 1) * st);
-          v10 = ld_rec(A, pa + (size_t)(ba.i00 + n0) * st);
-          v11 = ld_rec(A, pa + (size_t)(ba.i00 + n0 + 1) * st);
-        }
-        const Corners w = corners(ba);
-        rx = weigh(w, v00.x, v01.x, v10.x, v11.x);
-        ry = weigh(w, v00.y, v01.y, v10.y, v11.y);
+  double sx = 0.0, sy = 0.0;  // vector potential
+  if (A.has_vp) {
+    Bilinear ba;
+    if (column_lookup(F.xa, F.ya, Y, P.cA, P.sA, n0, ba)) {
+      if (!(one && inD && ba.i00 == b.i00)) {
+        const size_t pa = (size_t)A.nc;
+        ca[0] = ld_rec(A, pa + (size_t)ba.i00 * st);
+        ca[1] = ld_rec(A, pa + (size_t)(ba.i00 + 1) * st);
+        ca[2] = ld_rec(A, pa + (size_t)(ba.i00 + n0) * st);
+        ca[3] = ld_rec(A, pa + (size_t)(ba.i00 + n0 + 1) * st);
       }
-      rx *= A.lam_scale;
-      ry *= A.lam_scale;
-      es = A.q * (P.vx * (rx + ax) + P.vy * (ry + ay));
-    } else {
-      es = A.q * (P.vx * ax + P.vy * ay);
+      const Corners w = corners(ba, A.lam_scale);
+      sx = weigh(w, ca[0].x, ca[1].x, ca[2].x, ca[3].x);
+      sy = weigh(w, ca[0].y, ca[1].y, ca[2].y, ca[3].y);
     }
   }
+  if (A.has_ext) {
+    const double Yh = Y * A.h;
+    double ax, ay;
+    gauge_potential(A.gauge, A.flux_b, A.area, fma(-Yh, P.sE, F.xe), fma(Yh, P.cE, F.ye), ax, ay);
+    sx += ax;
+    sy += ay;
+  }
+  es = A.q * (P.vx * sx + P.vy * sy);
 }
 
 __device__ __forceinline__ void group_sum(double &v, int groups, unsigned mask) {
@@ -330,17 +353,18 @@ __device__ __forceinline__ void group_sum(double &v, int groups, unsigned mask) 
 // the reference grid (a warp along one row touched ~20 sectors per gather).
 constexpr int FF_COLS = 8, FF_ROWS = 16;
 template <typename R>
-__global__ void __launch_bounds__(FF_COLS * FF_ROWS, sizeof(R) == 4 ? 6 : 1) k_frame_fields(const SweepArgs<R> A, int rows_per_block) {
+__global__ void __launch_bounds__(FF_COLS * FF_ROWS, 5) k_frame_fields(const SweepArgs<R> A, int rows_per_block) {
   const int item = blockIdx.x * FF_COLS + threadIdx.x;
   if (item >= A.n_items) return;
   const int4 it = A.items[item];
   const int a = it.x, x = it.y, lo = it.z, hi = it.w;
   const AngleParams &P = A.ang[a];  // read in place (a local copy went to the stack)
+  const FrameColumn F = frame_column(A, P, x);
   const int r0 = blockIdx.y * rows_per_block;
   const int r1 = min(r0 + rows_per_block, hi - lo + 1);
   for (int r = r0 + threadIdx.y; r < r1; r += FF_ROWS) {
     double dre, dim, es;
-    frame_fields(A, P, x, lo + r, dre, dim, es);
+    frame_fields(A, P, F, lo + r, dre, dim, es);
     int code = A.labels[(size_t)a * A.n1 * A.n1 + (size_t)(lo + r) * A.n1 + x];
     if (!fields_allow_fast((float)dre, (float)dim, (float)es, (float)P.hs, A.e_re_max)) code |= SITE_GENERAL;
     typedef typename Rec4<R>::type V4;
@@ -577,32 +601,35 @@ __device__ __forceinline__ void res_add(double *q, double o, double n) {
 }
 
 // Block reduction of N sums held in registers (slots listed in max_mask are
-// maxima), written to out[0..N): a shuffle tree per warp, then one thread per
-// slot adds the warps' values in order.  One barrier for all slots instead of
-// ten per slot: the 48-slot reduction of k_finalize took 44 of its 44 us on a
-// 86 x 86 lattice through 480 barriers.
+// maxima), written to out[0..N): 16 slots at a time through shared memory, a
+// warp adding up two of them (eight values a lane, then a shuffle tree).  The
+// serial tree of the whole block took ten barriers per slot (44 us on a 86 x 86
+// lattice for 48 slots), a shuffle tree of every slot in every warp 85 dependent
+// shuffle steps for 17 slots.
 template <int N>
 __device__ __forceinline__ void block_reduce(double (&q)[N], unsigned long long max_mask, double *out) {
-  __shared__ double sh[N][REDUCE_THREADS / 32];
+  constexpr int CH = N < 16 ? N : 16;
+  __shared__ double sh[CH][REDUCE_THREADS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-    const bool mx = (max_mask >> k) & 1ull;
-    double v = q[k];
+  for (int k0 = 0; k0 < N; k0 += CH) {
+    if (k0) __syncthreads();
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double u = __shfl_xor_sync(0xffffffffu, v, o);
-      v = mx ? max_nan(v, u) : v + u;
+    for (int k = 0; k < CH; ++k)
+      if (k0 + k < N) sh[k][threadIdx.x] = q[k0 + k < N ? k0 + k : 0];
+    __syncthreads();
+    for (int k = w; k < CH && k0 + k < N; k += REDUCE_THREADS / 32) {
+      const bool mx = (max_mask >> (k0 + k)) & 1ull;
+      double v = sh[k][lane];
+#pragma unroll
+      for (int i = 1; i < REDUCE_THREADS / 32; ++i) v = mx ? max_nan(v, sh[k][32 * i + lane]) : v + sh[k][32 * i + lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double u = __shfl_xor_sync(0xffffffffu, v, o);
+        v = mx ? max_nan(v, u) : v + u;
+      }
+      if (lane == 0) out[k0 + k] = v;
     }
-    if (lane == 0) sh[k][w] = v;
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < N; k += REDUCE_THREADS) {
-    const bool mx = (max_mask >> k) & 1ull;
-    double v = sh[k][0];
-#pragma unroll
-    for (int i = 1; i < REDUCE_THREADS / 32; ++i) v = mx ? max_nan(v, sh[k][i]) : v + sh[k][i];
-    out[k] = v;
   }
 }
 
@@ -879,7 +906,7 @@ __global__ void k_boundary_initial(int n_out, int ne, int is_g, const int *__res
   const int k = (int)(t / ne), e = (int)(t % ne);
   const AngleParams P = A.ang[node_a[k]];
   double dre, dim, es;
-  frame_fields(A, P, node_x[k], node_y[k], dre, dim, es);
+  frame_fields(A, P, frame_column(A, P, node_x[k]), node_y[k], dre, dim, es);
   Cx<R> g, gt;
   riccati_homogeneous<R>((R)dre, (R)dim, (R)(es + A.e_re[e]), (R)A.e_im[e], g, gt);
   bout[t] = is_g ? g : gt;
@@ -1681,11 +1708,14 @@ void launch_sweep_kel(sc_ctx *c, const SweepArgs<R> &A, unsigned blocks) {
     if (c->ept == 1) launch_sweep_lg<R, 1, 5, KEL, false>(c, A, blocks);
     else if (c->ept == 2) launch_sweep_lg<R, 2, 3, KEL, false>(c, A, blocks);
     else if (c->ept == 4) launch_sweep_lg<R, 4, 3, KEL, false>(c, A, blocks);
+    else if (c->ept == 5) launch_sweep_lg<R, 5, 2, KEL, false>(c, A, blocks);
+    else if (c->ept == 6) launch_sweep_lg<R, 6, 2, KEL, false>(c, A, blocks);
     else launch_sweep_lg<R, 7, 2, KEL, false>(c, A, blocks);
   } else {
     if (c->ept == 1) launch_sweep_lg<R, 1, 4, KEL, false>(c, A, blocks);
     else if (c->ept == 2) launch_sweep_lg<R, 2, 4, KEL, true>(c, A, blocks);
     else if (c->ept == 4) launch_sweep_lg<R, 4, 3, KEL, true>(c, A, blocks);
+    else if (c->ept == 6) launch_sweep_lg<R, 6, 3, KEL, true>(c, A, blocks);
     else launch_sweep_lg<R, 8, 3, KEL, true>(c, A, blocks);
   }
 }
@@ -2259,10 +2289,42 @@ void plan_chunks(sc_ctx *c, std::vector<int4> &items) {
   }
 }
 
+// Energies per thread that the sweep kernels exist for.
+constexpr int EPT64[] = {1, 2, 4, 5, 6, 7}, EPT32[] = {1, 2, 4, 6, 8};
+
+// Energies of one sweep pass.  All of them up to SWEEP_MAX_ENERGIES; above
+// that passes of ENERGY_PASS, except on grains whose columns leave the GPU
+// short of warps in such a pass (fewer than six per scheduler): these take all
+// energies at once as far as 16 threads per column hold them, in equal passes
+// beyond (81 energies on a 103 x 103 square, 2.6 warps per scheduler: one pass
+// in the place of three serial ones).
+int sweep_pass(const sc_ctx *c) {
+  const HostSetup &S = c->S;
+  if (S.ne <= SWEEP_MAX_ENERGIES) return S.ne;
+  if (c->batch_member || std::getenv("SCB_ENERGY_GROUPS")) return ENERGY_PASS;
+  size_t columns = 0;
+  for (int lo : S.col_lo) columns += lo >= 0;
+  if (c->pair) columns /= 2;
+  int dev = 0, n_sm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  const double warps = (double)columns * 2 * 8 / 32 / (4.0 * n_sm);  // eight threads per column and function
+  if (warps >= 6.0) return ENERGY_PASS;
+  const int most = 16 * (c->mode == SC_MODE_MIXED ? 8 : 7), passes = (S.ne + most - 1) / most;
+  return (S.ne + passes - 1) / passes;
+}
+
 // Threads per column and function (groups = 2^log_groups) and energies per
-// thread (ept) of the context's sweeps.
+// thread (ept, or more where 16 threads do not hold the pass) of the context's
+// sweeps.
 void set_mapping(sc_ctx *c, int ept) {
-  while (16 * ept < c->e_pass) ept *= 2;  // at most 16 threads per column and function
+  if (c->mode == SC_MODE_MIXED) {
+    for (int e : EPT32)
+      if (16 * ept < c->e_pass && e > ept) ept = e;
+  } else {
+    for (int e : EPT64)
+      if (16 * ept < c->e_pass && e > ept) ept = e;
+  }
   c->ept = ept;
   c->log_groups = 0;
   while ((ept << c->log_groups) < c->e_pass && c->log_groups < 4) c->log_groups++;
@@ -2287,8 +2349,8 @@ void plan_mapping(sc_ctx *c) {
     int ept;
     double cost, warps;  // per energy slot; wanted per scheduler
   };
-  const Option fp64_opt[] = {{1, 1.64, 0.0}, {2, 1.23, 1.5}, {4, 1.0, 1.5}, {7, 1.06, 3.0}};
-  const Option fp32_opt[] = {{1, 1.6, 0.0}, {2, 1.32, 1.5}, {4, 1.0, 1.5}, {8, kel ? 1.15 : 0.95, 5.0}};
+  const Option fp64_opt[] = {{1, 1.64, 0.0}, {2, 1.23, 1.5}, {4, 1.0, 1.5}, {5, 1.06, 2.5}, {6, 1.06, 2.5}, {7, 1.06, 3.0}};
+  const Option fp32_opt[] = {{1, 1.6, 0.0}, {2, 1.32, 1.5}, {4, 1.0, 1.5}, {6, kel ? 1.1 : 0.98, 3.0}, {8, kel ? 1.15 : 0.95, 5.0}};
   const Option *opt = fp32 ? fp32_opt : fp64_opt;
   const char *eg = std::getenv("SCB_ENERGY_GROUPS");
   const int cap = fp32 ? 8 : 7;
@@ -2298,7 +2360,6 @@ void plan_mapping(sc_ctx *c) {
     set_mapping(c, need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : cap);
     return;
   }
-  if (const char *ee = std::getenv("SCB_EPT")) return set_mapping(c, std::atoi(ee));
   int dev = 0, n_sm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
@@ -2306,7 +2367,7 @@ void plan_mapping(sc_ctx *c) {
   for (const Chunk &ch : c->chunks) items = std::max(items, (size_t)(ch.item_end - ch.item_begin));
   double best = 1e300;
   int ept = 1;
-  for (int k = 0; k < 4; ++k) {
+  for (int k = 0; k < (fp32 ? 5 : 6); ++k) {
     set_mapping(c, opt[k].ept);
     if (c->ept != opt[k].ept) continue;  // more than 16 threads per column
     const double warps = (double)items * 2 * c->groups / 32 / (4.0 * n_sm);
@@ -2316,10 +2377,6 @@ void plan_mapping(sc_ctx *c) {
       best = cost;
       ept = opt[k].ept;
     }
-  }
-  if (best == 1e300) {  // one energy per thread does not fit 16 threads: the fewest that do
-    ept = 2;
-    while (16 * ept < c->e_pass) ept *= 2;
   }
   set_mapping(c, ept);
 }
@@ -2446,7 +2503,7 @@ void upload_static(sc_ctx *c) {
     }
     if (ok) c->pair = na / 2;
   }
-  c->e_pass = S.ne <= SWEEP_MAX_ENERGIES ? S.ne : ENERGY_PASS;
+  c->e_pass = sweep_pass(c);
   std::vector<int4> items;
   plan_chunks(c, items);
   c->items.upload(items, s);
@@ -3334,7 +3391,7 @@ void launch_batch_sweep(sc_batch *b, sc_batch::Wave &w, int wi) {
     } else {
       if (ept == 1) run(k_sweep_batch<R, 1, 4, false>, SweepRing<R, 1, 4, false>::BYTES);
       else if (ept == 2) run(k_sweep_batch<R, 2, 4, true>, SweepRing<R, 2, 4, true>::BYTES);
-      else if (ept == 4) run(k_sweep_batch<R, 4, 3, true>, SweepRing<R, 4, 3, true>::BYTES);
+      else if (ept == 4) run(k_sweep_batch<R, 4, 4, true>, SweepRing<R, 4, 4, true>::BYTES);
       else run(k_sweep_batch<R, 8, 3, true>, SweepRing<R, 8, 3, true>::BYTES);
     }
     b->launches++;
