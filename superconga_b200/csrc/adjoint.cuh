@@ -401,32 +401,59 @@ __global__ void __launch_bounds__(128, 3) k_adjoint(const AdjArgs J) {
   }
 }
 
-// Seeds on the frame lattice of the angles [a_begin, a_end): the transpose of
-// the rotation back (k_rotate_back) applied to the reference-grid weights
-// alpha (of Re I, already times the integrand factor's partner T h^2 w_omega)
-// and beta (of j_x, j_y, already times the current's factor).
-__global__ void k_adj_seeds(int n0, int n1, int a_begin, int a_end, const AngleParams *__restrict__ ang,
-                            const double *__restrict__ alpha, const double *__restrict__ beta, double2 *seed) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= n0 || y >= n0) return;
+// The transposes of the bilinear lookups are gathers: the sites of the lattice
+// `from` (side n_from) whose lookup in the lattice `to` (side n_to, rotation c,
+// s) has site (x, y) among its four corners lie within sqrt(2) of (x, y)
+// rotated the other way, so the 3 x 3 sites from `base` on are looked up the
+// way the forward kernels do and the matching corner's weight is taken.
+// Against scattering with FP64 atomics into cleared buffers (456^2 grain, 128
+// angles, with the clearing): seeds 1.18 -> 1.07 ms, fields 2.41 -> 1.44 ms.
+struct Transposed {
+  int bx, by;  // first candidate
+};
+__device__ __forceinline__ Transposed transposed_lookup(int x, int y, int n_from, int n_to, double c, double s) {
+  const double ct = (double)(n_to - 1) / 2.0, cf = (double)(n_from - 1) / 2.0;
+  const double X = (double)x - ct, Y = (double)y - ct;
+  // inverse rotation, then the smallest integer above the centre - sqrt(2)
+  const double xf = X * c + Y * s + cf, yf = Y * c - X * s + cf;
+  return Transposed{(int)ceil(xf - 1.4143), (int)ceil(yf - 1.4143)};
+}
+// The weight with which the lookup of from-site (u, v) reads to-site (x, y).
+__device__ __forceinline__ double corner_weight(int u, int v, int x, int y, int n_from, int n_to, double c, double s) {
+  Bilinear b;
+  if (!rotated_lookup(u, v, n_from, n_to, c, s, b)) return 0.0;
+  const int d = y * n_to + x - b.i00;
+  const double wx = (d == 0 || d == n_to) ? 1.0 - b.xf : b.xf, wy = (d == 0 || d == 1) ? 1.0 - b.yf : b.yf;
+  return (d == 0 || d == 1 || d == n_to || d == n_to + 1) ? wx * wy : 0.0;
+}
+
+// Seeds on the frame lattice of the angles from a_begin on (blockIdx.y): the
+// transpose of the rotation back (k_rotate_back) applied to the reference-grid
+// weights alpha (of Re I, already times the integrand factor's partner
+// T h^2 w_omega) and beta (of j_x, j_y, already times the current's factor).
+__global__ void __launch_bounds__(256) k_adj_seeds(int n0, int n1, int a_begin, const AngleParams *__restrict__ ang,
+                                                   const double *__restrict__ alpha, const double *__restrict__ beta,
+                                                   double2 *seed) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nn0 = (size_t)n0 * n0, nn1 = (size_t)n1 * n1;
-  const size_t i = (size_t)y * n0 + x;
-  const double al = alpha[i], bx = beta[i], by = beta[nn0 + i];
-  if (al == 0.0 && bx == 0.0 && by == 0.0) return;
-  for (int a = a_begin; a < a_end; ++a) {
-    const AngleParams &P = ang[a];
-    Bilinear b;
-    if (!rotated_lookup(x, y, n0, n1, P.cB, P.sB, b)) continue;
-    const double vi = al * P.w, vg = bx * P.sx + by * P.sy;
-    const double w[4] = {(1.0 - b.xf) * (1.0 - b.yf), b.xf * (1.0 - b.yf), (1.0 - b.xf) * b.yf, b.xf * b.yf};
-    const int off[4] = {b.i00, b.i00 + 1, b.i00 + n1, b.i00 + n1 + 1};
-    double *s = (double *)(seed + (size_t)(a - a_begin) * nn1);
-    for (int k = 0; k < 4; ++k) {
-      atomicAdd(s + 2 * (size_t)off[k], w[k] * vi);
-      atomicAdd(s + 2 * (size_t)off[k] + 1, w[k] * vg);
+  if (t >= (int)nn1) return;
+  const int x = t % n1, y = t / n1;
+  const AngleParams &P = ang[a_begin + blockIdx.y];
+  const Transposed T = transposed_lookup(x, y, n0, n1, P.cB, P.sB);
+  double si = 0.0, sg = 0.0;
+  if (T.bx > -3 && T.bx < n0 && T.by > -3 && T.by < n0) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int u = T.bx + k % 3, v = T.by + k / 3;
+      if (u < 0 || u >= n0 || v < 0 || v >= n0) continue;
+      const double w = corner_weight(u, v, x, y, n0, n1, P.cB, P.sB);
+      if (w == 0.0) continue;
+      const size_t i = (size_t)v * n0 + u;
+      si = fma(w, alpha[i], si);
+      sg = fma(w, beta[i] * P.sx + beta[nn0 + i] * P.sy, sg);
     }
   }
+  seed[(size_t)blockIdx.y * nn1 + t] = make_double2(si * P.w, sg);
 }
 
 // Transpose of the frame extension (k_halo): a halo site's seed moves to its
@@ -449,64 +476,97 @@ __global__ void k_adj_halo_t(int n_entries, int entry0, int n1, const int *__res
 }
 
 // Frame sensitivities back onto the reference grid: the transposes of the
-// bilinear lookups of frame_fields (order parameter, induced vector potential)
-// and the derivative of the gauge potential with respect to the field.
+// bilinear lookups of frame_fields (order parameter, induced vector
+// potential), gathered per reference site over the angles of one part
+// (blockIdx.z) and added to the gradients.  rows: first and last row of every
+// frame column (the sensitivities exist there only).
 __global__ void __launch_bounds__(256) k_adj_fields_t(SweepArgs<double> A, int a_begin, int a_end,
+                                                      const int2 *__restrict__ rows,
                                                       const double2 *__restrict__ grad_d,
                                                       const double *__restrict__ grad_e, double *g_dext,
-                                                      double *g_avec, double *g_b) {
+                                                      double *g_avec) {
   const int n1 = A.n1, n0 = A.n0;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+  if (x >= n0 || y >= n0) return;
   const size_t nn1 = (size_t)n1 * n1, nn0 = (size_t)n0 * n0;
-  const size_t site = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  const int a = a_begin + blockIdx.y;
-  double gb = 0.0;
-  if (site < nn1 && a < a_end) {
+  const int n = a_end - a_begin;
+  const int k0 = a_begin + (int)((long long)n * blockIdx.z / gridDim.z);
+  const int k1 = a_begin + (int)((long long)n * (blockIdx.z + 1) / gridDim.z);
+  double dr[MAX_COMP] = {0, 0, 0, 0}, di[MAX_COMP] = {0, 0, 0, 0}, ax = 0.0, ay = 0.0;
+  for (int a = k0; a < k1; ++a) {
     const AngleParams &P = A.ang[a];
-    const int x = (int)(site % n1), y = (int)(site / n1);
-    const double2 gd = grad_d[(size_t)(a - a_begin) * nn1 + site];
-    const double ge = grad_e[(size_t)(a - a_begin) * nn1 + site];
-    Bilinear b;
-    if ((gd.x != 0.0 || gd.y != 0.0) && rotated_lookup(x, y, n1, n0, P.cD, P.sD, b)) {
-      const double w[4] = {(1.0 - b.xf) * (1.0 - b.yf), b.xf * (1.0 - b.yf), (1.0 - b.xf) * b.yf, b.xf * b.yf};
-      const int off[4] = {b.i00, b.i00 + 1, b.i00 + n0, b.i00 + n0 + 1};
-      for (int c = 0; c < A.nc; ++c) {
-        double *pr = g_dext + (size_t)(2 * c) * nn0, *pi = pr + nn0;
-        const double et = P.eta[c];
-        for (int k = 0; k < 4; ++k) {
-          atomicAdd(pr + off[k], w[k] * et * gd.x);
-          atomicAdd(pi + off[k], w[k] * et * gd.y);
+    const Transposed T = transposed_lookup(x, y, n1, n0, P.cD, P.sD);
+    const size_t slot = (size_t)(a - a_begin) * nn1;
+    double gr = 0.0, gi = 0.0, ge = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int u = T.bx + i;
+      if (u < 0 || u >= n1) continue;
+      const int2 lh = rows[(size_t)a * n1 + u];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int v = T.by + j;
+        if (lh.x < 0 || v < lh.x || v > lh.y) continue;
+        const size_t f = slot + (size_t)v * n1 + u;
+        const double w = corner_weight(u, v, x, y, n1, n0, P.cD, P.sD);
+        if (w != 0.0) {
+          const double2 gd = grad_d[f];
+          gr = fma(w, gd.x, gr);
+          gi = fma(w, gd.y, gi);
+        }
+        if (A.has_vp) {
+          const double wa = corner_weight(u, v, x, y, n1, n0, P.cA, P.sA);
+          if (wa != 0.0) ge = fma(wa, grad_e[f], ge);
         }
       }
     }
-    if (ge != 0.0) {  // the shift depends on the field even where it is zero
-      const double off = -0.5 * (double)(n1 - 1);
-      const double xp = ((double)x + off) * A.h, yp = ((double)y + off) * A.h;
-      const double xr = xp * P.cE - yp * P.sE, yr = xp * P.sE + yp * P.cE;
-      double ax1 = 0.0, ay1 = 0.0;
-      gauge_potential(A.gauge, 1.0, A.area, xr, yr, ax1, ay1);
-      gb = ge * A.q * (P.vx * ax1 + P.vy * ay1);
-      Bilinear ba;
-      if (A.has_vp && rotated_lookup(x, y, n1, n0, P.cA, P.sA, ba)) {
-        const double w[4] = {(1.0 - ba.xf) * (1.0 - ba.yf), ba.xf * (1.0 - ba.yf), (1.0 - ba.xf) * ba.yf,
-                             ba.xf * ba.yf};
-        const int off4[4] = {ba.i00, ba.i00 + 1, ba.i00 + n0, ba.i00 + n0 + 1};
-        const double gx = ge * A.q * P.vx * A.lam_scale, gy = ge * A.q * P.vy * A.lam_scale;
-        for (int k = 0; k < 4; ++k) {
-          atomicAdd(g_avec + off4[k], w[k] * gx);
-          atomicAdd(g_avec + nn0 + off4[k], w[k] * gy);
-        }
+#pragma unroll
+    for (int c = 0; c < MAX_COMP; ++c)
+      if (c < A.nc) {
+        dr[c] = fma(P.eta[c], gr, dr[c]);
+        di[c] = fma(P.eta[c], gi, di[c]);
       }
+    ax = fma(P.vx, ge, ax);
+    ay = fma(P.vy, ge, ay);
+  }
+  const size_t i = (size_t)y * n0 + x;
+#pragma unroll
+  for (int c = 0; c < MAX_COMP; ++c)
+    if (c < A.nc) {
+      atomicAdd(g_dext + (size_t)(2 * c) * nn0 + i, dr[c]);
+      atomicAdd(g_dext + (size_t)(2 * c + 1) * nn0 + i, di[c]);
+    }
+  if (A.has_vp) {
+    atomicAdd(g_avec + i, A.q * A.lam_scale * ax);
+    atomicAdd(g_avec + nn0 + i, A.q * A.lam_scale * ay);
+  }
+}
+
+// dL/dB_ext: the Doppler shift's derivative with respect to the field (the
+// gauge potential of unit field) times its sensitivity, over the chunk's
+// trajectory columns (it does not vanish where the field is zero).
+__global__ void __launch_bounds__(256) k_adj_field(SweepArgs<double> A, const double *__restrict__ grad_e,
+                                                   double *g_b) {
+  const int n1 = A.n1, lane = threadIdx.x & 31;
+  const int item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // a warp per column
+  double gb = 0.0;
+  if (item < A.n_items) {
+    const int4 it = A.items[item];
+    const AngleParams &P = A.ang[it.x];
+    const double off = -0.5 * (double)(n1 - 1), xp = ((double)it.y + off) * A.h;
+    const double *g = grad_e + (size_t)(it.x - A.slot_base) * n1 * n1 + it.y;
+    for (int y = it.z + lane; y <= it.w; y += 32) {
+      const double yp = ((double)y + off) * A.h;
+      double ax1, ay1;
+      gauge_potential(A.gauge, 1.0, A.area, xp * P.cE - yp * P.sE, xp * P.sE + yp * P.cE, ax1, ay1);
+      gb += g[(size_t)y * n1] * A.q * (P.vx * ax1 + P.vy * ay1);
     }
   }
-  // block sum of the field sensitivity
-  __shared__ double sh[256];
-  sh[threadIdx.x] = gb;
+  double q[1] = {gb};
+  __shared__ double sum;
+  block_reduce(q, 0ull, &sum, 1);
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0 && sh[0] != 0.0) atomicAdd(g_b, sh[0]);
+  if (threadIdx.x == 0 && sum != 0.0) atomicAdd(g_b, sum);
 }
 
 // Transpose of extend_reference: an extension site's sensitivity moves to its
@@ -589,6 +649,7 @@ __global__ void k_adj_weights(size_t nn, const uint8_t *__restrict__ dom, double
 
 struct AdjBuffers {
   DevArray<double> g_all, grad_e, g_dext, g_avec, g_b, alpha, beta, beta_in;
+  DevArray<int2> rows;  // [angle][column]: first and last row
 };
 void AdjDeleter::operator()(AdjBuffers *p) const { delete p; }
 
@@ -647,6 +708,12 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_j)
   ensure(B.g_b, 1);
   ensure(B.alpha, nn);
   ensure(B.beta, 2 * nn);
+  if (!B.rows.n) {
+    std::vector<int2> rows((size_t)S.n_angles * S.n1);
+    for (size_t k = 0; k < rows.size(); ++k) rows[k] = make_int2(S.col_lo[k], S.col_hi[k]);
+    B.rows.upload(rows, c->stream);
+    CUDA_TRY(cudaStreamSynchronize(c->stream));
+  }
   B.g_dext.zero(c->stream);
   B.g_avec.zero(c->stream);
   B.g_b.zero(c->stream);
@@ -666,12 +733,9 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_j)
     // The frame-record buffer (two double2 per site and slot) holds both.
     double2 *seed = (double2 *)c->w_fr, *grad_d = seed + (size_t)nslots * nn1;
     c->frames_zeroed = false;  // the frame buffers serve as seed and gradient buffers
-    CUDA_TRY(cudaMemsetAsync(seed, 0, (size_t)nslots * nn1 * sizeof(double2), c->stream));
-    CUDA_TRY(cudaMemsetAsync(grad_d, 0, (size_t)nslots * nn1 * sizeof(double2), c->stream));
-    CUDA_TRY(cudaMemsetAsync(B.grad_e.p, 0, (size_t)nslots * nn1 * sizeof(double), c->stream));
     {
-      dim3 blk(32, 8), grid((S.n0 + 31) / 32, (S.n0 + 7) / 8);
-      k_adj_seeds<<<grid, blk, 0, c->stream>>>(S.n0, S.n1, ch.a_begin, ch.a_end, c->ang.p, B.alpha.p, B.beta.p, seed);
+      k_adj_seeds<<<dim3(grid1(nn1, 256), nslots), 256, 0, c->stream>>>(S.n0, S.n1, ch.a_begin, c->ang.p, B.alpha.p,
+                                                                        B.beta.p, seed);
       check_launch(c);
       const int h0 = S.halo_angle_off[ch.a_begin], h1 = S.halo_angle_off[ch.a_end];
       if (h1 > h0) {
@@ -705,9 +769,13 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_j)
         launch_adjoint<ADJ_EMAX>(c, P);
       }
     }
-    dim3 gridf(grid1(nn1, 256), nslots);
-    k_adj_fields_t<<<gridf, 256, 0, c->stream>>>(A, ch.a_begin, ch.a_end, grad_d, B.grad_e.p, B.g_dext.p,
-                                                  B.g_avec.p, B.g_b.p);
+    // As in k_rotate_back: 8 x 4 patches a warp, the angles in parts.
+    dim3 gridf((S.n0 + 7) / 8, (S.n0 + 31) / 32);
+    gridf.z = std::max(1, std::min<int>(8, (int)((32 * 148) / (gridf.x * gridf.y)) + 1));
+    k_adj_fields_t<<<gridf, dim3(8, 32), 0, c->stream>>>(A, ch.a_begin, ch.a_end, B.rows.p, grad_d, B.grad_e.p,
+                                                         B.g_dext.p, B.g_avec.p);
+    check_launch(c);
+    k_adj_field<<<grid1((size_t)A.n_items * 32, 256), 256, 0, c->stream>>>(A, B.grad_e.p, B.g_b.p);
     check_launch(c);
   }
   // Reference extension transpose, explicit terms, mask.

@@ -66,16 +66,69 @@ constexpr int NQ = 38;  // partial-sum slots of the finalize reduction (four com
 
 // ------------------------------------------------------------------ kernels --
 
+// The kernels of an iteration other than the sweeps are functors, K::run(block
+// index, grid size, arguments...), so that they run as a launch of their own
+// (k_one) and as one launch over the same kernel of many grains (k_many, the
+// batch): a grain of a few thousand sites fills a fraction of the GPU for a few
+// us per kernel, and 24 grains on eight streams still took 2 ms an iteration
+// outside the sweep.
+template <typename... P>
+struct Pack {};
+template <typename H, typename... T>
+struct Pack<H, T...> {
+  H h;
+  Pack<T...> t;
+};
+inline Pack<> make_pack() { return {}; }
+template <typename H, typename... T>
+Pack<H, T...> make_pack(H h, T... t) {
+  return Pack<H, T...>{h, make_pack(t...)};
+}
+template <typename K, typename... A>
+__device__ __forceinline__ void run_pack(uint3 bid, uint3 gdim, const Pack<> &, A... a) {
+  K::run(bid, gdim, a...);
+}
+template <typename K, typename H, typename... T, typename... A>
+__device__ __forceinline__ void run_pack(uint3 bid, uint3 gdim, const Pack<H, T...> &p, A... a) {
+  run_pack<K>(bid, gdim, p.t, a..., p.h);
+}
+template <typename K, typename... P>
+__global__ void __launch_bounds__(K::THREADS, K::BLOCKS) k_one(P... args) {
+  K::run(blockIdx, make_uint3(gridDim.x, gridDim.y, gridDim.z), args...);
+}
+// One grain's launch of a kernel: its grid and arguments, from block `first` of
+// the common launch on.
+template <typename... P>
+struct Task {
+  unsigned first;
+  uint3 grid;
+  Pack<P...> args;
+};
+template <typename K, typename... P>
+__global__ void __launch_bounds__(K::THREADS, K::BLOCKS) k_many(const Task<P...> *__restrict__ tasks, int n) {
+  int lo = 0, hi = n - 1;  // the last task that starts at or before this block
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (tasks[mid].first <= blockIdx.x) lo = mid;
+    else hi = mid - 1;
+  }
+  const Task<P...> &t = tasks[lo];
+  const unsigned l = blockIdx.x - t.first, gx = t.grid.x, gy = t.grid.y;
+  run_pack<K>(make_uint3(l % gx, l / gx % gy, l / gx / gy), t.grid, t.args);
+}
+
 // Reference-grid extension of the order parameter (domain_ops.h:11-69):
 // the order parameter everywhere, except label-0 sites next to the grain,
 // which get the mean of their nearest grain sites; written into the records
 // of k_advance_pack (field f = 2c + part of component c).
-__global__ void k_extend_reference(int n_fields, int nn, int n_sites, int stride, const int *__restrict__ site,
+struct k_extend_reference {
+  static constexpr int THREADS = 128, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, int n_fields, int nn, int n_sites, int stride, const int *__restrict__ site,
                                    const int *__restrict__ off, const int *__restrict__ src,
                                    const double *__restrict__ in, double *__restrict__ out,
                                    float *__restrict__ out32) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const int f = blockIdx.y;
+  const int k = bid.x * blockDim.x + threadIdx.x;
+  const int f = bid.y;
   if (k >= n_sites || f >= n_fields) return;
   const double *v = in + (size_t)f * nn;
   const int b = off[k], e = off[k + 1];
@@ -86,6 +139,7 @@ __global__ void k_extend_reference(int n_fields, int nn, int n_sites, int stride
   out[o] = v_ext;
   if (out32) out32[o] = (float)v_ext;
 }
+};
 
 // Element of the frame buffers: the per-angle Matsubara sums are accumulated in
 // FP64 in the sweep and stored in the stepping precision (FP64 frames for the
@@ -341,9 +395,6 @@ __device__ __forceinline__ void frame_fields(const SweepArgs<R> &A, const AngleP
   es = A.q * (P.vx * sx + P.vy * sy);
 }
 
-__device__ __forceinline__ void group_sum(double &v, int groups, unsigned mask) {
-  for (int o = groups >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
-}
 
 // Rotated order parameter and Doppler shift of every site of every trajectory
 // column of a chunk, written with the site's frame label as one record per
@@ -353,14 +404,16 @@ __device__ __forceinline__ void group_sum(double &v, int groups, unsigned mask) 
 // the reference grid (a warp along one row touched ~20 sectors per gather).
 constexpr int FF_COLS = 8, FF_ROWS = 16;
 template <typename R>
-__global__ void __launch_bounds__(FF_COLS * FF_ROWS, 5) k_frame_fields(const SweepArgs<R> A, int rows_per_block) {
-  const int item = blockIdx.x * FF_COLS + threadIdx.x;
+struct k_frame_fields {
+  static constexpr int THREADS = FF_COLS * FF_ROWS, BLOCKS = 5;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, const SweepArgs<R> A, int rows_per_block) {
+  const int item = bid.x * FF_COLS + threadIdx.x;
   if (item >= A.n_items) return;
   const int4 it = A.items[item];
   const int a = it.x, x = it.y, lo = it.z, hi = it.w;
   const AngleParams &P = A.ang[a];  // read in place (a local copy went to the stack)
   const FrameColumn F = frame_column(A, P, x);
-  const int r0 = blockIdx.y * rows_per_block;
+  const int r0 = bid.y * rows_per_block;
   const int r1 = min(r0 + rows_per_block, hi - lo + 1);
   for (int r = r0 + threadIdx.y; r < r1; r += FF_ROWS) {
     double dre, dim, es;
@@ -371,6 +424,7 @@ __global__ void __launch_bounds__(FF_COLS * FF_ROWS, 5) k_frame_fields(const Swe
     ((V4 *)A.scratch2)[rec_index(A, A.log_groups, item, r)] = V4{(R)dre, (R)dim, (R)es, code_bits(R(0), code)};
   }
 }
+};
 
 #include "sweep.cuh"
 
@@ -378,10 +432,12 @@ __global__ void __launch_bounds__(FF_COLS * FF_ROWS, 5) k_frame_fields(const Swe
 // (ComputeOrderParameter.h:180-181, ComputeCurrent.h:149-150,
 // ComputeFreeEnergy.h:265-266, all through domain_ops.h:11-69).
 template <typename F2>
-__global__ void k_halo(int n_entries, int entry0, int n1, const int *__restrict__ entry_angle,
+struct k_halo {
+  static constexpr int THREADS = 128, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, int n_entries, int entry0, int n1, const int *__restrict__ entry_angle,
                        int slot_base, const int *__restrict__ site, const int *__restrict__ off,
                        const int *__restrict__ src, F2 *fr) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = bid.x * blockDim.x + threadIdx.x;
   if (k >= n_entries) return;
   const int e = entry0 + k;
   F2 *slot = fr + (size_t)(entry_angle[e] - slot_base) * n1 * n1 * 2;  // records of two F2
@@ -398,6 +454,7 @@ __global__ void k_halo(int n_entries, int entry0, int n1, const int *__restrict_
   slot[2 * (size_t)site[e]] = frame_pair<F2>(__ddiv_rn(f.x, cnt), __ddiv_rn(f.y, cnt));
   slot[2 * (size_t)site[e] + 1] = frame_pair<F2>(__ddiv_rn(q.x, cnt), __ddiv_rn(q.y, cnt));
 }
+};
 
 // Rotation of the frame Green sums back to the reference grid, accumulated in
 // angle order (ComputeOrderParameter.h:174-210, ComputeCurrent.h:142-173,
@@ -416,21 +473,23 @@ __global__ void k_halo(int n_entries, int entry0, int n1, const int *__restrict_
 // registers); NC = 0 takes it from nc.  One component: four resident blocks
 // per SM (64 registers) measured fastest on B200; more: three.
 template <typename F2, int NC>
-__global__ void __launch_bounds__(256, NC == 1 ? 4 : 3) k_rotate_back(int n0, int n1, int nc_, int first, int a_begin,
+struct k_rotate_back {
+  static constexpr int THREADS = 256, BLOCKS = NC == 1 ? 4 : 3;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, int n0, int n1, int nc_, int first, int a_begin,
                                                      int a_end, int pair, const AngleParams *__restrict__ ang,
                                                      const F2 *__restrict__ fr,
                                                      double *acc_d, double *acc_j, double *acc_fe) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
+  const int x = bid.x * blockDim.x + threadIdx.x;
+  const int y = bid.y * blockDim.y + threadIdx.y;
   if (x >= n0 || y >= n0) return;
   const size_t nn0 = (size_t)n0 * n0, nn1 = (size_t)n1 * n1;
   const size_t i = (size_t)y * n0 + x;
   const int nc = NC > 0 ? NC : nc_;
-  acc_d += blockIdx.z * (size_t)(2 * nc) * nn0;
-  acc_j += blockIdx.z * 2 * nn0;
-  acc_fe += blockIdx.z * nn0;
+  acc_d += bid.z * (size_t)(2 * nc) * nn0;
+  acc_j += bid.z * 2 * nn0;
+  acc_fe += bid.z * nn0;
   const int n_ang = a_end - a_begin;
-  const int k0 = (int)((long long)n_ang * blockIdx.z / gridDim.z), k1 = (int)((long long)n_ang * (blockIdx.z + 1) / gridDim.z);
+  const int k0 = (int)((long long)n_ang * bid.z / gdim.z), k1 = (int)((long long)n_ang * (bid.z + 1) / gdim.z);
   double dr[NC > 0 ? NC : MAX_COMP], di[NC > 0 ? NC : MAX_COMP];
 #pragma unroll
   for (int c = 0; c < nc; ++c) {
@@ -489,6 +548,7 @@ __global__ void __launch_bounds__(256, NC == 1 ? 4 : 3) k_rotate_back(int n0, in
   acc_j[nn0 + i] = jy;
   acc_fe[i] = fe;
 }
+};
 
 // LDOS frame extension next to the boundary, every energy of the block
 // (ComputeLDOS.h:137-138 through domain_ops.h:11-69).
@@ -601,13 +661,16 @@ __device__ __forceinline__ void res_add(double *q, double o, double n) {
 }
 
 // Block reduction of N sums held in registers (slots listed in max_mask are
-// maxima), written to out[0..N): 16 slots at a time through shared memory, a
+// maxima), written to out[k * stride] (the partial sums of a kernel are
+// [slot][block], which the final sums read in whole lines): 16 slots at a time
+// through shared memory, a
 // warp adding up two of them (eight values a lane, then a shuffle tree).  The
 // serial tree of the whole block took ten barriers per slot (44 us on a 86 x 86
 // lattice for 48 slots), a shuffle tree of every slot in every warp 85 dependent
 // shuffle steps for 17 slots.
 template <int N>
-__device__ __forceinline__ void block_reduce(double (&q)[N], unsigned long long max_mask, double *out) {
+__device__ __forceinline__ void block_reduce(double (&q)[N], unsigned long long max_mask, double *out,
+                                             size_t stride) {
   constexpr int CH = N < 16 ? N : 16;
   __shared__ double sh[CH][REDUCE_THREADS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -628,7 +691,7 @@ __device__ __forceinline__ void block_reduce(double (&q)[N], unsigned long long 
         const double u = __shfl_xor_sync(0xffffffffu, v, o);
         v = mx ? max_nan(v, u) : v + u;
       }
-      if (lane == 0) out[k0 + k] = v;
+      if (lane == 0) out[(k0 + k) * stride] = v;
     }
   }
 }
@@ -685,12 +748,11 @@ __device__ double residual_from(const double *t, size_t n_elem, int norm) {
   return numer / fmax(denom, eps);
 }
 
-// Sums (or maxima, for the slots set in max_mask) of the first nq of `stride`
-// slots over the nblocks rows of block partials: warp w reduces slots w,
+// Sums (or maxima, for the slots set in max_mask) of nq slots over the block
+// partials [slot][nblocks]: warp w reduces slots w,
 // w + nwarps, ... in a fixed order (lane-strided with four loads in flight,
 // then a shuffle tree); results in t[0..nq).
-__device__ void reduce_slots(const double *partial, int nblocks, int stride, int nq, unsigned long long max_mask,
-                             double *t) {
+__device__ void reduce_slots(const double *partial, int nblocks, int nq, unsigned long long max_mask, double *t) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int k = w; k < nq; k += nw) {
     const bool mx = (max_mask >> k) & 1ull;
@@ -698,7 +760,7 @@ __device__ void reduce_slots(const double *partial, int nblocks, int stride, int
     for (int b0 = lane; b0 < nblocks; b0 += 128) {
       double p[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) p[u] = b0 + 32 * u < nblocks ? partial[(size_t)(b0 + 32 * u) * stride + k] : 0.0;
+      for (int u = 0; u < 4; ++u) p[u] = b0 + 32 * u < nblocks ? partial[(size_t)k * nblocks + b0 + 32 * u] : 0.0;
 #pragma unroll
       for (int u = 0; u < 4; ++u) v = mx ? max_nan(v, p[u]) : v + p[u];
     }
@@ -724,7 +786,7 @@ struct FinalizeConsts {
 // By the last block of k_finalize.
 __device__ __forceinline__ void finalize_scalars(const FinalizeConsts &C, const double *partial, int nblocks, Scalars *S) {
   __shared__ double t[NQ];
-  reduce_slots(partial, nblocks, NQ, FIN_HEAD + FIN_COMP * C.nc, FIN_MAX_MASK, t);
+  reduce_slots(partial, nblocks, FIN_HEAD + FIN_COMP * C.nc, FIN_MAX_MASK, t);
   if (threadIdx.x != 0) return;
   double rop = 0.0;
   for (int c = 0; c < C.nc; ++c) rop = max_nan(rop, residual_from(&t[FIN_HEAD + FIN_COMP * c], C.n_elem_field, C.norm));
@@ -759,7 +821,9 @@ __device__ __forceinline__ void finalize_scalars(const FinalizeConsts &C, const 
 // component count is fixed at compile time (NC = 0: up to MAX_COMP at run
 // time), so that the sums stay in registers and only used slots are reduced.
 template <int NC>
-__global__ void __launch_bounds__(REDUCE_THREADS) k_finalize(
+struct k_finalize {
+  static constexpr int THREADS = REDUCE_THREADS, BLOCKS = NC == 1 ? 3 : 2;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, 
     int n0, int nc_, double h, double jfactor, int has_vp, const uint8_t *__restrict__ dom,
     const double *__restrict__ coupling, const double *__restrict__ acc_d,
     const double *__restrict__ acc_j, const double *__restrict__ acc_fe,
@@ -772,55 +836,65 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_finalize(
 #pragma unroll
   for (int k = 0; k < FIN_HEAD + FIN_COMP * NCM; ++k) q[k] = 0.0;
   const double inv_h = 1.0 / h;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
+  for (unsigned i = bid.x * blockDim.x + threadIdx.x; i < nn; i += gdim.x * blockDim.x) {
+    // All loads of the site first: the stores below may alias them as far as
+    // the compiler knows, and a load after a store waits out its own latency.
     const bool in = dom[i] != 0;
+    double o[2 * NCM], sum[2 * NCM], oj[2], sj[2], sf = acc_fe[i];
 #pragma unroll
-    for (int c = 0; c < NCM; ++c) {
-      if (c >= nc) break;
-      double *qc = &q[FIN_HEAD + FIN_COMP * c];
-      const double lc = coupling[c];
-      const size_t kr = (size_t)(2 * c) * nn + i, ki = kr + nn;
-      const double o_re = delta[kr], o_im = delta[ki];
-      double s_re = acc_d[kr], s_im = acc_d[ki];  // the parts of k_rotate_back in order
-      for (int p = 1; p < parts; ++p) {
-        s_re += acc_d[p * (size_t)(2 * nc) * nn + kr];
-        s_im += acc_d[p * (size_t)(2 * nc) * nn + ki];
-      }
-      const double n_re = in ? s_re * lc : 0.0, n_im = in ? s_im * lc : 0.0;
-      delta_new[kr] = n_re;
-      delta_new[ki] = n_im;
-      res_add(qc, o_re, n_re);
-      res_add(qc, o_im, n_im);
-      if (in) qc[6] += o_re * o_re + o_im * o_im;
+    for (int k = 0; k < 2 * NCM; ++k) {
+      o[k] = k < 2 * nc ? delta[(size_t)k * nn + i] : 0.0;
+      sum[k] = k < 2 * nc ? acc_d[(size_t)k * nn + i] : 0.0;
     }
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
-      const size_t k = (size_t)d * nn + i;
-      double sj = acc_j[k];
-      for (int p = 1; p < parts; ++p) sj += acc_j[p * 2 * (size_t)nn + k];
-      const double nv = in ? sj * jfactor : 0.0;
-      res_add(&q[0], j_real[k], nv);
-      j_real[k] = nv;
-      q[8 + d] += nv;
+      oj[d] = j_real[(size_t)d * nn + i];
+      sj[d] = acc_j[(size_t)d * nn + i];
     }
-    double sf = acc_fe[i];
-    for (int p = 1; p < parts; ++p) sf += acc_fe[p * (size_t)nn + i];
-    if (in) q[6] += sf;
+    double bz = 0.0;
     if (has_vp) {
-      // curl_kernel, GridFunctions_GPU.h:326-352.
+      // curl_kernel, GridFunctions_GPU.h:326-352, over one or two spacings.
       const int x = (int)(i % (unsigned)n0), y = (int)(i / (unsigned)n0);
       const int xn = min(x + 1, n0 - 1), xp = max(x - 1, 0);
       const int yn = min(y + 1, n0 - 1), yp = max(y - 1, 0);
       const double *ax = avec, *ay = avec + nn;
-      const double dAydx = (ay[(size_t)y * n0 + xn] - ay[(size_t)y * n0 + xp]) / (double)(xn - xp);
-      const double dAxdy = (ax[(size_t)yn * n0 + x] - ax[(size_t)yp * n0 + x]) / (double)(yn - yp);
-      const double bz = (dAydx - dAxdy) * inv_h;
-      q[7] += bz * bz;
+      const double dAydx = (ay[(size_t)y * n0 + xn] - ay[(size_t)y * n0 + xp]) * (xn - xp == 2 ? 0.5 : 1.0);
+      const double dAxdy = (ax[(size_t)yn * n0 + x] - ax[(size_t)yp * n0 + x]) * (yn - yp == 2 ? 0.5 : 1.0);
+      bz = (dAydx - dAxdy) * inv_h;
     }
+    for (int p = 1; p < parts; ++p) {  // the parts of k_rotate_back in order
+#pragma unroll
+      for (int k = 0; k < 2 * NCM; ++k)
+        if (k < 2 * nc) sum[k] += acc_d[((size_t)p * 2 * nc + k) * nn + i];
+#pragma unroll
+      for (int d = 0; d < 2; ++d) sj[d] += acc_j[((size_t)p * 2 + d) * nn + i];
+      sf += acc_fe[(size_t)p * nn + i];
+    }
+#pragma unroll
+    for (int c = 0; c < NCM; ++c)
+      if (c < nc) {
+        const double lc = coupling[c];
+        const double n_re = in ? sum[2 * c] * lc : 0.0, n_im = in ? sum[2 * c + 1] * lc : 0.0;
+        delta_new[(size_t)(2 * c) * nn + i] = n_re;
+        delta_new[(size_t)(2 * c + 1) * nn + i] = n_im;
+        res_add(&q[FIN_HEAD + FIN_COMP * c], o[2 * c], n_re);
+        res_add(&q[FIN_HEAD + FIN_COMP * c], o[2 * c + 1], n_im);
+        if (in) q[FIN_HEAD + FIN_COMP * c + 6] += o[2 * c] * o[2 * c] + o[2 * c + 1] * o[2 * c + 1];
+      }
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+      const double nv = in ? sj[d] * jfactor : 0.0;
+      res_add(&q[0], oj[d], nv);
+      j_real[(size_t)d * nn + i] = nv;
+      q[8 + d] += nv;
+    }
+    if (in) q[6] += sf;
+    q[7] += bz * bz;
   }
-  block_reduce(q, FIN_MAX_MASK, partial + (size_t)blockIdx.x * NQ);
-  if (last_block(counter, gridDim.x)) finalize_scalars(C, partial, gridDim.x, S);
+  block_reduce(q, FIN_MAX_MASK, partial + bid.x, gdim.x);
+  if (last_block(counter, gdim.x)) finalize_scalars(C, partial, gdim.x, S);
 }
+};
 
 __global__ void __launch_bounds__(256) k_ldos_finalize(int n0, int n_fields, const uint8_t *__restrict__ dom,
                                                        const double *__restrict__ acc, double *ldos,
@@ -848,7 +922,7 @@ __global__ void __launch_bounds__(256) k_ldos_finalize(int n0, int n_fields, con
         }
     }
   }
-  block_reduce(q, 0x30ull, partial + (size_t)blockIdx.x * 6);
+  block_reduce(q, 0x30ull, partial + blockIdx.x, gridDim.x);
 }
 
 // Specular boundary condition through the precomputed gather table
@@ -865,11 +939,13 @@ struct BoundarySide {
   double *partial;
 };
 template <typename R>
-__global__ void __launch_bounds__(REDUCE_THREADS) k_boundary(int ne, BoundarySide<R> g, BoundarySide<R> gt) {
-  const BoundarySide<R> &B = blockIdx.y ? gt : g;
+struct k_boundary {
+  static constexpr int THREADS = REDUCE_THREADS, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, int ne, BoundarySide<R> g, BoundarySide<R> gt) {
+  const BoundarySide<R> &B = bid.y ? gt : g;
   double q[6] = {0, 0, 0, 0, 0, 0};
   const unsigned total = (unsigned)B.n_in * ne;
-  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+  for (unsigned t = bid.x * blockDim.x + threadIdx.x; t < total; t += gdim.x * blockDim.x) {
     const unsigned k = t / (unsigned)ne, e = t - k * ne;
     const int4 src = ((const int4 *)B.src)[k];
     const double2 w01 = ((const double2 *)B.w)[2 * (size_t)k], w23 = ((const double2 *)B.w)[2 * (size_t)k + 1];
@@ -891,8 +967,9 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_boundary(int ne, BoundarySid
     res_add(q, (double)ov.im, (double)nv.im);
     B.in[t] = nv;
   }
-  block_reduce(q, 0x30ull, B.partial + (size_t)blockIdx.x * 6);
+  block_reduce(q, 0x30ull, B.partial + bid.x, gdim.x);
 }
+};
 
 // Initial boundary values: homogeneous solutions at every exit node
 // (computeGammaFunctionInitialBoundaryTemplate_kernel,
@@ -937,10 +1014,9 @@ __global__ void k_boundary_initial(int n_out, int ne, int is_g, const int *__res
 // x[j + r P/R], twiddles it by w^(r k), k = j mod Ns, w = exp(-2 pi i / (Ns R)),
 // takes the R-point DFT and writes y[(j / Ns) Ns R + k + r Ns].
 // tw[q] = exp(-2 pi i q / P), q < P (conjugated for the inverse).
-struct FftPlan {
-  int n_stages;
-  int radix[16];
-};
+// The radices of a plan, first stage in the lowest four bits (an array would be
+// copied to the stack to be indexed).
+using FftPlan = unsigned long long;
 
 __device__ __forceinline__ double2 cmul_d2(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -1026,11 +1102,11 @@ __device__ __forceinline__ void fft_stage(const double2 *a, double2 *b, int P, i
 // The P-point transforms of `cols` arrays in shared memory, ping-ponging
 // between a and b (the data is in a on return).  The caller has filled a and
 // synchronised.
-__device__ __forceinline__ void fft_shared(const FftPlan &plan, int P, int cols, const double2 *__restrict__ tw,
+__device__ __forceinline__ void fft_shared(FftPlan plan, int P, int cols, const double2 *__restrict__ tw,
                                            double2 *&a, double2 *&b, int inverse) {
   int ns = 1;
-  for (int st = 0; st < plan.n_stages; ++st) {
-    const int R = plan.radix[st];
+  for (; plan; plan >>= 4) {
+    const int R = (int)(plan & 15);
     if (R == 4) fft_stage<4>(a, b, P, cols, ns, tw, inverse);
     else if (R == 2) fft_stage<2>(a, b, P, cols, ns, tw, inverse);
     else if (R == 3) fft_stage<3>(a, b, P, cols, ns, tw, inverse);
@@ -1046,14 +1122,16 @@ __device__ __forceinline__ void fft_shared(const FftPlan &plan, int P, int cols,
 // Row r of the padded current s_x + i s_y, s = j - mean inside the n x n
 // lattice (ComputeVectorPotential.h:575-591; mean null: j is mean-free),
 // transformed into z[r].  j null: the row of z itself, in place.
-__global__ void __launch_bounds__(512) k_pois_rows(FftPlan plan, int n, int P, const double2 *__restrict__ tw,
+struct k_pois_rows {
+  static constexpr int THREADS = 512, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, FftPlan plan, int n, int P, const double2 *__restrict__ tw,
                                                    const double *__restrict__ j, const double *__restrict__ mean,
                                                    double2 *z) {
   extern __shared__ double2 fft_sm[];
   double2 *a = fft_sm, *b = fft_sm + P;
-  double2 *row = z + (size_t)blockIdx.x * P;
+  double2 *row = z + (size_t)bid.x * P;
   if (j) {
-    const size_t nn = (size_t)n * n, r = (size_t)blockIdx.x * n;
+    const size_t nn = (size_t)n * n, r = (size_t)bid.x * n;
     const double mx = mean ? mean[0] : 0.0, my = mean ? mean[1] : 0.0;
     for (int i = threadIdx.x; i < P; i += blockDim.x)
       a[i] = i < n ? make_double2(j[r + i] - mx, j[nn + r + i] - my) : make_double2(0.0, 0.0);
@@ -1064,17 +1142,20 @@ __global__ void __launch_bounds__(512) k_pois_rows(FftPlan plan, int n, int P, c
   fft_shared(plan, P, 1, tw, a, b, 0);
   for (int i = threadIdx.x; i < P; i += blockDim.x) row[i] = a[i];
 }
+};
 
 // `cols` neighbouring columns of z, of which the first rows_in rows are not
 // zero: transformed, times their spectrum kf[column][row], transformed back,
 // and the first rows_in rows written in place.  out not null (set-up):
 // transformed only, written to out[column][row].
-__global__ void __launch_bounds__(512) k_pois_cols(FftPlan plan, int P, int rows_in, int cols,
+struct k_pois_cols {
+  static constexpr int THREADS = 512, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, FftPlan plan, int P, int rows_in, int cols,
                                                    const double2 *__restrict__ tw, const double2 *__restrict__ kf,
                                                    double2 *z, double2 *out) {
   extern __shared__ double2 fft_sm[];
   double2 *a = fft_sm, *b = fft_sm + cols * P;
-  const int c0 = blockIdx.x * cols;
+  const int c0 = bid.x * cols;
   for (int t = threadIdx.x; t < cols * P; t += blockDim.x) {
     const int r = t / cols, c = t - r * cols;
     a[c * P + r] = r < rows_in ? z[(size_t)r * P + c0 + c] : make_double2(0.0, 0.0);
@@ -1093,22 +1174,25 @@ __global__ void __launch_bounds__(512) k_pois_cols(FftPlan plan, int P, int rows
     z[(size_t)r * P + c0 + c] = a[c * P + r];
   }
 }
+};
 
 // Row r of the result: a_x = Re z / P^2, a_y = Im z / P^2 on the n x n
 // lattice, and (old not null) the row's residual sums against the old vector
 // potential.
-__global__ void __launch_bounds__(REDUCE_THREADS) k_pois_back(FftPlan plan, int n, int P, double inv,
+struct k_pois_back {
+  static constexpr int THREADS = REDUCE_THREADS, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, FftPlan plan, int n, int P, double inv,
                                                               const double2 *__restrict__ tw,
                                                               const double2 *__restrict__ z,
                                                               const double *__restrict__ old, double *av,
                                                               double *partial) {
   extern __shared__ double2 fft_sm[];
   double2 *a = fft_sm, *b = fft_sm + P;
-  const double2 *row = z + (size_t)blockIdx.x * P;
+  const double2 *row = z + (size_t)bid.x * P;
   for (int i = threadIdx.x; i < P; i += blockDim.x) a[i] = row[i];
   __syncthreads();
   fft_shared(plan, P, 1, tw, a, b, 1);
-  const size_t nn = (size_t)n * n, r = (size_t)blockIdx.x * n;
+  const size_t nn = (size_t)n * n, r = (size_t)bid.x * n;
   double q[6] = {0, 0, 0, 0, 0, 0};
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double x = a[i].x * inv, y = a[i].y * inv;
@@ -1119,19 +1203,22 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_pois_back(FftPlan plan, int 
       res_add(q, old[nn + r + i], y);
     }
   }
-  if (old) block_reduce(q, 0x30ull, partial + (size_t)blockIdx.x * 6);
+  if (old) block_reduce(q, 0x30ull, partial + bid.x, gdim.x);
 }
+};
 
 // Boundary and vector-potential residuals, total residual (Context.h:462-483).
-__global__ void k_scalars_b(int norm, size_t n_elem_g, size_t n_elem_gt, size_t n_elem_vp,
+struct k_scalars_b {
+  static constexpr int THREADS = 1024, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, int norm, size_t n_elem_g, size_t n_elem_gt, size_t n_elem_vp,
                             int do_bc, int do_vp, int compute_mode, const double *p_bg, int nb_g,
                             const double *p_bgt, int nb_gt, const double *p_vp, int nb_vp, Scalars *S) {
   __shared__ double t[18];
   if (do_bc) {
-    reduce_slots(p_bg, nb_g, 6, 6, 0x30ull, &t[0]);
-    reduce_slots(p_bgt, nb_gt, 6, 6, 0x30ull, &t[6]);
+    reduce_slots(p_bg, nb_g, 6, 0x30ull, &t[0]);
+    reduce_slots(p_bgt, nb_gt, 6, 0x30ull, &t[6]);
   }
-  if (do_vp) reduce_slots(p_vp, nb_vp, 6, 6, 0x30ull, &t[12]);
+  if (do_vp) reduce_slots(p_vp, nb_vp, 6, 0x30ull, &t[12]);
   if (threadIdx.x != 0) return;
   if (do_bc) S->res_bc = max_nan(residual_from(&t[0], n_elem_g, norm), residual_from(&t[6], n_elem_gt, norm));
   if (do_vp) S->res_vp = residual_from(&t[12], n_elem_vp, norm);
@@ -1144,6 +1231,7 @@ __global__ void k_scalars_b(int norm, size_t n_elem_g, size_t n_elem_gt, size_t 
   }
   S->residual = r;
 }
+};
 
 // ---------------------------------------------------------- accelerators --
 constexpr int AND_MAX_RANK = 16;
@@ -1200,7 +1288,7 @@ __device__ __forceinline__ void acc_scalars(const AccConsts &C, const double *pa
   __shared__ double t[48];
   const int nf = C.nf;
   const bool init = !st->initialized;  // read before the barrier in reduce_slots
-  reduce_slots(partial, nblocks, 3 * nf, 3 * nf, 0ull, t);
+  reduce_slots(partial, nblocks, 3 * nf, 0ull, t);
   const int f = threadIdx.x;
   if (f >= nf) return;
   if (C.kind == ACC_CONGACC) {
@@ -1242,35 +1330,40 @@ __device__ __forceinline__ void acc_scalars(const AccConsts &C, const double *pa
 // Per-field sums for CongAcc (CongAcc.h:371-385) and Barzilai-Borwein
 // (BarzilaiBorwein.h:214-229): slots [3f] sum d^2, [3f+1] sum m^2, [3f+2] sum d m,
 // where d = g - x and m is the running mean (CongAcc) or the previous d (BB).
-__global__ void __launch_bounds__(REDUCE_THREADS) k_acc_sums(AccConsts C, size_t nn, const double *__restrict__ x,
+struct k_acc_sums {
+  static constexpr int THREADS = REDUCE_THREADS, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, AccConsts C, size_t nn, const double *__restrict__ x,
                                                              const double *__restrict__ gx,
                                                              const double *__restrict__ m, double *partial,
                                                              AccState *st, unsigned *counter) {
-  const int f = blockIdx.y;
+  const int f = bid.y;
   double q[3] = {0, 0, 0};
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nn;
-       i += (size_t)gridDim.x * blockDim.x) {
+  for (size_t i = bid.x * (size_t)blockDim.x + threadIdx.x; i < nn;
+       i += (size_t)gdim.x * blockDim.x) {
     const size_t k = (size_t)f * nn + i;
     const double d = gx[k] - x[k], mv = m[k];
     q[0] += d * d;
     q[1] += mv * mv;
     q[2] += d * mv;
   }
-  block_reduce(q, 0, partial + ((size_t)blockIdx.x * C.nf + f) * 3);
-  if (last_block(counter, gridDim.x * gridDim.y)) acc_scalars(C, partial, gridDim.x, st);
+  block_reduce(q, 0, partial + (size_t)3 * f * gdim.x + bid.x, gdim.x);
+  if (last_block(counter, gdim.x * gdim.y)) acc_scalars(C, partial, gdim.x, st);
 }
+};
 
 // Anderson::set (Anderson.h:267-289): the iterate and its residual
 // d = g(x) - x go to slot iter mod rank (the oldest once all are used), and
 // the block partials of |d|^2 and of d . D_j with the other stored residuals.
-__global__ void __launch_bounds__(REDUCE_THREADS) k_and_store(size_t tot, int rank, const double *__restrict__ x,
+struct k_and_store {
+  static constexpr int THREADS = REDUCE_THREADS, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, size_t tot, int rank, const double *__restrict__ x,
                                                               const double *__restrict__ gx, double *hx,
                                                               double *hd, const AccState *st, double *partial) {
   const int it = st->and_iter, slot = it % rank, m = min(it + 1, rank);
   double q[AND_MAX_RANK];
 #pragma unroll
   for (int j = 0; j < AND_MAX_RANK; ++j) q[j] = 0.0;
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < tot; k += (size_t)gridDim.x * blockDim.x) {
+  for (size_t k = bid.x * (size_t)blockDim.x + threadIdx.x; k < tot; k += (size_t)gdim.x * blockDim.x) {
     const double d = gx[k] - x[k];
     hx[(size_t)slot * tot + k] = x[k];
     hd[(size_t)slot * tot + k] = d;
@@ -1278,15 +1371,18 @@ __global__ void __launch_bounds__(REDUCE_THREADS) k_and_store(size_t tot, int ra
     for (int j = 0; j < AND_MAX_RANK; ++j)
       if (j < m) q[j] += d * (j == slot ? d : hd[(size_t)j * tot + k]);
   }
-  block_reduce(q, 0, partial + (size_t)blockIdx.x * AND_MAX_RANK);
+  block_reduce(q, 0, partial + bid.x, gdim.x);
 }
+};
 
 // Anderson::solve (Anderson.h:291-333): the bordered least-squares system
 // [A 1; 1 0] [w; l] = [0; 1] with A_ij = D_i . D_j / mean |D|^2, solved by
 // Gaussian elimination with partial pivoting; then the iteration count.
-__global__ void k_and_solve(int rank, const double *partial, int nblocks, AccState *st) {
+struct k_and_solve {
+  static constexpr int THREADS = 256, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, int rank, const double *partial, int nblocks, AccState *st) {
   __shared__ double t[AND_MAX_RANK];
-  reduce_slots(partial, nblocks, AND_MAX_RANK, rank, 0ull, t);
+  reduce_slots(partial, nblocks, rank, 0ull, t);
   if (threadIdx.x != 0) return;
   const int it = st->and_iter, slot = it % rank, m = min(it + 1, rank), mt = m + 1;
   for (int j = 0; j < m; ++j) {
@@ -1342,17 +1438,21 @@ __global__ void k_and_solve(int rank, const double *partial, int nblocks, AccSta
   for (int i = 0; i < AND_MAX_RANK; ++i) st->and_w[i] = i < m ? w[i] : 0.0;
   st->and_iter = it + 1;
 }
+};
 
 // Anderson::computeInternal (Anderson.h:336-355): x = sum_i w_i (X_i + step D_i).
-__global__ void k_and_update(size_t tot, int rank, double step, const double *__restrict__ hx,
+struct k_and_update {
+  static constexpr int THREADS = 256, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, size_t tot, int rank, double step, const double *__restrict__ hx,
                              const double *__restrict__ hd, const AccState *st, double *x) {
-  const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t k = bid.x * (size_t)blockDim.x + threadIdx.x;
   if (k >= tot) return;
   const int m = min(st->and_iter, rank);  // already counts this iteration
   double v = 0.0;
   for (int i = 0; i < m; ++i) v += (hx[(size_t)i * tot + k] + hd[(size_t)i * tot + k] * step) * st->and_w[i];
   x[k] = v;
 }
+};
 
 // One site's new value of field f: CongAcc (CongAcc.h:271-297), Picard
 // (Picard.h:133-138), Polyak (Polyak.h:214-239), Barzilai-Borwein
@@ -1384,11 +1484,13 @@ __device__ __forceinline__ double acc_advance(const AccConsts &C, const AccState
 // mixed-precision lookups (the FP32 sweep rounds the frame fields to FP32
 // anyway).  With nf > 0 the first nf of the 2 nc + 2 fields of the state first
 // take the accelerator's step.
-__global__ void __launch_bounds__(256) k_advance_pack(AccConsts C, int nf, int nc, int nn,
+struct k_advance_pack {
+  static constexpr int THREADS = 256, BLOCKS = 1;
+  static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, AccConsts C, int nf, int nc, int nn,
                                                       const double *__restrict__ gx, double *x, double *m,
                                                       const AccState *st, double2 *__restrict__ rf,
                                                       float2 *__restrict__ rf32) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = bid.x * blockDim.x + threadIdx.x;
   if (i >= nn) return;
   const size_t r = (size_t)i * (nc + 1);
   for (int c = 0; c <= nc; ++c) {
@@ -1404,6 +1506,7 @@ __global__ void __launch_bounds__(256) k_advance_pack(AccConsts C, int nf, int n
     if (rf32) rf32[r + c] = make_float2((float)v0, (float)v1);
   }
 }
+};
 
 // Zero outside the reference domain (GeometryGroup::zeroValuesOutsideDomainRef).
 __global__ void k_mask(int n_fields, size_t nn, const uint8_t *__restrict__ dom, double *v) {
@@ -1470,6 +1573,7 @@ struct DevArray {
   }
 };
 
+struct Recorder;    // a phase's launches, for a batch
 struct AdjBuffers;  // adjoint work buffers (adjoint.cuh)
 struct AdjDeleter {
   void operator()(AdjBuffers *p) const;
@@ -1505,8 +1609,6 @@ struct sc_ctx {
   DevArray<int4> items;
   DevArray<double> e_re, e_im, res, res2, coupling;
   float e_re_max = 0.0f;  // over all LDOS energies
-  DevArray<double> filters;
-  DevArray<int> filter_pos;
   DevArray<int> onode_a_g, onode_x_g, onode_y_g, onode_a_gt, onode_x_gt, onode_y_gt;
   std::vector<Chunk> chunks;
   int groups = 1, log_groups = 0, ept = 1;
@@ -1529,7 +1631,7 @@ struct sc_ctx {
   // Poisson transform: side P = 32 * 2^a 3^b 5^c (radix plan), twiddles,
   // kernel spectrum, work arrays (complex).
   int fft_p = 0;
-  FftPlan fft_plan{};
+  FftPlan fft_plan = 0;
   DevArray<double> fft_tw, fft_kf, fft_z;
   DevArray<double> acc_m;
   DevArray<double> and_x, and_d;  // Anderson history [rank][fields][N0*N0] (iterates, residuals)
@@ -1542,6 +1644,7 @@ struct sc_ctx {
   // Work buffers of the sweep (scratch, fields, frame buffers): the
   // context's own arrays, or a batch's shared pool (batch_member).
   bool batch_member = false;
+  int shared_by = 1;  // grains whose kernels are launched together (the batch's)
   // Frame buffers hold zeros wherever the sweep and the extension do not
   // write; with one chunk every slot always holds the same angle, so they are
   // cleared once instead of before every sweep.
@@ -1549,6 +1652,7 @@ struct sc_ctx {
   double *w_scratch = nullptr, *w_scratch2 = nullptr, *w_fr = nullptr;
   size_t need_scratch = 0, need_scratch2 = 0, need_frame = 0;  // bytes of each (frame: fg and gi each)
 
+  Recorder *rec = nullptr;  // set while the launches of a phase are collected
   std::unique_ptr<AdjBuffers, AdjDeleter> adj;  // allocated by the first sc_adjoint
 
   // LDOS postprocess: frame buffer, block accumulator, all energies.
@@ -1612,6 +1716,58 @@ void check_launch(sc_ctx *c) {
   c->launches++;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw EngineError(SC_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
+}
+
+// One launch of a kernel for many grains: the tasks in device memory.
+struct MergedLaunch {
+  const void *kernel = nullptr;
+  dim3 block;
+  size_t smem = 0;
+  unsigned blocks = 0;
+  int n = 0;
+  size_t task_size = 0;
+  std::vector<unsigned char> bytes;  // the tasks until they are uploaded
+  DevArray<unsigned char> tasks;
+  void (*go)(const MergedLaunch &, cudaStream_t) = nullptr;
+};
+// The launches of one grain's phase, kept instead of issued (sc_ctx::rec).
+struct Recorder {
+  struct Entry {
+    const void *kernel;
+    dim3 block;
+    size_t smem;
+    unsigned blocks;
+    std::vector<unsigned char> task;
+    void (*go)(const MergedLaunch &, cudaStream_t);
+  };
+  std::vector<Entry> entries;
+};
+
+template <typename K, typename... P>
+void allow_smem(void (*kernel)(P...), size_t smem) {
+  if (smem > 32 * 1024)  // with the static shared memory possibly above the default 48 KB
+    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+}
+
+// Launches kernel K on the context's stream, or records it when the context
+// collects a phase for a batch.
+template <typename K, typename... P>
+void enqueue(sc_ctx *c, dim3 grid, dim3 block, size_t smem, P... args) {
+  if (c->rec) {
+    Task<P...> t{0u, make_uint3(grid.x, grid.y, grid.z), make_pack(args...)};
+    Recorder::Entry e{(const void *)k_many<K, P...>, block, smem, grid.x * grid.y * grid.z, {}, nullptr};
+    e.task.resize(sizeof(t));
+    std::memcpy(e.task.data(), &t, sizeof(t));
+    e.go = [](const MergedLaunch &m, cudaStream_t s) {
+      allow_smem<K>(k_many<K, P...>, m.smem);
+      k_many<K, P...><<<m.blocks, m.block, m.smem, s>>>((const Task<P...> *)m.tasks.p, m.n);
+    };
+    c->rec->entries.push_back(std::move(e));
+    return;
+  }
+  allow_smem<K>(k_one<K, P...>, smem);
+  k_one<K, P...><<<grid, block, smem, c->stream>>>(args...);
+  check_launch(c);
 }
 
 unsigned grid1(size_t n, int threads) { return (unsigned)std::max<size_t>(1, (n + threads - 1) / threads); }
@@ -1681,8 +1837,7 @@ void launch_frame_fields(sc_ctx *c, const Chunk &ch, const SweepArgs<R> &A) {
   const int rows = 64 * FF_ROWS;
   dim3 grid(grid1(A.n_items, FF_COLS), (unsigned)((ch.kmax + rows - 1) / rows));
   ProfScope prof(c, 4);
-  k_frame_fields<R><<<grid, dim3(FF_COLS, FF_ROWS), 0, c->stream>>>(A, rows);
-  check_launch(c);
+  enqueue<k_frame_fields<R>>(c, grid, dim3(FF_COLS, FF_ROWS), 0, A, rows);
 }
 
 // One launch of the sweep, with the kernel of the context's mapping: EMAX
@@ -1777,17 +1932,15 @@ void extend_reference(sc_ctx *c, bool advance = false) {
   const HostSetup &S = c->S;
   const int nn = (int)c->nn0();
   const AccConsts C = acc_consts(c);
-  k_advance_pack<<<grid1(nn, 256), 256, 0, c->stream>>>(C, advance ? C.nf : 0, S.nc, nn, c->gstate.p, c->xstate.p,
+  enqueue<k_advance_pack>(c, grid1(nn, 256), 256, 0, C, advance ? C.nf : 0, S.nc, nn, c->gstate.p, c->xstate.p,
                                                        c->acc_m.p, c->acc_state.p, (double2 *)c->rfields.p,
                                                        (float2 *)c->rfields32.p);
-  check_launch(c);
   const int ns = (int)S.rext_site.size();
   if (ns) {
     dim3 grid(grid1(ns, 128), 2 * S.nc);
-    k_extend_reference<<<grid, 128, 0, c->stream>>>(2 * S.nc, nn, ns, S.nc + 1, c->rext_site.p, c->rext_off.p,
+    enqueue<k_extend_reference>(c, grid, 128, 0, 2 * S.nc, nn, ns, S.nc + 1, c->rext_site.p, c->rext_off.p,
                                                     c->rext_src.p, c->xstate.p, c->rfields.p,
                                                     (float *)c->rfields32.p);
-    check_launch(c);
   }
 }
 
@@ -1799,8 +1952,7 @@ void boundary_condition(sc_ctx *c) {
                           (Cx<R> *)c->bnd_ptr(0), c->partial_bg.p};
   const BoundarySide<R> gt{S.n_in_gt, c->bc_src_gt.p, c->bc_w_gt.p, c->bc_ws_gt.p, (const Cx<R> *)c->bnd_ptr(3),
                            (Cx<R> *)c->bnd_ptr(2), c->partial_bgt.p};
-  k_boundary<R><<<dim3(c->nb_bnd, 2), REDUCE_THREADS, 0, c->stream>>>(S.ne, g, gt);
-  check_launch(c);
+  enqueue<k_boundary<R>>(c, dim3(c->nb_bnd, 2), REDUCE_THREADS, 0, S.ne, g, gt);
 }
 
 template <typename R>
@@ -1827,21 +1979,24 @@ void boundary_initial(sc_ctx *c) {
 void launch_scalars_b(sc_ctx *c, int do_bc, int do_vp, int compute_mode, size_t n_elem_vp = 0) {
   const HostSetup &S = c->S;
   if (!n_elem_vp) n_elem_vp = 2 * c->nn0();
-  k_scalars_b<<<1, 1024, 0, c->stream>>>(S.norm, (size_t)2 * S.n_in_g * S.ne,
+  enqueue<k_scalars_b>(c, 1, 1024, 0, S.norm, (size_t)2 * S.n_in_g * S.ne,
                                          (size_t)2 * S.n_in_gt * S.ne, n_elem_vp, do_bc, do_vp,
                                          compute_mode, c->partial_bg.p, c->nb_bnd, c->partial_bgt.p,
                                          c->nb_bnd, c->partial_vp.p, c->nb_vp, c->scalars.p);
-  check_launch(c);
 }
 
 // Columns of one block of k_pois_cols: as many as leave a block per SM (four
 // neighbouring columns are a 64-byte run of every row) and about 100 KB of
-// shared memory a block.
-int pois_cols(int P) {
-  int cols = P >= 4 * 148 ? 4 : P >= 2 * 148 ? 2 : 1;
-  while (cols > 1 && (size_t)2 * cols * P * sizeof(double2) > 104 * 1024) cols /= 2;
+// shared memory a block; in a batch, where blocks abound, 28 KB (eight blocks of
+// 256 threads per SM: the transforms' stages wait for one another).
+int pois_cols(const sc_ctx *c) {
+  const int P = c->fft_p;
+  const bool many = c->shared_by > 1;
+  int cols = many || P >= 4 * 148 ? 4 : P >= 2 * 148 ? 2 : 1;
+  while (cols > 1 && (size_t)2 * cols * P * sizeof(double2) > (many ? 28 : 104) * 1024) cols /= 2;
   return cols;
 }
+int pois_threads(int P, int cols) { return cols * P <= 1024 ? 256 : 512; }
 
 // A of the current j: old not null: its residual against old goes to
 // partial_vp (one row of sums per lattice row), and the mean of j is taken
@@ -1851,17 +2006,14 @@ void poisson(sc_ctx *c, const double *j, double *a_out, const double *old) {
   ProfScope prof(c, 2);
   double2 *z = (double2 *)c->fft_z.p;
   const double2 *tw = (const double2 *)c->fft_tw.p;
-  const int cols = pois_cols(P);
+  const int cols = pois_cols(c);
   const size_t row = 2 * (size_t)P * sizeof(double2);
-  k_pois_rows<<<n, P > 1024 ? 512 : 256, row, c->stream>>>(c->fft_plan, n, P, tw, j,
-                                                           old ? c->scalars.p->j_mean : nullptr, z);
-  check_launch(c);
-  k_pois_cols<<<P / cols, 512, cols * row, c->stream>>>(c->fft_plan, P, n, cols, tw, (const double2 *)c->fft_kf.p, z,
-                                                         nullptr);
-  check_launch(c);
-  k_pois_back<<<n, REDUCE_THREADS, row, c->stream>>>(c->fft_plan, n, P, 1.0 / ((double)P * (double)P), tw, z, old,
+  const double *mean = old ? c->scalars.p->j_mean : nullptr;
+  enqueue<k_pois_rows>(c, n, P > 1024 ? 512 : 256, row, c->fft_plan, n, P, tw, j, mean, z);
+  enqueue<k_pois_cols>(c, P / cols, pois_threads(P, cols), cols * row, c->fft_plan, P, n, cols, tw, (const double2 *)c->fft_kf.p, z,
+                       (double2 *)nullptr);
+  enqueue<k_pois_back>(c, n, REDUCE_THREADS, row, c->fft_plan, n, P, 1.0 / ((double)P * (double)P), tw, z, old,
                                                     a_out, c->partial_vp.p);
-  check_launch(c);
 }
 
 // The kernel K(u, v) = -h^2 scale sum_k (+/-) f_k(u) f_k(v), reflected
@@ -1882,14 +2034,15 @@ void poisson_setup(sc_ctx *c) {
   const int P = 32 * m;
   if (P > 4096) throw EngineError(SC_ERR_ARG, "lattice too large for the Poisson transform (N0 > 2048)");
   c->fft_p = P;
-  FftPlan plan{};
+  FftPlan plan = 0;
   {
-    int r = P, twos = 0;
+    int r = P, twos = 0, n = 0;
+    auto stage = [&](unsigned long long radix) { plan |= radix << (4 * n++); };
     while (r % 2 == 0) r /= 2, ++twos;
-    for (int k = 0; k < twos / 2; ++k) plan.radix[plan.n_stages++] = 4;
-    if (twos % 2) plan.radix[plan.n_stages++] = 2;
-    while (r % 3 == 0) r /= 3, plan.radix[plan.n_stages++] = 3;
-    while (r % 5 == 0) r /= 5, plan.radix[plan.n_stages++] = 5;
+    for (int k = 0; k < twos / 2; ++k) stage(4);
+    if (twos % 2) stage(2);
+    while (r % 3 == 0) r /= 3, stage(3);
+    while (r % 5 == 0) r /= 5, stage(5);
   }
   c->fft_plan = plan;
   std::vector<double> tw(2 * (size_t)P);  // exp(-2 pi i q / P), q < P
@@ -1915,17 +2068,13 @@ void poisson_setup(sc_ctx *c) {
   c->fft_z.alloc(2 * pp);
   c->fft_kf.alloc(2 * pp);
   CUDA_TRY(cudaMemcpyAsync(c->fft_z.p, kr.data(), 2 * pp * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  const int cols = pois_cols(P);
+  const int cols = pois_cols(c);
   const size_t row = 2 * (size_t)P * sizeof(double2);
-  for (const void *k : {(const void *)k_pois_rows, (const void *)k_pois_back, (const void *)k_pois_cols})
-    CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
   double2 *z = (double2 *)c->fft_z.p;
-  k_pois_rows<<<P, P > 1024 ? 512 : 256, row, c->stream>>>(c->fft_plan, n, P, (const double2 *)c->fft_tw.p, nullptr,
-                                                           nullptr, z);
-  check_launch(c);
-  k_pois_cols<<<P / cols, 512, cols * row, c->stream>>>(c->fft_plan, P, P, cols, (const double2 *)c->fft_tw.p,
-                                                         nullptr, z, (double2 *)c->fft_kf.p);
-  check_launch(c);
+  enqueue<k_pois_rows>(c, P, P > 1024 ? 512 : 256, row, c->fft_plan, n, P, (const double2 *)c->fft_tw.p,
+                       (const double *)nullptr, (const double *)nullptr, z);
+  enqueue<k_pois_cols>(c, P / cols, pois_threads(P, cols), cols * row, c->fft_plan, P, P, cols, (const double2 *)c->fft_tw.p,
+                       (const double2 *)nullptr, z, (double2 *)c->fft_kf.p);
   CUDA_TRY(cudaStreamSynchronize(c->stream));
 }
 
@@ -1938,21 +2087,17 @@ bool accelerate(sc_ctx *c) {
   if (C.kind == ACC_ANDERSON) {
     const size_t tot = (size_t)C.nf * nn;
     const int rank = S.acc.rank;
-    k_and_store<<<c->nb_acc, REDUCE_THREADS, 0, c->stream>>>(tot, rank, c->xstate.p, c->gstate.p, c->and_x.p,
+    enqueue<k_and_store>(c, c->nb_acc, REDUCE_THREADS, 0, tot, rank, c->xstate.p, c->gstate.p, c->and_x.p,
                                                              c->and_d.p, c->acc_state.p, c->partial_acc.p);
-    check_launch(c);
-    k_and_solve<<<1, 256, 0, c->stream>>>(rank, c->partial_acc.p, c->nb_acc, c->acc_state.p);
-    check_launch(c);
-    k_and_update<<<grid1(tot, 256), 256, 0, c->stream>>>(tot, rank, C.step_size, c->and_x.p, c->and_d.p,
+    enqueue<k_and_solve>(c, 1, 256, 0, rank, c->partial_acc.p, c->nb_acc, c->acc_state.p);
+    enqueue<k_and_update>(c, grid1(tot, 256), 256, 0, tot, rank, C.step_size, c->and_x.p, c->and_d.p,
                                                          c->acc_state.p, c->xstate.p);
-    check_launch(c);
     return false;
   }
   if (C.kind == ACC_CONGACC || C.kind == ACC_BB) {
     dim3 grid(c->nb_acc, C.nf);
-    k_acc_sums<<<grid, REDUCE_THREADS, 0, c->stream>>>(C, nn, c->xstate.p, c->gstate.p, c->acc_m.p,
+    enqueue<k_acc_sums>(c, grid, REDUCE_THREADS, 0, C, nn, c->xstate.p, c->gstate.p, c->acc_m.p,
                                                         c->partial_acc.p, c->acc_state.p, c->counters.p + 1);
-    check_launch(c);
   }
   return true;
 }
@@ -1974,19 +2119,21 @@ void frame_to_reference(sc_ctx *c, const Chunk &ch) {
   const int a_stored = ch.a_begin + chunk_slots(c, ch);
   const int h0 = S.halo_angle_off[ch.a_begin], h1 = S.halo_angle_off[a_stored];
   if (h1 > h0) {
-    k_halo<<<grid1(h1 - h0, 128), 128, 0, c->stream>>>(h1 - h0, h0, S.n1, c->halo_angle.p, ch.a_begin,
+    enqueue<k_halo<Fr>>(c, grid1(h1 - h0, 128), 128, 0, h1 - h0, h0, S.n1, c->halo_angle.p, ch.a_begin,
                                                         c->halo_site.p, c->halo_off.p, c->halo_src.p,
                                                         (Fr *)c->w_fr);
-    check_launch(c);
   }
   // A warp covers an 8 x 4 patch of the reference grid (its rotated corners
   // share cache lines of the frame).
   dim3 blk(8, 32), grid((S.n0 + 7) / 8, (S.n0 + 31) / 32, c->rb_parts);
   ProfScope prof(c, 1);
-  auto kern = S.nc == 1 ? k_rotate_back<Fr, 1> : S.nc == 2 ? k_rotate_back<Fr, 2> : k_rotate_back<Fr, 0>;
-  kern<<<grid, blk, 0, c->stream>>>(S.n0, S.n1, S.nc, ch.a_begin == 0, ch.a_begin, a_stored, pair, c->ang.p, (const Fr *)c->w_fr,
-                                    c->acc_d.p, c->acc_j.p, c->acc_fe.p);
-  check_launch(c);
+  auto go = [&](auto k) {
+    enqueue<decltype(k)>(c, grid, blk, 0, S.n0, S.n1, S.nc, (int)(ch.a_begin == 0), ch.a_begin, a_stored, pair,
+                         (const AngleParams *)c->ang.p, (const Fr *)c->w_fr, c->acc_d.p, c->acc_j.p, c->acc_fe.p);
+  };
+  if (S.nc == 1) go(k_rotate_back<Fr, 1>{});
+  else if (S.nc == 2) go(k_rotate_back<Fr, 2>{});
+  else go(k_rotate_back<Fr, 0>{});
 }
 
 // Lanes per reference site: the smallest of 8, 16, 32 that holds the block's
@@ -2142,11 +2289,14 @@ void launch_finalize(sc_ctx *c, const double *delta, const double *avec) {
   F.sum_inv = si * S.temperature;
   for (int k = 0; k < S.nc; ++k) F.log_t_tc[k] = std::log(S.temperature / S.tc[k]);
   const double jfactor = (double)(2 * S.charge_sign) * S.temperature;
-  auto fin = S.nc == 1 ? k_finalize<1> : S.nc == 2 ? k_finalize<2> : k_finalize<0>;
-  fin<<<c->nb_fin, REDUCE_THREADS, 0, c->stream>>>(
-      S.n0, S.nc, S.h, jfactor, c->has_vp() ? 1 : 0, c->dom.p, c->coupling.p, c->acc_d.p, c->acc_j.p, c->acc_fe.p,
-      delta, avec, c->gstate.p, c->j_real.p, c->partial_fin.p, F, c->scalars.p, c->counters.p, c->rb_parts);
-  check_launch(c);
+  auto go = [&](auto k) {
+    enqueue<decltype(k)>(c, c->nb_fin, REDUCE_THREADS, 0, S.n0, S.nc, S.h, jfactor, c->has_vp() ? 1 : 0, c->dom.p,
+                         c->coupling.p, c->acc_d.p, c->acc_j.p, c->acc_fe.p, delta, avec, c->gstate.p, c->j_real.p,
+                         c->partial_fin.p, F, c->scalars.p, c->counters.p, c->rb_parts);
+  };
+  if (S.nc == 1) go(k_finalize<1>{});
+  else if (S.nc == 2) go(k_finalize<2>{});
+  else go(k_finalize<0>{});
 }
 
 template <typename R>
@@ -2439,10 +2589,6 @@ void upload_static(sc_ctx *c) {
   c->res2.upload(res2, s);
   for (double v : S.ldos_energies) c->e_re_max = std::max(c->e_re_max, (float)std::fabs(v) * 1.001f);
   c->coupling.upload(S.coupling, s);
-  if (S.n_filters) {
-    c->filters.upload(S.filters, s);
-    c->filter_pos.upload(S.filter_pos, s);
-  }
   // Exit nodes (for the homogeneous initial boundary values).
   std::vector<int> ag, xg, yg, agt, xgt, ygt;
   ag.resize(S.n_out_g);
@@ -2545,7 +2691,8 @@ void upload_static(sc_ctx *c) {
   // 12 us, one 31).
   if (!S.keldysh) {
     const size_t tiles = (size_t)((S.n0 + 7) / 8) * ((S.n0 + 31) / 32);
-    const int want = (int)std::min<size_t>(8, (32 * 148 + tiles - 1) / tiles);
+    const size_t all = tiles * c->shared_by;
+    const int want = (int)std::min<size_t>(8, (32 * 148 + all - 1) / all);
     c->rb_parts = std::max(1, std::min(want, max_slots / 4));
     c->acc_d.alloc((size_t)2 * S.nc * nn * c->rb_parts);
     c->acc_j.alloc(2 * nn * c->rb_parts);
@@ -2574,10 +2721,13 @@ void upload_static(sc_ctx *c) {
     c->frames.alloc((size_t)max_slots * n1 * n1 * 4);  // FP64-sized records (the adjoint's buffers too)
     c->w_fr = c->frames.p;
   }
-  c->nb_fin = std::min<int>(592, (int)grid1(nn, REDUCE_THREADS));
-  c->nb_bnd = std::min<int>(592, (int)grid1((size_t)std::max(S.n_in_g, S.n_in_gt) * S.ne, REDUCE_THREADS));
+  // Blocks of the reductions: up to four per SM, shared with the batch's other
+  // grains.
+  const int share = std::max(8, 592 / c->shared_by), share_acc = std::max(4, 148 / c->shared_by);
+  c->nb_fin = std::min<int>(share, (int)grid1(nn, REDUCE_THREADS));
+  c->nb_bnd = std::min<int>(share, (int)grid1((size_t)std::max(S.n_in_g, S.n_in_gt) * S.ne, REDUCE_THREADS));
   c->nb_vp = S.keldysh ? std::min<int>(592, (int)grid1(nn, REDUCE_THREADS)) : S.n0;  // LDOS finalize blocks; Poisson rows
-  c->nb_acc = std::min<int>(148, (int)grid1(nn, REDUCE_THREADS));
+  c->nb_acc = std::min<int>(share_acc, (int)grid1(nn, REDUCE_THREADS));
   c->partial_fin.alloc((size_t)c->nb_fin * NQ);
   c->partial_bg.alloc((size_t)c->nb_bnd * 6);
   c->partial_bgt.alloc((size_t)c->nb_bnd * 6);
@@ -3235,6 +3385,13 @@ struct sc_batch {
     std::vector<std::unique_ptr<Pass>> passes;  // energy passes, swept one after another
   };
   std::vector<std::unique_ptr<Wave>> waves;
+  // The kernels of a steady iteration other than the sweeps, each one launch
+  // over all grains that run it: before the sweeps, before and after the sweep
+  // of every wave, after all.  Built for a plan by batch_program.
+  using Phase = std::vector<std::unique_ptr<MergedLaunch>>;
+  Phase pre, post;
+  std::vector<Phase> wave_pre, wave_post;
+  bool program_dirty = true;
   DevArray<int> counters;
   DevArray<const Scalars *> scalar_src;
   DevArray<Scalars> scalars;  // gathered [grain] after every iteration
@@ -3366,6 +3523,89 @@ void batch_plan(sc_batch *b) {
   b->counters.alloc(std::max<size_t>(1, b->waves.size()));
   CUDA_TRY(cudaStreamSynchronize(b->stream));
   b->graph_dirty = true;
+  b->program_dirty = true;
+}
+
+// Records what `issue` launches for every listed grain and merges the recorded
+// sequences: as long as a grain has launches left, the first one's next kernel
+// is launched for all grains whose next kernel it is too, so that every grain's
+// kernels keep their order.
+template <typename F>
+void batch_phase(sc_batch *b, const std::vector<int> &grains, sc_batch::Phase &out, F issue) {
+  std::vector<Recorder> recs(grains.size());
+  for (size_t k = 0; k < grains.size(); ++k) {
+    sc_ctx *c = b->grains[grains[k]];
+    c->rec = &recs[k];
+    try {
+      issue(c);
+    } catch (...) {
+      c->rec = nullptr;
+      throw;
+    }
+    c->rec = nullptr;
+  }
+  out.clear();
+  std::vector<size_t> at(grains.size(), 0);
+  for (;;) {
+    size_t first = 0;
+    while (first < recs.size() && at[first] == recs[first].entries.size()) ++first;
+    if (first == recs.size()) break;
+    const Recorder::Entry &head = recs[first].entries[at[first]];
+    auto m = std::make_unique<MergedLaunch>();
+    m->kernel = head.kernel;
+    m->block = head.block;
+    m->go = head.go;
+    m->task_size = head.task.size();
+    for (size_t k = first; k < recs.size(); ++k) {
+      if (at[k] == recs[k].entries.size()) continue;
+      Recorder::Entry &e = recs[k].entries[at[k]];
+      if (e.kernel != m->kernel || e.block.x != m->block.x || e.block.y != m->block.y || e.block.z != m->block.z) continue;
+      ++at[k];
+      std::memcpy(e.task.data(), &m->blocks, sizeof(unsigned));  // Task::first
+      m->bytes.insert(m->bytes.end(), e.task.begin(), e.task.end());
+      m->blocks += e.blocks;
+      m->smem = std::max(m->smem, e.smem);
+      ++m->n;
+    }
+    m->tasks.upload(m->bytes, b->stream);
+    out.push_back(std::move(m));
+  }
+  CUDA_TRY(cudaStreamSynchronize(b->stream));  // the host copies of the tasks are done with
+}
+void run_phase(sc_batch *b, const sc_batch::Phase &ph) {
+  for (const auto &m : ph) {
+    m->go(*m, b->stream);
+    b->launches++;
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) throw EngineError(SC_ERR_CUDA, std::string("batch launch: ") + cudaGetErrorString(e));
+  }
+}
+
+// The merged launches of a steady iteration of the active grains; frame
+// buffers that a new plan moved are cleared here.
+template <typename R>
+void batch_program(sc_batch *b) {
+  std::vector<int> all;
+  for (int g = 0; g < (int)b->grains.size(); ++g)
+    if (b->active[g]) all.push_back(g);
+  for (int g : all) {
+    sc_ctx *c = b->grains[g];
+    if (c->frames_zeroed) continue;
+    const size_t nn1 = (size_t)c->S.n1 * c->S.n1;
+    CUDA_TRY(cudaMemsetAsync(c->w_fr, 0, (size_t)chunk_slots(c, c->chunks[0]) * nn1 * c->frame_rec(), b->stream));
+    c->frames_zeroed = true;
+  }
+  batch_phase(b, all, b->pre, [](sc_ctx *c) { compute_pre<R>(c); });
+  b->wave_pre.resize(b->waves.size());
+  b->wave_post.resize(b->waves.size());
+  for (size_t w = 0; w < b->waves.size(); ++w) {
+    batch_phase(b, b->waves[w]->grains, b->wave_pre[w], [](sc_ctx *c) {
+      launch_frame_fields<R>(c, c->chunks[0], sweep_args<R>(c, &c->chunks[0], 0));
+    });
+    batch_phase(b, b->waves[w]->grains, b->wave_post[w], [](sc_ctx *c) { frame_to_reference<R>(c, c->chunks[0]); });
+  }
+  batch_phase(b, all, b->post, [](sc_ctx *c) { compute_post<R>(c); });
+  b->program_dirty = false;
 }
 
 template <typename R>
@@ -3465,13 +3705,34 @@ void batch_iteration(sc_batch *b) {
   b->launches++;
 }
 
+// A steady iteration through the merged launches.
+template <typename R>
+void batch_steady(sc_batch *b) {
+  run_phase(b, b->pre);
+  for (size_t w = 0; w < b->waves.size(); ++w) {
+    run_phase(b, b->wave_pre[w]);
+    launch_batch_sweep<R>(b, *b->waves[w], (int)w);
+    run_phase(b, b->wave_post[w]);
+  }
+  run_phase(b, b->post);
+  k_gather_scalars<<<grid1(b->grains.size(), 128), 128, 0, b->stream>>>((int)b->grains.size(), b->scalar_src.p,
+                                                                          b->scalars.p);
+  b->launches++;
+}
+
 template <typename R>
 void batch_step(sc_batch *b) {
   bool first = false;
   for (size_t g = 0; g < b->grains.size(); ++g)
     if (b->active[g] && (b->grains[g]->first_compute || !b->grains[g]->boundary_initialized)) first = true;
-  if (!b->use_graph || first) {
+  if (!first && b->program_dirty) {
+    batch_program<R>(b);
+    b->graph_dirty = true;  // the graph launches the old program's tasks
+  }
+  if (first) {
     batch_iteration<R>(b);  // first iterations differ (no accelerator step, initial boundary)
+  } else if (!b->use_graph) {
+    batch_steady<R>(b);
   } else {
     if (b->graph_dirty || !b->exec) {
       if (b->exec) {
@@ -3484,7 +3745,7 @@ void batch_step(sc_batch *b) {
       for (const sc_ctx *c : b->grains) grain_launches0 += c->launches;
       CUDA_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
       try {
-        batch_iteration<R>(b);
+        batch_steady<R>(b);
       } catch (...) {
         cudaStreamEndCapture(b->stream, &graph);
         if (graph) cudaGraphDestroy(graph);
@@ -3568,6 +3829,7 @@ int sc_batch_create(const char *const *configs, int n, int mode, sc_batch **out)
       b->grains.push_back(c);
       c->mode = mode;
       c->batch_member = true;
+      c->shared_by = n;
     }
     // Host set-up of the grains in parallel (pure host work).
     std::vector<std::string> errs(n);

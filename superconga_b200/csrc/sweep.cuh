@@ -374,7 +374,7 @@ __device__ __forceinline__ void sweep_tile(const SweepArgs<R> &A, const double *
       ldo += o_step * A.ne_stride;
     } else {
       // Sums over this thread's energies of r (f + f~*), r Re g and
-      // r Im(conj(D) g - D gt) (local_greens): with p = g gt,
+      // r Im(conj(D) g - D gt): with p = g gt,
       // i 2 / (1 + p) = (fre, fim), and d = (other - own), v = (own + other),
       //   f + f~* = (+-(fre d.re - fim d.im), -(fre v.im + fim v.re)),
       //   Re g = -fre,   Im I = -(D_own.re d.im + D.im v.re),
@@ -516,11 +516,8 @@ __device__ __forceinline__ void sweep_tile(const SweepArgs<R> &A, const double *
       if constexpr (LATE)
         if (green) greens(pdre, pdim, (pcode & SITE_LABEL) != 0);
       if (step) {
-#ifndef NOFASTGEN
         if (fast) fast_steps(dre, dim, es);
-        else
-#endif
-          general_steps(code & SITE_LABEL, dre, dim, es);
+        else general_steps(code & SITE_LABEL, dre, dim, es);
         if (!want_gt && !burn_in) store();
       }
       if constexpr (!LATE)
