@@ -944,9 +944,10 @@ struct k_boundary {
   static __device__ __forceinline__ void run(uint3 bid, uint3 gdim, int ne, BoundarySide<R> g, BoundarySide<R> gt) {
   const BoundarySide<R> &B = bid.y ? gt : g;
   double q[6] = {0, 0, 0, 0, 0, 0};
-  const unsigned total = (unsigned)B.n_in * ne;
-  for (unsigned t = bid.x * blockDim.x + threadIdx.x; t < total; t += gdim.x * blockDim.x) {
-    const unsigned k = t / (unsigned)ne, e = t - k * ne;
+  const size_t total = (size_t)B.n_in * ne;
+  const bool narrow = total >> 32 == 0;  // a 32-bit division where it is enough
+  for (size_t t = bid.x * blockDim.x + threadIdx.x; t < total; t += gdim.x * blockDim.x) {
+    const unsigned k = narrow ? (unsigned)t / (unsigned)ne : (unsigned)(t / (unsigned)ne), e = (unsigned)(t - (size_t)k * ne);
     const int4 src = ((const int4 *)B.src)[k];
     const double2 w01 = ((const double2 *)B.w)[2 * (size_t)k], w23 = ((const double2 *)B.w)[2 * (size_t)k + 1];
     const int si[4] = {src.x, src.y, src.z, src.w};
@@ -3923,6 +3924,8 @@ int sc_batch_compute(sc_batch *b, int n, int *n_active) {
     }
   } catch (const EngineError &e) {
     return batch_fail(b, e);
+  } catch (const std::exception &e) {
+    return batch_fail(b, EngineError(SC_ERR_ARG, e.what()));
   }
   return SC_OK;
 }
@@ -4020,13 +4023,11 @@ extern "C" {
 
 // Autotuner of the persistent batch sweep: tries the mappings of trajectory
 // columns to threads (at most 1, 2, 4 or 8 energies per thread, each grain
-// taking the fewest threads per column that allow it, up to 8) with the
-// resident-block variants that fit them (registers capped at 80, 128 or 255
-// per thread), times the sweeps of all waves for each on the current state,
-// keeps the fastest and returns it.
+// taking the fewest threads per column that allow it), times the sweeps of all
+// waves for each on the current state, keeps the fastest and returns it.
 int sc_batch_autotune(sc_batch *b, int *energies_per_thread, int *minb, double *best_ms) {
   if (!b) return SC_ERR_ARG;
-  const int cand[][2] = {{1, 4}, {2, 4}, {2, 6}, {4, 3}, {4, 4}, {4, 1}, {8, 1}};
+  const int cand[][2] = {{1, 4}, {2, 4}, {4, 4}, {8, 1}};
   int best_e = b->ept_max, best_mb = b->minb;
   double best = 1e300;
   for (const auto &cd : cand) {

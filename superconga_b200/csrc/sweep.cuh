@@ -254,6 +254,9 @@ __device__ __forceinline__ void sweep_tile(const SweepArgs<R> &A, const double *
   const size_t site0 = (size_t)(a - A.slot_base) * nn1 + (size_t)(lo + (down ? n_rows - 1 - first : first)) * n1 + x;
   Fr *rec = A.fr + 2 * site0;
   typename LdosOf<R>::type *ldo = A.ldf + site0 * A.ne_stride + e0;
+  // 16-byte stores of four energies: the frame's base (an energy pass's slice
+  // starts anywhere) and its sites must be aligned; e0 is a multiple of four.
+  const bool ldos_vec = KEL && EMAX == 4 && (A.ne_stride & 3) == 0 && ((size_t)A.ldf & 15) == 0;
   bool bounded = true;  // every entering value inside the unit disc
   int pcode = SITE_GENERAL, slot = 0;
   R pdre = 0, pdim = 0, pes = 0;
@@ -360,7 +363,7 @@ __device__ __forceinline__ void sweep_tile(const SweepArgs<R> &A, const double *
         }
         bool done = false;
         if constexpr (PK && EMAX == 4) {
-          if (ecount == 4 && (A.ne_stride & 3) == 0) {
+          if (ldos_vec && ecount == 4) {
             *(float4 *)ldo = make_float4(im[0], im[1], im[2], im[3]);
             done = true;
           }

@@ -138,6 +138,34 @@ def test_entering_values_outside_the_unit_disc(engine_lib):
     assert _rel(e.boundary(3), o.boundary(3)) < 1e-8
 
 
+@pytest.mark.parametrize("per_block", [80, 132])
+def test_ldos_blocks_in_one_pass_and_two(engine_lib, per_block):
+    """Blocks of 80 and 132 real energies on a small grain: one pass, and two
+    of 66 whose slice of the frame is not 16-byte aligned; mixed against FP64
+    (1e-4 of the largest value, the bound of the other LDOS tests), FP64 against
+    the passes of 32 (another order of nothing but the boundary: 1e-12)."""
+    import os
+    import superconga_b200 as sb
+    sim = _grain(0.3, True, angles=16)
+    out = {}
+    for key, mode, env in (("fp64", "fp64", None), ("passes", "fp64", "8"), ("mixed", "mixed", None)):
+        if env:
+            os.environ["SCB_ENERGY_GROUPS"] = env
+        try:
+            e = sb.LdosContext(sim, configs.ldos_postprocess(0.2, n_energies=per_block, per_block=per_block, n_angles=16),
+                               mode=mode)
+        finally:
+            os.environ.pop("SCB_ENERGY_GROUPS", None)
+        d, a = configs.seeded_state(1, e.dims.n0, 0.2, 3, 0.05, True, 0.02)
+        e.set_state(d, a)
+        e.begin_block(0)
+        e.burn_in(1)
+        e.iterate(2)
+        out[key] = e.ldos()
+    assert _rel(out["passes"], out["fp64"]) < 1e-12
+    assert _rel(out["mixed"], out["fp64"]) < 1e-4
+
+
 @pytest.mark.parametrize("mode", ["fp64", "mixed"])
 def test_batch_of_unlike_grains(engine_lib, mode):
     """Merged launches over grains whose kernels differ: one and two
