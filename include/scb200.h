@@ -129,8 +129,8 @@ int sc_get_external_field(const sc_ctx *ctx, double *b_ext);
  * sc_get_results then returns that pass's Delta, j and A. */
 int sc_evaluate(sc_ctx *ctx, double *free_energy);
 
-/* Reverse-mode derivative of L at the current state (checkpointed adjoint
- * Riccati sweeps, gamma kept every 16 sites).  beta_j [2][N0][N0] host (NULL:
+/* Reverse-mode derivative of L at the current state (adjoint Riccati sweeps
+ * over both coherence functions, stored at every site).  beta_j [2][N0][N0] host (NULL:
  * no current term); outputs, host, any may be NULL: g_delta [Nc][2][N0][N0]
  * = dL/dRe Delta, dL/dIm Delta; g_a [2][N0][N0] = dL/dA (internal units);
  * *g_b = dL/dB_ext. */
@@ -287,12 +287,11 @@ int sc_batch_grain_state(const sc_batch *b, int *state);
 /* CUDA-graph replay of the iteration on (default) or off. */
 int sc_batch_set_graph(sc_batch *b, int enable);
 /* Mapping of the persistent sweep: each grain takes the fewest threads per
- * trajectory column (1, 2, 4 or 8) that keep at most energies_per_thread
- * energies on a thread, and minb selects the resident-block variant (1: up
- * to 255 registers per thread, 3: at most 168, 4: at most 128, 6: at most 80;
- * 3 with at most four energies per thread, 6 with at most two; the default is four energies per thread and
- * minb 4).  In mixed precision a cap of two or four runs the packed FP32 sweep (each grain's energies per thread
- * rounded up to even).  sc_batch_autotune times the feasible choices on the current state (after at least one
+ * trajectory column and coherence function (1, 2, 4, 8 or 16) that keep at most
+ * energies_per_thread energies on a thread (a cap of eight or 16: seven in
+ * FP64, eight in mixed precision).  minb (1, 3, 4 or 6) is accepted and
+ * reported; every mapping has one register variant.  The default is four
+ * energies per thread and minb 4.  sc_batch_autotune times the feasible choices on the current state (after at least one
  * iteration) and keeps the fastest. */
 int sc_batch_config(sc_batch *b, int energies_per_thread, int minb);
 int sc_batch_get_config(const sc_batch *b, int *energies_per_thread, int *minb, int *n_waves);

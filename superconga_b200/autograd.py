@@ -7,7 +7,7 @@ L = w_omega * Omega + sum(beta_j * j) for the complex order parameter
 (0-d float64, B0 units), evaluated on the engine context ``ctx`` with its
 incoming boundary values held fixed (one frozen-boundary pass of the
 self-consistency map, ComputeFreeEnergy.h:281-414, ComputeCurrent.h:175-222).
-``backward`` runs the adjoint sweep (gamma checkpointed every 16 sites) and
+``backward`` runs the adjoint sweep and
 returns dL/dDelta, dL/dA and dL/dB_ext in PyTorch's convention for complex
 inputs (dL/dRe + i dL/dIm).
 
