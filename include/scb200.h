@@ -289,7 +289,9 @@ int sc_batch_set_graph(sc_batch *b, int enable);
 /* Mapping of the persistent sweep: each grain takes the fewest threads per
  * trajectory column and coherence function (1, 2, 4, 8 or 16) that keep at most
  * energies_per_thread energies on a thread (a cap of eight or 16: seven in
- * FP64, eight in mixed precision).  minb (1, 3, 4 or 6) is accepted and
+ * FP64, eight in mixed precision).  Where 16 threads do not hold a grain's
+ * energies (17 to 32 under a cap of one, 33 to 64 under one or two), the grains
+ * swept together with it take two or four per thread.  minb (1, 3, 4 or 6) is accepted and
  * reported; every mapping has one register variant.  The default is four
  * energies per thread and minb 4.  sc_batch_autotune times the feasible choices on the current state (after at least one
  * iteration) and keeps the fastest. */

@@ -3383,6 +3383,7 @@ struct sc_batch {
   };
   struct Wave {
     std::vector<int> grains;
+    int ept = 1;  // energies per thread of the wave's sweep kernel (EMAX) and of all its grains' mappings
     std::vector<std::unique_ptr<Pass>> passes;  // energy passes, swept one after another
   };
   std::vector<std::unique_ptr<Wave>> waves;
@@ -3470,10 +3471,20 @@ void batch_plan(sc_batch *b) {
     auto wv = std::make_unique<sc_batch::Wave>();
     wv->grains = m;
     int n_passes = 1;
+    // One kernel sweeps the wave, so all its grains take the same energies per
+    // thread: the batch's cap, or the least above it for which 16 threads hold
+    // every grain's pass (cap 1 holds 16 energies, cap 2 holds 32).
+    wv->ept = b->ept();
+    for (int g : m) {
+      set_mapping(b->grains[g], wv->ept);
+      wv->ept = b->grains[g]->ept;
+    }
     for (int k = 0; k < (int)m.size(); ++k) {
       sc_ctx *c = b->grains[m[k]];
       const int ne = c->e_pass;  // energies per pass: all of them up to 64, else 32
-      set_mapping(c, b->ept());
+      set_mapping(c, wv->ept);
+      if (c->ept != wv->ept || (c->ept << c->log_groups) < ne)
+        throw EngineError(SC_ERR_STATE, "batch: the sweep's mapping does not hold a grain's energies");
       n_passes = std::max(n_passes, (c->S.ne + ne - 1) / ne);
     }
     for (int p = 0; p < n_passes; ++p) {
@@ -3623,7 +3634,7 @@ void launch_batch_sweep(sc_batch *b, sc_batch::Wave &w, int wi) {
       const int blocks = std::max(1, per_sm) * b->n_sm;
       kernel<<<blocks, 128, smem, b->stream>>>(args, ps.units.p, ps.n_units, counter);
     };
-    const int ept = b->ept();
+    const int ept = w.ept;
     if constexpr (sizeof(R) == 8) {
       if (ept == 1) run(k_sweep_batch<R, 1, 5, false>, SweepRing<R, 1, 5, false>::BYTES);
       else if (ept == 2) run(k_sweep_batch<R, 2, 3, false>, SweepRing<R, 2, 3, false>::BYTES);

@@ -521,8 +521,9 @@ class Batch:
 
     def config(self, energies_per_thread: int, minb: int):
         """Each grain takes the fewest threads per column that keep at most
-        ``energies_per_thread`` energies on a thread; ``minb`` is accepted and
-        reported (every mapping has one register variant)."""
+        ``energies_per_thread`` energies on a thread (more where 16 threads do
+        not hold a grain's energies); ``minb`` is accepted and reported (every
+        mapping has one register variant)."""
         self._check(_lib.load().sc_batch_config(self._h, int(energies_per_thread), int(minb)))
 
     def get_config(self):

@@ -239,3 +239,52 @@ def test_nan_state_never_reads_as_converged(engine_lib):
         res, conv = e.compute(2)
         assert not np.isfinite(res) and not conv, norm
         e.close()
+
+
+def _study(counts=((0.5, 8.0, 7), (0.05, 8.0, 20), (0.01, 8.0, 45), (0.005, 16.0, 89))):
+    """Small discs of (temperature, cutoff) with the given numbers of Ozaki energies."""
+    from oracle import oracle as O
+    cfgs, states = [], []
+    for i, (t, cut, ne) in enumerate(counts):
+        c = configs.small_disc()
+        c["physics"]["temperature"] = t
+        c["numerics"]["energy_cutoff"] = cut
+        s = O.make_setup(c)
+        assert s.n_energies == ne
+        cfgs.append(c)
+        states.append(configs.seeded_state(s.n_comp, s.n0, O.delta_bulk(t, s.symmetries[0]), 20 + i, 0.05, True, 0.02))
+    return cfgs, states
+
+
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+@pytest.mark.parametrize("cap", [1, 2, 4, 8, "autotune"])
+def test_batch_sweeps_every_energy_under_every_cap(engine_lib, mode, cap):
+    """Grains of 7, 20, 45 and 89 energies: 16 threads of one or two energies
+    do not hold 17 to 64, and the sweep takes more per thread then.  State,
+    current, free energy and outgoing boundary values are those of the grains
+    run alone (mixed: of another mapping of energies to threads, as in the
+    low-temperature test)."""
+    import superconga_b200 as sb
+    cfgs, states = _study()
+    b = sb.Batch(cfgs, mode=mode)
+    for g, (d, a) in zip(b.grains, states):
+        g.set_state(d, a)
+    if cap == "autotune":
+        b.compute(1)
+        b.autotune()
+        b.compute(2)
+    else:
+        b.config(cap, 4)
+        b.compute(3)
+    tol = 1e-11 if mode == "fp64" else 1e-4
+    for g, c, (d, a) in zip(b.grains, cfgs, states):
+        e = sb.Context(c, mode=mode)
+        e.set_state(d, a)
+        e.compute(3)
+        assert _rel(g.results()[0], e.results()[0]) < tol
+        assert _rel(g.results()[1], e.results()[1]) < 100 * tol
+        assert abs(g.scalars()["free_energy"] - e.scalars()["free_energy"]) <= tol * abs(e.scalars()["free_energy"])
+        for which in range(4):
+            assert _rel(g.boundary(which), e.boundary(which)) < tol
+        e.close()
+    b.close()
