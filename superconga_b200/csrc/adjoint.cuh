@@ -96,15 +96,15 @@ __device__ __forceinline__ void riccati_step_adj(double dre, double dim, double 
 //                                          B1 = (i h e - 1) / 2)
 // the reverse is a dozen complex products on values the forward step has too;
 // |w| and 1 / |w| come from one estimate.
-__device__ __forceinline__ Cx<double> step_fast_adj(const SiteConst<double> &S, double s0h, double sh, double bh,
+__device__ __forceinline__ Cx<double> step_fast_adj(const SiteConst<double> &S, double s0, double sh, double d,
                                                     double h, Cx<double> g0, Cx<double> gw, Cx<double> &gD,
                                                     double &ge) {
   typedef Cx<double> C;
-  const double ure = S.ar * g0.re - S.ai * g0.im, uim = S.ar * g0.im + S.ai * g0.re;
-  const double br = ure + bh, bi = uim + sh;
-  const double tr = br + (bh + 2.0), ti = bi + sh;
+  const double urd = S.ar * g0.re - (S.ai * g0.im + d), uim = S.ar * g0.im + S.ai * g0.re;
+  const double br = urd - 0.5, bi = uim + sh;
+  const double tr = (urd - d) + 1.0, ti = bi + sh;
   const double cre = tr * g0.re - (ti * g0.im + S.hdi), cim = tr * g0.im + (ti * g0.re + S.hdr);
-  const double xh = (0.5 * bh * bh + s0h) - ure, y = bh * sh - uim;
+  const double xh = (0.5 * ((d * d + s0) - d) - urd) + 0.125, y = -(d * sh + (0.5 * sh + uim));
   const double xx = xh * xh + (y * y + 1e-300);  // |w|^2 / 4
   const double rm = rsqrt_(xx), m = xx * rm;     // 2 / |w|, |w| / 2
   const double U = m + xh, rho = rsqrt_pos(U);
@@ -124,8 +124,8 @@ __device__ __forceinline__ Cx<double> step_fast_adj(const SiteConst<double> &S, 
   G0.re += S.ar * Gu.re + S.ai * Gu.im;  // conj(a) Gu
   G0.im += S.ar * Gu.im - S.ai * Gu.re;
   // Re e through i h e: B1 carries half of it, t a further half.
-  //   G of i h e = Gt + Gb / 2 + conj(B1) Gw, B1 = (bh, sh); its imaginary part
-  ge += h * (Gt.im + 0.5 * Gb.im + (bh * Gw.im - sh * Gw.re));
+  //   G of i h e = Gt + Gb / 2 + conj(B1) Gw, B1 = (-1/2 - d, sh); its imaginary part
+  ge += h * (Gt.im + 0.5 * Gb.im - ((0.5 + d) * Gw.im + sh * Gw.re));
   // P = (-hdi, hdr): G_P = Gc - conj(a) Gw;  a: G_a = conj(g0) Gu - conj(P) Gw
   const C GP{Gc.re - (S.ar * Gw.re + S.ai * Gw.im), Gc.im - (S.ar * Gw.im - S.ai * Gw.re)};
   const C Ga{g0.re * Gu.re + g0.im * Gu.im + (S.hdi * Gw.re - S.hdr * Gw.im),
@@ -166,10 +166,10 @@ __global__ void __launch_bounds__(128, 3) k_adjoint(const AdjArgs J) {
   const size_t nn1 = (size_t)n1 * n1;
   const double h = A.ang[a].hs;
   const int e0 = g * EMAX, ecount = min(max(ne - e0, 0), EMAX);
-  double bh[EMAX], rr[EMAX];
+  double hd[EMAX], rr[EMAX];  // h e_im / 2, residue
 #pragma unroll
   for (int j = 0; j < EMAX; ++j) {
-    bh[j] = -0.5 - 0.5 * h * ((j < ecount) ? A.e_im[e0 + j] : 1.0);
+    hd[j] = 0.5 * h * ((j < ecount) ? A.e_im[e0 + j] : 1.0);
     rr[j] = (j < ecount) ? A.res[e0 + j] : 0.0;
   }
   const size_t ax = (size_t)a * n1 + x;
@@ -206,9 +206,9 @@ __global__ void __launch_bounds__(128, 3) k_adjoint(const AdjArgs J) {
     const double dre = down ? -fr.x : fr.x, dim = fr.y, es = fr.z;
     if (code == 1 && pcode < SITE_GENERAL && bounded) {
       const SiteConst<double> S = site_const<double>((dre + p0) * 0.5, (dim + p1) * 0.5, (es + p2) * 0.5, h);
-      const double s0h = S.s0h - 0.5 * S.sh * S.sh;
+      const double s0 = 2.0 * S.s0h - S.sh * S.sh;
 #pragma unroll
-      for (int j = 0; j < EMAX; ++j) coh[j] = step_fast<double>(S, s0h, S.sh, bh[j], coh[j]);
+      for (int j = 0; j < EMAX; ++j) coh[j] = step_fast(S, s0, S.sh, hd[j], coh[j]);
     } else {
       const bool entry = l == l_entry;
       const double st = entry ? dist_in[in_base + n_in] * h : h;
@@ -341,9 +341,9 @@ __global__ void __launch_bounds__(128, 3) k_adjoint(const AdjArgs J) {
         double nE = 0.0;
         if (code == 1 && has && bcode < SITE_GENERAL && bounded) {
           const SiteConst<double> S = site_const<double>(mre, mim, mes, h);
-          const double s0h = S.s0h - 0.5 * S.sh * S.sh;
+          const double s0 = 2.0 * S.s0h - S.sh * S.sh;
 #pragma unroll
-          for (int j = 0; j < EMAX; ++j) lam[j] = step_fast_adj(S, s0h, S.sh, bh[j], h, gin[j], lam[j], nD, nE);
+          for (int j = 0; j < EMAX; ++j) lam[j] = step_fast_adj(S, s0, S.sh, hd[j], h, gin[j], lam[j], nD, nE);
         } else {
 #pragma unroll
           for (int j = 0; j < EMAX; ++j)

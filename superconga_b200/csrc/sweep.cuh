@@ -138,8 +138,8 @@ __device__ __forceinline__ void sweep_tile(const SweepArgs<R> &A, const double *
   const int e0 = g * EMAX;
   const int ecount = min(max(ne - e0, 0), EMAX);
 
-  // Interior constants of the energies: FP64 bh = -(1 + h e_im) / 2, FP32
-  // d = h e_im / 2 (rounded from FP64) and what step_fast2 takes of it.
+  // Interior constants of the energies: d = h e_im / 2 (rounded from FP64) and
+  // what step_fast2 takes of it.
   constexpr int NP = PK ? EMAX / 2 : 1;
   R ec[PK ? 1 : EMAX], ere[KEL ? EMAX : 1];
   EnergyConst2 ec2[NP];
@@ -147,7 +147,7 @@ __device__ __forceinline__ void sweep_tile(const SweepArgs<R> &A, const double *
   for (int j = 0; j < EMAX; ++j) {
     const double d = 0.5 * A.ang[a].hs * ((j < ecount) ? A.e_im[e0 + j] : 1.0);
     if constexpr (KEL) ere[j] = (j < ecount) ? (R)A.e_re[e0 + j] : R(0);
-    if constexpr (!PK) ec[j] = sizeof(R) == 8 ? R(-0.5 - d) : R(d);
+    if constexpr (!PK) ec[j] = R(d);
     if constexpr (PK) {
       const float c[4] = {(float)(0.5 + d), (float)(1.0 + d), (float)(0.5 * (d + d * d)), (float)(3.0 * d)};
       EnergyConst2 &E = ec2[j / 2];
@@ -278,16 +278,18 @@ __device__ __forceinline__ void sweep_tile(const SweepArgs<R> &A, const double *
         coh2[p] = step_fast2(S2, s0h, nsh, n3sh, ec2[p], coh2[p]);
       }
     } else {
-      const R s0h_site = S.s0h - R(0.5) * S.sh * S.sh;
+      // FP64: s0; FP32: half of it.
+      constexpr R c2 = sizeof(R) == 8 ? 2 : 1, c1 = sizeof(R) == 8 ? 1 : 0.5;
+      const R s0_site = c2 * S.s0h - c1 * S.sh * S.sh;
 #pragma unroll
       for (int j = 0; j < EMAX; ++j) {
-        R sh = S.sh, s0h = s0h_site;
+        R sh = S.sh, s0 = s0_site;
         if constexpr (KEL) {
           sh += R(0.5) * h * ere[j];
-          s0h = S.s0h - R(0.5) * sh * sh;
+          s0 = c2 * S.s0h - c1 * sh * sh;
         }
-        if constexpr (sizeof(R) == 8) coh[j] = step_fast<R>(S, s0h, sh, ec[j], coh[j]);
-        else coh[j] = step_fast_f32(S, s0h, sh, ec[j], coh[j]);
+        if constexpr (sizeof(R) == 8) coh[j] = step_fast(S, s0, sh, ec[j], coh[j]);
+        else coh[j] = step_fast_f32(S, s0, sh, ec[j], coh[j]);
       }
     }
   };

@@ -240,3 +240,29 @@ def test_autograd_takes_tensors_of_any_place_and_layout(engine_lib):
         assert c.device.type == "cpu" and g.device.type == "cuda"
         assert _rel(c.detach().numpy(), r.detach().cpu().numpy()) < 1e-12
         assert _rel(g.detach().cpu().numpy(), r.detach().cpu().numpy()) < 1e-12
+
+
+@pytest.mark.parametrize("broadening", [0.05, 0.02, 0.008])
+def test_short_step_rounds_like_the_general_one(engine_lib, broadening):
+    """The LDOS of a disc in FP64 against the oracle, which takes the general
+    step everywhere.  A step rounds at about 2^-53 in both, a column remembers
+    the last 1 / (2 h delta) sites (broadening delta), and independent errors
+    add up as the square root of their number; the bound is 1.5 of that (B200:
+    0.2).  An error that all steps of an energy share adds up in proportion to
+    the sites (a rounded 1 + h e: 2 to 2.9)."""
+    from oracle import oracle as O
+    import superconga_b200 as sb
+    points = 12.0
+    sim = _grain(0.5, True, ppxi=points, size=6.0, angles=16)
+    db = O.delta_bulk(0.5, "s")
+    pp = configs.ldos_postprocess(db, n_energies=12, per_block=12, n_angles=16, broadening=broadening)
+    L = O.LdosOracle(sim, pp)
+    e = sb.LdosContext(sim, pp, mode="fp64")
+    d, a = configs.seeded_state(1, e.dims.n0, db, 6, 0.05, True, 0.02)
+    for c in (L, e):
+        c.set_state(d, a)
+        c.begin_block(0)
+    L.iterate()
+    e.iterate(1)
+    diff = np.linalg.norm(e.ldos() - L.ldos) / np.linalg.norm(L.ldos)
+    assert diff < 1.5 * 2.0 ** -53 * np.sqrt(points / (2.0 * broadening))
