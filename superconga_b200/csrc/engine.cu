@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "../../include/scb200.h"
+#include "dev_array.hpp"
 #include "device.cuh"
 #include "setup.hpp"
 
@@ -41,19 +42,6 @@ using namespace scb;
 namespace {
 
 thread_local std::string g_create_error;
-
-#define CUDA_TRY(expr)                                                          \
-  do {                                                                          \
-    cudaError_t _e = (expr);                                                    \
-    if (_e != cudaSuccess)                                                      \
-      throw EngineError(SC_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(_e)); \
-  } while (0)
-
-struct EngineError {
-  int code;
-  std::string msg;
-  EngineError(int c, std::string m) : code(c), msg(std::move(m)) {}
-};
 
 constexpr int REDUCE_THREADS = 256;
 // Ozaki energies one sweep pass takes (the residues sit in shared memory);
@@ -1547,33 +1535,6 @@ __global__ void __launch_bounds__(256) k_fma_peak(int iters, T a, T b, T *out) {
 }
 
 // --------------------------------------------------------------- helpers --
-template <typename T>
-struct DevArray {
-  T *p = nullptr;
-  size_t n = 0;
-  DevArray() = default;
-  DevArray(const DevArray &) = delete;
-  DevArray &operator=(const DevArray &) = delete;
-  ~DevArray() { free(); }
-  void alloc(size_t count) {
-    free();
-    n = count;
-    if (count) CUDA_TRY(cudaMalloc(&p, count * sizeof(T)));
-  }
-  void upload(const std::vector<T> &v, cudaStream_t s) {
-    alloc(v.size());
-    if (n) CUDA_TRY(cudaMemcpyAsync(p, v.data(), n * sizeof(T), cudaMemcpyHostToDevice, s));
-  }
-  void zero(cudaStream_t s) {
-    if (n) CUDA_TRY(cudaMemsetAsync(p, 0, n * sizeof(T), s));
-  }
-  void free() {
-    if (p) cudaFree(p);
-    p = nullptr;
-    n = 0;
-  }
-};
-
 struct Recorder;    // a phase's launches, for a batch
 struct AdjBuffers;  // adjoint work buffers (adjoint.cuh)
 struct AdjDeleter {
