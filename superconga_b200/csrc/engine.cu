@@ -1705,10 +1705,19 @@ struct Recorder {
   std::vector<Entry> entries;
 };
 
-template <typename K, typename... P>
+// Allows kernel K's launch form the dynamic shared memory that a block can have
+// beside its static one.  Always the same value: threads with contexts of
+// different lattices share the kernel, and a smaller one set by one of them
+// between another's setting and its launch would fail that launch.
+template <typename... P>
 void allow_smem(void (*kernel)(P...), size_t smem) {
-  if (smem > 32 * 1024)  // with the static shared memory possibly above the default 48 KB
-    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem <= 32 * 1024) return;  // with the static shared memory below the default 48 KB
+  int dev = 0, most = 0;
+  cudaFuncAttributes fa{};
+  CUDA_TRY(cudaGetDevice(&dev));
+  CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
+  CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes));
 }
 
 // Launches kernel K on the context's stream, or records it when the context
@@ -1721,13 +1730,13 @@ void enqueue(sc_ctx *c, dim3 grid, dim3 block, size_t smem, P... args) {
     e.task.resize(sizeof(t));
     std::memcpy(e.task.data(), &t, sizeof(t));
     e.go = [](const MergedLaunch &m, cudaStream_t s) {
-      allow_smem<K>(k_many<K, P...>, m.smem);
+      allow_smem(k_many<K, P...>, m.smem);
       k_many<K, P...><<<m.blocks, m.block, m.smem, s>>>((const Task<P...> *)m.tasks.p, m.n);
     };
     c->rec->entries.push_back(std::move(e));
     return;
   }
-  allow_smem<K>(k_one<K, P...>, smem);
+  allow_smem(k_one<K, P...>, smem);
   k_one<K, P...><<<grid, block, smem, c->stream>>>(args...);
   check_launch(c);
 }

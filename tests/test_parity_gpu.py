@@ -663,3 +663,40 @@ def test_group_sizes_match_oracle(engine_lib, monkeypatch, groups):
         assert np.max(np.abs(d_m - d_e)) / db <= 1e-5, (groups, it)
     e.close()
     m.close()
+
+
+def test_threads_with_lattices_of_different_sizes(engine_lib):
+    """Contexts of different lattices in threads of their own: their Poisson
+    kernels are the same ones with different amounts of shared memory, and no
+    thread's setting may fail another's launch.  Every solve equals the same
+    solve alone."""
+    import threading
+    import superconga_b200 as sb
+
+    def context(points):
+        cfg = configs.small_square_d()
+        cfg["geometry"][0]["regular_polygon"]["side_length"] = 20.0
+        cfg["numerics"]["points_per_coherence_length"] = points
+        cfg["numerics"]["num_fermi_momenta"] = 4
+        return sb.Context(cfg, mode="mixed")
+
+    failed = []
+
+    def solves(e, j, want):
+        for _ in range(300):
+            try:
+                if not np.array_equal(e.poisson(j), want):
+                    failed.append("differs")
+            except Exception as x:
+                failed.append(repr(x))
+
+    threads = []
+    for points in (14.0, 19.0, 14.0, 19.0, 16.0, 18.0):  # 20 to 102 KB a block
+        e = context(points)
+        j = np.random.default_rng(0).standard_normal((2, e.dims.n0, e.dims.n0))
+        threads.append(threading.Thread(target=solves, args=(e, j, e.poisson(j))))
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, (len(failed), failed[:3])
