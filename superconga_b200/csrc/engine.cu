@@ -3588,6 +3588,7 @@ void batch_program(sc_batch *b) {
   }
   batch_phase(b, all, b->post, [](sc_ctx *c) { compute_post<R>(c); });
   b->program_dirty = false;
+  b->graph_dirty = true;  // the graph launches the old program's tasks
 }
 
 template <typename R>
@@ -3702,17 +3703,35 @@ void batch_steady(sc_batch *b) {
   b->launches++;
 }
 
+// Whether the next iteration launches every grain's kernels by themselves: an
+// active grain's first one differs (no accelerator step, initial boundary).
+bool batch_apart(const sc_batch *b) {
+  for (size_t g = 0; g < b->grains.size(); ++g)
+    if (b->active[g] && (b->grains[g]->first_compute || !b->grains[g]->boundary_initialized)) return true;
+  return false;
+}
+
+// The sweeps of all waves with the frame fields before and the rotation back
+// after them, as the next iteration will launch them.
+template <typename R>
+void batch_time_step(sc_batch *b) {
+  if (batch_apart(b)) {
+    batch_sweeps<R>(b);
+    return;
+  }
+  for (size_t w = 0; w < b->waves.size(); ++w) {
+    run_phase(b, b->wave_pre[w]);
+    launch_batch_sweep<R>(b, *b->waves[w], (int)w);
+    run_phase(b, b->wave_post[w]);
+  }
+}
+
 template <typename R>
 void batch_step(sc_batch *b) {
-  bool first = false;
-  for (size_t g = 0; g < b->grains.size(); ++g)
-    if (b->active[g] && (b->grains[g]->first_compute || !b->grains[g]->boundary_initialized)) first = true;
-  if (!first && b->program_dirty) {
-    batch_program<R>(b);
-    b->graph_dirty = true;  // the graph launches the old program's tasks
-  }
-  if (first) {
-    batch_iteration<R>(b);  // first iterations differ (no accelerator step, initial boundary)
+  const bool apart = batch_apart(b);
+  if (!apart && b->program_dirty) batch_program<R>(b);
+  if (apart) {
+    batch_iteration<R>(b);
   } else if (!b->use_graph) {
     batch_steady<R>(b);
   } else {
@@ -3961,21 +3980,26 @@ int sc_batch_get_config(const sc_batch *b, int *energies_per_thread, int *minb, 
   return SC_OK;
 }
 
-// Times the sweeps of all waves for the current configuration (no state
-// changes: the sweeps rewrite the same outgoing boundary values and frames).
+// Times the sweeps of all waves for the current configuration, through the
+// launches of the iteration that follows (no state changes: the sweeps rewrite
+// the same outgoing boundary values and frames).
 int sc_batch_time_sweeps(sc_batch *b, int repeats, double *ms) {
   if (!b || repeats < 1 || !ms) return SC_ERR_ARG;
   try {
     for (size_t g = 0; g < b->grains.size(); ++g)
       if (b->active[g] && !b->grains[g]->boundary_initialized)
         throw EngineError(SC_ERR_STATE, "sc_batch_time_sweeps: run one iteration first");
+    if (b->program_dirty && !batch_apart(b)) {
+      if (b->mode == SC_MODE_FP64) batch_program<double>(b);
+      else batch_program<float>(b);
+    }
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
     CUDA_TRY(cudaEventCreate(&e1));
     CUDA_TRY(cudaEventRecord(e0, b->stream));
     for (int r = 0; r < repeats; ++r) {
-      if (b->mode == SC_MODE_FP64) batch_sweeps<double>(b);
-      else batch_sweeps<float>(b);
+      if (b->mode == SC_MODE_FP64) batch_time_step<double>(b);
+      else batch_time_step<float>(b);
     }
     CUDA_TRY(cudaEventRecord(e1, b->stream));
     CUDA_TRY(cudaEventSynchronize(e1));

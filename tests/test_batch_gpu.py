@@ -288,3 +288,33 @@ def test_batch_sweeps_every_energy_under_every_cap(engine_lib, mode, cap):
             assert _rel(g.boundary(which), e.boundary(which)) < tol
         e.close()
     b.close()
+
+
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+def test_batch_times_the_launches_that_it_runs(engine_lib, mode):
+    """time_sweeps of a steady batch launches what its iteration launches
+    around the sweep, for all grains together: fewer launches per repeat than
+    grains, and fewer than an iteration.  The state and what follows are those
+    of a batch that was not timed."""
+    import superconga_b200 as sb
+    cfgs, states = _grains()
+    cfgs, states = cfgs * 3, states * 3  # more grains than launches in a repeat
+    batches = [sb.Batch(cfgs, mode=mode) for _ in range(2)]
+    for b in batches:
+        for g, (d, a) in zip(b.grains, states):
+            g.set_state(d, a)
+        b.compute(2)
+    b, untimed = batches
+    n = b.launch_count()
+    assert b.time_sweeps(1) > 0.0
+    timed = b.launch_count() - n
+    n = b.launch_count()
+    b.compute(1)
+    untimed.compute(1)
+    assert 0 < timed < len(cfgs) and timed < b.launch_count() - n
+    b.compute(1)
+    untimed.compute(1)
+    for g, u in zip(b.grains, untimed.grains):
+        assert np.array_equal(g.results()[0], u.results()[0])
+    for x in batches:
+        x.close()
