@@ -311,7 +311,9 @@ int sc_measure_fma_peak(int precision, double *flops_per_second);
  * sweep, 1 rotation back to the reference grid, 2 Poisson filters, 3 boundary
  * condition, 4 frame fields (the rotated order parameter, Doppler shift and
  * labels of each chunk's trajectory sites).  sc_profile_read returns the summed device time and number of
- * timed launches since the last read, and resets them. */
+ * timed launches since the last read, and resets them.  A batch runs kernels 1
+ * to 4 for all its grains together; while a grain is timed it launches every
+ * grain's by themselves.  The sweep (0) of a batch belongs to no grain. */
 int sc_profile(sc_ctx *ctx, int enable);
 int sc_profile_read(sc_ctx *ctx, int kernel, double *total_ms, long long *launches);
 

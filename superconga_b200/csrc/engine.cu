@@ -3704,10 +3704,13 @@ void batch_steady(sc_batch *b) {
 }
 
 // Whether the next iteration launches every grain's kernels by themselves: an
-// active grain's first one differs (no accelerator step, initial boundary).
+// active grain's first one differs (no accelerator step, initial boundary), and
+// a grain whose kernels are timed (sc_profile) needs launches of its own.
 bool batch_apart(const sc_batch *b) {
-  for (size_t g = 0; g < b->grains.size(); ++g)
-    if (b->active[g] && (b->grains[g]->first_compute || !b->grains[g]->boundary_initialized)) return true;
+  for (size_t g = 0; g < b->grains.size(); ++g) {
+    const sc_ctx *c = b->grains[g];
+    if (b->active[g] && (c->first_compute || !c->boundary_initialized || c->profiling)) return true;
+  }
   return false;
 }
 

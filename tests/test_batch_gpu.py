@@ -318,3 +318,38 @@ def test_batch_times_the_launches_that_it_runs(engine_lib, mode):
         assert np.array_equal(g.results()[0], u.results()[0])
     for x in batches:
         x.close()
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_a_batch_grain_can_be_timed(engine_lib, graph):
+    """sc_profile on one grain: its rotation back, Poisson solve, boundary and
+    frame-field kernels are timed once per iteration, with the results of a
+    batch that is not timed; afterwards the batch runs as before."""
+    import superconga_b200 as sb
+    cfgs, states = _grains()
+    batches = [sb.Batch(cfgs, mode="fp64") for _ in range(2)]
+    for b in batches:
+        b.set_graph(graph)
+        for g, (d, a) in zip(b.grains, states):
+            g.set_state(d, a)
+        b.compute(2)
+    timed, plain = batches
+    g = timed.grains[1]
+    g.profile(True)
+    timed.compute(3)
+    plain.compute(3)
+    for kernel in (1, 2, 3, 4):
+        ms, n = g.profile_read(kernel)
+        assert n == 3 and ms > 0.0, kernel
+    g.profile(False)
+    n = timed.launch_count()
+    timed.compute(2)
+    n2 = plain.launch_count()
+    plain.compute(2)
+    assert timed.launch_count() - n == plain.launch_count() - n2
+    for kernel in (1, 2, 3, 4):
+        assert g.profile_read(kernel)[1] == 0
+    for x, y in zip(timed.grains, plain.grains):
+        assert np.array_equal(x.results()[0], y.results()[0])
+    for b in batches:
+        b.close()
