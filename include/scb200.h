@@ -130,8 +130,11 @@ int sc_get_external_field(const sc_ctx *ctx, double *b_ext);
 int sc_evaluate(sc_ctx *ctx, double *free_energy);
 
 /* Reverse-mode derivative of L at the current state (adjoint Riccati sweeps
- * over both coherence functions, stored at every site).  beta_j [2][N0][N0] host (NULL:
- * no current term); outputs, host, any may be NULL: g_delta [Nc][2][N0][N0]
+ * over both coherence functions, stored at every site).  The first call takes
+ * device memory for one of them, at most 40% of what is then free, and the
+ * context keeps it until sc_destroy; where that is not room for all of it, a
+ * call runs in several launches and a later one takes more if it is there.
+ * beta_j [2][N0][N0] host (NULL: no current term); outputs, host, any may be NULL: g_delta [Nc][2][N0][N0]
  * = dL/dRe Delta, dL/dIm Delta; g_a [2][N0][N0] = dL/dA (internal units);
  * *g_b = dL/dB_ext. */
 int sc_adjoint(sc_ctx *ctx, double w_omega, const double *beta_j, double *g_delta, double *g_a,

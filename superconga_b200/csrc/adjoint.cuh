@@ -694,13 +694,24 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_j)
   }
   // gamma of as many tiles as fit 40% of the free memory (all of them unless
   // the sweep's own scratch already takes most of the device), at least one.
-  if (!B.g_all.n && tiles) {
+  // The buffer is kept for the next gradient; one that was made when memory
+  // was short grows once all tiles, or twice as many as before, would fit.
+  const size_t held = B.g_all.n * sizeof(double);
+  if (held < tiles * tile_bytes) {
     size_t free_b = 0, total_b = 0;
     CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-    double budget = 0.4 * (double)free_b;
+    double budget = 0.4 * (double)(free_b + held);
     if (const char *env = std::getenv("SCB_SCRATCH_MB")) budget = std::min(budget, std::atof(env) * 1048576.0);
     const size_t fit = std::max<size_t>(1, (size_t)budget / tile_bytes);
-    B.g_all.alloc(std::min(tiles, fit) * tile_bytes / sizeof(double));
+    const size_t want = std::min(tiles, fit) * tile_bytes;
+    if (!held || want == tiles * tile_bytes || want >= 2 * held) {
+      try {
+        B.g_all.alloc(want / sizeof(double));
+      } catch (const EngineError &) {  // no piece of that size: as before
+        if (!held) throw;
+        B.g_all.alloc(held / sizeof(double));
+      }
+    }
   }
   if (B.grad_e.n < slots * nn1) B.grad_e.alloc(slots * nn1);
   ensure(B.g_dext, (size_t)2 * S.nc * nn);

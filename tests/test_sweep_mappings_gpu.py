@@ -266,3 +266,30 @@ def test_short_step_rounds_like_the_general_one(engine_lib, broadening):
     e.iterate(1)
     diff = np.linalg.norm(e.ldos() - L.ldos) / np.linalg.norm(L.ldos)
     assert diff < 1.5 * 2.0 ** -53 * np.sqrt(points / (2.0 * broadening))
+
+
+def test_the_adjoints_buffer_grows_when_memory_is_there(engine_lib, monkeypatch):
+    """A first gradient with room for a few tiles only takes many launches; once
+    the room is there, the next one takes as many as a context that always had
+    it, and they agree."""
+    cfg = _grain(0.3, True)
+    e, f = _pair(cfg)[1], _pair(cfg)[1]
+    for c in (e, f):
+        c.boundary_initial()
+    beta = np.random.default_rng(3).standard_normal((2, e.dims.n0, e.dims.n0))
+
+    def gradient(c):
+        n = c.launch_count()
+        out = c.adjoint(0.7, beta)
+        return out, c.launch_count() - n
+
+    monkeypatch.setenv("SCB_SCRATCH_MB", "0.05")
+    first, bounded = gradient(e)
+    still, held = gradient(e)
+    monkeypatch.delenv("SCB_SCRATCH_MB")
+    again, free = gradient(e)
+    want, launches = gradient(f)
+    assert bounded == held > launches and free == launches
+    for got in (first, still, again):
+        for x, y in zip(got, want):
+            assert _rel(x, y) < 1e-11
