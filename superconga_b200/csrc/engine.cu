@@ -166,6 +166,11 @@ __device__ __forceinline__ void ldg_d2x2(const double2 *p, double2 &a, double2 &
       : "l"(p));
 }
 
+// Four consecutive doubles in one 256-bit store (sm_100); p must be 32-byte aligned.
+__device__ __forceinline__ void st_d4(double *p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
 // A frame site's record is two frame elements, (Re F, Im F) then (Re g, Re I):
 // 16 bytes in FP32, 32 in FP64, read with one load (the buffers are 256-byte
 // aligned and the records packed).

@@ -254,9 +254,12 @@ __device__ __forceinline__ void sweep_tile(const SweepArgs<R> &A, const double *
   const size_t site0 = (size_t)(a - A.slot_base) * nn1 + (size_t)(lo + (down ? n_rows - 1 - first : first)) * n1 + x;
   Fr *rec = A.fr + 2 * site0;
   typename LdosOf<R>::type *ldo = A.ldf + site0 * A.ne_stride + e0;
-  // 16-byte stores of four energies: the frame's base (an energy pass's slice
-  // starts anywhere) and its sites must be aligned; e0 is a multiple of four.
-  const bool ldos_vec = KEL && EMAX == 4 && (A.ne_stride & 3) == 0 && ((size_t)A.ldf & 15) == 0;
+  // One store of four energies (16 or 32 bytes): the frame's base (an energy
+  // pass's slice starts anywhere) and its sites must be aligned; e0 is a
+  // multiple of four.  In FP64 four stores of 8 bytes write every 32-byte sector
+  // of the frame four times (64 angles, 32 energies: sweep of a 286^2 disc 2.20
+  // -> 1.93 ms, of a 487^2 square 8.34 -> 7.37 ms).
+  const bool ldos_vec = KEL && EMAX == 4 && (A.ne_stride & 3) == 0 && ((size_t)A.ldf & (4 * sizeof(*ldo) - 1)) == 0;
   bool bounded = true;  // every entering value inside the unit disc
   int pcode = SITE_GENERAL, slot = 0;
   R pdre = 0, pdim = 0, pes = 0;
@@ -364,9 +367,10 @@ __device__ __forceinline__ void sweep_tile(const SweepArgs<R> &A, const double *
           for (int j = 0; j < EMAX; ++j) im[j] = greens_g_im<R>(coh[j], gt[j]);
         }
         bool done = false;
-        if constexpr (PK && EMAX == 4) {
+        if constexpr (EMAX == 4) {
           if (ldos_vec && ecount == 4) {
-            *(float4 *)ldo = make_float4(im[0], im[1], im[2], im[3]);
+            if constexpr (PK) *(float4 *)ldo = make_float4(im[0], im[1], im[2], im[3]);
+            else st_d4((double *)ldo, im[0], im[1], im[2], im[3]);
             done = true;
           }
         }

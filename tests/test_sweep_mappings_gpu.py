@@ -293,3 +293,28 @@ def test_the_adjoints_buffer_grows_when_memory_is_there(engine_lib, monkeypatch)
     for got in (first, still, again):
         for x, y in zip(got, want):
             assert _rel(x, y) < 1e-11
+
+
+@pytest.mark.parametrize("per_block,groups", [(13, 4), (16, 4), (18, 8), (32, 8), (66, 8)])
+def test_ldos_frames_of_four_energies_a_thread(engine_lib, monkeypatch, per_block, groups):
+    """FP64 LDOS with four energies a thread: blocks whose sites are 32-byte
+    aligned in the frame and blocks whose sites are not, a last thread with
+    fewer than four, and a last pass of two: against the oracle (1e-10, as in
+    the other parity tests)."""
+    from oracle import oracle as O
+    import superconga_b200 as sb
+    monkeypatch.setenv("SCB_ENERGY_GROUPS", str(groups))
+    sim = _grain(0.5, True, angles=16)
+    db = O.delta_bulk(0.5, "s")
+    pp = configs.ldos_postprocess(db, n_energies=per_block, per_block=per_block, n_angles=16)
+    L = O.LdosOracle(sim, pp)
+    e = sb.LdosContext(sim, pp, mode="fp64")
+    d, a = configs.seeded_state(1, e.dims.n0, db, 6, 0.05, True, 0.02)
+    for c in (L, e):
+        c.set_state(d, a)
+        c.begin_block(0)
+    L.burn_in()
+    e.burn_in(1)
+    L.iterate()
+    e.iterate(1)
+    assert _rel(e.ldos(), L.ldos) < TOL
