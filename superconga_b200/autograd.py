@@ -47,8 +47,9 @@ class FreeEnergy(torch.autograd.Function):
         av = _on_gpu(a, torch.float64, 2 * n0 * n0, "a").resolve_neg().reshape(2, n0, n0).clone(
             memory_format=torch.contiguous_format)
         b = float(b_ext.detach().cpu())
+        # In C order whatever the weight's own: backward hands its address on.
         beta = None if beta_j is None else torch.from_numpy(
-            np.array(beta_j, np.float64)).to(d.device)
+            np.array(beta_j, np.float64, order="C")).to(d.device)
         torch.cuda.current_stream().synchronize()
         ctx.set_state_device(d.data_ptr(), av.data_ptr())
         ctx.set_external_field(b)

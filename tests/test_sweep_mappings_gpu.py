@@ -221,11 +221,12 @@ def test_autograd_takes_tensors_of_any_place_and_layout(engine_lib):
     d, a = configs.seeded_state(1, n0, 0.2, 4, 0.05, True, 0.02)
     e.set_state(d, a)
     e.boundary_initial()
-    beta = np.random.default_rng(1).standard_normal((2, n0, n0))
+    row = np.random.default_rng(1).standard_normal((2, 1, n0))
+    beta, spread = np.repeat(row, n0, axis=1), np.broadcast_to(row, (2, n0, n0))
     z = torch.from_numpy(d[:, 0] + 1j * d[:, 1])
 
-    def grads(delta, av, b):
-        loss = autograd.FreeEnergy.apply(delta, av, b, e, 1.0, beta)
+    def grads(delta, av, b, weight=beta):
+        loss = autograd.FreeEnergy.apply(delta, av, b, e, 1.0, weight)
         return (loss, *torch.autograd.grad(loss, [delta, av, b]))
 
     b0 = e.external_field()
@@ -235,7 +236,7 @@ def test_autograd_takes_tensors_of_any_place_and_layout(engine_lib):
                 torch.tensor(b0, dtype=torch.float64, requires_grad=True))
     view = z.conj().resolve_conj().cuda().conj().detach().requires_grad_()  # lazily conjugated
     at = torch.from_numpy(a).cuda().transpose(1, 2).contiguous().transpose(1, 2).detach().requires_grad_()
-    got = grads(view, at, torch.tensor(b0, dtype=torch.float64, device="cuda", requires_grad=True))
+    got = grads(view, at, torch.tensor(b0, dtype=torch.float64, device="cuda", requires_grad=True), spread)
     for r, c, g in zip(ref, cpu, got):
         assert c.device.type == "cpu" and g.device.type == "cuda"
         assert _rel(c.detach().numpy(), r.detach().cpu().numpy()) < 1e-12
