@@ -739,7 +739,6 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_j)
     SweepArgs<double> A = sweep_args<double>(c, &ch, 0);
     if (!A.n_items) continue;
     A.log_groups = lg;  // the records in the adjoint's tiles
-    A.groups = 1 << lg;
     launch_frame_fields<double>(c, ch, A);
     // The frame-record buffer (two double2 per site and slot) holds both.
     double2 *seed = (double2 *)c->w_fr, *grad_d = seed + (size_t)nslots * nn1;
@@ -782,7 +781,7 @@ void adjoint_run(sc_ctx *c, AdjBuffers &B, double w_omega, const double *beta_j)
     }
     // As in k_rotate_back: 8 x 4 patches a warp, the angles in parts.
     dim3 gridf((S.n0 + 7) / 8, (S.n0 + 31) / 32);
-    gridf.z = std::max(1, std::min<int>(8, (int)((32 * 148) / (gridf.x * gridf.y)) + 1));
+    gridf.z = std::max(1, std::min<int>(8, (int)((32 * c->n_sm) / (gridf.x * gridf.y)) + 1));
     k_adj_fields_t<<<gridf, dim3(8, 32), 0, c->stream>>>(A, ch.a_begin, ch.a_end, B.rows.p, grad_d, B.grad_e.p,
                                                          B.g_dext.p, B.g_avec.p);
     check_launch(c);

@@ -8,9 +8,10 @@
 //                     packed with A into one record per reference site
 //   per angle chunk:
 //     frame_fields    order parameter and Doppler shift along every column
-//     sweep           gammaTilde down every trajectory column (stored), gamma up,
-//                     Green sums over the Ozaki energies -> frame buffers;
-//                     outgoing boundary values written in sparse order
+//     sweep           gammaTilde down and gamma up every trajectory column at
+//                     the same time, each stored until they meet; then Green
+//                     sums over the Ozaki energies -> frame buffers; outgoing
+//                     boundary values written in sparse order
 //     halo            frame extension next to the boundary (domain_ops.h:11-69)
 //     rotate_back     frame -> reference grid, accumulated angle by angle
 //   finalize          Delta, j, free energy, residuals (ComputeOrderParameter.h,
@@ -189,7 +190,7 @@ __device__ __forceinline__ FrameRec load_rec(const double2 *fr, size_t i) {
 
 template <typename R>
 struct SweepArgs {
-  int n0, n1, ne, nc, groups, log_groups, ept, n_items;
+  int n0, n1, ne, nc, log_groups, n_items;
   int ne_stride;   // energies per boundary entry (all of them; ne counts this pass's)
   int accumulate;  // add the pass's Matsubara sums to the frame instead of storing them
   int burn_in, has_vp, has_ext, gauge;
@@ -1571,7 +1572,7 @@ struct sc_ctx {
   cudaStream_t own_stream = nullptr;  // the stream this context created
   std::string err;
   long long launches = 0;
-  int device = 0;
+  int device = 0, n_sm = 148;
 
   // static data
   DevArray<AngleParams> ang;
@@ -1766,9 +1767,7 @@ SweepArgs<R> sweep_args(sc_ctx *c, const Chunk *ch, int burn_in) {
   A.ne = S.ne;
   A.ne_stride = S.ne;
   A.nc = S.nc;
-  A.groups = c->groups;
   A.log_groups = c->log_groups;
-  A.ept = c->ept;
   A.n_items = ch ? ch->item_end - ch->item_begin : 0;
   A.burn_in = burn_in;
   A.has_vp = c->has_vp();
@@ -1977,7 +1976,7 @@ void launch_scalars_b(sc_ctx *c, int do_bc, int do_vp, int compute_mode, size_t 
 int pois_cols(const sc_ctx *c) {
   const int P = c->fft_p;
   const bool many = c->shared_by > 1;
-  int cols = many || P >= 4 * 148 ? 4 : P >= 2 * 148 ? 2 : 1;
+  int cols = many || P >= 4 * c->n_sm ? 4 : P >= 2 * c->n_sm ? 2 : 1;
   while (cols > 1 && (size_t)2 * cols * P * sizeof(double2) > (many ? 28 : 104) * 1024) cols /= 2;
   return cols;
 }
@@ -2007,8 +2006,8 @@ void poisson(sc_ctx *c, const double *j, double *a_out, const double *old) {
 void poisson_setup(sc_ctx *c) {
   const HostSetup &S = c->S;
   const int n = S.n0;
-  // The smallest side P >= 2 N0 - 1 of the form 32 * 2^a 3^b 5^c (a multiple
-  // of the 32-wide transpose tiles whose rows the mixed-radix FFT handles).
+  // The smallest side P >= 2 N0 - 1 of the form 32 * 2^a 3^b 5^c: the
+  // transform's radices, and a multiple of the columns of a block of k_pois_cols.
   auto smooth = [](int m) {
     for (int f : {2, 3, 5})
       while (m % f == 0) m /= f;
@@ -2440,10 +2439,7 @@ int sweep_pass(const sc_ctx *c) {
   size_t columns = 0;
   for (int lo : S.col_lo) columns += lo >= 0;
   if (c->pair) columns /= 2;
-  int dev = 0, n_sm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-  const double warps = (double)columns * 2 * 8 / 32 / (4.0 * n_sm);  // eight threads per column and function
+  const double warps = (double)columns * 2 * 8 / 32 / (4.0 * c->n_sm);  // eight threads per column and function
   if (warps >= 6.0) return ENERGY_PASS;
   const int most = 16 * (c->mode == SC_MODE_MIXED ? 8 : 7), passes = (S.ne + most - 1) / most;
   return (S.ne + passes - 1) / passes;
@@ -2468,16 +2464,27 @@ void set_mapping(sc_ctx *c, int ept) {
 // The mapping of a single context.  A thread with more energies interleaves
 // more independent recursions and shares the site's loads, reductions and
 // bookkeeping among them; a thread with fewer leaves more warps for a grain of
-// few columns.  Measured on B200 (sweep of the 606 x 606 d-wave square, 14
-// energies, per energy slot, relative): FP64 one energy 1.64, two 1.23, four
-// 1.00, seven 1.06; FP32 two 1.32, four 1.00, eight 0.95 (real energies, whose
-// constants are per energy: eight 1.15).  Slots round the energies up to
-// EMAX * 2^lg, so 14 energies on seven a thread beat 16 slots on four, 20 real
-// energies 21 slots on seven (5.3 ms) 32 slots on four (6.4 ms).  The cheapest
-// product is taken among the mappings that give every scheduler enough warps
-// (1.5 to 5, by the mapping's own parallelism), else the one with the most
-// warps: a 4 xi0 disc in FP32, 0.5 warps per scheduler at two energies, takes
-// 37 us per sweep with one, 46 with two and 55 with four.
+// few columns.  Threads per column are a power of two, so the slots are
+// EMAX * 2^lg: 14 energies take 14 slots on seven a thread and 16 on four, 20
+// take 20 on five, 24 on six, 28 on seven and 32 on four.
+// Cost per slot relative to four energies a thread in 16 slots, measured on B200
+// (sweep of the 606 x 606 d-wave square, 256 angles; the energies that fill
+// the slots best: 14 of 16 on one, two and four, 14 on seven, 10 on five, 12 on
+// six; 1.11 and 0.308 ms a slot):
+//   FP64  one 1.50, two 1.24, five 1.07, six 1.00, seven 1.03
+//   FP32  one 2.27, two 1.24, six 1.01 (10 of 12: 0.97), eight 0.95
+//   FP32, real energies (24 on six, 24 of 32 on four and eight): six 1.26 (20
+//         energies 1.12), eight 1.06
+// The costs below stand within 15% of these, but for FP32's one energy a thread,
+// which is taken for its warps alone.  With 10, 12 and 14 Ozaki energies and 20
+// and 24 real ones the rule takes the fastest mapping of those measured, within
+// 1%; two counts are left where it does not: seven Ozaki energies (FP64 seven a
+// thread 9.4 ms, four 8.9; FP32 eight 2.95, four 2.80) and 12 real ones (FP32
+// six 2.56 ms, four 2.16).
+// The cheapest product is taken among the mappings that give every scheduler
+// enough warps (1.5 to 5, by the mapping's own parallelism), else the one with
+// the most warps: a 4 xi0 disc in FP32, 0.5 warps per scheduler at two energies,
+// takes 37 us per sweep with one, 46 with two and 55 with four.
 void plan_mapping(sc_ctx *c) {
   const bool fp32 = c->mode == SC_MODE_MIXED, kel = c->S.keldysh;
   struct Option {
@@ -2495,9 +2502,6 @@ void plan_mapping(sc_ctx *c) {
     set_mapping(c, need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : cap);
     return;
   }
-  int dev = 0, n_sm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
   size_t items = 0;
   for (const Chunk &ch : c->chunks) items = std::max(items, (size_t)(ch.item_end - ch.item_begin));
   double best = 1e300;
@@ -2505,7 +2509,7 @@ void plan_mapping(sc_ctx *c) {
   for (int k = 0; k < (fp32 ? 5 : 6); ++k) {
     set_mapping(c, opt[k].ept);
     if (c->ept != opt[k].ept) continue;  // more than 16 threads per column
-    const double warps = (double)items * 2 * c->groups / 32 / (4.0 * n_sm);
+    const double warps = (double)items * 2 * c->groups / 32 / (4.0 * c->n_sm);
     if (warps < opt[k].warps) continue;
     const double cost = opt[k].cost * (opt[k].ept << c->log_groups);
     if (cost < best) {
@@ -2518,6 +2522,8 @@ void plan_mapping(sc_ctx *c) {
 
 void upload_static(sc_ctx *c) {
   HostSetup &S = c->S;
+  CUDA_TRY(cudaGetDevice(&c->device));
+  CUDA_TRY(cudaDeviceGetAttribute(&c->n_sm, cudaDevAttrMultiProcessorCount, c->device));
   cudaStream_t s = c->stream;
   const int na = S.n_angles;
   std::vector<AngleParams> ap(na);
@@ -2677,7 +2683,7 @@ void upload_static(sc_ctx *c) {
   if (!S.keldysh) {
     const size_t tiles = (size_t)((S.n0 + 7) / 8) * ((S.n0 + 31) / 32);
     const size_t all = tiles * c->shared_by;
-    const int want = (int)std::min<size_t>(8, (32 * 148 + all - 1) / all);
+    const int want = (int)std::min<size_t>(8, (32 * c->n_sm + all - 1) / all);
     c->rb_parts = std::max(1, std::min(want, max_slots / 4));
     c->acc_d.alloc((size_t)2 * S.nc * nn * c->rb_parts);
     c->acc_j.alloc(2 * nn * c->rb_parts);
@@ -2708,10 +2714,10 @@ void upload_static(sc_ctx *c) {
   }
   // Blocks of the reductions: up to four per SM, shared with the batch's other
   // grains.
-  const int share = std::max(8, 592 / c->shared_by), share_acc = std::max(4, 148 / c->shared_by);
+  const int share = std::max(8, 4 * c->n_sm / c->shared_by), share_acc = std::max(4, c->n_sm / c->shared_by);
   c->nb_fin = std::min<int>(share, (int)grid1(nn, REDUCE_THREADS));
   c->nb_bnd = std::min<int>(share, (int)grid1((size_t)std::max(S.n_in_g, S.n_in_gt) * S.ne, REDUCE_THREADS));
-  c->nb_vp = S.keldysh ? std::min<int>(592, (int)grid1(nn, REDUCE_THREADS)) : S.n0;  // LDOS finalize blocks; Poisson rows
+  c->nb_vp = S.keldysh ? std::min<int>(4 * c->n_sm, (int)grid1(nn, REDUCE_THREADS)) : S.n0;  // LDOS finalize blocks; Poisson rows
   c->nb_acc = std::min<int>(share_acc, (int)grid1(nn, REDUCE_THREADS));
   c->partial_fin.alloc((size_t)c->nb_fin * NQ);
   c->partial_bg.alloc((size_t)c->nb_bnd * 6);
@@ -2759,10 +2765,6 @@ int fail(sc_ctx *c, const EngineError &e) {
 
 }  // namespace
 
-extern "C" {
-
-}  // extern "C"
-
 namespace {
 // Shared part of sc_create / sc_ldos_create: the setup is built by `make`.
 template <typename F>
@@ -2783,7 +2785,6 @@ int create_context(int mode, sc_ctx **out, F make) {
     if (!e.empty()) throw EngineError(SC_ERR_ARG, e);
     if (c->S.nc > MAX_COMP) throw EngineError(SC_ERR_ARG, "at most 4 order-parameter components");
     if (2 * c->S.nc + 2 > 16) throw EngineError(SC_ERR_ARG, "too many accelerator fields");
-    CUDA_TRY(cudaGetDevice(&c->device));
     CUDA_TRY(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
     c->stream = c->own_stream;
     upload_static(c);
@@ -3858,7 +3859,6 @@ int sc_batch_create(const char *const *configs, int n, int mode, sc_batch **out)
       const std::string &e = errs[i];
       if (!e.empty()) throw EngineError(SC_ERR_ARG, "grain " + std::to_string(i) + ": " + e);
       if (c->S.nc > MAX_COMP) throw EngineError(SC_ERR_ARG, "at most 4 order-parameter components");
-      c->device = dev;
       c->stream = b->stream;
       upload_static(c);
     }
