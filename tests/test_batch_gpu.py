@@ -156,8 +156,8 @@ def test_batch_vs_oracle(engine_lib):
 @pytest.mark.parametrize("mode", ["fp64", "mixed"])
 def test_batch_low_temperature_grains(engine_lib, mode):
     """A temperature sweep in one batch: the small disc at T = 0.5 (7 Ozaki
-    energies), T = 0.01 at cutoff 8 (45: one pass, eight energies per thread
-    for some threads) and T = 0.005 at cutoff 16 (89: three energy passes of
+    energies), T = 0.01 at cutoff 8 (45: one pass, 16 threads of four per
+    column) and T = 0.005 at cutoff 16 (89: three energy passes of
     32, 32 and 25) give the results of the same grains run on their own."""
     import superconga_b200 as sb
     from oracle import oracle as O
