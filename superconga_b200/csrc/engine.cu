@@ -3379,6 +3379,7 @@ struct sc_batch {
   Phase pre, post;
   std::vector<Phase> wave_pre, wave_post;
   bool program_dirty = true;
+  bool planned = false;  // the waves are those of the active grains and the mapping
   DevArray<int> counters;
   DevArray<const Scalars *> scalar_src;
   DevArray<Scalars> scalars;  // gathered [grain] after every iteration
@@ -3423,6 +3424,11 @@ size_t grain_footprint(const sc_ctx *c) {
 // every grain's work buffers into the pool at its wave offset.
 template <typename R>
 void batch_plan(sc_batch *b) {
+  // Nothing of the old plan runs again from here on, also when this one fails
+  // half-way: the graph and the program launch on the old lists.
+  b->planned = false;
+  b->graph_dirty = true;
+  b->program_dirty = true;
   std::vector<int> order;
   for (int g = 0; g < (int)b->grains.size(); ++g)
     if (b->active[g]) order.push_back(g);
@@ -3519,8 +3525,7 @@ void batch_plan(sc_batch *b) {
   }
   b->counters.alloc(std::max<size_t>(1, b->waves.size()));
   CUDA_TRY(cudaStreamSynchronize(b->stream));
-  b->graph_dirty = true;
-  b->program_dirty = true;
+  b->planned = true;
 }
 
 // Records what `issue` launches for every listed grain and merges the recorded
@@ -3746,6 +3751,7 @@ void batch_time_step(sc_batch *b) {
 
 template <typename R>
 void batch_step(sc_batch *b) {
+  if (!b->planned) batch_plan<R>(b);  // the last one failed
   const bool apart = batch_apart(b);
   if (!apart && b->program_dirty) batch_program<R>(b);
   if (apart) {
@@ -3985,6 +3991,8 @@ int sc_batch_config(sc_batch *b, int energies_per_thread, int minb) {
     else batch_plan<float>(b);
   } catch (const EngineError &e) {
     return batch_fail(b, e);
+  } catch (const std::exception &e) {
+    return batch_fail(b, EngineError(SC_ERR_ARG, e.what()));
   }
   return SC_OK;
 }
@@ -4006,6 +4014,10 @@ int sc_batch_time_sweeps(sc_batch *b, int repeats, double *ms) {
     for (size_t g = 0; g < b->grains.size(); ++g)
       if (b->active[g] && !b->grains[g]->boundary_initialized)
         throw EngineError(SC_ERR_STATE, "sc_batch_time_sweeps: run one iteration first");
+    if (!b->planned) {
+      if (b->mode == SC_MODE_FP64) batch_plan<double>(b);
+      else batch_plan<float>(b);
+    }
     if (b->program_dirty && !batch_apart(b)) {
       if (b->mode == SC_MODE_FP64) batch_program<double>(b);
       else batch_program<float>(b);
@@ -4027,6 +4039,8 @@ int sc_batch_time_sweeps(sc_batch *b, int repeats, double *ms) {
     *ms = (double)t / repeats;
   } catch (const EngineError &e) {
     return batch_fail(b, e);
+  } catch (const std::exception &e) {
+    return batch_fail(b, EngineError(SC_ERR_ARG, e.what()));
   }
   return SC_OK;
 }
